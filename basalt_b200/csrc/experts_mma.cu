@@ -32,7 +32,6 @@ constexpr int kStages = 4;
 constexpr int kRowBytes = 144;                 // 4 NVFP4 blocks = 256 columns of one row
 constexpr int kRows = 16;                      // weight rows per warp
 constexpr int kStageBytes = kRows * kRowBytes; // 2304
-constexpr int kPieces = kStageBytes / 16;      // 144 16-byte pieces a stage
 constexpr int kCols = 8;                       // MMA n: activation columns per pass
 
 enum { MODE_GU = 0, MODE_DOWN = 1 };
@@ -41,6 +40,11 @@ __device__ __forceinline__ void cp_async16(uint32_t smem_addr, const void* gmem)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int BYTES>
+__device__ __forceinline__ void cp_async_piece(uint32_t smem_addr, const void* gmem) {   // BYTES 16, 8 or 4, both addresses aligned to it
+    if constexpr (BYTES == 16) cp_async16(smem_addr, gmem);
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(smem_addr), "l"(gmem), "n"(BYTES) : "memory");
+}
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
@@ -195,7 +199,10 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
 // MODE_GU:  rows = 8 gate rows r0.. paired with up rows r0..; columns = the entries' x images; writes h (fp32).
 // MODE_DOWN: rows = 16 down rows; columns = the entries' h images; writes out rows through ent_dst.
 // TERMS = 1: 8 entries a pass; TERMS = 2: 4 entries a pass, each as hi + lo fp16 columns.
-template <int MODE, int TERMS>
+// PIECE: bytes of one weight copy = the rows' alignment.  16 where K is whole 256-column chunks; a row of any other K (whole
+// 64-column NVFP4 blocks, 36 bytes each) starts on 8 bytes (K % 128 == 0) or 4, and its last chunk holds fewer than four blocks:
+// those pieces are not requested and those blocks not multiplied.
+template <int MODE, int TERMS, int PIECE>
 __global__ void __launch_bounds__(kThreads, 2)
 nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __restrict__ inv, const int2* __restrict__ items,
                  int* __restrict__ n_items, int tiles_per_warp, int n_row_blocks) {
@@ -224,17 +231,19 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
     constexpr int kTileRows = MODE == MODE_GU ? 8 : 16;
     constexpr int tile_stride = kWarps * kTileRows;
     __shared__ int s_work;
-    const int n_chunks = n_gran >> 2;
+    const int n_chunks = (n_gran + 3) >> 2;
+    const int last_bytes = PIECE == 16 ? kRowBytes : (n_gran - 4 * (n_chunks - 1)) * 36;   // bytes of a row in the last chunk
     const int pieces_per_col = (int) (K >> 3);               // 16-byte pieces of one image
 
-    // this lane's copy duty inside a stage: pieces lane, lane + 32, ... (< 144); row = piece / 9
-    int cp_row[5], cp_off[5];
-    uint32_t cp_dst[5];
+    // this lane's copy duty inside a stage: pieces lane, lane + 32, ...; row = piece / kRowPieces
+    constexpr int kRowPieces = kRowBytes / PIECE, kPieces = kRows * kRowPieces, kCopies = (kPieces + 31) / 32;
+    int cp_row[kCopies], cp_off[kCopies];
+    uint32_t cp_dst[kCopies];
 #pragma unroll
-    for (int j = 0; j < 5; ++j) {
+    for (int j = 0; j < kCopies; ++j) {
         const int p = lane + 32 * j;
-        cp_row[j] = p / 9;
-        cp_off[j] = (p % 9) * 16;
+        cp_row[j] = p / kRowPieces;
+        cp_off[j] = (p % kRowPieces) * PIECE;
         cp_dst[j] = (uint32_t) (cp_row[j] * kRowBytes + cp_off[j]);
     }
 
@@ -256,9 +265,9 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
         const float* tail = reinterpret_cast<const float*>(blob + a.L.bytes - 16);
         const int e1 = min(a.grp_start[grp + 1], (int) a.cap_entries);
         // global address of this lane's pieces at chunk 0
-        const uint8_t* src[5];
+        const uint8_t* src[kCopies];
 #pragma unroll
-        for (int j = 0; j < 5; ++j) {
+        for (int j = 0; j < kCopies; ++j) {
             const int row = cp_row[j];
             const uint8_t* rp;
             if (MODE == MODE_GU)
@@ -274,9 +283,10 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
         auto issue = [&]() {
             if (iss_unit < n_units) {
                 const uint32_t dst = wring_s + (uint32_t) (iss_unit & (kStages - 1)) * kStageBytes;
+                const int row_bytes = iss_chunk + 1 < n_chunks ? kRowBytes : last_bytes;
 #pragma unroll
-                for (int j = 0; j < 5; ++j)
-                    if (lane + 32 * j < kPieces) cp_async16(dst + cp_dst[j], src[j] + iss_off);
+                for (int j = 0; j < kCopies; ++j)
+                    if (lane + 32 * j < kPieces && (PIECE == 16 || cp_off[j] < row_bytes)) cp_async_piece<PIECE>(dst + cp_dst[j], src[j] + iss_off);
                 ++iss_unit;
                 if (++iss_chunk == n_chunks) {
                     iss_chunk = 0;
@@ -346,6 +356,7 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
                 const uint4* bp = bcol + (size_t) chunk * 4 * bstep;
 #pragma unroll
                 for (int blk = 0; blk < 4; ++blk) {
+                    if (PIECE != 16 && 4 * chunk + blk >= n_gran) break;   // past the row's last block
                     const uint4 b0 = bp[blk * bstep], b1 = bp[blk * bstep + bhalf];
                     const uint32_t sa = lut[reinterpret_cast<const uint8_t*>(ra)[36 * blk + t]];
                     const uint32_t sb = lut[reinterpret_cast<const uint8_t*>(rb)[36 * blk + t]];
@@ -407,7 +418,7 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
 size_t smem_bytes(int64_t K) { return (size_t) K * kCols * 2 + 1152 + (size_t) kWarps * kStages * kStageBytes; }
 size_t align256(size_t v) { return (v + 255) & ~(size_t) 255; }
 
-template <int MODE, int TERMS>
+template <int MODE, int TERMS, int PIECE = 16>
 int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const int2* items, int* n_items, cudaStream_t st) {
     const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff;
     const size_t smem = smem_bytes(K);
@@ -415,7 +426,7 @@ int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const i
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(nvfp4_mma_kernel<MODE, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        const cudaError_t e = cudaFuncSetAttribute(nvfp4_mma_kernel<MODE, TERMS, PIECE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
@@ -430,7 +441,7 @@ int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const i
     const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
     const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
     const int n_row_blocks = (int) ((n_tiles + tpw - 1) / tpw);
-    nvfp4_mma_kernel<MODE, TERMS><<<(unsigned) (2 * sm_count()), kThreads, smem, st>>>(a, img, inv, items, n_items, tpw, n_row_blocks);
+    nvfp4_mma_kernel<MODE, TERMS, PIECE><<<(unsigned) (2 * sm_count()), kThreads, smem, st>>>(a, img, inv, items, n_items, tpw, n_row_blocks);
     return launch_status();
 }
 
@@ -446,8 +457,9 @@ size_t experts_mma_scratch_bytes(int64_t cap_entries, int64_t n_embd, int64_t n_
 int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     const bsx_expert_layout& L = a.L;
     if (L.gu_type != kTypeNVFP4 || L.up_type != kTypeNVFP4 || L.d_type != kTypeNVFP4) return BSX_E_TYPE;
-    // 16-byte row chunks: both K dimensions must be whole 256-column chunks; the activation image must fit shared memory
-    if (L.n_embd % 256 || L.n_ff % 256 || L.n_ff % 8 || L.n_embd % 16) return BSX_E_TYPE;
+    // gate and up rows are whole 256-column chunks (n_embd % 256 == 0 in every layout), down rows whole 64-column blocks; the
+    // activation image must fit shared memory
+    if (L.n_embd % 256 || L.n_ff % 64) return BSX_E_TYPE;
     if (smem_bytes(L.n_embd) > 200 * 1024 || smem_bytes(L.n_ff) > 200 * 1024) return BSX_E_TYPE;
     // scratch: [h fp32][x images][h images][x inverse scales][h inverse scales]
     uint8_t* p = reinterpret_cast<uint8_t*>(a.h) + align256((size_t) a.cap_entries * L.n_ff * 4);
@@ -475,7 +487,12 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     }
     if (rc != BSX_OK || phase == 1) return rc;
     prep_image_kernel<true, 2><<<nbh, 256, 0, st>>>(a, himg, hinv, items, n_items);
-    return launch<MODE_DOWN, 2>(a, himg, hinv, items, n_items, st);
+    // Down rows of n_ff columns: the copies' width is what their start is aligned to.  An n_ff that is not whole 256-column chunks
+    // went to the warp-per-row kernels before (2 % of the copy bandwidth: fp32 decode and FMA for every weight and entry); here
+    // the same 27-token step (2560 x 640, 512 + 1 experts, top-10) takes 205 us instead of 3648.
+    if (L.n_ff % 256 == 0) return launch<MODE_DOWN, 2>(a, himg, hinv, items, n_items, st);
+    if (L.n_ff % 128 == 0) return launch<MODE_DOWN, 2, 8>(a, himg, hinv, items, n_items, st);
+    return launch<MODE_DOWN, 2, 4>(a, himg, hinv, items, n_items, st);
 }
 
 }  // namespace bsx
