@@ -159,12 +159,12 @@ moe_plan_kernel(const int32_t* __restrict__ ids, int n, int k, int E, const unsi
                 int32_t* __restrict__ n_groups, int32_t* __restrict__ dst, int32_t* __restrict__ tok, PassRec* __restrict__ items,
                 int* __restrict__ n_items) {
     extern __shared__ unsigned long long smb[];
-    const PlanSmem ps = plan_smem(smb, E);
+    const PlanSmem ps = plan_smem(smb, E, plan_masks(E, n, n_tok));
     plan_load_blobs(ps, blobs, E);       // constant addresses: before the wait for the kernel that wrote the ids
     pdl_wait();
     pdl_launch_dependents();
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) plan_note_pair(ps, i, ids[i], E);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) plan_note_pair(ps, i, i / k, ids[i], E);
     __syncthreads();
     plan_finish(ps, n, k, E, shared_blob, n_tok, ptr, start, n_groups, dst, tok, items, n_items);
 }
@@ -183,7 +183,7 @@ ep_plan_kernel(const int32_t* __restrict__ ids, int n, int k, int blk, int blk_s
                int32_t* __restrict__ n_groups, int32_t* __restrict__ dst, int32_t* __restrict__ tok, const uint8_t* __restrict__ replicated,
                int own_lo, int own_n) {
     extern __shared__ unsigned long long smb[];
-    const PlanSmem ps = plan_smem(smb, E);
+    const PlanSmem ps = plan_smem(smb, E, false);
     plan_load_blobs(ps, blobs, E);
     pdl_wait();
     pdl_launch_dependents();
@@ -192,7 +192,7 @@ ep_plan_kernel(const int32_t* __restrict__ ids, int n, int k, int blk, int blk_s
         const int at = blk > 0 ? (i / blk) * blk_stride + (i % blk) : i;
         int e = ids[at];
         if (replicated && (unsigned) e < (unsigned) E && replicated[e] && (i < own_lo || i >= own_lo + own_n)) e = -1;   // its token's owner runs it
-        plan_note_pair(ps, i, e, E);
+        plan_note_pair(ps, i, 0, e, E);
     }
     __syncthreads();
     plan_finish<false>(ps, n, k, E, shared_blob, tok_n, ptr, start, n_groups, dst, tok, nullptr, nullptr, tok_lo);
@@ -336,9 +336,9 @@ static int32_t plan_launch(const int32_t* ids, int32_t T, int32_t k, int32_t E, 
     const int64_t n = (int64_t) T * k;
     if (n <= 0) return BSX_OK;   // the reference returns without touching its outputs (ops.cu:491)
     if (n > BSX_PLAN_MAX_PAIRS) return BSX_E_LIMIT;
-    if (E < 1 || E > BSX_PLAN_MAX_EXPERTS) return BSX_E_GEOMETRY;   // E * 16 + n * 4 bytes of shared memory must stay below 48 KB
+    if (E < 1 || E > BSX_PLAN_MAX_EXPERTS) return BSX_E_GEOMETRY;   // the tables must fit 48 KB of shared memory
     if (!ids || !blob_table || !ptr || !start || !n_groups || !dst || !tok) return BSX_E_POINTER;
-    const size_t smem = (size_t) E * (sizeof(unsigned long long) + 2 * sizeof(int32_t)) + (size_t) n * sizeof(int32_t);
+    const size_t smem = plan_smem_bytes(E, (int) n, plan_masks(E, (int) n, T));
     launch_k(moe_plan_kernel, dim3(1), dim3(1024), smem, (cudaStream_t) stream, ids, (int) n, k, E, blob_table, shared_blob, (int) T, ptr, start, n_groups, dst, tok, items, n_items);
     return launch_status();
 }
@@ -383,8 +383,8 @@ extern "C" int32_t bsx_ep_plan(const int32_t* ids, int64_t n_pairs, int32_t k, i
                                int32_t* ent_tok, void* stream) {
     if (!stream) return BSX_E_STREAM;
     if (E < 1 || E > BSX_PLAN_MAX_EXPERTS || k < 1 || n_pairs < 0 || tok_lo < 0 || tok_n < 0 || pairs_per_block < 0) return BSX_E_GEOMETRY;
-    const size_t smem = plan_smem_bytes(E, (int) n_pairs);
-    if (n_pairs > BSX_EP_PLAN_MAX_PAIRS || smem > 48 * 1024) return BSX_E_LIMIT;
+    if (n_pairs > BSX_EP_PLAN_MAX_PAIRS || (size_t) E * 16 + (size_t) n_pairs * 4 > kPlanSmemMax) return BSX_E_LIMIT;
+    const size_t smem = plan_smem_bytes(E, (int) n_pairs, false);
     if (!ids || !blob_table || !ptr || !start || !n_groups || !ent_dst || !ent_tok) return BSX_E_POINTER;
     launch_k(ep_plan_kernel, dim3(1), dim3(1024), smem, (cudaStream_t) stream, ids, (int) n_pairs, (int) k, (int) pairs_per_block, (int) block_stride, (int) E,
              blob_table, shared_blob, (int) tok_lo, (int) tok_n, ptr, start, n_groups, ent_dst, ent_tok, replicated, (int) (tok_lo * k), (int) (tok_n * k));
