@@ -66,6 +66,40 @@ __device__ __forceinline__ uint32_t scale_pair_bits(uint32_t byte) {
     return v | (v << 16);
 }
 
+__device__ __forceinline__ uint32_t hadd2_bits(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+// IQ1_M weights as fp16(16 w), packed arithmetic throughout.  A weight is d m (g + delta), g = c - 1 with c the codebook's 2-bit
+// code, m = 2 s + 1 <= 15, delta = +-1/8.  8 m (g + delta) is an integer of at most 135 and exact in fp16 at every step below; the
+// product with 2 d rounds once, so the stored value is the same fp16 the fp32 product would round to.
+// A code becomes its value by masking it where it lies in the codebook word and or-ing in an exponent that makes its place worth
+// one: bits 4-5 under 2^6, 6-7 under 2^4, 8-9 under 2^2 (the constants -(2^E + 1) +- 1/8 stay within fp16's 11 bits only there), so
+// two shifts bring all eight pairs into place and a pair costs one logic and three fp16x2 operations.
+// q16: the two index bytes of 16 values; h8: their high bits and delta signs; s3: the scale field; d2: 2 d twice.
+// out[i] = values i (low half) and i + 8 (high half): the k order both operands are stored in.
+__device__ __forceinline__ void iq1m_16(uint32_t q16, uint32_t h8, uint32_t s3, uint32_t d2, const uint16_t* grid, uint32_t (&out)[8]) {
+    const uint32_t ia = (q16 & 0xFFu) | ((h8 & 7u) << 8), ib = (q16 >> 8) | ((h8 & 0x70u) << 4);
+    const uint32_t x = (uint32_t) grid[ia] | ((uint32_t) grid[ib] << 16);
+    const uint32_t delta = 0x30003000u | ((h8 & 8u) << 12) | ((h8 & 0x80u) << 24);       // +-0.125 each
+    const uint32_t k2 = hadd2_bits(delta, 0xC500C500u), k4 = hadd2_bits(delta, 0xCC40CC40u), k6 = hadd2_bits(delta, 0xD410D410u);   // -5, -17, -65
+    const uint32_t m8 = hadd2_bits((0x6408u | (s3 << 4)) * 0x10001u, 0xE400E400u);       // 1024 + 16 s + 8 - 1024
+    const uint32_t y = x << 4, z = x >> 6;
+    const uint32_t v[8] = {hadd2_bits((y & 0x00300030u) | 0x54005400u, k6), hadd2_bits((y & 0x00C000C0u) | 0x4C004C00u, k4),
+                           hadd2_bits((x & 0x00300030u) | 0x54005400u, k6), hadd2_bits((x & 0x00C000C0u) | 0x4C004C00u, k4),
+                           hadd2_bits((x & 0x03000300u) | 0x44004400u, k2), hadd2_bits((z & 0x00300030u) | 0x54005400u, k6),
+                           hadd2_bits((z & 0x00C000C0u) | 0x4C004C00u, k4), hadd2_bits((z & 0x03000300u) | 0x44004400u, k2)};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[i] = hmul2_bits(hmul2_bits(v[i], m8), d2);
+}
+// the block's fp16 super-scale, from the top nibbles of its four scale words, times two, in both halves
+__device__ __forceinline__ uint32_t iq1m_twice_d(uint2 sc) {
+    const uint32_t d = (((sc.x >> 12) & 0x000Fu) | ((sc.x >> 24) & 0x00F0u) | ((sc.y >> 4) & 0x0F00u) | ((sc.y >> 16) & 0xF000u)) * 0x10001u;
+    return hadd2_bits(d, d);
+}
+
 struct PrefillArgs {
     bsx_expert_layout L;
     const unsigned long long* blob_table;   // [E] device addresses
@@ -340,11 +374,63 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                 item = nxt;
                 it = itn;
             }
+        } else if constexpr (WT == WT_IQ1M) {
+            // IQ1_M rows: half a block (128 values: 16 index bytes, 8 bytes of high bits, the 8 scale bytes) is one pair of k-blocks.
+            // The next half is requested before this one is decoded, across items too; the decode runs ahead of the wait for the
+            // stage, so it overlaps the tensor core.
+            uint2 nx[4];
+            auto load_half = [&](const uint8_t* wrow, int q) {
+                const uint8_t* blk = wrow + (size_t) (q >> 1) * 56;
+                const int hb = q & 1;
+                nx[0] = *reinterpret_cast<const uint2*>(blk + 16 * hb);
+                nx[1] = *reinterpret_cast<const uint2*>(blk + 16 * hb + 8);
+                nx[2] = *reinterpret_cast<const uint2*>(blk + 32 + 8 * hb);
+                nx[3] = *reinterpret_cast<const uint2*>(blk + 48);
+            };
+            uint32_t kc = 0;
+            int item = blockIdx.x;
+            Item it;
+            while (item < n_items && !get_item(item, it)) item += gridDim.x;
+            if (item < n_items && grp < npair) load_half(weight_row(it), grp);
+            while (item < n_items && ok) {
+                const uint8_t* wrow = weight_row(it);
+                int nxt = item + gridDim.x;
+                Item itn;
+                while (nxt < n_items && !get_item(nxt, itn)) nxt += gridDim.x;
+                for (int q = grp; q < npair && ok; q += 2) {
+                    const uint32_t qs[4] = {nx[0].x, nx[0].y, nx[1].x, nx[1].y}, qh[2] = {nx[2].x, nx[2].y};
+                    const uint2 sc = nx[3];
+                    if (q + 2 < npair) load_half(wrow, q + 2);
+                    else if (nxt < n_items) load_half(weight_row(itn), grp);
+                    const uint32_t d2 = iq1m_twice_d(sc);
+                    const uint32_t scw = (q & 1) ? sc.y : sc.x;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int kb = 2 * q + j;
+                        uint32_t p[4][8];
+#pragma unroll
+                        for (int sub = 0; sub < 4; ++sub)
+                            iq1m_16((qs[2 * j + (sub >> 1)] >> (16 * (sub & 1))) & 0xFFFFu, (qh[j] >> (8 * sub)) & 0xFFu, (scw >> (16 * j + 3 * sub)) & 7u, d2, s_grid, p[sub]);
+                        const uint32_t kk = kc + (uint32_t) kb, s = kk % kStagesP;
+                        ok = mbar_wait(&empty[s], ((kk / kStagesP) & 1u) ^ 1u);
+                        if (!ok) break;
+                        uint4* brow = reinterpret_cast<uint4*>(smem + s * kStage + row_off);
+#pragma unroll
+                        for (int sub = 0; sub < 4; ++sub) {
+                            brow[(2 * sub) ^ swz] = make_uint4(p[sub][0], p[sub][1], p[sub][2], p[sub][3]);
+                            brow[(2 * sub + 1) ^ swz] = make_uint4(p[sub][4], p[sub][5], p[sub][6], p[sub][7]);
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                        mbar_arrive(&full[s]);
+                    }
+                }
+                kc += (uint32_t) nkb;
+                item = nxt;
+                it = itn;
+            }
         } else {
-            // K- and I-quant rows (Q6_K: 210 bytes per 256 values, IQ1_M: 56): the thread decodes its row's 64 values of a k-block
-            // exactly (formats.cuh), stores them as fp16(16 w) - the rounding, 2^-11 relative, is the only one - in the permuted
-            // k order, and hands the stage over.  The decode runs before the wait for the stage, so it overlaps the tensor core.
-            constexpr int kBB = WT == WT_Q6K ? 210 : 56;
+            // Q6_K rows (210 bytes per 256 values): the thread decodes its row's 64 values of a k-block exactly (formats.cuh), stores
+            // them as fp16(16 w) - the rounding, 2^-11 relative, is the only one - in the permuted k order, and hands the stage over.
             uint32_t kc = 0;
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
                 Item it;
@@ -356,15 +442,10 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                         const int kb = 2 * q + j;
                         if (kb >= nkb || !ok) continue;
                         float v[64];
-                        const uint8_t* blk = wrow + (size_t) (kb >> 2) * kBB;
+                        const uint8_t* blk = wrow + (size_t) (kb >> 2) * 210;
                         const int u0 = 2 * (kb & 3);
-                        if (WT == WT_Q6K) {
-                            decode_q6k_32(blk, u0, v);
-                            decode_q6k_32(blk, u0 + 1, v + 32);
-                        } else {
-                            decode_iq1m_32(blk, u0, s_grid, v);
-                            decode_iq1m_32(blk, u0 + 1, s_grid, v + 32);
-                        }
+                        decode_q6k_32(blk, u0, v);
+                        decode_q6k_32(blk, u0 + 1, v + 32);
                         const uint32_t kk = kc + (uint32_t) kb, s = kk % kStagesP;
                         ok = mbar_wait(&empty[s], ((kk / kStagesP) & 1u) ^ 1u);
                         if (!ok) break;
