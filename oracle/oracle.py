@@ -34,7 +34,7 @@ def build(force: bool = False) -> None:
     if force or not so.exists() or so.stat().st_mtime < src.stat().st_mtime or not (HERE / "libstdrandn.so").exists():
         subprocess.check_call(["make", "-C", str(HERE), "oracle"], stdout=subprocess.DEVNULL)
     ref = reference_checkout()
-    if ref.is_dir() and (force or not (HERE / "_ref" / "libref_cpu.so").exists() or not (HERE / "_ref" / "libref_gpu.so").exists()):
+    if (ref / "src").is_dir() and (force or not (HERE / "_ref" / "libref_cpu.so").exists() or not (HERE / "_ref" / "libref_gpu.so").exists()):
         subprocess.check_call(["make", "-C", str(HERE), "-j8", "ref", f"REF={ref}"], stdout=subprocess.DEVNULL)
 
 
