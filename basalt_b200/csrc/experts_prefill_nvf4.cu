@@ -10,13 +10,16 @@
 // That is what Basalt's sm_120 kernel does with ONE term (and an optional second) at ~1e-1 .. 1e-2; four terms cost the
 // tensor time of an fp16 product and meet the 2e-3 bar.
 //
-// Persistent CTAs, one per SM, static round-robin over work items (128-row tile of one expert, N weight rows):
-//   gate/up: N = 256 = the tile's 128 gate rows and their 128 up rows (two packed blocks), one accumulator of 256 columns;
-//   down:    N = 128 (one packed block), two accumulators, so the epilogue of one item overlaps the next item's stream.
-// Warp 0: per K-step the scale copies (tcgen05.cp shared -> tensor memory) and the four MMAs (M = 128 rows); warp 1: the
-// weights (one lane, bulk copies, completion in bytes); warps 2-5: the tile's activation rows - codes by 16-byte cp.async
-// gathers into four swizzled A tiles, scale words through registers into the lane-major order tcgen05.cp reads; warps 6-9:
-// epilogue (thread = TMEM lane = row).  Two stages of 256 columns; every wait is time-bounded with a status word.
+// Persistent CTAs, one per SM, static round-robin over work items (128-row tile of one expert x 256 weight rows: gate/up 128 gate
+// rows and their 128 up rows, down 256 rows; one accumulator of 256 columns).  Every operand is a bulk copy: the rows of a tile are
+// laid out beforehand as the images a stage holds (tile_images_kernel for x, h_images_kernel for the SwiGLU rows).  Warp 0: per
+// 64-column K-step the scale copies (tcgen05.cp shared -> tensor memory) and one MMA a term (M = 128 rows); warp 1: weights, two
+// stages of 256 columns; warp 2: activations, a slot a (chunk, term), eight of them, so that a slot is refilled as soon as its four
+// MMAs have read it; warps 4-11: epilogue (thread = TMEM lane = row).  Every wait is time-bounded with a status word.
+// Bound: operands from L2, 108 KB a (tile, 256 rows, 256 columns) against 2048 tensor-core cycles; the copies alone run at 10.6 TB/s
+// over the chip.  Measured, gate/up product of the 7168 x 2048 layer at 8192 tokens (256 experts + the shared one): 4.88 ms with
+// rows gathered by cp.async and MMAs issued under `lane == 0`, 4.59 with bulk copies, 3.52 with the issue under elect.sync too
+// (tc5.cuh); its down product 3.80 -> 2.33 (256 instead of 128 rows an item) -> 1.87.
 // With n_ff <= 512 the down product runs as prefill_down_resident_kernel instead (the tile's rows stay in shared memory).
 #include <atomic>
 #include <cuda_fp16.h>
@@ -24,51 +27,79 @@
 #include "common.cuh"
 #include "experts.cuh"
 #include "nvf4.cuh"
+#include "plan.cuh"
 #include "tc5.cuh"
 
 namespace bsx {
 namespace {
 
-constexpr int kStagesQ = 2;
-constexpr int kThreadsQ = 32 * 10;
-constexpr int kATileQ = 128 * 128;                 // one term's A tile of a stage: 128 rows x 128 bytes
-constexpr int kSFQ = 4 * 512;                      // four K-steps of 32 x 4 scale words
+constexpr int kThreadsQ = 32 * 12;
+constexpr int kATileQ = 128 * 128;                 // code tile of 128 rows x 256 columns
+constexpr int kSFQ = 4 * 512;                      // its scale words: four K-steps of 32 lanes x 4 words
+constexpr int kSlotQ = kSFQ + kATileQ;             // an activation slot: [scale words | codes], 18,432 bytes = a packed block's size
+constexpr int kBStages = 2, kASlots = kBStages * kTermsF;
 enum { QMODE_GU = 0, QMODE_DOWN = 1 };
 
-template <int MODE>
-struct Geo {
-    static constexpr int kN = MODE == QMODE_GU ? 256 : 128;           // weight rows (accumulator columns) of an item
-    static constexpr int kBlocks = kN / 128;                           // packed blocks of the B operand
-    static constexpr int kAccSets = MODE == QMODE_GU ? 1 : 2;
-    // a stage: [A term 0..3 | SFA term 0..3 | B codes (kBlocks x 16 KB) | SFB (kBlocks x 2 KB)]
-    static constexpr int kOffSFA = kTermsF * kATileQ;
-    static constexpr int kOffB = kOffSFA + kTermsF * kSFQ;
-    static constexpr int kOffSFB = kOffB + kBlocks * kATileQ;
-    static constexpr int kStage = kOffSFB + kBlocks * kSFQ;            // 110,592 (gate/up) or 92,160 (down): multiples of 1024
-    static constexpr size_t kSmem = 1024 + (size_t) kStagesQ * kStage + 256;
-    // tensor memory: accumulators first, then per stage the scale columns: SFA 4 terms x 4 steps x 4, SFB 4 steps x 4 kBlocks
-    static constexpr uint32_t kTmemSF = kAccSets * kN;
-    static constexpr uint32_t kSFACols = kTermsF * 16, kSFBCols = 16 * kBlocks, kSFStage = kSFACols + kSFBCols;
-    static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((uint32_t) (kN >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+struct GeoQ {
+    // shared memory: kBStages x [codes 0 | codes 1 | scales 0 | scales 1], then kASlots x [scales | codes], then the barriers
+    static constexpr int kBStage = 2 * kBlockF;
+    static constexpr int kOffA = kBStages * kBStage;
+    static constexpr int kBars = kOffA + kASlots * kSlotQ;
+    static constexpr size_t kSmem = 1024 + (size_t) kBars + 256;
+    // tensor memory: one accumulator of 256 columns, 16 scale columns per activation slot, 32 per weight stage
+    static constexpr uint32_t kTmemSFA = 256, kTmemSFB = kTmemSFA + 16 * kASlots;
+    static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((uint32_t) (256 >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
 };
 
-// a 128-row tile of one expert with everything the kernels need about it in one 16-byte load (blob 0: held elsewhere)
+// a 128-row tile of one expert with everything the kernels need about it (blob 0: held elsewhere)
 struct __align__(16) TileRec {
     unsigned long long blob;
     int row0, rows;
+    int64_t base;          // units (of atoms) before this tile's in the tile images, see image_block
+    int64_t pad;
 };
 
-__global__ void __launch_bounds__(256) tile_records_kernel(const int32_t* __restrict__ tiles, const int32_t* __restrict__ n_tiles,
-                                                           const int32_t* __restrict__ off, const unsigned long long* __restrict__ blob_table,
-                                                           TileRec* __restrict__ recs, int64_t cap_tiles) {
-    const int64_t t = (int64_t) blockIdx.x * 256 + threadIdx.x;
-    if (t >= cap_tiles || t >= *n_tiles) return;
-    const int expert = tiles[2 * t], row0 = tiles[2 * t + 1];
-    TileRec r;
-    r.blob = blob_table[expert];
-    r.row0 = row0;
-    r.rows = min(128, off[expert + 1] - row0);
-    recs[t] = r;
+// Tile images.  The activation rows a tile multiplies lie in dispatch order, in the form a stage has in shared memory: for each
+// (chunk of 256 columns, FP4 term) one run of [2 KB scale words, as tcgen05.cp reads them for 128 rows | 1 KB per eight rows of
+// codes, 128-byte swizzled], so that a stage of a tile is one bulk copy and a tile with few rows is a short one.  A tile takes
+// `units` = ceil(rows / 8) + 2 KB per (chunk, term); rows and scale words past its last row are never written (each only
+// reaches its own accumulator row, which is not stored).
+__host__ __device__ __forceinline__ int tile_units(int rows) { return (rows + 7) / 8 + 2; }
+__device__ __forceinline__ size_t image_block(const TileRec& r, int n_chunk, int c, int t) {
+    return ((size_t) r.base * n_chunk * kTermsF + (size_t) (c * kTermsF + t) * tile_units(r.rows)) * 1024;
+}
+// units that cap_rows rows in cap_tiles tiles can take
+__host__ __device__ inline int64_t image_units(int64_t cap_rows, int64_t cap_tiles) { return cap_rows / 8 + 3 * cap_tiles; }
+
+// one block: the units are a running sum over the tiles
+__global__ void __launch_bounds__(1024) tile_records_kernel(const int32_t* __restrict__ tiles, const int32_t* __restrict__ n_tiles,
+                                                            const int32_t* __restrict__ off, const unsigned long long* __restrict__ blob_table,
+                                                            TileRec* __restrict__ recs, int64_t cap_tiles, int64_t cap_units, int32_t* status) {
+    __shared__ unsigned long long sh[32];
+    const int64_t n = min(cap_tiles, (int64_t) *n_tiles);
+    int64_t at = 0;
+    for (int64_t t0 = 0; t0 < n; t0 += 1024) {
+        const int64_t t = t0 + threadIdx.x;
+        TileRec r = {0ull, 0, 0, 0, 0};
+        if (t < n) {
+            const int expert = tiles[2 * t], row0 = tiles[2 * t + 1];
+            r.blob = blob_table[expert];
+            r.row0 = row0;
+            r.rows = min(128, off[expert + 1] - row0);
+        }
+        const int u = r.rows > 0 ? tile_units(r.rows) : 0;
+        unsigned long long total = 0;
+        r.base = at + (int64_t) block_excl_sum<unsigned long long>((unsigned long long) u, &total, sh);
+        at += (int64_t) total;
+        if (t < n) {
+            if (r.rows <= 0 || r.base + u > cap_units) {      // no rows; or tiles that overlap, which no dispatch makes
+                if (r.rows > 0) atomicOr(status, 1);
+                r.blob = 0ull;
+                r.rows = 0;
+            }
+            recs[t] = r;
+        }
+    }
 }
 
 struct PrefillFArgs {
@@ -76,8 +107,7 @@ struct PrefillFArgs {
     const TileRec* recs;                     // [n_tiles]
     const int32_t* src;                      // [rows] token of each row
     const int32_t* n_tiles;
-    const uint8_t* codes;                    // activation images of this product's A operand
-    const uint8_t* sfs;
+    const uint8_t* img;                      // tile images of this product's A operand
     const float* inv;
     float* h;                                // [rows + 128][I] fp32 SwiGLU output
     float* dm;                               // [rows][H] fp32
@@ -87,319 +117,148 @@ struct PrefillFArgs {
 __device__ __forceinline__ uint64_t sf_desc_q(uint32_t addr) {   // 32 rows x 16 bytes, 8-row groups 128 bytes apart, no swizzle
     return (uint64_t) ((addr & 0x3FFFFu) >> 4) | ((uint64_t) (128 >> 4) << 16) | ((uint64_t) (128 >> 4) << 32) | ((uint64_t) 1 << 46);
 }
+__device__ __forceinline__ void sf_copy_q(uint32_t tmem_addr, uint64_t desc) {
+    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tmem_addr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void mma_nvf4_q(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accum) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
+                 "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(d),
+                 "l"(ad), "l"(bd), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accum)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_copy_q(uint32_t dst, const uint8_t* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void expect_bytes_q(uint32_t bar, uint32_t bytes) {
+    asm volatile("{\n.reg .b64 t;\nmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n}\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+// descriptors count addresses in 16 bytes: a K-step further is 32 bytes of codes, 512 of scale words
+constexpr uint64_t kStepCode = 2, kStepSF = 32;
+// eight consecutive floats of one row.  A thread of the epilogue owns a row, so a store instruction touches 32 rows: 32 bytes each
+// fill a sector, 16 bytes (rows whose base is only 16-byte aligned) would write every sector in two halves.
+__device__ __forceinline__ void store8_q(float* p, const float (&v)[8], bool wide) {
+    if (wide) {
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
+                     "f"(v[6]), "f"(v[7])
+                     : "memory");
+    } else {
+        reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+}
 
-// activation rows -> FP4 images.  FROM_H = false: rows of x (fp32 or bf16), image row = token; true: rows of h, image row =
-// dispatch row, as many as the dispatch has (off[E], read on the device).
-template <bool FROM_H, int TPR>
-__global__ void __launch_bounds__(256) prefill_images_kernel(const void* __restrict__ src, int kind, int64_t n_rows, const int32_t* __restrict__ n_rows_dev,
-                                                              int64_t K, uint8_t* __restrict__ codes, uint8_t* __restrict__ sfs, float* __restrict__ inv) {
+// rows of x (fp32 or bf16) -> FP4 terms, one image row per token: codes [token][term][H / 2], scales [token][term][H / 16]
+template <int TPR>
+__global__ void __launch_bounds__(256) prefill_images_kernel(const void* __restrict__ src, int kind, int64_t n, int64_t K, uint8_t* __restrict__ codes,
+                                                              uint8_t* __restrict__ sfs, float* __restrict__ inv) {
     __shared__ float shf[8];
-    const int64_t n = n_rows_dev ? min(n_rows, (int64_t) *n_rows_dev) : n_rows;
     const int64_t i = (int64_t) blockIdx.x * (256 / TPR) + threadIdx.x / TPR;
-    if ((int64_t) blockIdx.x * (256 / TPR) >= n) return;       // whole block past the end
     fp4_image_row<TPR>(src, kind, i < n ? i : 0, K, i < n, (int) i, codes, sfs, inv, shf);
 }
 
-template <bool FROM_H>
-void launch_images(const void* src, int kind, int64_t rows, const int32_t* rows_dev, int64_t K, uint8_t* codes, uint8_t* sfs, float* inv, cudaStream_t st) {
-    const int64_t n_sb = K / 16;
-    if (n_sb <= 32) prefill_images_kernel<FROM_H, 32><<<(unsigned) ((rows + 7) / 8), 256, 0, st>>>(src, kind, rows, rows_dev, K, codes, sfs, inv);
-    else if (n_sb <= 128) prefill_images_kernel<FROM_H, 128><<<(unsigned) ((rows + 1) / 2), 256, 0, st>>>(src, kind, rows, rows_dev, K, codes, sfs, inv);
-    else prefill_images_kernel<FROM_H, 256><<<(unsigned) rows, 256, 0, st>>>(src, kind, rows, rows_dev, K, codes, sfs, inv);
+// token images -> tile images of the gate/up product.  Block = one (tile, chunk): every row's four 128-byte code runs move in
+// 16-byte pieces (eight lanes a run), the scale words are transposed through shared memory.  Bound: HBM writes of 2.25 bytes a
+// value (180,224 rows x 2048: 830 MB); reads come from L2.
+__global__ void __launch_bounds__(256) tile_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ n_tiles, int tile0,
+                                                          const int32_t* __restrict__ src, const uint8_t* __restrict__ codes, const uint8_t* __restrict__ sfs, int64_t K,
+                                                          uint8_t* __restrict__ img) {
+    __shared__ __align__(16) uint32_t sf[kTermsF * kSFQ / 4];
+    const int tile = tile0 + blockIdx.y;
+    if (tile >= *n_tiles) return;
+    const TileRec r = recs[tile];
+    if (r.blob == 0ull) return;
+    const int c = blockIdx.x, n_chunk = gridDim.x;
+    uint8_t* out = img + image_block(r, n_chunk, c, 0);
+    const size_t term_bytes = (size_t) tile_units(r.rows) * 1024;
+    for (int i = threadIdx.x; i < r.rows * kTermsF; i += 256) {        // a row's 16 scale bytes of a term: one word into each K-step's block
+        const int row = i >> 2, t = i & 3;
+        const uint4 v = *reinterpret_cast<const uint4*>(sfs + ((size_t) src[r.row0 + row] * kTermsF + t) * (size_t) (K >> 4) + (size_t) c * 16);
+        uint32_t* d = sf + t * (kSFQ / 4) + (row & 31) * 4 + (row >> 5);
+        d[0] = v.x;
+        d[128] = v.y;
+        d[256] = v.z;
+        d[384] = v.w;
+    }
+    const int p = threadIdx.x & 7;
+    for (int row0 = threadIdx.x >> 5; row0 < r.rows; row0 += 32) {     // a warp: a row's four terms, four rows in flight
+        const int t = (threadIdx.x >> 3) & 3;
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int row = min(row0 + 8 * j, r.rows - 1);
+            v[j] = *reinterpret_cast<const uint4*>(codes + ((size_t) src[r.row0 + row] * kTermsF + t) * (size_t) (K >> 1) + (size_t) c * 128 + p * 16);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int row = row0 + 8 * j;
+            if (row < r.rows) *reinterpret_cast<uint4*>(out + t * term_bytes + kSFQ + (row >> 3) * 1024 + (row & 7) * 128 + ((p ^ (row & 7)) << 4)) = v[j];
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kTermsF * kSFQ / 16; i += 256) {
+        const int t = i / (kSFQ / 16), q = i - t * (kSFQ / 16);
+        reinterpret_cast<uint4*>(out + t * term_bytes)[q] = reinterpret_cast<const uint4*>(sf)[i];
+    }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs a) {
-    using G = Geo<MODE>;
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStagesQ * G::kStage);
-    uint64_t* empty = full + kStagesQ;
-    uint64_t* acc_full = empty + kStagesQ;
-    uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
-    const int n_chunk = (int) (K >> 8);
-    const int n_out = MODE == QMODE_GU ? (int) a.L.n_ff : (int) a.L.n_embd;       // neurons, or down rows
-    const int n_n = n_out / 128;                                                    // items per row tile
-    const int n_items = *a.n_tiles * n_n;
-    const PackedGeom geo = packed_geom(a.L.n_embd, a.L.n_ff);
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kStagesQ; ++s) {
-            mbar_init(&full[s], 1 + 128);    // the weight loader's expect_tx arrival + the 128 activation-loader lanes
-            mbar_init(&empty[s], 1);
-        }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], 128);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+// rows of h (fp32, dispatch order) -> tile images of the down product.  Block = eight rows of a tile, a warp a row: a lane makes
+// one sub-block of 16 values at a time, and four lanes' scale bytes make the word tcgen05.cp reads.
+__global__ void __launch_bounds__(256) h_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ n_tiles, const float* __restrict__ h, int64_t K,
+                                                       uint8_t* __restrict__ img, float* __restrict__ inv) {
+    const int tile = blockIdx.x >> 4, row = (blockIdx.x & 15) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (tile >= *n_tiles) return;
+    const TileRec r = recs[tile];
+    if (r.blob == 0ull || row >= r.rows) return;
+    const int64_t i = r.row0 + row;
+    const int n_sb = (int) (K >> 4), n_chunk = (int) (K >> 8);
+    float amax = 0.f;
+    for (int sb = lane; sb < n_sb; sb += 32) {
+        float v[16];
+        load16(h, BSX_X_F32, i, K, sb, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[j]));
     }
+    amax = warp_max_xor(amax);
+    const Pow2Scale ps = fp4_row_scale(amax);
+    if (lane == 0) inv[i] = ps.inv;
+    const size_t term_bytes = (size_t) tile_units(r.rows) * 1024;
+    for (int sb0 = 0; sb0 < n_sb; sb0 += 32) {       // n_sb is a multiple of 16: whole chunks, four lanes of a word together
+        const int sb = sb0 + lane;
+        const bool live = sb < n_sb;
+        float v[16];
+        if (live) load16(h, BSX_X_F32, i, K, sb, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = live ? v[j] * ps.s : 0.f;
+        uint8_t* out = img + image_block(r, n_chunk, sb >> 4, 0);
+        const int q = sb & 15;
+#pragma unroll
+        for (int t = 0; t < kTermsF; ++t) {
+            uint32_t w0, w1;
+            uint32_t sc = fp4_term(v, w0, w1) << (8 * (lane & 3));
+            sc |= __shfl_xor_sync(kFull, sc, 1);
+            sc |= __shfl_xor_sync(kFull, sc, 2);
+            if (!live) continue;
+            uint8_t* o = out + t * term_bytes;
+            *reinterpret_cast<uint2*>(o + kSFQ + (row >> 3) * 1024 + (row & 7) * 128 + (((q >> 1) ^ (row & 7)) << 4) + (q & 1) * 8) = make_uint2(w0, w1);
+            if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(o + (q >> 2) * 512 + (row & 31) * 16 + (row >> 5) * 4) = sc;
+        }
+    }
+}
+
+// the common start and end of the product kernels: tensor memory for the CTA
+__device__ __forceinline__ uint32_t tmem_take_q(uint32_t* slot, int warp) {
     if (warp == 0) {
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
-    bool ok = true;
-
-    // item -> (tile: expert, first row, live rows; first neuron / down row n0); items of experts held elsewhere are skipped by
-    // every role alike
-    struct Item { const uint8_t* blob; int row0, rows, n0; };
-    auto get_item = [&](int item, Item& it) -> bool {
-        const int tile = item / n_n;
-        const TileRec r = a.recs[tile];
-        if (r.blob == 0ull) return false;
-        it.blob = reinterpret_cast<const uint8_t*>(r.blob);
-        it.row0 = r.row0;
-        it.rows = r.rows;
-        it.n0 = (item - tile * n_n) * 128;
-        return true;
-    };
-
-    if (warp == 0) {
-        // ---- MMA issuer
-        if (lane == 0) {
-            uint32_t kc = 0, ti = 0;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                Item it;
-                if (!get_item(item, it)) continue;
-                const uint32_t acc = ti % G::kAccSets;
-                ok = mbar_wait(&acc_empty[acc], ((ti / G::kAccSets) & 1u) ^ 1u);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t d = tmem + acc * G::kN;
-                for (int c = 0; c < n_chunk; ++c, ++kc) {
-                    const uint32_t s = kc % kStagesQ;
-                    ok = mbar_wait(&full[s], (kc / kStagesQ) & 1u);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const uint32_t st = smem_u32(smem + s * G::kStage);
-                    const uint32_t tsfa = tmem + G::kTmemSF + s * G::kSFStage, tsfb = tsfa + G::kSFACols;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-#pragma unroll
-                        for (int b = 0; b < G::kBlocks; ++b)
-                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsfb + (uint32_t) (4 * G::kBlocks * k + 4 * b)),
-                                         "l"(sf_desc_q(st + (uint32_t) G::kOffSFB + b * kSFQ + k * 512))
-                                         : "memory");
-                        const uint64_t bd = smem_desc_sw128(st + (uint32_t) G::kOffB + k * 32);
-#pragma unroll
-                        for (int t = 0; t < kTermsF; ++t) {
-                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsfa + (uint32_t) (16 * t + 4 * k)),
-                                         "l"(sf_desc_q(st + (uint32_t) G::kOffSFA + t * kSFQ + k * 512))
-                                         : "memory");
-                            const uint32_t accum = (c | k | t) ? 1u : 0u;
-                            asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
-                                         "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(d),
-                                         "l"(smem_desc_sw128(st + (uint32_t) (t * kATileQ) + k * 32)), "l"(bd), "r"(G::kIdesc), "r"(tsfa + (uint32_t) (16 * t + 4 * k)),
-                                         "r"(tsfb + (uint32_t) (4 * G::kBlocks * k)), "r"(accum)
-                                         : "memory");
-                        }
-                    }
-                    umma_commit(&empty[s]);
-                }
-                if (!ok) break;
-                umma_commit(&acc_full[acc]);
-                ++ti;
-            }
-            if (!ok) atomicOr(a.status, 1);
-        }
-    } else if (warp == 1) {
-        // ---- weight loader: one lane; per stage each packed block of the item as two bulk copies (codes, scale words)
-        if (lane == 0) {
-            uint32_t issued = 0;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                Item it;
-                if (!get_item(item, it)) continue;
-                const int tile = it.n0 >> 7;
-                const uint8_t* blk[G::kBlocks];
-                if (MODE == QMODE_GU) {
-                    blk[0] = it.blob + geo.gate + (size_t) tile * n_chunk * kBlockF;
-                    if (G::kBlocks > 1) blk[G::kBlocks - 1] = it.blob + geo.up + (size_t) tile * n_chunk * kBlockF;
-                } else {
-                    blk[0] = it.blob + geo.down + (size_t) tile * n_chunk * kBlockF;
-                }
-                for (int c = 0; c < n_chunk; ++c, ++issued) {
-                    const uint32_t s = issued % kStagesQ;
-                    ok = mbar_wait(&empty[s], ((issued / kStagesQ) & 1u) ^ 1u);
-                    if (!ok) break;
-                    const uint32_t st = smem_u32(smem + s * G::kStage), bar = smem_u32(&full[s]);
-                    asm volatile("{\n.reg .b64 t;\nmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n}\n" ::"r"(bar), "r"((uint32_t) (G::kBlocks * kBlockF))
-                                 : "memory");
-#pragma unroll
-                    for (int b = 0; b < G::kBlocks; ++b) {
-                        const uint8_t* g = blk[b] + (size_t) c * kBlockF;
-                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(st + (uint32_t) G::kOffB + b * kATileQ),
-                                     "l"(g), "r"((uint32_t) kATileQ), "r"(bar)
-                                     : "memory");
-                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(st + (uint32_t) G::kOffSFB + b * kSFQ),
-                                     "l"(g + kATileQ), "r"((uint32_t) kSFQ), "r"(bar)
-                                     : "memory");
-                    }
-                }
-            }
-            if (!ok) atomicOr(a.status, 1);
-        }
-    } else if (warp <= 5) {
-        // ---- activation loaders (128 lanes).  Codes: lane = (16-byte piece c8, row group r16); rows r16 + 16 i, every term.
-        // Scales: lane = row m; for each term and K-step one word into slot (m % 32, m / 32) of that step's block.  A lane
-        // arrives on a stage when its copies there have landed.
-        const int tl = threadIdx.x - 64;
-        const int c8 = tl & 7, r16 = tl >> 3;
-        uint32_t issued = 0, arrived = 0;
-        // Software pipeline over items so that no item starts with a chain of dependent loads: the tile record of the item after
-        // next and the row indices of the next item are requested while this item streams.
-        auto next_valid = [&](int from, TileRec& r) {     // first item >= from (in this CTA's stride) whose expert is held here
-            int it = from;
-            for (; it < n_items; it += gridDim.x) {
-                r = a.recs[it / n_n];
-                if (r.blob != 0ull) break;
-            }
-            return it;
-        };
-        auto load_idx = [&](const TileRec& r, int (&idx)[9]) {   // image rows of this lane's 8 code rows and its scale row
-#pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                const int rw = i < 8 ? r16 + 16 * i : tl;
-                const int rr = rw < r.rows ? rw : 0;
-                idx[i] = MODE == QMODE_GU ? a.src[r.row0 + rr] : r.row0 + rr;
-            }
-        };
-        TileRec rec0, rec1, rec2;
-        int idx0[9], idx1[9];
-        int item = next_valid(blockIdx.x, rec0);
-        int item1 = item < n_items ? next_valid(item + gridDim.x, rec1) : n_items;
-        if (item < n_items) load_idx(rec0, idx0);
-        if (item1 < n_items) load_idx(rec1, idx1);
-        while (item < n_items && ok) {
-            const int item2 = item1 < n_items ? next_valid(item1 + gridDim.x, rec2) : n_items;
-            Item it;
-            it.blob = reinterpret_cast<const uint8_t*>(rec0.blob);
-            it.row0 = rec0.row0;
-            it.rows = rec0.rows;
-            it.n0 = (item - (item / n_n) * n_n) * 128;
-            // image rows behind the tile's rows: the row's token (gate/up) or the dispatch row itself (down); rows past the
-            // expert's last row read the tile's first row (their results are never stored)
-            const uint8_t* crow[8];
-            uint32_t cdst[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = r16 + 16 * i;
-                crow[i] = a.codes + (size_t) idx0[i] * kTermsF * (size_t) (K >> 1) + c8 * 16;
-                cdst[i] = (uint32_t) ((r >> 3) * 1024 + (r & 7) * 128 + ((c8 ^ (r & 7)) << 4));
-            }
-            const uint8_t* srow = a.sfs + (size_t) idx0[8] * kTermsF * (size_t) (K >> 4);
-            const uint32_t sdst = (uint32_t) (G::kOffSFA + (tl & 31) * 16 + (tl >> 5) * 4);
-            for (int c = 0; c < n_chunk; ++c) {
-                // hand over what is already on its way before blocking on the next slot (it frees only when the tensor core has
-                // consumed the stage before this one)
-                if (issued > arrived) {
-                    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    for (; arrived < issued; ++arrived) mbar_arrive(&full[arrived % kStagesQ]);
-                }
-                const uint32_t s = issued % kStagesQ;
-                ok = mbar_wait(&empty[s], ((issued / kStagesQ) & 1u) ^ 1u);
-                if (!ok) break;
-                const uint32_t st = smem_u32(smem + s * G::kStage);
-#pragma unroll
-                for (int t = 0; t < kTermsF; ++t) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(st + (uint32_t) (t * kATileQ) + cdst[i]),
-                                     "l"(crow[i] + (size_t) t * (size_t) (K >> 1) + (size_t) c * 128)
-                                     : "memory");
-                }
-                // this row's scale words: 16 bytes a term (the chunk's four K-steps) through registers, then one word into slot
-                // (m % 32, m / 32) of each step's block (four rows share a 16-byte slot, so no 16-byte copy can place them)
-                uint4 sv[kTermsF];
-#pragma unroll
-                for (int t = 0; t < kTermsF; ++t) sv[t] = *reinterpret_cast<const uint4*>(srow + (size_t) t * (size_t) (K >> 4) + (size_t) c * 16);
-#pragma unroll
-                for (int t = 0; t < kTermsF; ++t) {
-                    const uint32_t w[4] = {sv[t].x, sv[t].y, sv[t].z, sv[t].w};
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(st + sdst + (uint32_t) (t * kSFQ + k * 512)), "r"(w[k]) : "memory");
-                }
-                asm volatile("cp.async.commit_group;\n" ::: "memory");
-                ++issued;
-            }
-            // advance the pipeline: the next item's indices were requested one item ago; request those of the item after it
-            item = item1;
-            item1 = item2;
-            rec0 = rec1;
-            rec1 = rec2;
-#pragma unroll
-            for (int i = 0; i < 9; ++i) idx0[i] = idx1[i];
-            if (item1 < n_items) load_idx(rec1, idx1);
-        }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        for (; arrived < issued; ++arrived) mbar_arrive(&full[arrived % kStagesQ]);
-        if (!ok) atomicOr(a.status, 1);
-    } else {
-        // ---- epilogue: thread p reads TMEM lane p (= tile row p).  A warp may only read lanes 32 (warp % 4) .. + 31.
-        const int p = (warp & 3) * 32 + lane;
-        const uint32_t lane_base = (uint32_t) ((warp & 3) * 32) << 16;
-        uint32_t ti = 0;
-        for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-            Item it;
-            if (!get_item(item, it)) continue;
-            const bool row_live = p < it.rows;
-            const float* tail = reinterpret_cast<const float*>(it.blob + geo.tail);
-            const int64_t ir = !row_live ? 0 : (MODE == QMODE_GU ? (int64_t) a.src[it.row0 + p] : (int64_t) (it.row0 + p));
-            const float f = row_live ? a.inv[ir] : 0.f;
-            const float sg = tail[0] * f, su = tail[1] * f, sd = tail[2] * f;
-            const uint32_t acc = ti % G::kAccSets;
-            ok = __all_sync(kFull, mbar_wait(&acc_full[acc], (ti / G::kAccSets) & 1u));
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t tbase = tmem + lane_base + acc * G::kN;
-            if (MODE == QMODE_GU) {
-                float* hrow = a.h + (size_t) (it.row0 + p) * a.L.n_ff + it.n0;
-#pragma unroll 1
-                for (int c0 = 0; c0 < 128; c0 += 16) {
-                    uint32_t g[16], u[16];
-                    tmem_ld16(tbase + (uint32_t) c0, g);
-                    tmem_ld16(tbase + (uint32_t) (128 + c0), u);
-                    if (row_live) {
-#pragma unroll
-                        for (int v = 0; v < 4; ++v)
-                            reinterpret_cast<float4*>(hrow + c0)[v] =
-                                make_float4(swiglu(__uint_as_float(g[4 * v]) * sg, __uint_as_float(u[4 * v]) * su, a.L),
-                                            swiglu(__uint_as_float(g[4 * v + 1]) * sg, __uint_as_float(u[4 * v + 1]) * su, a.L),
-                                            swiglu(__uint_as_float(g[4 * v + 2]) * sg, __uint_as_float(u[4 * v + 2]) * su, a.L),
-                                            swiglu(__uint_as_float(g[4 * v + 3]) * sg, __uint_as_float(u[4 * v + 3]) * su, a.L));
-                    }
-                }
-            } else {
-                float* orow = a.dm + (size_t) (it.row0 + p) * a.L.n_embd + it.n0;
-#pragma unroll 1
-                for (int c0 = 0; c0 < 128; c0 += 32) {
-                    uint32_t d[32];
-                    tmem_ld32(tbase + (uint32_t) c0, d);
-                    if (row_live) {
-#pragma unroll
-                        for (int v = 0; v < 8; ++v)
-                            reinterpret_cast<float4*>(orow + c0)[v] = make_float4(__uint_as_float(d[4 * v]) * sd, __uint_as_float(d[4 * v + 1]) * sd,
-                                                                                 __uint_as_float(d[4 * v + 2]) * sd, __uint_as_float(d[4 * v + 3]) * sd);
-                    }
-                }
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            mbar_arrive(&acc_empty[acc]);
-            ++ti;
-        }
-        if (!ok && lane == 0) atomicOr(a.status, 1);
-    }
+    return *slot;
+}
+__device__ __forceinline__ void tmem_give_q(uint32_t tmem, int warp) {
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     if (warp == 0) {
@@ -407,6 +266,193 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
     }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs a) {
+    using G = GeoQ;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
+    uint64_t* a_full = reinterpret_cast<uint64_t*>(smem + G::kBars);
+    uint64_t* a_empty = a_full + kASlots;
+    uint64_t* b_full = a_empty + kASlots;
+    uint64_t* b_empty = b_full + kBStages;
+    uint64_t* acc_full = b_empty + kBStages;
+    uint64_t* acc_empty = acc_full + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const int n_chunk = (int) ((MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff) >> 8);
+    const int n_n = (int) (MODE == QMODE_GU ? a.L.n_ff / 128 : a.L.n_embd / 256);   // items per row tile: 128 neurons, or 256 down rows
+    const int n_items = *a.n_tiles * n_n;
+    const PackedGeom geo = packed_geom(a.L.n_embd, a.L.n_ff);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kASlots; ++s) {
+            mbar_init(&a_full[s], 1);
+            mbar_init(&a_empty[s], 1);
+        }
+        for (int s = 0; s < kBStages; ++s) {
+            mbar_init(&b_full[s], 1);
+            mbar_init(&b_empty[s], 1);
+        }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, 256);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    const uint32_t tmem = tmem_take_q(tmem_slot, warp);
+    const uint32_t sbase = smem_u32(smem);
+    bool ok = true;
+
+    // items of experts held elsewhere are skipped by every role alike
+    if (warp == 0) {
+        // ---- MMA issuer
+        if (elect_one()) {
+            uint32_t kb = 0, ti = 0;
+            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                if (a.recs[item / n_n].blob == 0ull) continue;
+                ok = mbar_wait(acc_empty, (ti & 1u) ^ 1u);
+                if (!ok) break;
+                for (int c = 0; c < n_chunk && ok; ++c, ++kb) {
+                    const uint32_t sb = kb % kBStages;
+                    ok = mbar_wait(&b_full[sb], (kb / kBStages) & 1u);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    const uint32_t bst = sbase + sb * G::kBStage, tsfb = tmem + G::kTmemSFB + sb * 32;
+                    const uint64_t bd = smem_desc_sw128(bst), bs = sf_desc_q(bst + 2 * kATileQ);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) sf_copy_q(tsfb + (uint32_t) (8 * k + 4 * b), bs + b * (kSFQ / 16) + k * kStepSF);
+#pragma unroll
+                    for (int t = 0; t < kTermsF; ++t) {
+                        const uint32_t sa = (kb & 1u) * kTermsF + t;
+                        ok = ok && mbar_wait(&a_full[sa], (kb >> 1) & 1u);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                        const uint32_t ast = sbase + G::kOffA + sa * kSlotQ, tsfa = tmem + G::kTmemSFA + sa * 16;
+                        const uint64_t ad = smem_desc_sw128(ast + kSFQ), as = sf_desc_q(ast);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            sf_copy_q(tsfa + (uint32_t) (4 * k), as + k * kStepSF);
+                            mma_nvf4_q(tmem, ad + k * kStepCode, bd + k * kStepCode, G::kIdesc, tsfa + (uint32_t) (4 * k), tsfb + (uint32_t) (8 * k),
+                                       (t | k) ? 1u : (c ? 1u : 0u));
+                        }
+                        umma_commit(&a_empty[sa]);
+                    }
+                    if (ok) umma_commit(&b_empty[sb]);
+                }
+                if (!ok) break;
+                umma_commit(acc_full);
+                ++ti;
+            }
+            if (!ok) atomicOr(a.status, 1);
+        }
+    } else if (warp == 1) {
+        // ---- weight loader: one lane; a stage is two packed blocks (gate and up rows, or two blocks of down rows)
+        if (elect_one()) {
+            uint32_t kb = 0;
+            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                const int tile = item / n_n, n = item - tile * n_n;
+                const unsigned long long bp = a.recs[tile].blob;
+                if (bp == 0ull) continue;
+                const uint8_t* blob = reinterpret_cast<const uint8_t*>(bp);
+                const size_t mat = (size_t) n_chunk * kBlockF;             // a 128-row block over all of K
+                const uint8_t* b0 = MODE == QMODE_GU ? blob + geo.gate + n * mat : blob + geo.down + 2 * n * mat;
+                const uint8_t* b1 = MODE == QMODE_GU ? blob + geo.up + n * mat : b0 + mat;
+                for (int c = 0; c < n_chunk; ++c, ++kb) {
+                    const uint32_t s = kb % kBStages;
+                    ok = mbar_wait(&b_empty[s], ((kb / kBStages) & 1u) ^ 1u);
+                    if (!ok) break;
+                    const uint32_t st = sbase + s * G::kBStage, bar = smem_u32(&b_full[s]);
+                    expect_bytes_q(bar, 2 * kBlockF);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const uint8_t* g = (b ? b1 : b0) + (size_t) c * kBlockF;
+                        bulk_copy_q(st + (uint32_t) (b * kATileQ), g, kATileQ, bar);
+                        bulk_copy_q(st + (uint32_t) (2 * kATileQ + b * kSFQ), g + kATileQ, kSFQ, bar);
+                    }
+                }
+            }
+            if (!ok) atomicOr(a.status, 1);
+        }
+    } else if (warp == 2) {
+        // ---- activation loader: one lane, one copy a slot
+        if (elect_one()) {
+            uint32_t ka = 0;
+            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                const TileRec r = a.recs[item / n_n];
+                if (r.blob == 0ull) continue;
+                const uint32_t bytes = (uint32_t) tile_units(r.rows) * 1024u;
+                const uint8_t* g = a.img + image_block(r, n_chunk, 0, 0);
+                for (int i = 0; i < n_chunk * kTermsF; ++i, ++ka, g += bytes) {
+                    const uint32_t s = ka % kASlots;
+                    ok = mbar_wait(&a_empty[s], ((ka / kASlots) & 1u) ^ 1u);
+                    if (!ok) break;
+                    const uint32_t bar = smem_u32(&a_full[s]);
+                    expect_bytes_q(bar, bytes);
+                    bulk_copy_q(sbase + (uint32_t) (G::kOffA + s * kSlotQ), g, bytes, bar);
+                }
+            }
+            if (!ok) atomicOr(a.status, 1);
+        }
+    } else if (warp >= 4) {
+        // ---- epilogue: thread p reads TMEM lane p (= tile row p), warps 4-7 the first and 8-11 the second half of the item's
+        // columns.  A warp may only read lanes 32 (warp % 4) .. + 31.  All of a thread's 128 values go to registers first, so the
+        // one accumulator is back with the tensor core before any of them is worked on.
+        const int p = (warp & 3) * 32 + lane, half = warp >= 8 ? 1 : 0;
+        const uint32_t tbase = tmem + ((uint32_t) ((warp & 3) * 32) << 16);
+        const bool wide = MODE == QMODE_GU || (reinterpret_cast<uintptr_t>(a.dm) & 31) == 0;
+        uint32_t ti = 0;
+        for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+            const int tile = item / n_n, n = item - tile * n_n;
+            const TileRec r = a.recs[tile];
+            if (r.blob == 0ull) continue;
+            const bool row_live = p < r.rows;
+            const float* tail = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(r.blob) + geo.tail);
+            const int64_t ir = !row_live ? 0 : (MODE == QMODE_GU ? (int64_t) a.src[r.row0 + p] : (int64_t) (r.row0 + p));
+            const float f = row_live ? a.inv[ir] : 0.f;
+            const float sg = tail[0] * f, su = tail[1] * f, sd = tail[2] * f;
+            ok = __all_sync(kFull, mbar_wait(acc_full, ti & 1u));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            uint32_t v[4][32];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int col = MODE == QMODE_GU ? (i >> 1) * 128 + half * 64 + (i & 1) * 32 : half * 128 + i * 32;
+                tmem_ld32(tbase + (uint32_t) col, v[i]);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            mbar_arrive(acc_empty);
+            ++ti;
+            if (!row_live) continue;
+            if (MODE == QMODE_GU) {
+                float* hrow = a.h + (size_t) (r.row0 + p) * a.L.n_ff + n * 128 + half * 64;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float o[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o[e] = swiglu(__uint_as_float(v[i][8 * j + e]) * sg, __uint_as_float(v[2 + i][8 * j + e]) * su, a.L);
+                        store8_q(hrow + 32 * i + 8 * j, o, wide);
+                    }
+            } else {
+                float* orow = a.dm + (size_t) (r.row0 + p) * a.L.n_embd + n * 256 + half * 128;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float o[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(v[i][8 * j + e]) * sd;
+                        store8_q(orow + 32 * i + 8 * j, o, wide);
+                    }
+            }
+        }
+        if (!ok && lane == 0) atomicOr(a.status, 1);
+    }
+    tmem_give_q(tmem, warp);
 }
 
 // ---------------------------------------------------------------- down product with the tile's rows resident
@@ -418,9 +464,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
 // per stage the weight scales.
 template <int KC>
 struct GeoR {
-    static constexpr int kABytes = KC * kTermsF * kATileQ;          // [chunk][term] code tiles
-    static constexpr int kOffSFA = kABytes;                           // [chunk][term][step] scale blocks
-    static constexpr int kOffB = kOffSFA + KC * kTermsF * kSFQ;       // two stages of KC packed blocks
+    static constexpr int kOffB = KC * kTermsF * kSlotQ;             // [chunk][term] slots, then two stages of KC packed blocks
     static constexpr int kStageB = KC * kBlockF;
     static constexpr int kBars = kOffB + 2 * kStageB;
     static constexpr size_t kSmem = 1024 + (size_t) kBars + 256;
@@ -441,8 +485,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
     uint64_t* a_empty = a_full + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(a_empty + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t K = a.L.n_ff;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_nb = (int) (a.L.n_embd / 128);            // blocks of 128 down rows = stages per tile
     const int n_tiles = *a.n_tiles;
     const PackedGeom geo = packed_geom(a.L.n_embd, a.L.n_ff);
@@ -452,26 +495,18 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
             mbar_init(&b_full[s], 1);
             mbar_init(&b_empty[s], 1);
             mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], 128);
+            mbar_init(&acc_empty[s], 256);
         }
-        mbar_init(a_full, 128);
+        mbar_init(a_full, 1);
         mbar_init(a_empty, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if (warp == 0) {
-        __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = tmem_take_q(tmem_slot, warp);
     const uint32_t sbase = smem_u32(smem);
     bool ok = true;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t ti = 0, nbc = 0;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
                 if (a.recs[tile].blob == 0ull) continue;
@@ -480,14 +515,12 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 // the tile's activation scales: shared -> tensor memory, once
 #pragma unroll
-                for (int c = 0; c < KC; ++c)
+                for (int q = 0; q < KC * kTermsF; ++q) {
+                    const uint64_t as = sf_desc_q(sbase + (uint32_t) (q * kSlotQ));
 #pragma unroll
-                    for (int t = 0; t < kTermsF; ++t)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tmem + G::kTmemSFA + (uint32_t) (64 * c + 16 * t + 4 * k)),
-                                         "l"(sf_desc_q(sbase + (uint32_t) G::kOffSFA + (uint32_t) (((c * kTermsF + t) * 4 + k) * 512)))
-                                         : "memory");
+                    for (int k = 0; k < 4; ++k) sf_copy_q(tmem + G::kTmemSFA + (uint32_t) (16 * q + 4 * k), as + k * kStepSF);
+                }
+                const uint64_t ad = smem_desc_sw128(sbase + kSFQ);
                 for (int nb = 0; nb < n_nb; ++nb, ++nbc) {
                     const uint32_t s = nbc & 1u, par = (nbc >> 1) & 1u;
                     ok = mbar_wait(&acc_empty[s], par ^ 1u);
@@ -498,23 +531,17 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
                     const uint32_t tsfb = tmem + G::kTmemSFB + s * G::kSFBStage;
                     const uint32_t d = tmem + s * 128;
 #pragma unroll
-                    for (int c = 0; c < KC; ++c)
+                    for (int c = 0; c < KC; ++c) {
+                        const uint64_t bd = smem_desc_sw128(sb + (uint32_t) (c * kBlockF)), bs = sf_desc_q(sb + (uint32_t) (c * kBlockF + kATileQ));
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
-                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsfb + (uint32_t) (16 * c + 4 * k)),
-                                         "l"(sf_desc_q(sb + (uint32_t) (c * kBlockF + kATileQ + k * 512)))
-                                         : "memory");
-                            const uint64_t bd = smem_desc_sw128(sb + (uint32_t) (c * kBlockF) + k * 32);
+                            sf_copy_q(tsfb + (uint32_t) (16 * c + 4 * k), bs + k * kStepSF);
 #pragma unroll
-                            for (int t = 0; t < kTermsF; ++t) {
-                                const uint32_t accum = (c | k | t) ? 1u : 0u;
-                                asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
-                                             "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(d),
-                                             "l"(smem_desc_sw128(sbase + (uint32_t) ((c * kTermsF + t) * kATileQ) + k * 32)), "l"(bd), "r"(G::kIdesc),
-                                             "r"(tmem + G::kTmemSFA + (uint32_t) (64 * c + 16 * t + 4 * k)), "r"(tsfb + (uint32_t) (16 * c + 4 * k)), "r"(accum)
-                                             : "memory");
-                            }
+                            for (int t = 0; t < kTermsF; ++t)
+                                mma_nvf4_q(d, ad + (uint64_t) ((c * kTermsF + t) * (kSlotQ / 16)) + k * kStepCode, bd + k * kStepCode, G::kIdesc,
+                                           tmem + G::kTmemSFA + (uint32_t) (64 * c + 16 * t + 4 * k), tsfb + (uint32_t) (16 * c + 4 * k), (c | k | t) ? 1u : 0u);
                         }
+                    }
                     umma_commit(&b_empty[s]);
                     umma_commit(&acc_full[s]);
                 }
@@ -525,7 +552,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
             if (!ok) atomicOr(a.status, 1);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t nbc = 0;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
                 const unsigned long long bp = a.recs[tile].blob;
@@ -536,113 +563,69 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
                     ok = mbar_wait(&b_empty[s], ((nbc >> 1) & 1u) ^ 1u);
                     if (!ok) break;
                     const uint32_t bar = smem_u32(&b_full[s]);
-                    asm volatile("{\n.reg .b64 t;\nmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n}\n" ::"r"(bar), "r"((uint32_t) G::kStageB) : "memory");
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(sbase + (uint32_t) G::kOffB + s * G::kStageB),
-                                 "l"(down + (size_t) nb * G::kStageB), "r"((uint32_t) G::kStageB), "r"(bar)
-                                 : "memory");
+                    expect_bytes_q(bar, (uint32_t) G::kStageB);
+                    bulk_copy_q(sbase + (uint32_t) G::kOffB + s * G::kStageB, down + (size_t) nb * G::kStageB, (uint32_t) G::kStageB, bar);
                 }
             }
             if (!ok) atomicOr(a.status, 1);
         }
-    } else if (warp <= 5) {
-        // ---- the tile's rows (images of dispatch rows row0 ..): codes by 16-byte cp.async, scale words through registers
-        const int tl = threadIdx.x - 64;
-        const int c8 = tl & 7, r16 = tl >> 3;
-        const uint32_t sdst = sbase + (uint32_t) (G::kOffSFA + (tl & 31) * 16 + (tl >> 5) * 4);
-        uint32_t ti = 0;
-        TileRec rec, nrec;
-        int tile = blockIdx.x;
-        for (; tile < n_tiles; tile += gridDim.x) {
-            rec = a.recs[tile];
-            if (rec.blob != 0ull) break;
+    } else if (warp == 2) {
+        // ---- the tile's rows: one copy per (chunk, term)
+        if (elect_one()) {
+            uint32_t ti = 0;
+            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+                const TileRec r = a.recs[tile];
+                if (r.blob == 0ull) continue;
+                ok = mbar_wait(a_empty, (ti & 1u) ^ 1u);
+                if (!ok) break;
+                const uint32_t bytes = (uint32_t) tile_units(r.rows) * 1024u, bar = smem_u32(a_full);
+                expect_bytes_q(bar, (uint32_t) (KC * kTermsF) * bytes);
+                const uint8_t* g = a.img + image_block(r, KC, 0, 0);
+#pragma unroll
+                for (int q = 0; q < KC * kTermsF; ++q) bulk_copy_q(sbase + (uint32_t) (q * kSlotQ), g + (size_t) q * bytes, bytes, bar);
+                ++ti;
+            }
+            if (!ok) atomicOr(a.status, 1);
         }
-        while (tile < n_tiles && ok) {
-            int ntile = tile + gridDim.x;             // the next tile's record is requested while this one loads
-            for (; ntile < n_tiles; ntile += gridDim.x) {
-                nrec = a.recs[ntile];
-                if (nrec.blob != 0ull) break;
-            }
-            ok = mbar_wait(a_empty, (ti & 1u) ^ 1u);
-            if (!ok) break;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = r16 + 16 * i;
-                const int64_t ir = rec.row0 + (r < rec.rows ? r : 0);
-                const uint8_t* g = a.codes + (size_t) ir * kTermsF * (size_t) (K >> 1) + c8 * 16;
-                const uint32_t dst = sbase + (uint32_t) ((r >> 3) * 1024 + (r & 7) * 128 + ((c8 ^ (r & 7)) << 4));
-#pragma unroll
-                for (int c = 0; c < KC; ++c)
-#pragma unroll
-                    for (int t = 0; t < kTermsF; ++t)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (uint32_t) ((c * kTermsF + t) * kATileQ)),
-                                     "l"(g + (size_t) t * (size_t) (K >> 1) + (size_t) c * 128)
-                                     : "memory");
-            }
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-            {
-                const int64_t ir = rec.row0 + (tl < rec.rows ? tl : 0);
-                const uint8_t* srow = a.sfs + (size_t) ir * kTermsF * (size_t) (K >> 4);
-#pragma unroll
-                for (int c = 0; c < KC; ++c)
-#pragma unroll
-                    for (int t = 0; t < kTermsF; ++t) {
-                        const uint4 sv = *reinterpret_cast<const uint4*>(srow + (size_t) t * (size_t) (K >> 4) + (size_t) c * 16);
-                        const uint32_t w[4] = {sv.x, sv.y, sv.z, sv.w};
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(sdst + (uint32_t) (((c * kTermsF + t) * 4 + k) * 512)), "r"(w[k]) : "memory");
-                    }
-            }
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            mbar_arrive(a_full);
-            ++ti;
-            tile = ntile;
-            rec = nrec;
-        }
-        if (!ok) atomicOr(a.status, 1);
-    } else {
-        // ---- epilogue: thread p = tile row p reads TMEM lane p of each finished accumulator (128 down rows at a time)
-        const int p = (warp & 3) * 32 + lane;
-        const uint32_t lane_base = (uint32_t) ((warp & 3) * 32) << 16;
+    } else if (warp >= 4) {
+        // ---- epilogue: thread p = tile row p reads TMEM lane p of each finished accumulator, half of its 128 columns
+        const int p = (warp & 3) * 32 + lane, half = warp >= 8 ? 1 : 0;
+        const uint32_t tbase = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + (uint32_t) (half * 64);
+        const bool wide = (reinterpret_cast<uintptr_t>(a.dm) & 31) == 0;
         uint32_t nbc = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            const TileRec rec = a.recs[tile];
-            if (rec.blob == 0ull) continue;
-            const bool row_live = p < rec.rows;
-            const float* tail = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(rec.blob) + geo.tail);
-            const float sd = row_live ? tail[2] * a.inv[rec.row0 + p] : 0.f;
-            float* orow = a.dm + (size_t) (rec.row0 + p) * a.L.n_embd;
+            const TileRec r = a.recs[tile];
+            if (r.blob == 0ull) continue;
+            const bool row_live = p < r.rows;
+            const float* tail = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(r.blob) + geo.tail);
+            const float sd = row_live ? tail[2] * a.inv[r.row0 + p] : 0.f;
+            float* orow = a.dm + (size_t) (r.row0 + p) * a.L.n_embd + half * 64;
             for (int nb = 0; nb < n_nb; ++nb, ++nbc) {
                 const uint32_t s = nbc & 1u;
                 ok = __all_sync(kFull, mbar_wait(&acc_full[s], (nbc >> 1) & 1u));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll 1
-                for (int c0 = 0; c0 < 128; c0 += 32) {
-                    uint32_t d[32];
-                    tmem_ld32(tmem + lane_base + s * 128 + (uint32_t) c0, d);
-                    if (row_live) {
-#pragma unroll
-                        for (int v = 0; v < 8; ++v)
-                            reinterpret_cast<float4*>(orow + nb * 128 + c0)[v] = make_float4(__uint_as_float(d[4 * v]) * sd, __uint_as_float(d[4 * v + 1]) * sd,
-                                                                                            __uint_as_float(d[4 * v + 2]) * sd, __uint_as_float(d[4 * v + 3]) * sd);
-                    }
-                }
+                uint32_t v[2][32];
+                tmem_ld32(tbase + s * 128, v[0]);
+                tmem_ld32(tbase + s * 128 + 32, v[1]);
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 mbar_arrive(&acc_empty[s]);
+                if (!row_live) continue;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float o[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(v[i][8 * j + e]) * sd;
+                        store8_q(orow + nb * 128 + 32 * i + 8 * j, o, wide);
+                    }
             }
             if (!ok) break;
         }
         if (!ok && lane == 0) atomicOr(a.status, 1);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0) {
-        __syncwarp();
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
-    }
+    tmem_give_q(tmem, warp);
 }
 
 template <int KC>
@@ -667,11 +650,11 @@ int32_t launch_q(const PrefillFArgs& a, cudaStream_t st) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(prefill_nvf4_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) Geo<MODE>::kSmem);
+        const cudaError_t e = cudaFuncSetAttribute(prefill_nvf4_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GeoQ::kSmem);
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
-    prefill_nvf4_kernel<MODE><<<(unsigned) sm_count(), kThreadsQ, Geo<MODE>::kSmem, st>>>(a);
+    prefill_nvf4_kernel<MODE><<<(unsigned) sm_count(), kThreadsQ, GeoQ::kSmem, st>>>(a);
     return launch_status();
 }
 
@@ -680,11 +663,15 @@ int32_t launch_q(const PrefillFArgs& a, cudaStream_t st) {
 
 using namespace bsx;
 
+// the tiles that rows of up to 1024 experts can make
+static int64_t prefill_cap_tiles(int64_t cap_rows) { return cap_rows < 1025 ? cap_rows : cap_rows / 128 + 1025; }
+
 extern "C" size_t bsx_experts_prefill_packed_scratch_bytes(const bsx_expert_layout* L, int64_t n_tokens, int64_t cap_rows) {
     if (!L || n_tokens < 0 || cap_rows < 0 || !bsx_expert_packed_bytes(L)) return 0;
     const size_t H = (size_t) L->n_embd, I = (size_t) L->n_ff, R = (size_t) cap_rows + 128;
+    const size_t units = (size_t) image_units(cap_rows, prefill_cap_tiles(cap_rows));
     return al256q((size_t) n_tokens * kTermsF * H / 2) + al256q((size_t) n_tokens * kTermsF * H / 16) + al256q((size_t) n_tokens * 4) + al256q(R * I * 4) +
-           al256q(R * kTermsF * I / 2) + al256q(R * kTermsF * I / 16) + al256q(R * 4) + al256q(((size_t) cap_rows / 128 + 1025) * sizeof(TileRec)) + 256;
+           units * 1024 * kTermsF * (H / 256 + I / 256) + al256q(R * 4) + al256q(((size_t) cap_rows / 128 + 1025) * sizeof(TileRec)) + 256;
 }
 
 extern "C" int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, const unsigned long long* blob_table, const int32_t* off,
@@ -710,15 +697,16 @@ extern "C" int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, c
     p += al256q((size_t) n_tokens * 4);
     float* h = reinterpret_cast<float*>(p);
     p += al256q(R * I * 4);
-    uint8_t* hcodes = p;
-    p += al256q(R * kTermsF * I / 2);
-    uint8_t* hsf = p;
-    p += al256q(R * kTermsF * I / 16);
+    const int64_t units = image_units(cap_rows, prefill_cap_tiles(cap_rows));
+    uint8_t* ximg = p;
+    p += (size_t) units * 1024 * kTermsF * (H / 256);
+    uint8_t* himg = p;
+    p += (size_t) units * 1024 * kTermsF * (I / 256);
     float* hinv = reinterpret_cast<float*>(p);
     p += al256q(R * 4);
     TileRec* recs = reinterpret_cast<TileRec*>(p);
     if (cap_tiles > cap_rows / 128 + 1025) return BSX_E_LIMIT;      // more tiles than rows / 128 + experts can make
-    tile_records_kernel<<<(unsigned) ((cap_tiles + 255) / 256), 256, 0, st>>>(tiles, n_tiles, off, blob_table, recs, cap_tiles);
+    tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, recs, cap_tiles, units, status);
     PrefillFArgs a;
     a.L = L;
     a.recs = recs;
@@ -727,15 +715,16 @@ extern "C" int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, c
     a.h = h;
     a.dm = dm;
     a.status = status;
-    launch_images<false>(x, x_kind, n_tokens, nullptr, (int64_t) H, xcodes, xsf, xinv, st);
-    a.codes = xcodes;
-    a.sfs = xsf;
+    if (H <= 2048) prefill_images_kernel<128><<<(unsigned) ((n_tokens + 1) / 2), 256, 0, st>>>(x, x_kind, n_tokens, (int64_t) H, xcodes, xsf, xinv);
+    else prefill_images_kernel<256><<<(unsigned) n_tokens, 256, 0, st>>>(x, x_kind, n_tokens, (int64_t) H, xcodes, xsf, xinv);
+    for (int64_t t0 = 0; t0 < cap_tiles; t0 += 65535)
+        tile_images_kernel<<<dim3((unsigned) (H / 256), (unsigned) (cap_tiles - t0 < 65535 ? cap_tiles - t0 : 65535)), 256, 0, st>>>(recs, n_tiles, (int) t0, src, xcodes, xsf, (int64_t) H, ximg);
+    a.img = ximg;
     a.inv = xinv;
     int32_t rc = launch_q<QMODE_GU>(a, st);
     if (rc != BSX_OK) return rc;
-    launch_images<true>(h, BSX_X_F32, cap_rows, off + n_expert, (int64_t) I, hcodes, hsf, hinv, st);
-    a.codes = hcodes;
-    a.sfs = hsf;
+    h_images_kernel<<<(unsigned) (cap_tiles * 16), 256, 0, st>>>(recs, n_tiles, h, (int64_t) I, himg, hinv);
+    a.img = himg;
     a.inv = hinv;
     // n_ff <= 512: the tile's rows stay in shared memory and only weights stream
     if (I == 256) return launch_down_resident<1>(a, st);

@@ -63,11 +63,48 @@ __device__ __forceinline__ float2 e2m1x2_values(uint32_t c) {
     return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
 
+// A row times a power of two (largest magnitude into [2^7, 2^8), so block scales sit well inside UE4M3's range).
+struct Pow2Scale {
+    float s, inv;
+};
+__device__ __forceinline__ Pow2Scale fp4_row_scale(float amax) {
+    Pow2Scale r = {1.f, 1.f};
+    if (amax > 0.f && amax <= 3.0e38f) {
+        int ex = 0;
+        frexpf(amax, &ex);                          // amax = f 2^ex, f in [0.5, 1)
+        ex = max(-100, min(100, 8 - ex));
+        r.s = ldexpf(1.f, ex);
+        r.inv = ldexpf(1.f, -ex);
+    }
+    return r;
+}
+// One FP4 term of a sub-block of 16 values: scale = the smallest UE4M3 value s with 6 s >= the largest magnitude (its byte is
+// returned), codes = rn(v / s) in w0, w1, v -= code value x s.
+__device__ __forceinline__ uint32_t fp4_term(float (&v)[16], uint32_t& w0, uint32_t& w1) {
+    float m = 0.f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) m = fmaxf(m, fabsf(v[j]));
+    const uint32_t sb8 = ue4m3_cover(m);
+    const float sv = ue4m3_value(sb8);
+    w0 = w1 = 0u;
+    if (sv > 0.f) {
+        const float rs = 1.f / sv;          // 6 sv >= every |v|, so |v rs| <= 6 up to rounding, which the conversion saturates
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const uint32_t c = e2m1x2(v[b] * rs, v[b + 8] * rs);
+            const float2 q = e2m1x2_values(c);
+            v[b] -= q.x * sv;
+            v[b + 8] -= q.y * sv;
+            if (b < 4) w0 |= c << (8 * b);
+            else w1 |= c << (8 * (b - 4));
+        }
+    }
+    return sb8;
+}
+
 // TPR threads per activation row (32, 128 or 256: a thread per 16-value sub-block where the row allows), 256 / TPR rows a
 // block; every thread of the block must call (the row maximum is reduced through `shf`, 8 floats of shared memory).
-// The row times a power of two (largest magnitude into [2^7, 2^8), so block scales sit well inside UE4M3's range) becomes
-// kTermsF FP4 terms.  Term t of a sub-block: scale = the smallest UE4M3 value s with 6 s >= the largest residual, codes =
-// rn(residual / s), residual -= code value x s.  Layout: codes [image row][term][K / 2] bytes with ggml's nibble order
+// The scaled row becomes kTermsF FP4 terms, term t of a sub-block from the residual of the ones before.  Layout: codes [image row][term][K / 2] bytes with ggml's nibble order
 // (byte b of a sub-block = values b and b + 8), scales [image row][term][K / 16] bytes, inv[image row] undoes the power of two.
 template <int TPR>
 __device__ __forceinline__ void fp4_image_row(const void* src, int kind, int64_t row, int64_t K, bool live, int i, uint8_t* __restrict__ codes,
@@ -94,40 +131,17 @@ __device__ __forceinline__ void fp4_image_row(const void* src, int kind, int64_t
         for (int w = 1; w < TPR / 32; ++w) amax = fmaxf(amax, shf[w0 + w]);
     }
     if (!live) return;
-    int ex = 0;
-    float s = 1.f, iv = 1.f;
-    if (amax > 0.f && amax <= 3.0e38f) {
-        frexpf(amax, &ex);                          // amax = f 2^ex, f in [0.5, 1)
-        ex = max(-100, min(100, 8 - ex));
-        s = ldexpf(1.f, ex);
-        iv = ldexpf(1.f, -ex);
-    }
-    if (tr == 0) inv[i] = iv;
+    const Pow2Scale ps = fp4_row_scale(amax);
+    if (tr == 0) inv[i] = ps.inv;
     for (int sb = tr; sb < n_sb; sb += TPR) {
         float v[16];
         load16(src, kind, row, K, sb, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] *= s;
+        for (int j = 0; j < 16; ++j) v[j] *= ps.s;
 #pragma unroll
         for (int t = 0; t < kTermsF; ++t) {
-            float m = 0.f;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) m = fmaxf(m, fabsf(v[j]));
-            const uint32_t sb8 = ue4m3_cover(m);
-            const float sv = ue4m3_value(sb8);
-            uint32_t w0 = 0u, w1 = 0u;
-            if (sv > 0.f) {
-                const float rs = 1.f / sv;          // 6 sv >= every |v|, so |v rs| <= 6 up to rounding, which the conversion saturates
-#pragma unroll
-                for (int b = 0; b < 8; ++b) {
-                    const uint32_t c = e2m1x2(v[b] * rs, v[b + 8] * rs);
-                    const float2 q = e2m1x2_values(c);
-                    v[b] -= q.x * sv;
-                    v[b + 8] -= q.y * sv;
-                    if (b < 4) w0 |= c << (8 * b);
-                    else w1 |= c << (8 * (b - 4));
-                }
-            }
+            uint32_t w0, w1;
+            const uint32_t sb8 = fp4_term(v, w0, w1);
             const size_t r4 = (size_t) i * kTermsF + t;
             *reinterpret_cast<uint2*>(codes + r4 * (K / 2) + (size_t) sb * 8) = make_uint2(w0, w1);
             sfs[r4 * (K / 16) + sb] = (uint8_t) sb8;

@@ -1,0 +1,49 @@
+"""Packed prompt experts at the row counts where a 128-row tile's image changes its length (whole groups of eight rows, one more,
+one less, one row, two tiles), at one and several chunks of either product, and with an output that is only 16-byte aligned.
+Bound 7e-4: four times the four-term FP4 error of a row (1.8e-4)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from basalt_b200 import capi, moe
+from oracle import oracle as O
+from tests.helpers import make_expert_blobs, rel_l2, stack_blobs
+from tests.test_experts_gpu import dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,I,shift", [(256, 256, 0), (512, 512, 16), (768, 768, 0), (256, 1024, 16), (2048, 512, 0)])
+def test_tile_row_counts(lib, cuda, H, I, shift):
+    rng = np.random.default_rng(H * 3 + I)
+    counts = [1, 0, 7, 8, 9, 127, 128, 129, 0, 260]
+    E = len(counts)
+    Lo, blobs = make_expert_blobs(rng, E, O.T_NVFP4, O.T_NVFP4, H, I)
+    L = moe.native_expert_layout(O.T_NVFP4, O.T_NVFP4, H, I)
+    packed = moe.pack_experts(L, dev(stack_blobs(blobs)))
+    n, T = sum(counts), 300
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    src = rng.integers(0, T, n).astype(np.int32)
+    tiles = np.array([(e, off[e] + 128 * i) for e in range(E) for i in range((counts[e] + 127) // 128)], np.int32)
+    x = rng.standard_normal((T, H)).astype(np.float32)
+    table = packed.data_ptr() + torch.arange(E, dtype=torch.int64, device="cuda") * packed.shape[1]
+    lb = capi.lib()
+    scratch = torch.empty(lb.bsx_experts_prefill_packed_scratch_bytes(C.byref(L), T, n), dtype=torch.uint8, device="cuda")
+    raw = torch.full((n * H * 4 + 256,), 0xFF, dtype=torch.uint8, device="cuda")
+    dm = raw[shift:shift + n * H * 4].view(torch.float32).view(n, H)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    o, s, t, nt, xd = dev(off), dev(src), dev(tiles), dev(np.array([len(tiles)], np.int32)), dev(x)
+    stream = moe._stream(None)
+    torch.cuda.synchronize()
+    capi.check("prefill packed", lb.bsx_experts_prefill_packed(C.byref(L), table.data_ptr(), o.data_ptr(), s.data_ptr(), t.data_ptr(), nt.data_ptr(),
+                                                               len(tiles), n, xd.data_ptr(), capi.X_F32, T, E, scratch.data_ptr(), dm.data_ptr(),
+                                                               status.data_ptr(), stream))
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    got = dm.cpu().numpy()
+    for e in range(E):
+        if counts[e]:
+            want = O.expert_forward(Lo, blobs[e], x[src[off[e]:off[e + 1]]], dtype=np.float64)
+            assert rel_l2(got[off[e]:off[e + 1]], want) < 7e-4, (e, counts[e])
