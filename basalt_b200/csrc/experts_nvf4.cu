@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) nvf4_stream_kernel(StreamArgs sa
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
     const ExpertArgs& a = sa.e;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int64_t K = MODE == FMODE_GU ? a.L.n_embd : a.L.n_ff;
     const int64_t R = MODE == FMODE_GU ? a.L.n_ff : a.L.n_embd;       // rows of each weight matrix
     const int n_chunk = (int) (K >> 8);                                 // stages (256 columns) per unit
@@ -299,7 +299,9 @@ __global__ void __launch_bounds__(kThreadsF, 1) nvf4_stream_kernel(StreamArgs sa
 
     if (warp == 0) {
         // ---- MMA issuer: per 64-column K-step the three scale copies (smem -> tensor memory), then one MMA per tile
-        if (lane == 0) {
+        // Twenty instructions a stage: under `lane == 0` their issue (~120 cycles each) held the stream below the memory rate (64-token
+        // step of 2048 x 512: 127.8 us, of 7168 x 2048: 848 us; under elect.sync 113.6 and 694)
+        if (elect_one()) {
             uint32_t kc = 0, ti = 0;
             for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
                 int rb0, rb1;
@@ -317,20 +319,23 @@ __global__ void __launch_bounds__(kThreadsF, 1) nvf4_stream_kernel(StreamArgs sa
                         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                         const uint32_t st = smem_u32(smem + s * kStageF);
                         const uint32_t tsf = tmem + kTmemSF + s * 48;
+                        // descriptors count addresses in 16 bytes: a K-step further is 32 bytes of codes, 512 of scale words
+                        const uint64_t a0 = smem_desc_sw128(st), a1 = smem_desc_sw128(st + kOffA1), bd0 = smem_desc_sw128(st + kOffB);
+                        const uint64_t f0 = sf_desc(st + kOffSFA0), f1 = sf_desc(st + kOffSFA1), fb = sf_desc(st + kOffSFB);
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
-                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsf + 4 * k), "l"(sf_desc(st + kOffSFA0 + k * 512)) : "memory");
-                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsf + 16 + 4 * k), "l"(sf_desc(st + kOffSFA1 + k * 512)) : "memory");
-                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsf + 32 + 4 * k), "l"(sf_desc(st + kOffSFB + k * 512)) : "memory");
-                            const uint64_t bd = smem_desc_sw128(st + kOffB + k * 32);
+                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsf + 4 * k), "l"(f0 + 32 * k) : "memory");
+                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsf + 16 + 4 * k), "l"(f1 + 32 * k) : "memory");
+                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsf + 32 + 4 * k), "l"(fb + 32 * k) : "memory");
+                            const uint64_t bd = bd0 + 2 * k;
                             const uint32_t accum = (c | k) ? 1u : 0u;
                             asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
                                          "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(d0),
-                                         "l"(smem_desc_sw128(st + k * 32)), "l"(bd), "r"(kIdescF), "r"(tsf + 4 * k), "r"(tsf + 32 + 4 * k), "r"(accum)
+                                         "l"(a0 + 2 * k), "l"(bd), "r"(kIdescF), "r"(tsf + 4 * k), "r"(tsf + 32 + 4 * k), "r"(accum)
                                          : "memory");
                             asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
                                          "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(d1),
-                                         "l"(smem_desc_sw128(st + kOffA1 + k * 32)), "l"(bd), "r"(kIdescF), "r"(tsf + 16 + 4 * k), "r"(tsf + 32 + 4 * k), "r"(accum)
+                                         "l"(a1 + 2 * k), "l"(bd), "r"(kIdescF), "r"(tsf + 16 + 4 * k), "r"(tsf + 32 + 4 * k), "r"(accum)
                                          : "memory");
                         }
                         umma_commit(&empty[s]);
@@ -346,7 +351,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) nvf4_stream_kernel(StreamArgs sa
         // ---- weight loader: one lane, two bulk copies a stage (each a whole block of the packed blob: 16 KB of codes already
         // in the stage's swizzled order + 2 KB of scales), completion counted in bytes on the stage's mbarrier.  The next
         // unit's pass record is requested while this unit streams.
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t issued = 0;
             PassRec nxt;
             nxt.blob = 0ull; nxt.eb = 0; nxt.ntok = 0;

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
     uint32_t* lut = tmem_slot + 2;                // [256] fp16 scale pairs
     uint16_t* s_grid = reinterpret_cast<uint16_t*>(lut + 256);   // [2048] the IQ1 codebook (IQ1_M rows only)
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int64_t K = MODE == PMODE_GU ? a.L.n_embd : a.L.n_ff;
     const int nkb = (int) (K / kBlockK);
     const int n_out = MODE == PMODE_GU ? (int) a.L.n_ff : (int) a.L.n_embd;      // neurons, or down rows
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
 
     if (warp == 0) {
         // ---- MMA issuer: one lane feeds the tensor core, four k = 16 instructions per 64-column k-block
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t kc = 0, ti = 0;
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
                 Item it;
@@ -219,9 +219,9 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     const uint32_t sa = smem_u32(smem + s * kStage), sb = sa + kABytes;
+                    const uint64_t ad = smem_desc_sw128(sa), bd = smem_desc_sw128(sb);      // addresses in 16 bytes: 2 a step
 #pragma unroll
-                    for (int k = 0; k < kBlockK / 16; ++k)
-                        umma_f16(tmem + acc * kTileN, smem_desc_sw128(sa + k * 32), smem_desc_sw128(sb + k * 32), kInstrDesc, (kb | k) ? 1u : 0u);
+                    for (int k = 0; k < kBlockK / 16; ++k) umma_f16(tmem + acc * kTileN, ad + 2 * k, bd + 2 * k, kInstrDesc, (kb | k) ? 1u : 0u);
                     umma_commit(&empty[s]);      // the stage may be refilled once these MMAs have read it
                 }
                 if (!ok) break;

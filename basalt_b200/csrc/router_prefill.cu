@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kThreadsR, 1) router_logits_tc_kernel(LogitsAr
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
     float* s_ginv = reinterpret_cast<float*>(smem + kStg * kStageR + 128);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int e0 = blockIdx.x * kTN;
     const int64_t t0 = (int64_t) blockIdx.y * kTM;
     const int nkb = a.H / kBK;
@@ -112,15 +112,16 @@ __global__ void __launch_bounds__(kThreadsR, 1) router_logits_tc_kernel(LogitsAr
     bool ok = true;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             for (int it = 0; it < n_it; ++it) {
                 const uint32_t s = (uint32_t) it % kStg;
                 ok = mbar_wait(&full[s], ((uint32_t) it / kStg) & 1u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t sa = smem_u32(smem + s * kStageR), sb = sa + kABytesR;
+                const uint64_t ad = smem_desc_sw128(sa), bd = smem_desc_sw128(sb);          // addresses in 16 bytes: 2 a step
 #pragma unroll
-                for (int k = 0; k < kBK / 16; ++k) umma_f16(tmem, smem_desc_sw128(sa + k * 32), smem_desc_sw128(sb + k * 32), kIdescR, (it | k) ? 1u : 0u);
+                for (int k = 0; k < kBK / 16; ++k) umma_f16(tmem, ad + 2 * k, bd + 2 * k, kIdescR, (it | k) ? 1u : 0u);
                 umma_commit(&empty[s]);
             }
             umma_commit(accum);
