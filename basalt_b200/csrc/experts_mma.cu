@@ -1,5 +1,5 @@
-// experts_mma.cu - decode-sized grouped experts for NVFP4 blobs: a bandwidth-bound weight stream through shared memory with
-// the dot products on the tensor cores.
+// experts_mma.cu - decode-sized grouped experts for NVFP4 and IQ3_S blobs: a bandwidth-bound weight stream through shared memory
+// with the dot products on the tensor cores.
 //
 // Shape of the work (HBM-bound): every touched expert's gate, up and down rows are read exactly once per pass of up to 8
 // activation columns.  Each warp owns 16 weight rows (8 gate rows paired with the 8 matching up rows, or 16 down rows) and
@@ -13,6 +13,10 @@
 // B-fragment order and copied into shared memory by cp.async.  Gate and up rows of one neuron land in the same thread's
 // accumulators, so SwiGLU is fused; a second small kernel turns the SwiGLU output into the down product's fp16 image.
 //
+// IQ3_S rows take the same stream with another decoder (iq3s_16): codebook points as four fp16 magnitudes in shared memory, signs
+// and the odd scales applied in packed fp16, exactly.  Bound by the decode's integer work and look-ups.  5 tokens through 512
+// experts of 2048 x 512, top-10: the layer's step takes 155 us, with the warp-per-row fp32 kernels it took 315.
+//
 // Semantics: Basalt's native_expert_grouped (include/basalt/kernels/iq_kernels.hpp:77-92; kernels src/kernels/cuda/iq_kernels.cu:
 // 1605-1658 gate/up, :2512-2524 SwiGLU, :2140-2164 down), NVFP4 decoding per src/kernels/cpu/ggml/ggml_quants.c:1397-1422,
 // tail scales per iq_kernels.cu:683-701 - but without the int8 rounding of x and h the reference applies.
@@ -22,6 +26,7 @@
 #include "common.cuh"
 #include "experts.cuh"
 #include "formats.cuh"
+#include "pdl.cuh"
 
 namespace bsx {
 namespace {
@@ -29,10 +34,22 @@ namespace {
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 constexpr int kStages = 4;
-constexpr int kRowBytes = 144;                 // 4 NVFP4 blocks = 256 columns of one row
 constexpr int kRows = 16;                      // weight rows per warp
-constexpr int kStageBytes = kRows * kRowBytes; // 2304
 constexpr int kCols = 8;                       // MMA n: activation columns per pass
+
+// The formats.  A chunk of a row is what a stage holds: 4 NVFP4 blocks of 64 columns, or 2 IQ3_S blocks of 256 (110 bytes, so every
+// second one starts on 4 bytes).  kTable: the shared-memory table, 256 fp16 scale pairs or 512 points of four fp16 magnitudes.
+enum { FMT_NVFP4 = 0, FMT_IQ3S = 1 };
+template <int FMT> struct Fmt;
+template <> struct Fmt<FMT_NVFP4> {
+    static constexpr int kRowBytes = 144, kGranules = 4, kTable = 1024;
+    static constexpr float kUnscale = 256.f;           // the block scales are used as scale / 2^8
+};
+template <> struct Fmt<FMT_IQ3S> {
+    static constexpr int kRowBytes = 220, kGranules = 8, kTable = 4096;
+    static constexpr float kUnscale = 1.f;
+};
+template <int FMT> constexpr int kStageBytes = kRows * Fmt<FMT>::kRowBytes;
 
 enum { MODE_GU = 0, MODE_DOWN = 1 };
 
@@ -84,6 +101,36 @@ __device__ __forceinline__ uint32_t scale_pair_bits(uint32_t byte) {
     return v | (v << 16);
 }
 
+// IQ3_S (include/basalt/ggml/ggml_common.h block_iq3_s: fp16 d, qs[64], qh[8], signs[32], scales[4]; decode rule
+// src/kernels/cpu/ggml/ggml_quants.c:1200-1239): a weight is d (2 s + 1) x +-(2 c + 1), c a 3-bit coordinate of a 512-point
+// codebook.  One thread decodes the 16 values [16 t, 16 t + 16) of granule `gr` (64 columns) of a row's block: four points, 16 sign
+// bits, one scale.  Magnitude x scale is an integer up to 465, exact in fp16; d stays outside the sums.  q[i]: values i and i + 8.
+__device__ __forceinline__ void iq3s_16(const uint8_t* blk, int gr, int t, const uint2* __restrict__ points, uint32_t (&q)[8]) {
+    const int ib = 2 * gr + (t >> 1), half = t & 1;
+    const uint16_t* qs = reinterpret_cast<const uint16_t*>(blk + 2 + 8 * ib + 4 * half);
+    const uint32_t q01 = qs[0], q23 = qs[1];
+    const uint32_t qh = (uint32_t) blk[66 + ib] >> (4 * half);
+    const uint32_t sg = *reinterpret_cast<const uint16_t*>(blk + 74 + 4 * ib + 2 * half);
+    const uint32_t s = ((uint32_t) blk[106 + gr] >> (4 * (t >> 1))) & 15u;      // 2 units of 32 columns a byte
+    // 2 s + 1 as an fp16 pair: 1024 + (2 s + 1) is a fp16 whose low bits are the integer
+    const __half2 m = __hsub2(__halves2half2(__ushort_as_half((unsigned short) (0x6400u + 2u * s + 1u)), __ushort_as_half((unsigned short) (0x6400u + 2u * s + 1u))),
+                              __float2half2_rn(1024.f));
+    const uint32_t mm = *reinterpret_cast<const uint32_t*>(&m);
+    const uint2 p0 = points[(q01 & 0xFFu) | ((qh & 1u) << 8)], p1 = points[(q01 >> 8) | ((qh & 2u) << 7)];
+    const uint2 p2 = points[(q23 & 0xFFu) | ((qh & 4u) << 6)], p3 = points[(q23 >> 8) | ((qh & 8u) << 5)];
+    const uint32_t sw = __byte_perm(sg, 0u, 0x4140);                             // signs of values 0-7 low, of 8-15 high half
+    q[0] = __byte_perm(p0.x, p2.x, 0x5410);
+    q[1] = __byte_perm(p0.x, p2.x, 0x7632);
+    q[2] = __byte_perm(p0.y, p2.y, 0x5410);
+    q[3] = __byte_perm(p0.y, p2.y, 0x7632);
+    q[4] = __byte_perm(p1.x, p3.x, 0x5410);
+    q[5] = __byte_perm(p1.x, p3.x, 0x7632);
+    q[6] = __byte_perm(p1.y, p3.y, 0x5410);
+    q[7] = __byte_perm(p1.y, p3.y, 0x7632);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = hmul2_bits(q[i] ^ ((sw << (15 - i)) & 0x80008000u), mm);
+}
+
 // Where column c of an activation row sits in its fp16 image, which is laid out so that a thread's B fragments are two
 // 16-byte pieces per 64 columns: piece (gran, h, t) holds, for sub-block t of granule gran, the values the thread with
 // id-in-group t needs for MMA steps 2h and 2h + 1.  Step s takes code bytes 2s and 2s + 1 of the sub-block's 8 bytes; byte b
@@ -115,6 +162,8 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 template <bool FROM_H, int TERMS>
 __global__ void __launch_bounds__(256)
 prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ inv, int2* __restrict__ items, int* __restrict__ n_items) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int ng = min(*a.n_groups, (int) a.cap_groups);
     const int total = min(a.grp_start[ng], (int) a.cap_entries);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -202,26 +251,38 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
 // PIECE: bytes of one weight copy = the rows' alignment.  16 where K is whole 256-column chunks; a row of any other K (whole
 // 64-column NVFP4 blocks, 36 bytes each) starts on 8 bytes (K % 128 == 0) or 4, and its last chunk holds fewer than four blocks:
 // those pieces are not requested and those blocks not multiplied.
-template <int MODE, int TERMS, int PIECE>
+template <int FMT, int MODE, int TERMS, int PIECE>
 __global__ void __launch_bounds__(kThreads, 2)
-nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __restrict__ inv, const int2* __restrict__ items,
+blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __restrict__ inv, const int2* __restrict__ items,
                  int* __restrict__ n_items, int tiles_per_warp, int n_row_blocks) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff;
     const int n_gran = (int) (K >> 6);                       // 64-column granules
     __half* xs = reinterpret_cast<__half*>(smem);            // [n_gran][2][8 cols][4][8]
-    uint32_t* lut = reinterpret_cast<uint32_t*>(smem + (size_t) K * kCols * 2);   // [256] scale pairs
-    uint4* zero = reinterpret_cast<uint4*>(smem + (size_t) K * kCols * 2 + 1024);   // 64 zero bytes: the B fragments of unused columns
-    uint8_t* wbase = smem + (size_t) K * kCols * 2 + 1152;
+    using F = Fmt<FMT>;
+    constexpr int kRowBytes = F::kRowBytes, kStageB = kStageBytes<FMT>;
+    uint32_t* lut = reinterpret_cast<uint32_t*>(smem + (size_t) K * kCols * 2);     // the format's table
+    uint4* zero = reinterpret_cast<uint4*>(smem + (size_t) K * kCols * 2 + F::kTable);   // 64 zero bytes: the B fragments of unused columns
+    uint8_t* wbase = smem + (size_t) K * kCols * 2 + F::kTable + 128;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    uint8_t* wring = wbase + (size_t) warp * kStages * kStageBytes;
+    uint8_t* wring = wbase + (size_t) warp * kStages * kStageB;
     const uint32_t wring_s = (uint32_t) __cvta_generic_to_shared(wring);
     const uint32_t xs_s = (uint32_t) __cvta_generic_to_shared(xs);
     constexpr int NTOK = kCols / TERMS;
 
     __shared__ int s_ir[kCols];                        // image row of each entry of the pass
-    lut[threadIdx.x] = scale_pair_bits(threadIdx.x);   // 256 threads, 256 entries; the first barrier below publishes it
+    // 256 threads; the first barrier below publishes the table
+    if constexpr (FMT == FMT_NVFP4) {
+        lut[threadIdx.x] = scale_pair_bits(threadIdx.x);
+    } else {
+        for (int i = threadIdx.x; i < 512; i += kThreads) {
+            const uint32_t pt = a.grid[kGridIQ3S + i];
+            const __half2 lo = __floats2half2_rn((float) (2u * (pt & 7u) + 1u), (float) (2u * ((pt >> 3) & 7u) + 1u));
+            const __half2 hi = __floats2half2_rn((float) (2u * ((pt >> 6) & 7u) + 1u), (float) (2u * ((pt >> 9) & 7u) + 1u));
+            reinterpret_cast<uint2*>(lut)[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        }
+    }
     if (threadIdx.x < 4) zero[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
 
     const int64_t n_rows = MODE == MODE_GU ? a.L.n_ff : a.L.n_embd;      // neurons (pairs) or down rows
@@ -231,12 +292,14 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
     constexpr int kTileRows = MODE == MODE_GU ? 8 : 16;
     constexpr int tile_stride = kWarps * kTileRows;
     __shared__ int s_work;
-    const int n_chunks = (n_gran + 3) >> 2;
-    const int last_bytes = PIECE == 16 ? kRowBytes : (n_gran - 4 * (n_chunks - 1)) * 36;   // bytes of a row in the last chunk
+    const int n_chunks = (n_gran + F::kGranules - 1) / F::kGranules;
+    const int last_bytes = FMT == FMT_IQ3S || PIECE == 16 ? kRowBytes : (n_gran - 4 * (n_chunks - 1)) * 36;   // bytes of a row in the last chunk
     const int pieces_per_col = (int) (K >> 3);               // 16-byte pieces of one image
 
     // this lane's copy duty inside a stage: pieces lane, lane + 32, ...; row = piece / kRowPieces
-    constexpr int kRowPieces = kRowBytes / PIECE, kPieces = kRows * kRowPieces, kCopies = (kPieces + 31) / 32;
+    // (IQ3_S: 55 words a row, a row at a time - lane and lane + 32 - so that no address lives in a register of its own)
+    constexpr bool kByRow = FMT == FMT_IQ3S;
+    constexpr int kRowPieces = kRowBytes / PIECE, kPieces = kRows * kRowPieces, kCopies = kByRow ? 1 : (kPieces + 31) / 32;
     int cp_row[kCopies], cp_off[kCopies];
     uint32_t cp_dst[kCopies];
 #pragma unroll
@@ -247,6 +310,8 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
         cp_dst[j] = (uint32_t) (cp_row[j] * kRowBytes + cp_off[j]);
     }
 
+    pdl_wait();      // the table does not depend on earlier kernels; everything below does
+    pdl_launch_dependents();
     const int n_work = n_items[0] * n_row_blocks;
     for (;;) {
         __syncthreads();   // the previous unit is done with xs and s_work
@@ -268,7 +333,7 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
         const uint8_t* src[kCopies];
 #pragma unroll
         for (int j = 0; j < kCopies; ++j) {
-            const int row = cp_row[j];
+            const int row = kByRow ? 0 : cp_row[j];
             const uint8_t* rp;
             if (MODE == MODE_GU)
                 rp = row < 8 ? blob + (size_t) (r0 + row) * a.L.gu_row : blob + a.L.up_off + (size_t) (r0 + row - 8) * a.L.up_row;
@@ -276,17 +341,30 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
                 rp = blob + a.L.down_off + (size_t) (r0 + row) * a.L.d_row;
             src[j] = rp + cp_off[j];
         }
+        // row 8's distance from row 0 (the first up row from the first gate row), and a row's from the one before it in each half
+        const size_t row8 = MODE == MODE_GU ? (size_t) a.L.up_off + (size_t) r0 * (a.L.up_row - a.L.gu_row) : 8 * (size_t) a.L.d_row;
+        const size_t pitch0 = MODE == MODE_GU ? (size_t) a.L.gu_row : (size_t) a.L.d_row, pitch1 = MODE == MODE_GU ? (size_t) a.L.up_row : (size_t) a.L.d_row;
         const size_t tile_bytes = (size_t) tile_stride * (MODE == MODE_GU ? a.L.gu_row : a.L.d_row);
         // the next (tile, chunk) unit to request and its global byte offset from the tile-0, chunk-0 addresses
         int iss_unit = 0, iss_chunk = 0;
         size_t iss_off = 0;
         auto issue = [&]() {
             if (iss_unit < n_units) {
-                const uint32_t dst = wring_s + (uint32_t) (iss_unit & (kStages - 1)) * kStageBytes;
+                const uint32_t dst = wring_s + (uint32_t) (iss_unit & (kStages - 1)) * kStageB;
                 const int row_bytes = iss_chunk + 1 < n_chunks ? kRowBytes : last_bytes;
+                if constexpr (kByRow) {
+#pragma unroll
+                    for (int row = 0; row < kRows; ++row) {
+                        const uint8_t* p = src[0] + iss_off + (row < 8 ? row * pitch0 : row8 + (row - 8) * pitch1);
+                        const uint32_t d = dst + (uint32_t) (row * kRowBytes + 4 * lane);
+                        cp_async_piece<PIECE>(d, p);
+                        if (lane < kRowPieces - 32) cp_async_piece<PIECE>(d + 128, p + 128);
+                    }
+                } else {
 #pragma unroll
                 for (int j = 0; j < kCopies; ++j)
-                    if (lane + 32 * j < kPieces && (PIECE == 16 || cp_off[j] < row_bytes)) cp_async_piece<PIECE>(dst + cp_dst[j], src[j] + iss_off);
+                    if (lane + 32 * j < kPieces && (FMT == FMT_IQ3S || PIECE == 16 || cp_off[j] < row_bytes)) cp_async_piece<PIECE>(dst + cp_dst[j], src[j] + iss_off);
+                }
                 ++iss_unit;
                 if (++iss_chunk == n_chunks) {
                     iss_chunk = 0;
@@ -327,8 +405,8 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
             int64_t o0 = 0, o1 = 0;
             {
                 const int j0 = TERMS == 1 ? 2 * t : t, j1 = 2 * t + 1;
-                if (j0 < ntok) f0 = inv[s_ir[j0]] * 256.f;
-                if (TERMS == 1 && j1 < ntok) f1 = inv[s_ir[j1]] * 256.f;
+                if (j0 < ntok) f0 = inv[s_ir[j0]] * F::kUnscale;
+                if (TERMS == 1 && j1 < ntok) f1 = inv[s_ir[j1]] * F::kUnscale;
                 if (MODE == MODE_GU) {
                     o0 = (int64_t) (eb + j0) * a.L.n_ff;
                     o1 = (int64_t) (eb + j1) * a.L.n_ff;
@@ -337,7 +415,8 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
                     if (TERMS == 1 && j1 < ntok) o1 = (int64_t) a.ent_dst[eb + j1] * a.L.n_embd;
                 }
             }
-            const float sg = tail[0], su = tail[1], sd = tail[2];
+            float sg = 1.f, su = 1.f, sd = 1.f;
+            if constexpr (FMT == FMT_NVFP4) { sg = tail[0]; su = tail[1]; sd = tail[2]; }
             // two accumulator sets, so that consecutive MMAs do not wait on each other
             float acc[4] = {0.f, 0.f, 0.f, 0.f}, acd[4] = {0.f, 0.f, 0.f, 0.f};
             // this lane's B fragments: its column's pieces, or (column unused in this pass) the zero area with stride 0
@@ -350,10 +429,34 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
                 issue();
                 cp_async_wait<kStages - 1>();
                 __syncwarp();
-                const uint8_t* st = wring + (size_t) (unit & (kStages - 1)) * kStageBytes;
+                const uint8_t* st = wring + (size_t) (unit & (kStages - 1)) * kStageB;
                 const uint32_t* ra = reinterpret_cast<const uint32_t*>(st + g * kRowBytes);          // row g
                 const uint32_t* rb = reinterpret_cast<const uint32_t*>(st + (g + 8) * kRowBytes);    // row g + 8
-                const uint4* bp = bcol + (size_t) chunk * 4 * bstep;
+                const uint4* bp = bcol + (size_t) chunk * F::kGranules * bstep;
+                if constexpr (FMT == FMT_IQ3S) {
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const uint8_t* ba = reinterpret_cast<const uint8_t*>(ra) + 110 * b;
+                        const uint8_t* bb = reinterpret_cast<const uint8_t*>(rb) + 110 * b;
+                        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                        for (int gr = 0; gr < 4; ++gr) {
+                            const uint4 b0 = bp[(4 * b + gr) * bstep], b1 = bp[(4 * b + gr) * bstep + bhalf];
+                            uint32_t qa[8], qb[8];
+                            iq3s_16(ba, gr, t, reinterpret_cast<const uint2*>(lut), qa);
+                            iq3s_16(bb, gr, t, reinterpret_cast<const uint2*>(lut), qb);
+                            mma_f16(s0, qa[0], qb[0], qa[1], qb[1], b0.x, b0.y);
+                            mma_f16(s1, qa[2], qb[2], qa[3], qb[3], b0.z, b0.w);
+                            mma_f16(s0, qa[4], qb[4], qa[5], qb[5], b1.x, b1.y);
+                            mma_f16(s1, qa[6], qb[6], qa[7], qb[7], b1.z, b1.w);
+                        }
+                        const float da = __half2float(*reinterpret_cast<const __half*>(ba)), db = __half2float(*reinterpret_cast<const __half*>(bb));
+                        acc[0] = fmaf(s0[0] + s1[0], da, acc[0]);
+                        acc[1] = fmaf(s0[1] + s1[1], da, acc[1]);
+                        acc[2] = fmaf(s0[2] + s1[2], db, acc[2]);
+                        acc[3] = fmaf(s0[3] + s1[3], db, acc[3]);
+                    }
+                } else {
 #pragma unroll
                 for (int blk = 0; blk < 4; ++blk) {
                     if (PIECE != 16 && 4 * chunk + blk >= n_gran) break;   // past the row's last block
@@ -376,6 +479,7 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
                     mma_f16(acd, qa0[2], qb0[2], qa0[3], qb0[3], b0.z, b0.w);
                     mma_f16(acc, qa1[0], qb1[0], qa1[1], qb1[1], b1.x, b1.y);
                     mma_f16(acd, qa1[2], qb1[2], qa1[3], qb1[3], b1.z, b1.w);
+                }
                 }
                 __syncwarp();   // every lane is done with this stage before a later issue overwrites it
                 if (++chunk != n_chunks) continue;
@@ -415,25 +519,26 @@ nvfp4_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __re
     cp_async_wait<0>();
 }
 
-size_t smem_bytes(int64_t K) { return (size_t) K * kCols * 2 + 1152 + (size_t) kWarps * kStages * kStageBytes; }
+template <int FMT>
+size_t smem_bytes(int64_t K) { return (size_t) K * kCols * 2 + Fmt<FMT>::kTable + 128 + (size_t) kWarps * kStages * kStageBytes<FMT>; }
 size_t align256(size_t v) { return (v + 255) & ~(size_t) 255; }
 
-template <int MODE, int TERMS, int PIECE = 16>
+template <int FMT, int MODE, int TERMS, int PIECE = 16>
 int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const int2* items, int* n_items, cudaStream_t st) {
     const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff;
-    const size_t smem = smem_bytes(K);
+    const size_t smem = smem_bytes<FMT>(K);
     static std::atomic<bool> configured[64];   // per device; threads of different devices call concurrently
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(nvfp4_mma_kernel<MODE, TERMS, PIECE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        const cudaError_t e = cudaFuncSetAttribute(blk_mma_kernel<FMT, MODE, TERMS, PIECE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
     const int64_t rows = MODE == MODE_GU ? a.L.n_ff : a.L.n_embd;
     // a work unit streams ~150 KB of weights (enough to hide its start-up: activation copy, first loads); the row tiles of an
     // expert are dealt evenly over the units
-    const int64_t tile_bytes = (int64_t) kWarps * 16 * (K / 64 * 36);
+    const int64_t tile_bytes = (int64_t) kWarps * 16 * (FMT == FMT_IQ3S ? K / 256 * 110 : K / 64 * 36);
     const int64_t tile_rows = MODE == MODE_GU ? kWarps * 8 : kWarps * 16;
     const int64_t n_tiles = (rows + tile_rows - 1) / tile_rows;
     int64_t tpw0 = (150 * 1024 + tile_bytes - 1) / tile_bytes;
@@ -441,7 +546,7 @@ int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const i
     const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
     const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
     const int n_row_blocks = (int) ((n_tiles + tpw - 1) / tpw);
-    nvfp4_mma_kernel<MODE, TERMS, PIECE><<<(unsigned) (2 * sm_count()), kThreads, smem, st>>>(a, img, inv, items, n_items, tpw, n_row_blocks);
+    launch_k(blk_mma_kernel<FMT, MODE, TERMS, PIECE>, dim3((unsigned) (2 * sm_count())), dim3(kThreads), smem, st, a, img, inv, items, n_items, tpw, n_row_blocks);
     return launch_status();
 }
 
@@ -456,11 +561,18 @@ size_t experts_mma_scratch_bytes(int64_t cap_entries, int64_t n_embd, int64_t n_
 
 int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     const bsx_expert_layout& L = a.L;
-    if (L.gu_type != kTypeNVFP4 || L.up_type != kTypeNVFP4 || L.d_type != kTypeNVFP4) return BSX_E_TYPE;
-    // gate and up rows are whole 256-column chunks (n_embd % 256 == 0 in every layout), down rows whole 64-column blocks; the
-    // activation image must fit shared memory
-    if (L.n_embd % 256 || L.n_ff % 64) return BSX_E_TYPE;
-    if (smem_bytes(L.n_embd) > 200 * 1024 || smem_bytes(L.n_ff) > 200 * 1024) return BSX_E_TYPE;
+    // NVFP4: gate and up rows are whole 256-column chunks (n_embd % 256 == 0 in every layout), down rows whole 64-column blocks.
+    // IQ3_S: rows of whole 512-column chunks (every other 110-byte block starts on 4 bytes, what the copies need).  The activation
+    // image must fit shared memory.
+    const int fmt = L.gu_type == kTypeNVFP4 ? FMT_NVFP4 : FMT_IQ3S;
+    if ((L.gu_type != kTypeNVFP4 && L.gu_type != kTypeIQ3S) || L.up_type != L.gu_type || L.d_type != L.gu_type) return BSX_E_TYPE;
+    if (fmt == FMT_NVFP4) {
+        if (L.n_embd % 256 || L.n_ff % 64) return BSX_E_TYPE;
+        if (smem_bytes<FMT_NVFP4>(L.n_embd) > 200 * 1024 || smem_bytes<FMT_NVFP4>(L.n_ff) > 200 * 1024) return BSX_E_TYPE;
+    } else {
+        if (L.n_embd % 512 || L.n_ff % 512) return BSX_E_TYPE;
+        if (smem_bytes<FMT_IQ3S>(L.n_embd) > 200 * 1024 || smem_bytes<FMT_IQ3S>(L.n_ff) > 200 * 1024) return BSX_E_TYPE;
+    }
     // scratch: [h fp32][x images][h images][x inverse scales][h inverse scales]
     uint8_t* p = reinterpret_cast<uint8_t*>(a.h) + align256((size_t) a.cap_entries * L.n_ff * 4);
     __half* ximg = reinterpret_cast<__half*>(p);
@@ -478,21 +590,22 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     int32_t rc = BSX_OK;
     if (phase != 2) {
         if (a.x_kind == BSX_X_BF16) {
-            prep_image_kernel<false, 1><<<nbx, 256, 0, st>>>(a, ximg, xinv, items, n_items);
-            rc = launch<MODE_GU, 1>(a, ximg, xinv, items, n_items, st);
+            launch_k(prep_image_kernel<false, 1>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
+            rc = fmt == FMT_NVFP4 ? launch<FMT_NVFP4, MODE_GU, 1>(a, ximg, xinv, items, n_items, st) : launch<FMT_IQ3S, MODE_GU, 1, 4>(a, ximg, xinv, items, n_items, st);
         } else {
-            prep_image_kernel<false, 2><<<nbx, 256, 0, st>>>(a, ximg, xinv, items, n_items);
-            rc = launch<MODE_GU, 2>(a, ximg, xinv, items, n_items, st);
+            launch_k(prep_image_kernel<false, 2>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
+            rc = fmt == FMT_NVFP4 ? launch<FMT_NVFP4, MODE_GU, 2>(a, ximg, xinv, items, n_items, st) : launch<FMT_IQ3S, MODE_GU, 2, 4>(a, ximg, xinv, items, n_items, st);
         }
     }
     if (rc != BSX_OK || phase == 1) return rc;
-    prep_image_kernel<true, 2><<<nbh, 256, 0, st>>>(a, himg, hinv, items, n_items);
+    launch_k(prep_image_kernel<true, 2>, dim3(nbh), dim3(256), 0, st, a, himg, hinv, items, n_items);
+    if (fmt == FMT_IQ3S) return launch<FMT_IQ3S, MODE_DOWN, 2, 4>(a, himg, hinv, items, n_items, st);
     // Down rows of n_ff columns: the copies' width is what their start is aligned to.  An n_ff that is not whole 256-column chunks
     // went to the warp-per-row kernels before (2 % of the copy bandwidth: fp32 decode and FMA for every weight and entry); here
     // the same 27-token step (2560 x 640, 512 + 1 experts, top-10) takes 205 us instead of 3648.
-    if (L.n_ff % 256 == 0) return launch<MODE_DOWN, 2>(a, himg, hinv, items, n_items, st);
-    if (L.n_ff % 128 == 0) return launch<MODE_DOWN, 2, 8>(a, himg, hinv, items, n_items, st);
-    return launch<MODE_DOWN, 2, 4>(a, himg, hinv, items, n_items, st);
+    if (L.n_ff % 256 == 0) return launch<FMT_NVFP4, MODE_DOWN, 2>(a, himg, hinv, items, n_items, st);
+    if (L.n_ff % 128 == 0) return launch<FMT_NVFP4, MODE_DOWN, 2, 8>(a, himg, hinv, items, n_items, st);
+    return launch<FMT_NVFP4, MODE_DOWN, 2, 4>(a, himg, hinv, items, n_items, st);
 }
 
 }  // namespace bsx
