@@ -41,16 +41,19 @@ constexpr float kTerm2 = 1.0f / 254.0f;
 
 enum { QMODE_GU = 0, QMODE_DOWN = 1 };
 
+// kChunkBlocks 256-column blocks of a row are a stage.  IQ1_M: two blocks (112 bytes), copied in 16-byte pieces.  Q6_K: one 210-byte
+// block as the 53 words that cover it (every second block starts on 2 bytes, so its copy starts 2 bytes early; none reaches past its
+// row), rows 60 words apart, which keeps a quarter-warp's reads in different banks.  One block a stage lets any power-of-two part
+// of a row be a warp's own (KS below) and two CTAs of eight warps share an SM.
 template <int TYPE> struct QT;
 template <> struct QT<kTypeIQ1M> {
-    static constexpr int kBlock = 56, kWarps = 16, kStages = 3, kPiece = 16, kPad = 32;
+    static constexpr int kBlock = 56, kWarps = 16, kPad = 32, kChunkBlocks = 2, kRowStage = 112;
     static constexpr bool kCorr = true;
 };
 template <> struct QT<kTypeQ6K> {
-    static constexpr int kBlock = 210, kWarps = 8, kStages = 3, kPiece = 4, kPad = 16;
+    static constexpr int kBlock = 210, kWarps = 8, kPad = 16, kChunkBlocks = 1, kRowStage = 240;
     static constexpr bool kCorr = false;
 };
-constexpr int kChunkBlocks = 2;   // 512 columns a stage
 
 __device__ __forceinline__ void cpa16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void cpa4(uint32_t dst, const void* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory"); }
@@ -190,6 +193,8 @@ kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ cor
 // activation columns; adds d / 8-scaled... the caller scales: tot[i] += I[i] * d[row] where I is the exact integer
 // 8 m c q - coefficient sums described at the top.  bcol: this lane's column, at the block's first byte plus 8 t;
 // ccol: the column's 64 correction bytes of this block.
+// tab: the lane's copy of the table (NC copies interleaved point by point).
+template <int NC>
 __device__ __forceinline__ void iq1m_block(const uint8_t* ra, const uint8_t* rb, const uint2* __restrict__ tab, const uint8_t* bcol,
                                            const uint8_t* ccol, int t, float (&tot)[4]) {
     uint32_t wa[14], wb[14];
@@ -212,8 +217,8 @@ __device__ __forceinline__ void iq1m_block(const uint8_t* ra, const uint8_t* rb,
         for (int r = 0; r < 2; ++r) {
             const uint32_t* w = r ? wb : wa;
             const uint32_t qsb = __byte_perm(w[u], 0u, sel);
-            const uint32_t nib = (w[8 + (u >> 1)] >> (16 * (u & 1) + s4)) & 0xFu;
-            const uint2 e = tab[nib * 256u + qsb];                                         // 12-bit index: the delta bit rides along
+            const uint32_t nib = (w[8 + (u >> 1)] >> (16 * (u & 1) + s4)) & 7u;
+            const uint2 e = tab[(nib * 256u + qsb) * NC];
             const uint32_t sw = w[12 + (u >> 2)] >> s3;                                    // the thread's scale field of unit u now sits at a fixed bit
             const int fb = 16 * ((u >> 1) & 1) + 6 * (u & 1);
             const uint32_t m = fb > 0 ? (((sw >> (fb - 1)) & 14u) | 1u) : (((sw << 1) & 14u) | 1u);   // 2 s + 1
@@ -294,16 +299,17 @@ __device__ __forceinline__ void q6k_block(const uint8_t* ra, const uint8_t* rb, 
 // ---------------------------------------------------------------- the product kernel
 // MODE GU: rows = 8 gate rows r0.. with the up rows r0..; columns = the entries' x images; writes h (fp32).
 // MODE DOWN: rows = 16 down rows; columns = the entries' h images; writes out rows through ent_dst.
-template <int TYPE, int MODE>
-__global__ void __launch_bounds__(QT<TYPE>::kWarps * 32, 1)
+// KS > 1: KS neighbouring warps share a row tile, each a part of its columns, and their sums meet in shared memory - for calls so
+// small that whole rows would leave most SMs without a unit (a shared expert of 2048 x 512 at 5 tokens: 16 units of 148; its two
+// products took 47 of the step's 155 us, with the split the step takes 121).
+template <int TYPE, int MODE, int KS, int NC, int ST>
+__global__ void __launch_bounds__(QT<TYPE>::kWarps * 32, TYPE == kTypeQ6K && ST == 3 ? 2 : 1)
 kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __restrict__ corr, const float* __restrict__ inv,
               const int2* __restrict__ items, int* __restrict__ n_items, int tiles_per_warp, int n_row_blocks) {
     using Q = QT<TYPE>;
-    constexpr int kWarps = Q::kWarps, kThreads = kWarps * 32, kStages = Q::kStages;
-    constexpr int kChunkBytes = kChunkBlocks * Q::kBlock;      // bytes of one row in a stage
-    constexpr int kStageBytes = kRowsQ * kChunkBytes;
-    constexpr int kPiecesRow = kChunkBytes / Q::kPiece, kPieces = kRowsQ * kPiecesRow;
-    constexpr int kCopies = (kPieces + 31) / 32;
+    constexpr int kWarps = Q::kWarps, kThreads = kWarps * 32, kStages = ST;
+    constexpr int kChunkBlocks = Q::kChunkBlocks, kChunkBytes = kChunkBlocks * Q::kBlock, kRowStage = Q::kRowStage;
+    constexpr int kStageBytes = kRowsQ * kRowStage;
     extern __shared__ __align__(128) uint8_t smem[];
     const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
     const int nblk = (int) (K >> 8);
@@ -311,8 +317,8 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
     const int xstride = nblk * 64 + 16;                                        // ... and between their correction columns
     uint8_t* xs = smem;                                                        // [8][cstride]
     uint8_t* cs = xs + (size_t) kColsQ * cstride;                              // [8][xstride] (IQ1_M)
-    uint2* tab = reinterpret_cast<uint2*>(cs + (Q::kCorr ? (size_t) kColsQ * xstride : 0));   // [4096] (IQ1_M)
-    uint8_t* wbase = reinterpret_cast<uint8_t*>(tab) + (Q::kCorr ? 32768 : 0);
+    uint2* tab = reinterpret_cast<uint2*>(cs + (Q::kCorr ? (size_t) kColsQ * xstride : 0));   // [2048][NC] (IQ1_M)
+    uint8_t* wbase = reinterpret_cast<uint8_t*>(tab) + (Q::kCorr ? 16384 * NC : 0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* wring = wbase + (size_t) warp * kStages * kStageBytes;
@@ -323,17 +329,20 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
 
     if (Q::kCorr) {
         // the codebook as 8 bytes per point, coordinate i's code c = g + 1 in byte i: the two words are the two MMA operand
-        // registers of an 8-weight group.  Indexed by the block's 12-bit (qh nibble, qs byte) pair, whose top bit (the group's
-        // delta sign) does not change the point: 4096 entries, each point twice.
-        for (int i = threadIdx.x; i < 4096; i += kThreads) {
-            const uint32_t p = a.grid[i & 2047];
+        // registers of an 8-weight group.  The look-ups are the kernel's scarce resource (16 data-dependent 8-byte reads a lane and
+        // block), and what they cost is bank conflicts.  NC copies, interleaved so that a lane's copy (lane % NC) lives in 1 / NC of the
+        // banks and only as many lanes compete there: sixteen lanes over sixteen bank pairs collide three deep on average, four
+        // over four two deep.  64-token step of the 7168 x 2048 layer: two copies 1602 us, four 1523.
+        for (int j = threadIdx.x; j < 2048 * NC; j += kThreads) {
+            const int i = j / NC;
+            const uint32_t p = a.grid[i];
             uint32_t lo = 0u, hi = 0u;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 lo |= ((p >> (2 * c)) & 3u) << (8 * c);
                 hi |= ((p >> (2 * c + 8)) & 3u) << (8 * c);
             }
-            tab[i] = make_uint2(lo, hi);
+            tab[j] = make_uint2(lo, hi);
         }
     }
     pdl_wait();
@@ -341,20 +350,22 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
 
     const int64_t n_rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd;
     constexpr int kTileRows = MODE == QMODE_GU ? 8 : 16;
-    constexpr int tile_stride = kWarps * kTileRows;
-    const int n_chunks = nblk / kChunkBlocks;
+    static_assert(kWarps % KS == 0, "");
+    constexpr int tile_stride = kWarps / KS * kTileRows;
+    const int n_chunks = nblk / kChunkBlocks / KS, chunk0 = (warp % KS) * n_chunks;      // this warp's part of a row
     const size_t row_bytes = MODE == QMODE_GU ? (size_t) a.L.gu_row : (size_t) a.L.d_row;
 
-    // this lane's copy duty inside a stage: pieces lane, lane + 32, ...; piece p -> row p / kPiecesRow
     const int n_work = n_items[0] * n_row_blocks;
+    // the next unit is drawn while this one streams: the counter's round trip is off the path from unit to unit
+    int drawn = threadIdx.x == 0 ? atomicAdd(&n_items[1], 1) : 0;
     for (;;) {
-        __syncthreads();   // the previous unit is done with xs, cs, s_ir and s_work
-        if (threadIdx.x == 0) s_work = atomicAdd(&n_items[1], 1);
-        __syncthreads();
+        if (threadIdx.x == 0) s_work = drawn;
+        __syncthreads();   // the previous unit is done with xs, cs and s_ir
         const int work = s_work;
         if (work >= n_work) break;
+        if (threadIdx.x == 0) drawn = atomicAdd(&n_items[1], 1);
         const int item = work / n_row_blocks, rb = work - item * n_row_blocks;
-        const int64_t r0 = (int64_t) rb * tiles_per_warp * tile_stride + warp * kTileRows;
+        const int64_t r0 = (int64_t) rb * tiles_per_warp * tile_stride + warp / KS * kTileRows;
         int live_tiles = 0;
         while (live_tiles < tiles_per_warp && r0 + (int64_t) live_tiles * tile_stride < n_rows) ++live_tiles;
         const int n_units = live_tiles * n_chunks;
@@ -383,39 +394,37 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
             }
             cpa_commit();
         }
-        // the weight stream: (tile, chunk) stages of this warp's 16 rows
-        const uint8_t* rowp[kCopies];
-        uint32_t dsto[kCopies];
-#pragma unroll
-        for (int j = 0; j < kCopies; ++j) {
-            const int p = lane + 32 * j;
-            const int row = p < kPieces ? p / kPiecesRow : 0, off = p < kPieces ? (p - row * kPiecesRow) * Q::kPiece : 0;
-            const uint8_t* rp;
-            if (MODE == QMODE_GU)
-                rp = row < 8 ? blob + (size_t) (r0 + row) * a.L.gu_row : blob + a.L.up_off + (size_t) (r0 + row - 8) * a.L.up_row;
-            else
-                rp = blob + a.L.down_off + (size_t) (r0 + row) * a.L.d_row;
-            rowp[j] = rp + off;
-            dsto[j] = (uint32_t) (row * kChunkBytes + off);
-        }
+        // the weight stream: (tile, chunk) stages of this warp's 16 rows; rows 0-7 `pitch` apart, row 8 `half` past row 0
+        const uint8_t* row0 = MODE == QMODE_GU ? blob + (size_t) r0 * a.L.gu_row : blob + a.L.down_off + (size_t) r0 * a.L.d_row;
+        const size_t pitch0 = row_bytes, pitch1 = MODE == QMODE_GU ? (size_t) a.L.up_row : row_bytes;
+        const size_t half = MODE == QMODE_GU ? (size_t) a.L.up_off + (size_t) r0 * (a.L.up_row - a.L.gu_row) : 8 * row_bytes;
         const size_t tile_bytes = (size_t) tile_stride * row_bytes;
         int iss_unit = 0, iss_chunk = 0;
-        size_t iss_off = 0;
+        size_t iss_tile = 0;
         auto issue = [&]() {
             if (iss_unit < n_units) {
                 const uint32_t dst = wring_s + (uint32_t) (iss_unit % kStages) * kStageBytes;
+                if constexpr (TYPE == kTypeIQ1M) {
+                    const uint8_t* src = row0 + iss_tile + (size_t) (chunk0 + iss_chunk) * kChunkBytes;
 #pragma unroll
-                for (int j = 0; j < kCopies; ++j)
-                    if (lane + 32 * j < kPieces) {
-                        if (Q::kPiece == 16) cpa16(dst + dsto[j], rowp[j] + iss_off);
-                        else cpa4(dst + dsto[j], rowp[j] + iss_off);
+                    for (int j = 0; j < 4; ++j) {                    // 7 pieces a row, 112 in all
+                        const int p = lane + 32 * j, row = p / 7, off = (p - row * 7) * 16;
+                        if (p < 112) cpa16(dst + (uint32_t) (row * kRowStage + off), src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1) + off);
                     }
+                } else {
+                    const uint8_t* src = row0 + iss_tile + (size_t) (chunk0 + iss_chunk) * kChunkBytes - 2 * ((chunk0 + iss_chunk) & 1) + 4 * lane;
+#pragma unroll
+                    for (int row = 0; row < kRowsQ; ++row) {
+                        const uint8_t* r = src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1);
+                        const uint32_t d = dst + (uint32_t) (row * kRowStage + 4 * lane);
+                        cpa4(d, r);
+                        if (lane < 53 - 32) cpa4(d + 128, r + 128);
+                    }
+                }
                 ++iss_unit;
                 if (++iss_chunk == n_chunks) {
                     iss_chunk = 0;
-                    iss_off += tile_bytes - (size_t) (n_chunks - 1) * kChunkBytes;
-                } else {
-                    iss_off += kChunkBytes;
+                    iss_tile += tile_bytes;
                 }
             }
             cpa_commit();
@@ -443,14 +452,16 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
             const uint8_t* st = wring + (size_t) (unit % kStages) * kStageBytes;
 #pragma unroll
             for (int b = 0; b < kChunkBlocks; ++b) {
-                const int blk = chunk * kChunkBlocks + b;
-                const uint8_t* ra = st + g * kChunkBytes + b * Q::kBlock;
-                const uint8_t* rbp = st + (g + 8) * kChunkBytes + b * Q::kBlock;
-                if constexpr (Q::kCorr) iq1m_block(ra, rbp, tab, bcol + 256 * blk, ccol + 64 * blk, t, tot);
+                const int blk = (chunk0 + chunk) * kChunkBlocks + b;
+                const int at = TYPE == kTypeIQ1M ? b * Q::kBlock : 2 * ((chunk0 + chunk) & 1);
+                const uint8_t* ra = st + g * kRowStage + at;
+                const uint8_t* rbp = st + (g + 8) * kRowStage + at;
+                if constexpr (Q::kCorr) iq1m_block<NC>(ra, rbp, tab + (lane & (NC - 1)), bcol + 256 * blk, ccol + 64 * blk, t, tot);
                 else q6k_block(ra, rbp, bcol + 256 * blk, t, tot);
             }
             __syncwarp();   // every lane is done with this stage before a later issue overwrites it
             if (++chunk != n_chunks) continue;
+            if constexpr (KS > 1) break;       // one tile a unit: the parts are put together below
             const int64_t rt = r0 + (int64_t) tile * tile_stride;
             chunk = 0;
             ++tile;
@@ -465,6 +476,26 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
                 }
             }
         }
+        if constexpr (KS > 1) {
+            __shared__ float4 part[kWarps][32];
+            if (n_units > 0) part[warp][lane] = make_float4(tot[0], tot[1], tot[2], tot[3]);
+            __syncthreads();
+            if (n_units > 0 && warp % KS == 0 && t < ntok) {
+                float4 v = part[warp][lane];
+#pragma unroll
+                for (int k = 1; k < KS; ++k) {
+                    const float4 o = part[warp + k][lane];
+                    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+                }
+                const float v0 = (v.x + v.y * kTerm2) * f, v1 = (v.z + v.w * kTerm2) * f;
+                if (MODE == QMODE_GU) {
+                    a.h[orow + r0 + g] = swiglu(v0, v1, a.L);
+                } else {
+                    store_out(a.out, a.out_kind, orow + r0 + g, v0);
+                    store_out(a.out, a.out_kind, orow + r0 + g + 8, v1);
+                }
+            }
+        }
         cpa_wait<0>();
     }
     cpa_wait<0>();
@@ -473,37 +504,65 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
 size_t al256q(size_t v) { return (v + 255) & ~(size_t) 255; }
 
 template <int TYPE>
-size_t kq_smem(int64_t K) {
+size_t kq_smem(int64_t K, int copies = 2, int stages = 3) {
     using Q = QT<TYPE>;
-    return (size_t) kColsQ * (K + Q::kPad) + (Q::kCorr ? (size_t) kColsQ * ((K >> 8) * 64 + 16) + 32768 : 0) +
-           (size_t) Q::kWarps * Q::kStages * kRowsQ * kChunkBlocks * Q::kBlock + 128;
+    return (size_t) kColsQ * (K + Q::kPad) + (Q::kCorr ? (size_t) kColsQ * ((K >> 8) * 64 + 16) + (size_t) 16384 * copies : 0) +
+           (size_t) Q::kWarps * stages * kRowsQ * Q::kRowStage + 128;
+}
+
+template <int TYPE, int MODE, int KS, int NC, int ST>
+int32_t kq_launch_split(const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const int2* items, int* n_items, int tpw, cudaStream_t st) {
+    using Q = QT<TYPE>;
+    const size_t smem = kq_smem<TYPE>(MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff, NC, ST);
+    static std::atomic<bool> configured[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
+    if (!configured[dev].load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(kq_mma_kernel<TYPE, MODE, KS, NC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, KS > 1 ? 220 * 1024 : 225 * 1024);
+        if (e != cudaSuccess) return (int32_t) e;
+        configured[dev].store(true, std::memory_order_release);
+    }
+    const int64_t rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd, tile_rows = (MODE == QMODE_GU ? 8 : 16) * Q::kWarps / KS;
+    const int64_t n_tiles = (rows + tile_rows - 1) / tile_rows;
+    const int n_row_blocks = (int) ((n_tiles + tpw - 1) / tpw);
+    const int per_sm = TYPE == kTypeQ6K && ST == 3 ? 2 : 1;
+    launch_k(kq_mma_kernel<TYPE, MODE, KS, NC, ST>, dim3((unsigned) (per_sm * sm_count())), dim3(Q::kWarps * 32), smem, st, a, img, corr, inv, items, n_items, tpw,
+             n_row_blocks);
+    return launch_status();
 }
 
 template <int TYPE, int MODE>
 int32_t kq_launch(const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const int2* items, int* n_items, cudaStream_t st) {
     using Q = QT<TYPE>;
     const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
-    const size_t smem = kq_smem<TYPE>(K);
-    static std::atomic<bool> configured[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
-    if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(kq_mma_kernel<TYPE, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-        if (e != cudaSuccess) return (int32_t) e;
-        configured[dev].store(true, std::memory_order_release);
-    }
     const int64_t rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd;
     const int64_t row_bytes = K / 256 * Q::kBlock;
     const int64_t tile_bytes = (int64_t) Q::kWarps * kRowsQ * row_bytes;                 // one row tile of every warp
     const int64_t tile_rows = (MODE == QMODE_GU ? 8 : 16) * Q::kWarps;
     const int64_t n_tiles = (rows + tile_rows - 1) / tile_rows;
-    int64_t tpw0 = (384 * 1024 + tile_bytes - 1) / tile_bytes;                           // a unit streams ~400 KB
-    tpw0 = tpw0 < 1 ? 1 : tpw0 > 8 ? 8 : tpw0;
-    const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
-    const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
-    const int n_row_blocks = (int) ((n_tiles + tpw - 1) / tpw);
-    launch_k(kq_mma_kernel<TYPE, MODE>, dim3((unsigned) sm_count()), dim3(Q::kWarps * 32), smem, st, a, img, corr, inv, items, n_items, tpw, n_row_blocks);
-    return launch_status();
+    if constexpr (TYPE == kTypeQ6K) {
+        // One row tile a warp, so that few passes still reach every SM; and where even these units cannot (at most a pass per group and
+        // one per four entries), the columns are split too.  cap_groups and cap_entries bound the passes on the host.
+        const int64_t passes = a.cap_groups + a.cap_entries / kEntQ, units = passes * n_tiles, chunks = K / 256;
+        const bool two = kq_smem<TYPE>(K, 0, 3) <= 108 * 1024;                           // two blocks an SM, else one with longer rings
+        if (units < sm_count() && two) {
+            if (chunks % 8 == 0) return kq_launch_split<TYPE, MODE, 8, 1, 3>(a, img, corr, inv, items, n_items, 1, st);
+            if (chunks % 4 == 0) return kq_launch_split<TYPE, MODE, 4, 1, 3>(a, img, corr, inv, items, n_items, 1, st);
+            return kq_launch_split<TYPE, MODE, 2, 1, 3>(a, img, corr, inv, items, n_items, 1, st);      // whole 512-column rows
+        }
+        if (two) return kq_launch_split<TYPE, MODE, 1, 1, 3>(a, img, corr, inv, items, n_items, 1, st);
+        if (units < sm_count() && chunks % 4 == 0 && kq_smem<TYPE>(K, 0, 5) <= 220 * 1024) return kq_launch_split<TYPE, MODE, 4, 1, 5>(a, img, corr, inv, items, n_items, 1, st);
+        if (kq_smem<TYPE>(K, 0, 5) <= 225 * 1024) return kq_launch_split<TYPE, MODE, 1, 1, 5>(a, img, corr, inv, items, n_items, 1, st);
+        return kq_launch_split<TYPE, MODE, 1, 1, 4>(a, img, corr, inv, items, n_items, 1, st);
+    } else {
+        int64_t tpw0 = (384 * 1024 + tile_bytes - 1) / tile_bytes;                       // a unit streams ~400 KB
+        tpw0 = tpw0 < 1 ? 1 : tpw0 > 8 ? 8 : tpw0;
+        const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
+        const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
+        // four copies of the codebook where they fit beside the columns and the stages (K up to 7680), else two
+        if (kq_smem<TYPE>(K, 4) <= 225 * 1024) return kq_launch_split<TYPE, MODE, 1, 4, 3>(a, img, corr, inv, items, n_items, tpw, st);
+        return kq_launch_split<TYPE, MODE, 1, 2, 3>(a, img, corr, inv, items, n_items, tpw, st);
+    }
 }
 
 bool kq_type(int t) { return t == kTypeIQ1M || t == kTypeQ6K; }
@@ -527,8 +586,8 @@ int32_t experts_grouped_kq(const ExpertArgs& a, cudaStream_t st) {
     const bsx_expert_layout& L = a.L;
     if (!kq_type(L.gu_type) || L.up_type != L.gu_type || !kq_type(L.d_type)) return BSX_E_TYPE;
     if (!kq_dim_ok(L.gu_type, L.n_embd, L.n_ff) || !kq_dim_ok(L.d_type, L.n_ff, L.n_embd) || L.n_embd % 16) return BSX_E_TYPE;
-    if ((L.gu_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_embd) : kq_smem<kTypeQ6K>(L.n_embd)) > 225 * 1024) return BSX_E_TYPE;
-    if ((L.d_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_ff) : kq_smem<kTypeQ6K>(L.n_ff)) > 225 * 1024) return BSX_E_TYPE;
+    if ((L.gu_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_embd) : kq_smem<kTypeQ6K>(L.n_embd, 0, 4)) > 225 * 1024) return BSX_E_TYPE;
+    if ((L.d_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_ff) : kq_smem<kTypeQ6K>(L.n_ff, 0, 4)) > 225 * 1024) return BSX_E_TYPE;
     const int64_t cap = a.cap_entries, H = L.n_embd, I = L.n_ff;
     uint8_t* p = reinterpret_cast<uint8_t*>(a.h) + al256q((size_t) cap * I * 4);
     int8_t* ximg = reinterpret_cast<int8_t*>(p);

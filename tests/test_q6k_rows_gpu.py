@@ -1,0 +1,30 @@
+"""Q6_K experts on the integer tensor-core stream where its launch changes: a few entries (the columns of a row split over two, four or
+eight warps), many groups (whole rows), odd and even numbers of 256-column blocks a part, rows that do not fill the last block of
+warps.  Bound 4e-4: four times the error of two int8 terms a row (1e-4)."""
+import numpy as np
+import pytest
+
+from basalt_b200 import moe
+from oracle import oracle as O
+from tests.helpers import make_expert_blobs, rel_l2, stack_blobs
+from tests.test_experts_gpu import dev, run_grouped
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,I", [(512, 512), (2048, 512), (1536, 1024), (3072, 512), (512, 2560)])
+@pytest.mark.parametrize("groups", [[[3]], [[4], list(range(13)), [0, 7]], [[i % 13] for i in range(60)]], ids=["one", "three", "sixty"])
+def test_q6k_rows(lib, cuda, H, I, groups):
+    rng = np.random.default_rng(H + I)
+    Lo, blobs = make_expert_blobs(rng, 3, O.T_Q6_K, O.T_Q6_K, H, I)
+    L = moe.native_expert_layout(O.T_Q6_K, O.T_Q6_K, H, I)
+    xd = dev(rng.standard_normal((13, H)).astype(np.float32))
+    x = xd.cpu().numpy()
+    ids = [i % 3 for i in range(len(groups))]
+    n = sum(len(g) for g in groups)
+    out = run_grouped(L, dev(stack_blobs(blobs)), ids, groups, xd, n).cpu().numpy()
+    at = 0
+    for e, toks in zip(ids, groups):
+        want = O.expert_forward(Lo, blobs[e], x[toks], dtype=np.float64)
+        assert rel_l2(out[at:at + len(toks)], want) < 4e-4, (e, rel_l2(out[at:at + len(toks)], want))
+        at += len(toks)
