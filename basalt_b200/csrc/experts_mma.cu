@@ -15,7 +15,7 @@
 //
 // IQ3_S rows take the same stream with another decoder (iq3s_16): codebook points as four fp16 magnitudes in shared memory, signs
 // and the odd scales applied in packed fp16, exactly.  Bound by the decode's integer work and look-ups.  5 tokens through 512
-// experts of 2048 x 512, top-10: the layer's step takes 155 us, with the warp-per-row fp32 kernels it took 315.
+// experts of 2048 x 512, top-10: the layer's step took 315 us with the warp-per-row fp32 kernels and 155 with this one.
 //
 // Semantics: Basalt's native_expert_grouped (include/basalt/kernels/iq_kernels.hpp:77-92; kernels src/kernels/cuda/iq_kernels.cu:
 // 1605-1658 gate/up, :2512-2524 SwiGLU, :2140-2164 down), NVFP4 decoding per src/kernels/cpu/ggml/ggml_quants.c:1397-1422,
@@ -417,8 +417,10 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
             }
             float sg = 1.f, su = 1.f, sd = 1.f;
             if constexpr (FMT == FMT_NVFP4) { sg = tail[0]; su = tail[1]; sd = tail[2]; }
-            // two accumulator sets, so that consecutive MMAs do not wait on each other
-            float acc[4] = {0.f, 0.f, 0.f, 0.f}, acd[4] = {0.f, 0.f, 0.f, 0.f};
+            // The tensor core truncates where it adds to an accumulator, so every MMA starts from zero and its sum goes to fp32
+            // arithmetic (rounded to nearest): chained over a row the result was 2 to 3 times as far from 64-bit sums as the
+            // warp-per-row fp32 kernel's
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
             // this lane's B fragments: its column's pieces, or (column unused in this pass) the zero area with stride 0
             const bool col_live = g < ncol;
             const uint4* bcol = col_live ? reinterpret_cast<const uint4*>(xs) + g * 4 + t : zero;
@@ -438,25 +440,27 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                     for (int b = 0; b < 2; ++b) {
                         const uint8_t* ba = reinterpret_cast<const uint8_t*>(ra) + 110 * b;
                         const uint8_t* bb = reinterpret_cast<const uint8_t*>(rb) + 110 * b;
-                        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+                        float part[4] = {0.f, 0.f, 0.f, 0.f};
+                        const float da = __half2float(*reinterpret_cast<const __half*>(ba)), db = __half2float(*reinterpret_cast<const __half*>(bb));
 #pragma unroll
                         for (int gr = 0; gr < 4; ++gr) {
                             const uint4 b0 = bp[(4 * b + gr) * bstep], b1 = bp[(4 * b + gr) * bstep + bhalf];
                             uint32_t qa[8], qb[8];
                             iq3s_16(ba, gr, t, reinterpret_cast<const uint2*>(lut), qa);
                             iq3s_16(bb, gr, t, reinterpret_cast<const uint2*>(lut), qb);
+                            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f}, s3[4] = {0.f, 0.f, 0.f, 0.f};
                             mma_f16(s0, qa[0], qb[0], qa[1], qb[1], b0.x, b0.y);
                             mma_f16(s1, qa[2], qb[2], qa[3], qb[3], b0.z, b0.w);
-                            mma_f16(s0, qa[4], qb[4], qa[5], qb[5], b1.x, b1.y);
-                            mma_f16(s1, qa[6], qb[6], qa[7], qb[7], b1.z, b1.w);
+                            mma_f16(s2, qa[4], qb[4], qa[5], qb[5], b1.x, b1.y);
+                            mma_f16(s3, qa[6], qb[6], qa[7], qb[7], b1.z, b1.w);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) part[i] += (s0[i] + s1[i]) + (s2[i] + s3[i]);
                         }
-                        const float da = __half2float(*reinterpret_cast<const __half*>(ba)), db = __half2float(*reinterpret_cast<const __half*>(bb));
-                        acc[0] = fmaf(s0[0] + s1[0], da, acc[0]);
-                        acc[1] = fmaf(s0[1] + s1[1], da, acc[1]);
-                        acc[2] = fmaf(s0[2] + s1[2], db, acc[2]);
-                        acc[3] = fmaf(s0[3] + s1[3], db, acc[3]);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[i] = fmaf(part[i], i < 2 ? da : db, acc[i]);
                     }
                 } else {
+                float part[4] = {0.f, 0.f, 0.f, 0.f};      // a chunk's sum, so that the row's is a short chain
 #pragma unroll
                 for (int blk = 0; blk < 4; ++blk) {
                     if (PIECE != 16 && 4 * chunk + blk >= n_gran) break;   // past the row's last block
@@ -475,11 +479,16 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                         qb0[i] = hmul2_bits(qb0[i], sb);
                         qb1[i] = hmul2_bits(qb1[i], sb);
                     }
-                    mma_f16(acc, qa0[0], qb0[0], qa0[1], qb0[1], b0.x, b0.y);
-                    mma_f16(acd, qa0[2], qb0[2], qa0[3], qb0[3], b0.z, b0.w);
-                    mma_f16(acc, qa1[0], qb1[0], qa1[1], qb1[1], b1.x, b1.y);
-                    mma_f16(acd, qa1[2], qb1[2], qa1[3], qb1[3], b1.z, b1.w);
+                    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f}, s3[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma_f16(s0, qa0[0], qb0[0], qa0[1], qb0[1], b0.x, b0.y);
+                    mma_f16(s1, qa0[2], qb0[2], qa0[3], qb0[3], b0.z, b0.w);
+                    mma_f16(s2, qa1[0], qb1[0], qa1[1], qb1[1], b1.x, b1.y);
+                    mma_f16(s3, qa1[2], qb1[2], qa1[3], qb1[3], b1.z, b1.w);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) part[i] += (s0[i] + s1[i]) + (s2[i] + s3[i]);
                 }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] += part[i];
                 }
                 __syncwarp();   // every lane is done with this stage before a later issue overwrites it
                 if (++chunk != n_chunks) continue;
@@ -487,9 +496,8 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                 const int64_t rt = r0 + (int64_t) tile * tile_stride;
                 chunk = 0;
                 ++tile;
-                const float c0 = acc[0] + acd[0], c1 = acc[1] + acd[1], c2 = acc[2] + acd[2], c3 = acc[3] + acd[3];
+                const float c0 = acc[0], c1 = acc[1], c2 = acc[2], c3 = acc[3];
                 acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-                acd[0] = acd[1] = acd[2] = acd[3] = 0.f;
                 if (MODE == MODE_GU) {
                     if (TERMS == 1) {
                         if (2 * t < ntok) a.h[o0 + rt + g] = swiglu(c0 * f0 * sg, c2 * f0 * su, a.L);
