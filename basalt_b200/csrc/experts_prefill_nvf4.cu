@@ -148,6 +148,41 @@ __device__ __forceinline__ void store8_q(float* p, const float (&v)[8], bool wid
     }
 }
 
+// 32 consecutive floats of each lane's row to memory.  A lane owns a row, so storing straight from the registers would touch 32
+// lines an instruction; a 4 x 4 transposition among neighbouring lanes makes four lanes hold one row's 128 bytes, eight lines an
+// instruction (the resident down product of 180,224 rows x 2048: 495 -> 458 us).  base: column 0 of the row of lane 0 of the
+// warp; rows beyond `live` are not stored.  wide: 32-byte aligned rows.
+__device__ __forceinline__ void store_rows32_q(float* base, size_t pitch, int live, int lane, float (&v)[32], bool wide) {
+#pragma unroll
+    for (int s = 1; s <= 2; s <<= 1)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (u & s) continue;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                float& lo = v[8 * u + e];
+                float& hi = v[8 * (u | s) + e];
+                const float r = __shfl_xor_sync(kFull, (lane & s) ? lo : hi, s);
+                if (lane & s) lo = r;
+                else hi = r;
+            }
+        }
+    const int row = lane & ~3;
+    float* p = base + (size_t) row * pitch + (lane & 3) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i, p += pitch) {
+        if (row + i >= live) break;
+        if (wide) {
+            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(p), "f"(v[8 * i]), "f"(v[8 * i + 1]), "f"(v[8 * i + 2]),
+                         "f"(v[8 * i + 3]), "f"(v[8 * i + 4]), "f"(v[8 * i + 5]), "f"(v[8 * i + 6]), "f"(v[8 * i + 7])
+                         : "memory");
+        } else {
+            reinterpret_cast<float4*>(p)[0] = make_float4(v[8 * i], v[8 * i + 1], v[8 * i + 2], v[8 * i + 3]);
+            reinterpret_cast<float4*>(p)[1] = make_float4(v[8 * i + 4], v[8 * i + 5], v[8 * i + 6], v[8 * i + 7]);
+        }
+    }
+}
+
 // rows of x (fp32 or bf16) -> FP4 terms, one image row per token: codes [token][term][H / 2], scales [token][term][H / 16]
 template <int TPR>
 __global__ void __launch_bounds__(256) prefill_images_kernel(const void* __restrict__ src, int kind, int64_t n, int64_t K, uint8_t* __restrict__ codes,
@@ -159,7 +194,7 @@ __global__ void __launch_bounds__(256) prefill_images_kernel(const void* __restr
 
 // token images -> tile images of the gate/up product.  Block = one (tile, chunk): every row's four 128-byte code runs move in
 // 16-byte pieces (eight lanes a run), the scale words are transposed through shared memory.  Bound: HBM writes of 2.25 bytes a
-// value (180,224 rows x 2048: 830 MB); reads come from L2.
+// value (180,224 rows x 2048: 830 MB); the stores are streaming, so that the token images they are read from stay in L2 (247 -> 215 us).
 __global__ void __launch_bounds__(256) tile_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ n_tiles, int tile0,
                                                           const int32_t* __restrict__ src, const uint8_t* __restrict__ codes, const uint8_t* __restrict__ sfs, int64_t K,
                                                           uint8_t* __restrict__ img) {
@@ -192,18 +227,21 @@ __global__ void __launch_bounds__(256) tile_images_kernel(const TileRec* __restr
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int row = row0 + 8 * j;
-            if (row < r.rows) *reinterpret_cast<uint4*>(out + t * term_bytes + kSFQ + (row >> 3) * 1024 + (row & 7) * 128 + ((p ^ (row & 7)) << 4)) = v[j];
+            if (row < r.rows) __stcs(reinterpret_cast<uint4*>(out + t * term_bytes + kSFQ + (row >> 3) * 1024 + (row & 7) * 128 + ((p ^ (row & 7)) << 4)), v[j]);
         }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kTermsF * kSFQ / 16; i += 256) {
         const int t = i / (kSFQ / 16), q = i - t * (kSFQ / 16);
-        reinterpret_cast<uint4*>(out + t * term_bytes)[q] = reinterpret_cast<const uint4*>(sf)[i];
+        __stcs(reinterpret_cast<uint4*>(out + t * term_bytes) + q, reinterpret_cast<const uint4*>(sf)[i]);
     }
 }
 
 // rows of h (fp32, dispatch order) -> tile images of the down product.  Block = eight rows of a tile, a warp a row: a lane makes
-// one sub-block of 16 values at a time, and four lanes' scale bytes make the word tcgen05.cp reads.
+// one sub-block of 16 values at a time, and four lanes' scale bytes make the word tcgen05.cp reads.  NIT = 1: a lane's one sub-block
+// stays in registers between the row's maximum and its codes (n_ff <= 512: 205 -> 174 us for 180,224 rows of 512); 0 reads the row
+// twice (four sub-blocks in registers were slower there: 274 -> 340 us for 73,728 rows of 2048).
+template <int NIT>
 __global__ void __launch_bounds__(256) h_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ n_tiles, const float* __restrict__ h, int64_t K,
                                                        uint8_t* __restrict__ img, float* __restrict__ inv) {
     const int tile = blockIdx.x >> 4, row = (blockIdx.x & 15) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -213,23 +251,37 @@ __global__ void __launch_bounds__(256) h_images_kernel(const TileRec* __restrict
     const int64_t i = r.row0 + row;
     const int n_sb = (int) (K >> 4), n_chunk = (int) (K >> 8);
     float amax = 0.f;
-    for (int sb = lane; sb < n_sb; sb += 32) {
-        float v[16];
-        load16(h, BSX_X_F32, i, K, sb, v);
+    float keep[NIT > 0 ? NIT : 1][16];
+    auto load = [&](int sb, float (&v)[16]) {
+        if (sb < n_sb) {
+            load16(h, BSX_X_F32, i, K, sb, v);
+        } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[j]));
+            for (int j = 0; j < 16; ++j) v[j] = 0.f;
+        }
+    };
+    if constexpr (NIT > 0) {
+#pragma unroll
+        for (int q = 0; q < NIT; ++q) load(32 * q + lane, keep[q]);
+#pragma unroll
+        for (int q = 0; q < NIT; ++q)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(keep[q][j]));
+    } else {
+        for (int sb = lane; sb < n_sb; sb += 32) {
+            load(sb, keep[0]);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(keep[0][j]));
+        }
     }
     amax = warp_max_xor(amax);
     const Pow2Scale ps = fp4_row_scale(amax);
     if (lane == 0) inv[i] = ps.inv;
     const size_t term_bytes = (size_t) tile_units(r.rows) * 1024;
-    for (int sb0 = 0; sb0 < n_sb; sb0 += 32) {       // n_sb is a multiple of 16: whole chunks, four lanes of a word together
-        const int sb = sb0 + lane;
+    auto write = [&](int sb, float (&v)[16]) {           // n_sb is a multiple of 16: whole chunks, four lanes of a word together
         const bool live = sb < n_sb;
-        float v[16];
-        if (live) load16(h, BSX_X_F32, i, K, sb, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = live ? v[j] * ps.s : 0.f;
+        for (int j = 0; j < 16; ++j) v[j] *= ps.s;
         uint8_t* out = img + image_block(r, n_chunk, sb >> 4, 0);
         const int q = sb & 15;
 #pragma unroll
@@ -242,6 +294,15 @@ __global__ void __launch_bounds__(256) h_images_kernel(const TileRec* __restrict
             uint8_t* o = out + t * term_bytes;
             *reinterpret_cast<uint2*>(o + kSFQ + (row >> 3) * 1024 + (row & 7) * 128 + (((q >> 1) ^ (row & 7)) << 4) + (q & 1) * 8) = make_uint2(w0, w1);
             if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(o + (q >> 2) * 512 + (row & 31) * 16 + (row >> 5) * 4) = sc;
+        }
+    };
+    if constexpr (NIT > 0) {
+#pragma unroll
+        for (int q = 0; q < NIT; ++q) write(32 * q + lane, keep[q]);
+    } else {
+        for (int sb = lane; sb - lane < n_sb; sb += 32) {
+            load(sb, keep[0]);
+            write(sb, keep[0]);
         }
     }
 }
@@ -599,7 +660,8 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
             const bool row_live = p < r.rows;
             const float* tail = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(r.blob) + geo.tail);
             const float sd = row_live ? tail[2] * a.inv[r.row0 + p] : 0.f;
-            float* orow = a.dm + (size_t) (r.row0 + p) * a.L.n_embd + half * 64;
+            const int w0 = (warp & 3) * 32;
+            float* orow = a.dm + (size_t) (r.row0 + w0) * a.L.n_embd + half * 64;
             for (int nb = 0; nb < n_nb; ++nb, ++nbc) {
                 const uint32_t s = nbc & 1u;
                 ok = __all_sync(kFull, mbar_wait(&acc_full[s], (nbc >> 1) & 1u));
@@ -610,16 +672,14 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
                 tmem_ld32(tbase + s * 128 + 32, v[1]);
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 mbar_arrive(&acc_empty[s]);
-                if (!row_live) continue;
+                if (w0 >= r.rows) continue;
 #pragma unroll
-                for (int i = 0; i < 2; ++i)
+                for (int i = 0; i < 2; ++i) {
+                    float o[32];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        float o[8];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(v[i][8 * j + e]) * sd;
-                        store8_q(orow + nb * 128 + 32 * i + 8 * j, o, wide);
-                    }
+                    for (int e = 0; e < 32; ++e) o[e] = __uint_as_float(v[i][e]) * sd;
+                    store_rows32_q(orow + nb * 128 + 32 * i, (size_t) a.L.n_embd, r.rows - w0, lane, o, wide);
+                }
             }
             if (!ok) break;
         }
@@ -718,12 +778,15 @@ extern "C" int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, c
     if (H <= 2048) prefill_images_kernel<128><<<(unsigned) ((n_tokens + 1) / 2), 256, 0, st>>>(x, x_kind, n_tokens, (int64_t) H, xcodes, xsf, xinv);
     else prefill_images_kernel<256><<<(unsigned) n_tokens, 256, 0, st>>>(x, x_kind, n_tokens, (int64_t) H, xcodes, xsf, xinv);
     for (int64_t t0 = 0; t0 < cap_tiles; t0 += 65535)
-        tile_images_kernel<<<dim3((unsigned) (H / 256), (unsigned) (cap_tiles - t0 < 65535 ? cap_tiles - t0 : 65535)), 256, 0, st>>>(recs, n_tiles, (int) t0, src, xcodes, xsf, (int64_t) H, ximg);
+        tile_images_kernel<<<dim3((unsigned) (H / 256), (unsigned) (cap_tiles - t0 < 65535 ? cap_tiles - t0 : 65535)), 256, 0, st>>>(recs, n_tiles, (int) t0, src, xcodes,
+                                                                                                                                     xsf, (int64_t) H, ximg);
     a.img = ximg;
     a.inv = xinv;
     int32_t rc = launch_q<QMODE_GU>(a, st);
     if (rc != BSX_OK) return rc;
-    h_images_kernel<<<(unsigned) (cap_tiles * 16), 256, 0, st>>>(recs, n_tiles, h, (int64_t) I, himg, hinv);
+    const unsigned hb = (unsigned) (cap_tiles * 16);
+    if (I <= 512) h_images_kernel<1><<<hb, 256, 0, st>>>(recs, n_tiles, h, (int64_t) I, himg, hinv);
+    else h_images_kernel<0><<<hb, 256, 0, st>>>(recs, n_tiles, h, (int64_t) I, himg, hinv);
     a.img = himg;
     a.inv = hinv;
     // n_ff <= 512: the tile's rows stay in shared memory and only weights stream
