@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) nvf4_stream_kernel(StreamArgs sa
                 const int e = u.eb + (j < u.ntok ? j : 0);
                 const int ir = (MODE == FMODE_GU && a.n_x_rows > 0) ? a.ent_tok[e] : e;
                 f[j] = sa.inv[ir];
-                orow[j] = MODE == FMODE_GU ? (int64_t) e * a.L.n_ff : (int64_t) a.ent_dst[e] * a.L.n_embd;
+                orow[j] = MODE == FMODE_GU ? (int64_t) e * a.L.n_ff : (int64_t) (a.ent_dst ? a.ent_dst[e] : e) * a.L.n_embd;
             }
             for (int rb = rb0; rb < rb1; ++rb) {
                 const int r0 = rb * kRowsPerBlock;
@@ -628,6 +628,35 @@ int32_t experts_grouped_packed(const ExpertArgs& a, int32_t* status, cudaStream_
     sa.inv = hinv;
     sa.early_weights = 1;
     return wide ? launch_stream<FMODE_DOWN, kEntWide>(sa, st) : launch_stream<FMODE_DOWN, kEntNarrow>(sa, st);
+}
+
+// The same two products over a pass list that is there already, entry e = row e: x rows ent_tok[e], output row e.  xcodes .. xinv and
+// hcodes .. hinv: room for the images of n_x_rows rows of n_embd and of a.cap_entries rows of n_ff.
+int32_t experts_packed_passes(const ExpertArgs& a, const PassRec* items, const int* n_items, int pass_entries, uint8_t* xcodes, uint8_t* xsf, float* xinv,
+                              uint8_t* hcodes, uint8_t* hsf, float* hinv, int32_t* status, cudaStream_t st) {
+    auto images = [&](const void* src, int kind, int64_t rows, int64_t K, uint8_t* codes, uint8_t* sfs, float* inv) {
+        const int64_t n_sb = K / 16;
+        if (n_sb <= 32) launch_k(x_images_kernel<32>, dim3((unsigned) ((rows + 7) / 8)), dim3(256), 0, st, src, kind, (int) rows, K, codes, sfs, inv);
+        else if (n_sb <= 128) launch_k(x_images_kernel<128>, dim3((unsigned) ((rows + 1) / 2)), dim3(256), 0, st, src, kind, (int) rows, K, codes, sfs, inv);
+        else launch_k(x_images_kernel<256>, dim3((unsigned) rows), dim3(256), 0, st, src, kind, (int) rows, K, codes, sfs, inv);
+    };
+    StreamArgs sa;
+    sa.e = a;
+    sa.items = items;
+    sa.n_items = n_items;
+    sa.status = status;
+    sa.early_weights = 0;
+    images(a.x, a.x_kind, a.n_x_rows, a.L.n_embd, xcodes, xsf, xinv);
+    sa.codes = xcodes;
+    sa.sfs = xsf;
+    sa.inv = xinv;
+    const int32_t rc = pass_entries == kEntWide ? launch_stream<FMODE_GU, kEntWide>(sa, st) : launch_stream<FMODE_GU, kEntNarrow>(sa, st);
+    if (rc != BSX_OK) return rc;
+    images(a.h, BSX_X_F32, a.cap_entries, a.L.n_ff, hcodes, hsf, hinv);
+    sa.codes = hcodes;
+    sa.sfs = hsf;
+    sa.inv = hinv;
+    return pass_entries == kEntWide ? launch_stream<FMODE_DOWN, kEntWide>(sa, st) : launch_stream<FMODE_DOWN, kEntNarrow>(sa, st);
 }
 
 }  // namespace bsx

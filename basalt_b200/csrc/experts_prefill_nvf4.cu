@@ -31,6 +31,10 @@
 #include "tc5.cuh"
 
 namespace bsx {
+
+int32_t experts_packed_passes(const ExpertArgs& a, const PassRec* items, const int* n_items, int pass_entries, uint8_t* xcodes, uint8_t* xsf, float* xinv,
+                              uint8_t* hcodes, uint8_t* hsf, float* hinv, int32_t* status, cudaStream_t st);
+
 namespace {
 
 constexpr int kThreadsQ = 32 * 12;
@@ -71,13 +75,16 @@ __device__ __forceinline__ size_t image_block(const TileRec& r, int n_chunk, int
 // units that cap_rows rows in cap_tiles tiles can take
 __host__ __device__ inline int64_t image_units(int64_t cap_rows, int64_t cap_tiles) { return cap_rows / 8 + 3 * cap_tiles; }
 
-// one block: the units are a running sum over the tiles
+// One block: the units are a running sum over the tiles.  items (optional): the tiles' rows as passes of up to pass_entries rows, for
+// the decode stream.
 __global__ void __launch_bounds__(1024) tile_records_kernel(const int32_t* __restrict__ tiles, const int32_t* __restrict__ n_tiles,
                                                             const int32_t* __restrict__ off, const unsigned long long* __restrict__ blob_table,
-                                                            TileRec* __restrict__ recs, int64_t cap_tiles, int64_t cap_units, int32_t* status) {
+                                                            TileRec* __restrict__ recs, int64_t cap_tiles, int64_t cap_units, int32_t* status,
+                                                            PassRec* __restrict__ items, int* __restrict__ n_items, int pass_entries) {
     __shared__ unsigned long long sh[32];
     const int64_t n = min(cap_tiles, (int64_t) *n_tiles);
     int64_t at = 0;
+    int passes = 0;
     for (int64_t t0 = 0; t0 < n; t0 += 1024) {
         const int64_t t = t0 + threadIdx.x;
         TileRec r = {0ull, 0, 0, 0, 0};
@@ -88,9 +95,19 @@ __global__ void __launch_bounds__(1024) tile_records_kernel(const int32_t* __res
             r.rows = min(128, off[expert + 1] - row0);
         }
         const int u = r.rows > 0 ? tile_units(r.rows) : 0;
+        const int np = items && r.rows > 0 && r.blob != 0ull ? (r.rows + pass_entries - 1) / pass_entries : 0;
         unsigned long long total = 0;
-        r.base = at + (int64_t) block_excl_sum<unsigned long long>((unsigned long long) u, &total, sh);
-        at += (int64_t) total;
+        const unsigned long long before = block_excl_sum<unsigned long long>((unsigned long long) u | ((unsigned long long) np << 32), &total, sh);
+        r.base = at + (int64_t) (before & 0xFFFFFFFFull);
+        for (int p = 0; p < np; ++p) {
+            PassRec q;
+            q.blob = r.blob;
+            q.eb = r.row0 + p * pass_entries;
+            q.ntok = min(pass_entries, r.rows - p * pass_entries);
+            items[passes + (int) (before >> 32) + p] = q;
+        }
+        at += (int64_t) (total & 0xFFFFFFFFull);
+        passes += (int) (total >> 32);
         if (t < n) {
             if (r.rows <= 0 || r.base + u > cap_units) {      // no rows; or tiles that overlap, which no dispatch makes
                 if (r.rows > 0) atomicOr(status, 1);
@@ -100,6 +117,7 @@ __global__ void __launch_bounds__(1024) tile_records_kernel(const int32_t* __res
             recs[t] = r;
         }
     }
+    if (items && threadIdx.x == 0) *n_items = passes;
 }
 
 struct PrefillFArgs {
@@ -723,6 +741,11 @@ int32_t launch_q(const PrefillFArgs& a, cudaStream_t st) {
 
 using namespace bsx;
 
+// Rows an expert, on average over the call, up to which the decode stream takes it.  Whole layer, stream against tiles: 2048 x 512 with
+// 512 + 1 experts at 1.4 rows an expert 207 : 310 us, 16.7 338 : 498, 32 443 : 547, 47 567 : 604; 5120 x 2304 with 384 + 1 at 14
+// rows 1500 : 2411, 27 2103 : 2780; 7168 x 2048 with 256 + 1 at 17.5 rows 1473 : 2203, 35 2112 : 2437.
+constexpr int64_t kShortRows = 48;
+
 // the tiles that rows of up to 1024 experts can make
 static int64_t prefill_cap_tiles(int64_t cap_rows) { return cap_rows < 1025 ? cap_rows : cap_rows / 128 + 1025; }
 
@@ -766,7 +789,32 @@ extern "C" int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, c
     p += al256q(R * 4);
     TileRec* recs = reinterpret_cast<TileRec*>(p);
     if (cap_tiles > cap_rows / 128 + 1025) return BSX_E_LIMIT;      // more tiles than rows / 128 + experts can make
-    tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, recs, cap_tiles, units, status);
+    // Few rows an expert: a tile's 128 tensor-core rows would be mostly padding and cost twice what the weights' bytes do, so the rows
+    // go through the decode stream instead (experts_nvf4.cu: passes of 8 or 16 rows as the MMA's narrow side, bound by the weights).
+    if (cap_rows <= kShortRows * n_expert && n_tokens <= 0x7FFFFFFF) {
+        const int pass_entries = cap_rows > kPassEntries / 2 * n_expert ? 2 * kPassEntries : kPassEntries;
+        int* n_items = reinterpret_cast<int*>(ximg);                 // the images' room holds the pass list: at most a pass a row
+        PassRec* items = reinterpret_cast<PassRec*>(ximg + 256);
+        tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, recs, cap_tiles, units, status, items, n_items, pass_entries);
+        ExpertArgs e;
+        e.L = L;
+        e.grp_ptr = nullptr;
+        e.grp_start = nullptr;
+        e.n_groups = nullptr;
+        e.ent_dst = nullptr;
+        e.ent_tok = src;
+        e.cap_groups = n_expert;
+        e.cap_entries = cap_rows;
+        e.x = x;
+        e.x_kind = x_kind;
+        e.h = h;
+        e.out = dm;
+        e.out_kind = BSX_OUT_F32;
+        e.n_x_rows = (int32_t) n_tokens;
+        e.grid = nullptr;
+        return experts_packed_passes(e, items, n_items, pass_entries, xcodes, xsf, xinv, himg, himg + al256q((size_t) cap_rows * kTermsF * I / 2), hinv, status, st);
+    }
+    tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, recs, cap_tiles, units, status, nullptr, nullptr, 1);
     PrefillFArgs a;
     a.L = L;
     a.recs = recs;

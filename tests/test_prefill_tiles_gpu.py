@@ -1,5 +1,6 @@
 """Packed prompt experts at the row counts where a 128-row tile's image changes its length (whole groups of eight rows, one more,
-one less, one row, two tiles), at one and several chunks of either product, and with an output that is only 16-byte aligned.
+one less, one row, two tiles), at one and several chunks of either product, and with an output that is only 16-byte aligned; and at
+the row counts where the short-prompt route's passes fill.
 Bound 7e-4: four times the four-term FP4 error of a row (1.8e-4)."""
 import ctypes as C
 
@@ -15,10 +16,15 @@ from tests.test_experts_gpu import dev
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("H,I,shift", [(256, 256, 0), (512, 512, 16), (768, 768, 0), (256, 1024, 16), (2048, 512, 0)])
-def test_tile_row_counts(lib, cuda, H, I, shift):
+TILES = [1, 0, 7, 8, 9, 127, 128, 129, 0, 260]                                    # 67 rows an expert: tiles
+SHORT16 = [0, 1, 8, 9, 15, 16, 17, 0, 130, 32, 33, 0, 0, 2, 0, 0]                # 16 an expert: the decode stream, passes of 16
+SHORT8 = [0, 1, 7, 8, 9, 0, 17, 0, 0, 0, 0, 0, 0, 1, 0, 0]                       # 3 an expert: passes of 8
+
+
+@pytest.mark.parametrize("H,I,shift,counts", [(256, 256, 0, TILES), (512, 512, 16, TILES), (768, 768, 0, TILES), (256, 1024, 16, TILES), (2048, 512, 0, TILES),
+                                              (256, 256, 16, SHORT16), (2048, 512, 0, SHORT16), (768, 1280, 0, SHORT16), (512, 512, 0, SHORT8), (768, 768, 16, SHORT8)])
+def test_tile_row_counts(lib, cuda, H, I, shift, counts):
     rng = np.random.default_rng(H * 3 + I)
-    counts = [1, 0, 7, 8, 9, 127, 128, 129, 0, 260]
     E = len(counts)
     Lo, blobs = make_expert_blobs(rng, E, O.T_NVFP4, O.T_NVFP4, H, I)
     L = moe.native_expert_layout(O.T_NVFP4, O.T_NVFP4, H, I)
