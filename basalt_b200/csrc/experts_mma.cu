@@ -610,7 +610,7 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     if (fmt == FMT_IQ3S) return launch<FMT_IQ3S, MODE_DOWN, 2, 4>(a, himg, hinv, items, n_items, st);
     // Down rows of n_ff columns: the copies' width is what their start is aligned to.  An n_ff that is not whole 256-column chunks
     // went to the warp-per-row kernels before (2 % of the copy bandwidth: fp32 decode and FMA for every weight and entry); here
-    // the same 27-token step (2560 x 640, 512 + 1 experts, top-10) takes 205 us instead of 3648.
+    // the same 27-token step (2560 x 640, 512 + 1 experts, top-10) takes 217 us instead of 3648.
     if (L.n_ff % 256 == 0) return launch<FMT_NVFP4, MODE_DOWN, 2>(a, himg, hinv, items, n_items, st);
     if (L.n_ff % 128 == 0) return launch<FMT_NVFP4, MODE_DOWN, 2, 8>(a, himg, hinv, items, n_items, st);
     return launch<FMT_NVFP4, MODE_DOWN, 2, 4>(a, himg, hinv, items, n_items, st);
