@@ -496,7 +496,7 @@ def decode_line(args, w, T, r, world=1):
     if "stage_ms" in r:
         gu_ms = r["stage_ms"]["experts_gate_up"]
         achieved = r["gu_bytes"] / (gu_ms * 1e-3) / 1e9
-        line["roofline"] = {"bound": "hbm", "kernel": ("nvf4_stream_kernel<gate/up>" if use_packed else "nvfp4_mma_kernel<gate/up>") +
+        line["roofline"] = {"bound": "hbm", "kernel": ("nvf4_stream_kernel<gate/up>" if use_packed else "blk_mma_kernel<gate/up>") +
                             " (routed + shared experts; the stage's CUDA events also span the one-block kernel that lists the passes)", "achieved": achieved, "peak": pk["hbm"],
                             "unit": "GB/s", "frac": achieved / pk["hbm"], "peak_source": pk["source"],
                             # dram__bytes_read.sum + dram__bytes_write.sum of one gate/up launch of this workload at 64 tokens (seeded, so the same
