@@ -19,6 +19,7 @@ namespace {
 constexpr int kChunk = 256;          // pairs per warp chunk
 constexpr int kWarpsPerBlock = 8;
 constexpr int kMaxExpert = 1024;
+constexpr size_t kEpPlanTables = 48 * 1024;      // bsx_ep_plan: 16 bytes an expert and 4 a pair (1024 experts: 8192 pairs)
 
 __host__ __device__ inline int64_t n_chunks_of(int64_t n) { return (n + kChunk - 1) / kChunk; }
 
@@ -383,9 +384,18 @@ extern "C" int32_t bsx_ep_plan(const int32_t* ids, int64_t n_pairs, int32_t k, i
                                int32_t* ent_tok, void* stream) {
     if (!stream) return BSX_E_STREAM;
     if (E < 1 || E > BSX_PLAN_MAX_EXPERTS || k < 1 || n_pairs < 0 || tok_lo < 0 || tok_n < 0 || pairs_per_block < 0) return BSX_E_GEOMETRY;
-    if (n_pairs > BSX_EP_PLAN_MAX_PAIRS || (size_t) E * 16 + (size_t) n_pairs * 4 > kPlanSmemMax) return BSX_E_LIMIT;
+    if (n_pairs > BSX_EP_PLAN_MAX_PAIRS || (size_t) E * 16 + (size_t) n_pairs * 4 > kEpPlanTables) return BSX_E_LIMIT;
     const size_t smem = plan_smem_bytes(E, (int) n_pairs, false);
     if (!ids || !blob_table || !ptr || !start || !n_groups || !ent_dst || !ent_tok) return BSX_E_POINTER;
+    // tables of up to 48 KB and the plan's few static words are more than a launch may have without an opt-in
+    static std::atomic<bool> configured[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
+    if (!configured[dev].load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(ep_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (kEpPlanTables + 16));
+        if (e != cudaSuccess) return (int32_t) e;
+        configured[dev].store(true, std::memory_order_release);
+    }
     launch_k(ep_plan_kernel, dim3(1), dim3(1024), smem, (cudaStream_t) stream, ids, (int) n_pairs, (int) k, (int) pairs_per_block, (int) block_stride, (int) E,
              blob_table, shared_blob, (int) tok_lo, (int) tok_n, ptr, start, n_groups, ent_dst, ent_tok, replicated, (int) (tok_lo * k), (int) (tok_n * k));
     return launch_status();

@@ -59,7 +59,9 @@ struct PlanSmem {
     int32_t* twice;             // a token named one expert twice: the masks do not give places
     int32_t* sid;               // [n]: the pairs' ids (-1: no entry)
 };
-constexpr size_t kPlanSmemMax = 48 * 1024;
+// A launch without an opt-in has 48 KB of shared memory in all, static (the scan's words in plan_finish) and dynamic together.
+constexpr size_t kPlanSmemStatic = 32 * sizeof(unsigned long long);
+constexpr size_t kPlanSmemMax = 48 * 1024 - kPlanSmemStatic;
 constexpr int kPlanMaskTokens = 64;
 __host__ __device__ inline size_t plan_smem_bytes(int E, int n, bool masks) { return (size_t) E * (masks ? 24 : 16) + 8 + (size_t) n * 4; }
 // whether a window of n_tok tokens gets masks
@@ -103,7 +105,7 @@ __device__ inline void plan_finish(const PlanSmem& s, int n, int k, int E, unsig
                                    unsigned long long* __restrict__ ptr, int32_t* __restrict__ start, int32_t* __restrict__ n_groups,
                                    int32_t* __restrict__ dst, int32_t* __restrict__ tok, PassRec* __restrict__ items, int* __restrict__ n_items,
                                    int tok_base = 0) {
-    __shared__ unsigned long long sh[32];
+    __shared__ unsigned long long sh[kPlanSmemStatic / sizeof(unsigned long long)];
     constexpr int kField = 20;                                // entries | groups << 20 | passes << 40: none reaches 2^20 here
     constexpr unsigned long long kLow = (1ull << kField) - 1;
     int at = 0, g = 0, np_total = 0;   // running totals over the expert chunks of blockDim.x
