@@ -153,8 +153,10 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 }
 
 // One warp per activation row: the row -> fp16 image(s) in fragment order plus the inverse of the power of two it was
-// scaled by (so that its largest magnitude lands in [2^13, 2^14), inside fp16 whatever the row's range).  A lane takes one
-// 16-value sub-block at a time, which is exactly two 16-byte pieces of the image (see image_index).
+// scaled by, so that its largest finite magnitude lands in [2^13, 2^14): inside fp16 and with all its bits for every fp32 row
+// (2^149 is the largest scale; it makes a row of nothing but the smallest numbers integers below 2^23, which the two terms hold
+// exactly).  An infinity is the first term alone: it reaches the sums as in fp32 and leaves the row's other values theirs.  A lane
+// takes one 16-value sub-block at a time, which is exactly two 16-byte pieces of the image (see image_index).
 // FROM_H = false: rows of x (kind x_kind, width n_embd) - row i of x when the caller gave the number of x rows, else the
 // row of entry i; true: row e of the SwiGLU output h (fp32, width n_ff).
 // The last block lists the passes of the product that follows: a pass is up to 8 / TERMS consecutive entries of one group,
@@ -212,24 +214,22 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
         float v[16];
         load16(src, kind, row, K, sb, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[j]));
+        for (int j = 0; j < 16; ++j) amax = fmaxf(amax, isfinite(v[j]) ? fabsf(v[j]) : 0.f);
     }
     amax = warp_max_xor(amax);
     int ex = 0;
-    float s = 1.f, iv = 1.f;
-    if (amax > 0.f && amax <= 3.0e38f) {
+    if (amax > 0.f) {
         frexpf(amax, &ex);                          // amax = f 2^ex, f in [0.5, 1)
-        ex = max(-100, min(100, 14 - ex));
-        s = ldexpf(1.f, ex);
-        iv = ldexpf(1.f, -ex);
+        ex = min(149, 14 - ex);
     }
-    if (lane == 0) inv[i] = iv;
+    const float s = ldexpf(1.f, min(ex, 100)), s_rest = ldexpf(1.f, max(ex - 100, 0));    // 2^149 is no fp32 number, its inverse is
+    if (lane == 0) inv[i] = ldexpf(1.f, -ex);
     uint4* out = reinterpret_cast<uint4*>(img + (size_t) i * K * TERMS);
     for (int sb = lane; sb < n_sb; sb += 32) {
         float v[16];
         load16(src, kind, row, K, sb, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] *= s;
+        for (int j = 0; j < 16; ++j) v[j] = v[j] * s * s_rest;
         // pieces (gran, 0, t) and (gran, 1, t): values {0,8,1,9,2,10,3,11} and {4,12,5,13,6,14,7,15}
         const int piece = ((sb >> 2) * 2) * 4 + (sb & 3);
         out[piece] = make_uint4(pack_half2(v[0], v[8]), pack_half2(v[1], v[9]), pack_half2(v[2], v[10]), pack_half2(v[3], v[11]));
@@ -237,7 +237,7 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
         if (TERMS == 2) {
             float r[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) r[j] = v[j] - __half2float(__float2half_rn(v[j]));
+            for (int j = 0; j < 16; ++j) r[j] = isinf(v[j]) ? 0.f : v[j] - __half2float(__float2half_rn(v[j]));
             uint4* lo = out + (K >> 3);
             lo[piece] = make_uint4(pack_half2(r[0], r[8]), pack_half2(r[1], r[9]), pack_half2(r[2], r[10]), pack_half2(r[3], r[11]));
             lo[piece + 4] = make_uint4(pack_half2(r[4], r[12]), pack_half2(r[5], r[13]), pack_half2(r[6], r[14]), pack_half2(r[7], r[15]));
