@@ -31,7 +31,7 @@ def rows(rng, K, names):
         if name in ("largest", "zero"):
             x[i] = 0
         if name == "largest":
-            x[i, 5], x[i, 90] = 3.3e38, 1e-30
+            x[i, 5], x[i, 90] = 3.3e38, 1e35        # (a value below 2^-38 of its row's largest would lie under both terms' last bit)
     return x
 
 
