@@ -155,8 +155,9 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 // One warp per activation row: the row -> fp16 image(s) in fragment order plus the inverse of the power of two it was
 // scaled by, so that its largest finite magnitude lands in [2^13, 2^14): inside fp16 and with all its bits for every fp32 row
 // (2^149 is the largest scale; it makes a row of nothing but the smallest numbers integers below 2^23, which the two terms hold
-// exactly).  An infinity is the first term alone: it reaches the sums as in fp32 and leaves the row's other values theirs.  A lane
-// takes one 16-value sub-block at a time, which is exactly two 16-byte pieces of the image (see image_index).
+// exactly; a value below 2^-38 of its row's largest is lost).  An infinity is the first term alone: it reaches the sums as in fp32
+// and leaves the row's other values theirs.  A lane takes one 16-value sub-block at a time, which is exactly two 16-byte pieces of
+// the image (see image_index).
 // FROM_H = false: rows of x (kind x_kind, width n_embd) - row i of x when the caller gave the number of x rows, else the
 // row of entry i; true: row e of the SwiGLU output h (fp32, width n_ff).
 // The last block lists the passes of the product that follows: a pass is up to 8 / TERMS consecutive entries of one group,
@@ -251,10 +252,15 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
 // PIECE: bytes of one weight copy = the rows' alignment.  16 where K is whole 256-column chunks; a row of any other K (whole
 // 64-column NVFP4 blocks, 36 bytes each) starts on 8 bytes (K % 128 == 0) or 4, and its last chunk holds fewer than four blocks:
 // those pieces are not requested and those blocks not multiplied.
-template <int FMT, int MODE, int TERMS, int PIECE>
+// CHAIN: MMAs that add up in one accumulator.  The tensor core truncates where it adds to an accumulator, fp32 arithmetic rounds to
+// nearest; distance to 64-bit sums of the 2048 x 512 layer's fp32 rows, and its 64-token step: a whole row chained 1.64e-6, 177 us;
+// 8 MMAs 2.9e-7, 179 us; 4 (a block of 64 columns) 2.1e-7, 186 us; 2 1.8e-7, 189 us; 1 1.7e-7, 192 us; the fp32 kernel 2.6e-7.
+// Four where no layout needs better.  IQ3_S and NVFP4 with ragged down rows, which the fp32 kernel had before, take one: with four,
+// bf16 rows would be further off than there (1.75e-7 against 1.6e-7 at 2560 x 640).
+template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN>
 __global__ void __launch_bounds__(kThreads, 2)
 blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __restrict__ inv, const int2* __restrict__ items,
-                 int* __restrict__ n_items, int tiles_per_warp, int n_row_blocks) {
+               int* __restrict__ n_items, int tiles_per_warp, int n_row_blocks) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff;
     const int n_gran = (int) (K >> 6);                       // 64-column granules
@@ -362,8 +368,8 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                     }
                 } else {
 #pragma unroll
-                for (int j = 0; j < kCopies; ++j)
-                    if (lane + 32 * j < kPieces && (FMT == FMT_IQ3S || PIECE == 16 || cp_off[j] < row_bytes)) cp_async_piece<PIECE>(dst + cp_dst[j], src[j] + iss_off);
+                    for (int j = 0; j < kCopies; ++j)
+                        if (lane + 32 * j < kPieces && (PIECE == 16 || cp_off[j] < row_bytes)) cp_async_piece<PIECE>(dst + cp_dst[j], src[j] + iss_off);
                 }
                 ++iss_unit;
                 if (++iss_chunk == n_chunks) {
@@ -417,9 +423,6 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
             }
             float sg = 1.f, su = 1.f, sd = 1.f;
             if constexpr (FMT == FMT_NVFP4) { sg = tail[0]; su = tail[1]; sd = tail[2]; }
-            // The tensor core truncates where it adds to an accumulator, so every MMA starts from zero and its sum goes to fp32
-            // arithmetic (rounded to nearest): chained over a row the result was 2 to 3 times as far from 64-bit sums as the
-            // warp-per-row fp32 kernel's
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
             // this lane's B fragments: its column's pieces, or (column unused in this pass) the zero area with stride 0
             const bool col_live = g < ncol;
@@ -460,35 +463,36 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                         for (int i = 0; i < 4; ++i) acc[i] = fmaf(part[i], i < 2 ? da : db, acc[i]);
                     }
                 } else {
-                float part[4] = {0.f, 0.f, 0.f, 0.f};      // a chunk's sum, so that the row's is a short chain
+                    float part[4] = {0.f, 0.f, 0.f, 0.f};      // a chunk's sum, so that the row's is a short chain
 #pragma unroll
-                for (int blk = 0; blk < 4; ++blk) {
-                    if (PIECE != 16 && 4 * chunk + blk >= n_gran) break;   // past the row's last block
-                    const uint4 b0 = bp[blk * bstep], b1 = bp[blk * bstep + bhalf];
-                    const uint32_t sa = lut[reinterpret_cast<const uint8_t*>(ra)[36 * blk + t]];
-                    const uint32_t sb = lut[reinterpret_cast<const uint8_t*>(rb)[36 * blk + t]];
-                    uint32_t qa0[4], qa1[4], qb0[4], qb1[4];
-                    cvt_e2m1x8(ra[9 * blk + 1 + 2 * t], qa0);
-                    cvt_e2m1x8(ra[9 * blk + 2 + 2 * t], qa1);
-                    cvt_e2m1x8(rb[9 * blk + 1 + 2 * t], qb0);
-                    cvt_e2m1x8(rb[9 * blk + 2 + 2 * t], qb1);
+                    for (int blk = 0; blk < 4; ++blk) {
+                        if (PIECE != 16 && 4 * chunk + blk >= n_gran) break;   // past the row's last block
+                        const uint4 b0 = bp[blk * bstep], b1 = bp[blk * bstep + bhalf];
+                        const uint32_t sa = lut[reinterpret_cast<const uint8_t*>(ra)[36 * blk + t]];
+                        const uint32_t sb = lut[reinterpret_cast<const uint8_t*>(rb)[36 * blk + t]];
+                        uint32_t qa0[4], qa1[4], qb0[4], qb1[4];
+                        cvt_e2m1x8(ra[9 * blk + 1 + 2 * t], qa0);
+                        cvt_e2m1x8(ra[9 * blk + 2 + 2 * t], qa1);
+                        cvt_e2m1x8(rb[9 * blk + 1 + 2 * t], qb0);
+                        cvt_e2m1x8(rb[9 * blk + 2 + 2 * t], qb1);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        qa0[i] = hmul2_bits(qa0[i], sa);
-                        qa1[i] = hmul2_bits(qa1[i], sa);
-                        qb0[i] = hmul2_bits(qb0[i], sb);
-                        qb1[i] = hmul2_bits(qb1[i], sb);
+                        for (int i = 0; i < 4; ++i) {
+                            qa0[i] = hmul2_bits(qa0[i], sa);
+                            qa1[i] = hmul2_bits(qa1[i], sa);
+                            qb0[i] = hmul2_bits(qb0[i], sb);
+                            qb1[i] = hmul2_bits(qb1[i], sb);
+                        }
+                        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f}, s3[4] = {0.f, 0.f, 0.f, 0.f};
+                        constexpr bool kOne = CHAIN == 1;
+                        mma_f16(s0, qa0[0], qb0[0], qa0[1], qb0[1], b0.x, b0.y);
+                        mma_f16(kOne ? s1 : s0, qa0[2], qb0[2], qa0[3], qb0[3], b0.z, b0.w);
+                        mma_f16(kOne ? s2 : s0, qa1[0], qb1[0], qa1[1], qb1[1], b1.x, b1.y);
+                        mma_f16(kOne ? s3 : s0, qa1[2], qb1[2], qa1[3], qb1[3], b1.z, b1.w);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) part[i] += kOne ? (s0[i] + s1[i]) + (s2[i] + s3[i]) : s0[i];
                     }
-                    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f}, s3[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_f16(s0, qa0[0], qb0[0], qa0[1], qb0[1], b0.x, b0.y);
-                    mma_f16(s1, qa0[2], qb0[2], qa0[3], qb0[3], b0.z, b0.w);
-                    mma_f16(s2, qa1[0], qb1[0], qa1[1], qb1[1], b1.x, b1.y);
-                    mma_f16(s3, qa1[2], qb1[2], qa1[3], qb1[3], b1.z, b1.w);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) part[i] += (s0[i] + s1[i]) + (s2[i] + s3[i]);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[i] += part[i];
+                    for (int i = 0; i < 4; ++i) acc[i] += part[i];
                 }
                 __syncwarp();   // every lane is done with this stage before a later issue overwrites it
                 if (++chunk != n_chunks) continue;
@@ -531,7 +535,7 @@ template <int FMT>
 size_t smem_bytes(int64_t K) { return (size_t) K * kCols * 2 + Fmt<FMT>::kTable + 128 + (size_t) kWarps * kStages * kStageBytes<FMT>; }
 size_t align256(size_t v) { return (v + 255) & ~(size_t) 255; }
 
-template <int FMT, int MODE, int TERMS, int PIECE = 16>
+template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN>
 int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const int2* items, int* n_items, cudaStream_t st) {
     const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff;
     const size_t smem = smem_bytes<FMT>(K);
@@ -539,7 +543,7 @@ int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const i
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(blk_mma_kernel<FMT, MODE, TERMS, PIECE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        const cudaError_t e = cudaFuncSetAttribute(blk_mma_kernel<FMT, MODE, TERMS, PIECE, CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
@@ -554,7 +558,7 @@ int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const i
     const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
     const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
     const int n_row_blocks = (int) ((n_tiles + tpw - 1) / tpw);
-    launch_k(blk_mma_kernel<FMT, MODE, TERMS, PIECE>, dim3((unsigned) (2 * sm_count())), dim3(kThreads), smem, st, a, img, inv, items, n_items, tpw, n_row_blocks);
+    launch_k(blk_mma_kernel<FMT, MODE, TERMS, PIECE, CHAIN>, dim3((unsigned) (2 * sm_count())), dim3(kThreads), smem, st, a, img, inv, items, n_items, tpw, n_row_blocks);
     return launch_status();
 }
 
@@ -573,6 +577,7 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     // IQ3_S: rows of whole 512-column chunks (every other 110-byte block starts on 4 bytes, what the copies need).  The activation
     // image must fit shared memory.
     const int fmt = L.gu_type == kTypeNVFP4 ? FMT_NVFP4 : FMT_IQ3S;
+    const bool whole = L.n_ff % 256 == 0;
     if ((L.gu_type != kTypeNVFP4 && L.gu_type != kTypeIQ3S) || L.up_type != L.gu_type || L.d_type != L.gu_type) return BSX_E_TYPE;
     if (fmt == FMT_NVFP4) {
         if (L.n_embd % 256 || L.n_ff % 64) return BSX_E_TYPE;
@@ -599,21 +604,25 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     if (phase != 2) {
         if (a.x_kind == BSX_X_BF16) {
             launch_k(prep_image_kernel<false, 1>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
-            rc = fmt == FMT_NVFP4 ? launch<FMT_NVFP4, MODE_GU, 1>(a, ximg, xinv, items, n_items, st) : launch<FMT_IQ3S, MODE_GU, 1, 4>(a, ximg, xinv, items, n_items, st);
+            rc = fmt == FMT_IQ3S ? launch<FMT_IQ3S, MODE_GU, 1, 4, 1>(a, ximg, xinv, items, n_items, st)
+                 : whole         ? launch<FMT_NVFP4, MODE_GU, 1, 16, 4>(a, ximg, xinv, items, n_items, st)
+                                 : launch<FMT_NVFP4, MODE_GU, 1, 16, 1>(a, ximg, xinv, items, n_items, st);
         } else {
             launch_k(prep_image_kernel<false, 2>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
-            rc = fmt == FMT_NVFP4 ? launch<FMT_NVFP4, MODE_GU, 2>(a, ximg, xinv, items, n_items, st) : launch<FMT_IQ3S, MODE_GU, 2, 4>(a, ximg, xinv, items, n_items, st);
+            rc = fmt == FMT_IQ3S ? launch<FMT_IQ3S, MODE_GU, 2, 4, 1>(a, ximg, xinv, items, n_items, st)
+                 : whole         ? launch<FMT_NVFP4, MODE_GU, 2, 16, 4>(a, ximg, xinv, items, n_items, st)
+                                 : launch<FMT_NVFP4, MODE_GU, 2, 16, 1>(a, ximg, xinv, items, n_items, st);
         }
     }
     if (rc != BSX_OK || phase == 1) return rc;
     launch_k(prep_image_kernel<true, 2>, dim3(nbh), dim3(256), 0, st, a, himg, hinv, items, n_items);
-    if (fmt == FMT_IQ3S) return launch<FMT_IQ3S, MODE_DOWN, 2, 4>(a, himg, hinv, items, n_items, st);
+    if (fmt == FMT_IQ3S) return launch<FMT_IQ3S, MODE_DOWN, 2, 4, 1>(a, himg, hinv, items, n_items, st);
     // Down rows of n_ff columns: the copies' width is what their start is aligned to.  An n_ff that is not whole 256-column chunks
     // went to the warp-per-row kernels before (2 % of the copy bandwidth: fp32 decode and FMA for every weight and entry); here
     // the same 27-token step (2560 x 640, 512 + 1 experts, top-10) takes 217 us instead of 3648.
-    if (L.n_ff % 256 == 0) return launch<FMT_NVFP4, MODE_DOWN, 2>(a, himg, hinv, items, n_items, st);
-    if (L.n_ff % 128 == 0) return launch<FMT_NVFP4, MODE_DOWN, 2, 8>(a, himg, hinv, items, n_items, st);
-    return launch<FMT_NVFP4, MODE_DOWN, 2, 4>(a, himg, hinv, items, n_items, st);
+    if (whole) return launch<FMT_NVFP4, MODE_DOWN, 2, 16, 4>(a, himg, hinv, items, n_items, st);
+    if (L.n_ff % 128 == 0) return launch<FMT_NVFP4, MODE_DOWN, 2, 8, 1>(a, himg, hinv, items, n_items, st);
+    return launch<FMT_NVFP4, MODE_DOWN, 2, 4, 1>(a, himg, hinv, items, n_items, st);
 }
 
 }  // namespace bsx
