@@ -40,6 +40,8 @@ constexpr int kEntQ = 4;
 constexpr float kTerm2 = 1.0f / 254.0f;
 
 enum { QMODE_GU = 0, QMODE_DOWN = 1 };
+// Q6_K rows beyond this go to the fp32 kernels: the images hold 15 bits of a row's largest value, not its 24
+constexpr int64_t kMaxColsQ6K = 8192;
 
 // kChunkBlocks 256-column blocks of a row are a stage.  IQ1_M: two blocks (112 bytes), copied in 16-byte pieces.  Q6_K: one 210-byte
 // block as the 53 words that cover it (every second block starts on 2 bytes, so its copy starts 2 bytes early; none reaches past its
@@ -551,9 +553,8 @@ int32_t kq_launch(const ExpertArgs& a, const int8_t* img, const int8_t* corr, co
             return kq_launch_split<TYPE, MODE, 2, 1, 3>(a, img, corr, inv, items, n_items, 1, st);      // whole 512-column rows
         }
         if (two) return kq_launch_split<TYPE, MODE, 1, 1, 3>(a, img, corr, inv, items, n_items, 1, st);
-        if (units < sm_count() && chunks % 4 == 0 && kq_smem<TYPE>(K, 0, 5) <= 220 * 1024) return kq_launch_split<TYPE, MODE, 4, 1, 5>(a, img, corr, inv, items, n_items, 1, st);
-        if (kq_smem<TYPE>(K, 0, 5) <= 225 * 1024) return kq_launch_split<TYPE, MODE, 1, 1, 5>(a, img, corr, inv, items, n_items, 1, st);
-        return kq_launch_split<TYPE, MODE, 1, 1, 4>(a, img, corr, inv, items, n_items, 1, st);
+        if (units < sm_count() && chunks % 4 == 0) return kq_launch_split<TYPE, MODE, 4, 1, 5>(a, img, corr, inv, items, n_items, 1, st);
+        return kq_launch_split<TYPE, MODE, 1, 1, 5>(a, img, corr, inv, items, n_items, 1, st);
     } else {
         int64_t tpw0 = (384 * 1024 + tile_bytes - 1) / tile_bytes;                       // a unit streams ~400 KB
         tpw0 = tpw0 < 1 ? 1 : tpw0 > 8 ? 8 : tpw0;
@@ -586,8 +587,8 @@ int32_t experts_grouped_kq(const ExpertArgs& a, cudaStream_t st) {
     const bsx_expert_layout& L = a.L;
     if (!kq_type(L.gu_type) || L.up_type != L.gu_type || !kq_type(L.d_type)) return BSX_E_TYPE;
     if (!kq_dim_ok(L.gu_type, L.n_embd, L.n_ff) || !kq_dim_ok(L.d_type, L.n_ff, L.n_embd) || L.n_embd % 16) return BSX_E_TYPE;
-    if ((L.gu_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_embd) : kq_smem<kTypeQ6K>(L.n_embd, 0, 4)) > 225 * 1024) return BSX_E_TYPE;
-    if ((L.d_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_ff) : kq_smem<kTypeQ6K>(L.n_ff, 0, 4)) > 225 * 1024) return BSX_E_TYPE;
+    if (L.gu_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_embd) > 225 * 1024 : L.n_embd > kMaxColsQ6K) return BSX_E_TYPE;
+    if (L.d_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_ff) > 225 * 1024 : L.n_ff > kMaxColsQ6K) return BSX_E_TYPE;
     const int64_t cap = a.cap_entries, H = L.n_embd, I = L.n_ff;
     uint8_t* p = reinterpret_cast<uint8_t*>(a.h) + al256q((size_t) cap * I * 4);
     int8_t* ximg = reinterpret_cast<int8_t*>(p);

@@ -28,3 +28,14 @@ def test_q6k_rows(lib, cuda, H, I, groups):
         want = O.expert_forward(Lo, blobs[e], x[toks], dtype=np.float64)
         assert rel_l2(out[at:at + len(toks)], want) < 4e-4, (e, rel_l2(out[at:at + len(toks)], want))
         at += len(toks)
+
+
+@pytest.mark.parametrize("H,I", [(8704, 512), (512, 8704)])
+def test_rows_beyond_the_integer_kernel_keep_their_24_bits(lib, cuda, H, I):
+    """Bound 1e-5: fp32 sums of exactly decoded weights."""
+    rng = np.random.default_rng(H)
+    Lo, blobs = make_expert_blobs(rng, 1, O.T_Q6_K, O.T_Q6_K, H, I)
+    L = moe.native_expert_layout(O.T_Q6_K, O.T_Q6_K, H, I)
+    x = rng.standard_normal((3, H)).astype(np.float32)
+    out = run_grouped(L, dev(stack_blobs(blobs)), [0], [[0, 1, 2]], dev(x), 3).cpu().numpy()
+    assert rel_l2(out, O.expert_forward(Lo, blobs[0], x, dtype=np.float64)) < 1e-5
