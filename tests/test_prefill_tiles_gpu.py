@@ -1,6 +1,6 @@
 """Packed prompt experts at the row counts where a 128-row tile's image changes its length (whole groups of eight rows, one more,
 one less, one row, two tiles), at one and several chunks of either product, and with an output that is only 16-byte aligned; and at
-the row counts where the short-prompt route's passes fill.
+the row counts where the short-prompt route's passes fill; and with experts that another device holds, whose rows stay as they are.
 Bound 7e-4: four times the four-term FP4 error of a row (1.8e-4)."""
 import ctypes as C
 
@@ -21,12 +21,10 @@ SHORT16 = [0, 1, 8, 9, 15, 16, 17, 0, 130, 32, 33, 0, 0, 2, 0, 0]               
 SHORT8 = [0, 1, 7, 8, 9, 0, 17, 0, 0, 0, 0, 0, 0, 1, 0, 0]                       # 3 an expert: passes of 8
 
 
-@pytest.mark.parametrize("H,I,shift,counts", [(256, 256, 0, TILES), (512, 512, 16, TILES), (768, 768, 0, TILES), (256, 1024, 16, TILES), (2048, 512, 0, TILES),
-                                              (256, 256, 16, SHORT16), (2048, 512, 0, SHORT16), (768, 1280, 0, SHORT16), (512, 512, 0, SHORT8), (768, 768, 16, SHORT8)])
-def test_tile_row_counts(lib, cuda, H, I, shift, counts):
+def run(H, I, shift, counts, held_elsewhere=()):
     rng = np.random.default_rng(H * 3 + I)
     E = len(counts)
-    Lo, blobs = make_expert_blobs(rng, E, O.T_NVFP4, O.T_NVFP4, H, I)
+    Lo, blobs = make_expert_blobs(rng, min(E, 10), O.T_NVFP4, O.T_NVFP4, H, I)
     L = moe.native_expert_layout(O.T_NVFP4, O.T_NVFP4, H, I)
     packed = moe.pack_experts(L, dev(stack_blobs(blobs)))
     n, T = sum(counts), 300
@@ -34,22 +32,44 @@ def test_tile_row_counts(lib, cuda, H, I, shift, counts):
     src = rng.integers(0, T, n).astype(np.int32)
     tiles = np.array([(e, off[e] + 128 * i) for e in range(E) for i in range((counts[e] + 127) // 128)], np.int32)
     x = rng.standard_normal((T, H)).astype(np.float32)
-    table = packed.data_ptr() + torch.arange(E, dtype=torch.int64, device="cuda") * packed.shape[1]
+    table = packed.data_ptr() + torch.arange(E, dtype=torch.int64, device="cuda") % len(blobs) * packed.shape[1]
+    table[list(held_elsewhere)] = 0
     lb = capi.lib()
-    scratch = torch.empty(lb.bsx_experts_prefill_packed_scratch_bytes(C.byref(L), T, n), dtype=torch.uint8, device="cuda")
+    scratch = torch.full((lb.bsx_experts_prefill_packed_scratch_bytes(C.byref(L), T, n),), 0xFF, dtype=torch.uint8, device="cuda")
     raw = torch.full((n * H * 4 + 256,), 0xFF, dtype=torch.uint8, device="cuda")
     dm = raw[shift:shift + n * H * 4].view(torch.float32).view(n, H)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     o, s, t, nt, xd = dev(off), dev(src), dev(tiles), dev(np.array([len(tiles)], np.int32)), dev(x)
     stream = moe._stream(None)
     torch.cuda.synchronize()
-    capi.check("prefill packed", lb.bsx_experts_prefill_packed(C.byref(L), table.data_ptr(), o.data_ptr(), s.data_ptr(), t.data_ptr(), nt.data_ptr(),
-                                                               len(tiles), n, xd.data_ptr(), capi.X_F32, T, E, scratch.data_ptr(), dm.data_ptr(),
-                                                               status.data_ptr(), stream))
+    for _ in range(2):          # again over the scratch that the first call left
+        capi.check("prefill packed", lb.bsx_experts_prefill_packed(C.byref(L), table.data_ptr(), o.data_ptr(), s.data_ptr(), t.data_ptr(), nt.data_ptr(),
+                                                                   len(tiles), n, xd.data_ptr(), capi.X_F32, T, E, scratch.data_ptr(), dm.data_ptr(),
+                                                                   status.data_ptr(), stream))
     torch.cuda.synchronize()
     assert int(status.item()) == 0
     got = dm.cpu().numpy()
+    assert (raw[:shift] == 0xFF).all() and (raw[shift + n * H * 4:] == 0xFF).all()
     for e in range(E):
-        if counts[e]:
-            want = O.expert_forward(Lo, blobs[e], x[src[off[e]:off[e + 1]]], dtype=np.float64)
-            assert rel_l2(got[off[e]:off[e + 1]], want) < 7e-4, (e, counts[e])
+        rows = got[off[e]:off[e + 1]]
+        if e in held_elsewhere:
+            assert (rows.view(np.uint32) == 0xFFFFFFFF).all(), e
+        elif counts[e]:
+            want = O.expert_forward(Lo, blobs[e % len(blobs)], x[src[off[e]:off[e + 1]]], dtype=np.float64)
+            assert rel_l2(rows, want) < 7e-4, (e, counts[e], rel_l2(rows, want))
+
+
+@pytest.mark.parametrize("H,I,shift,counts", [(256, 256, 0, TILES), (512, 512, 16, TILES), (768, 768, 0, TILES), (256, 1024, 16, TILES), (2048, 512, 0, TILES),
+                                              (256, 256, 16, SHORT16), (2048, 512, 0, SHORT16), (768, 1280, 0, SHORT16), (512, 512, 0, SHORT8), (768, 768, 16, SHORT8)])
+def test_tile_row_counts(lib, cuda, H, I, shift, counts):
+    run(H, I, shift, counts)
+
+
+MANY = [130, 500, 257] * 17                                                       # more tiles than an SM each
+
+
+@pytest.mark.parametrize("H,I,counts,away", [(256, 256, TILES, (0, 4, 9)), (512, 512, TILES, (9,)), (768, 768, TILES, (0, 1, 2, 3)), (256, 512, MANY, range(0, 51, 3)),
+                                             (256, 768, MANY, range(1, 51, 2)), (512, 512, SHORT16, (1, 8, 13)), (768, 2304, SHORT16, (8, 9)),
+                                             (512, 256, SHORT8, (1, 6, 13)), (768, 768, SHORT8, (4,)), (256, 256, SHORT8, range(16)), (256, 256, TILES, range(10))])
+def test_experts_held_elsewhere(lib, cuda, H, I, counts, away):
+    run(H, I, 0, counts, tuple(away))
