@@ -43,17 +43,19 @@ enum { QMODE_GU = 0, QMODE_DOWN = 1 };
 // Q6_K rows beyond this go to the fp32 kernels: the images hold 15 bits of a row's largest value, not its 24
 constexpr int64_t kMaxColsQ6K = 8192;
 
-// kChunkBlocks 256-column blocks of a row are a stage.  IQ1_M: two blocks (112 bytes), copied in 16-byte pieces.  Q6_K: one 210-byte
+// CB 256-column blocks of a row are a stage.  IQ1_M: two blocks (112 bytes), copied in 16-byte pieces.  Q6_K: one 210-byte
 // block as the 53 words that cover it (every second block starts on 2 bytes, so its copy starts 2 bytes early; none reaches past its
-// row), rows 60 words apart, which keeps a quarter-warp's reads in different banks.  One block a stage lets any power-of-two part
-// of a row be a warp's own (KS below) and two CTAs of eight warps share an SM.
+// row), rows 60 words apart, which keeps a quarter-warp's reads in different banks; or two blocks as 105 words.  One block a stage lets
+// any power-of-two part of a row be a warp's own (KS below) and, up to 2048 columns, two CTAs of eight warps share an SM; wider rows
+// leave room for one CTA and take two blocks (7168 x 2048, 256 experts: 64 tokens 2834 us, with one block and five stages 3239).
 template <int TYPE> struct QT;
+template <int TYPE, int CB> constexpr int kRowStage = TYPE == kTypeIQ1M ? 112 : CB == 1 ? 240 : 420;
 template <> struct QT<kTypeIQ1M> {
-    static constexpr int kBlock = 56, kWarps = 16, kPad = 32, kChunkBlocks = 2, kRowStage = 112;
+    static constexpr int kBlock = 56, kWarps = 16, kPad = 32;
     static constexpr bool kCorr = true;
 };
 template <> struct QT<kTypeQ6K> {
-    static constexpr int kBlock = 210, kWarps = 8, kPad = 16, kChunkBlocks = 1, kRowStage = 240;
+    static constexpr int kBlock = 210, kWarps = 8, kPad = 16;
     static constexpr bool kCorr = false;
 };
 
@@ -304,14 +306,13 @@ __device__ __forceinline__ void q6k_block(const uint8_t* ra, const uint8_t* rb, 
 // KS > 1: KS neighbouring warps share a row tile, each a part of its columns, and their sums meet in shared memory - for calls so
 // small that whole rows would leave most SMs without a unit (a shared expert of 2048 x 512 at 5 tokens: 16 units of 148; its two
 // products took 47 of the step's 155 us, with the split the step takes 121).
-template <int TYPE, int MODE, int KS, int NC, int ST>
-__global__ void __launch_bounds__(QT<TYPE>::kWarps * 32, TYPE == kTypeQ6K && ST == 3 ? 2 : 1)
+template <int TYPE, int MODE, int KS, int NC, int ST, int CB>
+__global__ void __launch_bounds__(QT<TYPE>::kWarps * 32, CB == 1 && ST == 3 ? 2 : 1)
 kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __restrict__ corr, const float* __restrict__ inv,
               const int2* __restrict__ items, int* __restrict__ n_items, int tiles_per_warp, int n_row_blocks) {
     using Q = QT<TYPE>;
     constexpr int kWarps = Q::kWarps, kThreads = kWarps * 32, kStages = ST;
-    constexpr int kChunkBlocks = Q::kChunkBlocks, kChunkBytes = kChunkBlocks * Q::kBlock, kRowStage = Q::kRowStage;
-    constexpr int kStageBytes = kRowsQ * kRowStage;
+    constexpr int kChunkBytes = CB * Q::kBlock, kRow = kRowStage<TYPE, CB>, kStageBytes = kRowsQ * kRow;
     extern __shared__ __align__(128) uint8_t smem[];
     const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
     const int nblk = (int) (K >> 8);
@@ -354,7 +355,7 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
     constexpr int kTileRows = MODE == QMODE_GU ? 8 : 16;
     static_assert(kWarps % KS == 0, "");
     constexpr int tile_stride = kWarps / KS * kTileRows;
-    const int n_chunks = nblk / kChunkBlocks / KS, chunk0 = (warp % KS) * n_chunks;      // this warp's part of a row
+    const int n_chunks = nblk / CB / KS, chunk0 = (warp % KS) * n_chunks;      // this warp's part of a row
     const size_t row_bytes = MODE == QMODE_GU ? (size_t) a.L.gu_row : (size_t) a.L.d_row;
 
     const int n_work = n_items[0] * n_row_blocks;
@@ -411,16 +412,29 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {                    // 7 pieces a row, 112 in all
                         const int p = lane + 32 * j, row = p / 7, off = (p - row * 7) * 16;
-                        if (p < 112) cpa16(dst + (uint32_t) (row * kRowStage + off), src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1) + off);
+                        if (p < 112) cpa16(dst + (uint32_t) (row * kRow + off), src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1) + off);
                     }
                 } else {
-                    const uint8_t* src = row0 + iss_tile + (size_t) (chunk0 + iss_chunk) * kChunkBytes - 2 * ((chunk0 + iss_chunk) & 1) + 4 * lane;
+                    const uint8_t* src = row0 + iss_tile + (size_t) (chunk0 + iss_chunk) * kChunkBytes - (CB == 1 ? 2 * ((chunk0 + iss_chunk) & 1) : 0) + 4 * lane;
+                    auto row_at = [&](int row) { return src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1); };
+                    if constexpr (CB == 1) {
 #pragma unroll
-                    for (int row = 0; row < kRowsQ; ++row) {
-                        const uint8_t* r = src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1);
-                        const uint32_t d = dst + (uint32_t) (row * kRowStage + 4 * lane);
-                        cpa4(d, r);
-                        if (lane < 53 - 32) cpa4(d + 128, r + 128);
+                        for (int row = 0; row < kRowsQ; ++row) {
+                            const uint8_t* r = row_at(row);
+                            const uint32_t d = dst + (uint32_t) (row * kRow + 4 * lane);
+                            cpa4(d, r);
+                            if (lane < 53 - 32) cpa4(d + 128, r + 128);
+                        }
+                    } else {
+                        // two rows as one run of 210 words: seven copies instead of four a row
+#pragma unroll
+                        for (int row = 0; row < kRowsQ; row += 2) {
+                            const uint8_t *ra = row_at(row), *rb = row_at(row + 1) - kRow;
+                            const uint32_t d = dst + (uint32_t) (row * kRow + 4 * lane);
+#pragma unroll
+                            for (int i = 0; i < 7; ++i)
+                                if (i < 6 || lane < 210 - 192) cpa4(d + 128 * i, (i > 3 || (i == 3 && lane >= 105 - 96) ? rb : ra) + 128 * i);
+                        }
                     }
                 }
                 ++iss_unit;
@@ -453,11 +467,11 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
             __syncwarp();
             const uint8_t* st = wring + (size_t) (unit % kStages) * kStageBytes;
 #pragma unroll
-            for (int b = 0; b < kChunkBlocks; ++b) {
-                const int blk = (chunk0 + chunk) * kChunkBlocks + b;
-                const int at = TYPE == kTypeIQ1M ? b * Q::kBlock : 2 * ((chunk0 + chunk) & 1);
-                const uint8_t* ra = st + g * kRowStage + at;
-                const uint8_t* rbp = st + (g + 8) * kRowStage + at;
+            for (int b = 0; b < CB; ++b) {
+                const int blk = (chunk0 + chunk) * CB + b;
+                const int at = CB == 2 ? b * Q::kBlock : 2 * ((chunk0 + chunk) & 1);
+                const uint8_t* ra = st + g * kRow + at;
+                const uint8_t* rbp = st + (g + 8) * kRow + at;
                 if constexpr (Q::kCorr) iq1m_block<NC>(ra, rbp, tab + (lane & (NC - 1)), bcol + 256 * blk, ccol + 64 * blk, t, tot);
                 else q6k_block(ra, rbp, bcol + 256 * blk, t, tot);
             }
@@ -506,29 +520,29 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
 size_t al256q(size_t v) { return (v + 255) & ~(size_t) 255; }
 
 template <int TYPE>
-size_t kq_smem(int64_t K, int copies = 2, int stages = 3) {
+size_t kq_smem(int64_t K, int copies = 2, int stages = 3, int cb = 2) {
     using Q = QT<TYPE>;
     return (size_t) kColsQ * (K + Q::kPad) + (Q::kCorr ? (size_t) kColsQ * ((K >> 8) * 64 + 16) + (size_t) 16384 * copies : 0) +
-           (size_t) Q::kWarps * stages * kRowsQ * Q::kRowStage + 128;
+           (size_t) Q::kWarps * stages * kRowsQ * (cb == 1 ? kRowStage<TYPE, 1> : kRowStage<TYPE, 2>) + 128;
 }
 
-template <int TYPE, int MODE, int KS, int NC, int ST>
+template <int TYPE, int MODE, int KS, int NC, int ST, int CB>
 int32_t kq_launch_split(const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const int2* items, int* n_items, int tpw, cudaStream_t st) {
     using Q = QT<TYPE>;
-    const size_t smem = kq_smem<TYPE>(MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff, NC, ST);
+    const size_t smem = kq_smem<TYPE>(MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff, NC, ST, CB);
     static std::atomic<bool> configured[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(kq_mma_kernel<TYPE, MODE, KS, NC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, KS > 1 ? 220 * 1024 : 225 * 1024);
+        const cudaError_t e = cudaFuncSetAttribute(kq_mma_kernel<TYPE, MODE, KS, NC, ST, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, KS > 1 ? 220 * 1024 : 225 * 1024);
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
     const int64_t rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd, tile_rows = (MODE == QMODE_GU ? 8 : 16) * Q::kWarps / KS;
     const int64_t n_tiles = (rows + tile_rows - 1) / tile_rows;
     const int n_row_blocks = (int) ((n_tiles + tpw - 1) / tpw);
-    const int per_sm = TYPE == kTypeQ6K && ST == 3 ? 2 : 1;
-    launch_k(kq_mma_kernel<TYPE, MODE, KS, NC, ST>, dim3((unsigned) (per_sm * sm_count())), dim3(Q::kWarps * 32), smem, st, a, img, corr, inv, items, n_items, tpw,
+    const int per_sm = CB == 1 && ST == 3 ? 2 : 1;
+    launch_k(kq_mma_kernel<TYPE, MODE, KS, NC, ST, CB>, dim3((unsigned) (per_sm * sm_count())), dim3(Q::kWarps * 32), smem, st, a, img, corr, inv, items, n_items, tpw,
              n_row_blocks);
     return launch_status();
 }
@@ -542,27 +556,31 @@ int32_t kq_launch(const ExpertArgs& a, const int8_t* img, const int8_t* corr, co
     const int64_t tile_bytes = (int64_t) Q::kWarps * kRowsQ * row_bytes;                 // one row tile of every warp
     const int64_t tile_rows = (MODE == QMODE_GU ? 8 : 16) * Q::kWarps;
     const int64_t n_tiles = (rows + tile_rows - 1) / tile_rows;
+    int64_t tpw0 = (384 * 1024 + tile_bytes - 1) / tile_bytes;                           // a unit streams ~400 KB
+    tpw0 = tpw0 < 1 ? 1 : tpw0 > 8 ? 8 : tpw0;
+    const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
+    const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
     if constexpr (TYPE == kTypeQ6K) {
-        // One row tile a warp, so that few passes still reach every SM; and where even these units cannot (at most a pass per group and
-        // one per four entries), the columns are split too.  cap_groups and cap_entries bound the passes on the host.
+        // Where even one row tile a warp and unit cannot reach every SM (at most a pass per group and one per four entries), the columns
+        // are split too.  cap_groups and cap_entries bound the passes on the host.
         const int64_t passes = a.cap_groups + a.cap_entries / kEntQ, units = passes * n_tiles, chunks = K / 256;
-        const bool two = kq_smem<TYPE>(K, 0, 3) <= 108 * 1024;                           // two blocks an SM, else one with longer rings
-        if (units < sm_count() && two) {
-            if (chunks % 8 == 0) return kq_launch_split<TYPE, MODE, 8, 1, 3>(a, img, corr, inv, items, n_items, 1, st);
-            if (chunks % 4 == 0) return kq_launch_split<TYPE, MODE, 4, 1, 3>(a, img, corr, inv, items, n_items, 1, st);
-            return kq_launch_split<TYPE, MODE, 2, 1, 3>(a, img, corr, inv, items, n_items, 1, st);      // whole 512-column rows
+        if (kq_smem<TYPE>(K, 0, 3, 1) <= 108 * 1024) {                                   // two blocks an SM
+            if (units >= sm_count()) {
+                // two tiles where one is less than 64 KB (down rows of 512 columns) and the units still go round the SMs four times:
+                // 2048 x 512, 512 experts, 64 tokens 331 us against 342 with one; at 32 tokens 226 against 230
+                const int two = tile_bytes < 64 * 1024 && units >= 2 * 4 * 2 * (int64_t) sm_count() ? 2 : 1;
+                return kq_launch_split<TYPE, MODE, 1, 1, 3, 1>(a, img, corr, inv, items, n_items, two, st);
+            }
+            if (chunks % 8 == 0) return kq_launch_split<TYPE, MODE, 8, 1, 3, 1>(a, img, corr, inv, items, n_items, 1, st);
+            if (chunks % 4 == 0) return kq_launch_split<TYPE, MODE, 4, 1, 3, 1>(a, img, corr, inv, items, n_items, 1, st);
+            return kq_launch_split<TYPE, MODE, 2, 1, 3, 1>(a, img, corr, inv, items, n_items, 1, st);      // whole 512-column rows
         }
-        if (two) return kq_launch_split<TYPE, MODE, 1, 1, 3>(a, img, corr, inv, items, n_items, 1, st);
-        if (units < sm_count() && chunks % 4 == 0) return kq_launch_split<TYPE, MODE, 4, 1, 5>(a, img, corr, inv, items, n_items, 1, st);
-        return kq_launch_split<TYPE, MODE, 1, 1, 5>(a, img, corr, inv, items, n_items, 1, st);
+        if (units < sm_count() && chunks % 4 == 0) return kq_launch_split<TYPE, MODE, 4, 1, 5, 1>(a, img, corr, inv, items, n_items, 1, st);
+        return kq_launch_split<TYPE, MODE, 1, 1, 3, 2>(a, img, corr, inv, items, n_items, tpw, st);
     } else {
-        int64_t tpw0 = (384 * 1024 + tile_bytes - 1) / tile_bytes;                       // a unit streams ~400 KB
-        tpw0 = tpw0 < 1 ? 1 : tpw0 > 8 ? 8 : tpw0;
-        const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
-        const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
         // four copies of the codebook where they fit beside the columns and the stages (K up to 7680), else two
-        if (kq_smem<TYPE>(K, 4) <= 225 * 1024) return kq_launch_split<TYPE, MODE, 1, 4, 3>(a, img, corr, inv, items, n_items, tpw, st);
-        return kq_launch_split<TYPE, MODE, 1, 2, 3>(a, img, corr, inv, items, n_items, tpw, st);
+        if (kq_smem<TYPE>(K, 4) <= 225 * 1024) return kq_launch_split<TYPE, MODE, 1, 4, 3, 2>(a, img, corr, inv, items, n_items, tpw, st);
+        return kq_launch_split<TYPE, MODE, 1, 2, 3, 2>(a, img, corr, inv, items, n_items, tpw, st);
     }
 }
 
