@@ -208,8 +208,9 @@ extern "C" int32_t bsx_moe_layer(const bsx_moe_layer_desc* d, const void* x, int
         rc = launch_status();
         if (rc != BSX_OK) return rc;
         // A shared expert sees every token.  From 16 tokens on, an NVFP4 one goes through the prompt-sized kernel (one pass over the
-        // blob for the whole window; the decode kernels take 4 or 8 entries a pass and would stream it several times).  K- and
-        // I-quant blobs stay on the decode kernels: the prompt kernel's decoders read those formats byte by byte and are slower.
+        // blob for the whole window; the decode kernels take 4 or 8 entries a pass and would stream it several times).  Q6_K blobs
+        // stay on the decode kernels, where a shared expert is faster at 64 tokens too: the prompt kernel reads that format byte
+        // by byte.  I-quant ones stay with them; that kernel's IQ1_M decoder has not been timed on a single blob.
         rc = BSX_E_TYPE;
         if (T >= 16 && status != nullptr && d->shared_layout.gu_type == kTypeNVFP4 && bsx_experts_prefill_group_scratch_bytes(&d->shared_layout, T, T) != 0) {
             const void* blob1[1] = {reinterpret_cast<const void*>((uintptr_t) d->shared_blob)};
