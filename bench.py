@@ -500,10 +500,11 @@ def decode_line(args, w, T, r, world=1):
                             " (routed + shared experts; the stage's CUDA events also span the one-block kernel that lists the passes)", "achieved": achieved, "peak": pk["hbm"],
                             "unit": "GB/s", "frac": achieved / pk["hbm"], "peak_source": pk["source"],
                             # dram__bytes_read.sum + dram__bytes_write.sum of one gate/up launch of this workload at 64 tokens (seeded, so the same
-                            # experts every run), from the ncu capture summarised in profiles/nvf4_stream_kernel_c1_t64.md; not measured by this run
-                            "traffic": ((450112000 if use_packed else 451744256) if (T == 64 and w.key == "c1") else None),
-                            "traffic_source": ("dram__bytes_read.sum + dram__bytes_write.sum of one launch, ncu capture of source revision b1578ff "
-                                               "(profiles/nvf4_stream_kernel_c1_t64.md); per launch on the same workload, not measured by this run"),
+                            # experts every run), from the ncu captures summarised in profiles/ (nvf4_stream_kernel_c1_t64.md, blk_mma_kernel_c1_t64.md);
+                            # not measured by this run
+                            "traffic": ((449978368 if use_packed else 450037248) if (T == 64 and w.key == "c1") else None),
+                            "traffic_source": ("dram__bytes_read.sum + dram__bytes_write.sum of one launch, ncu capture of source revision bb77e4a "
+                                               "(profiles/nvf4_stream_kernel_c1_t64.md, blk_mma_kernel_c1_t64.md); per launch on the same workload, not measured by this run"),
                             "algorithmic_bytes_per_launch": r["gu_bytes"], "kernel_ms": gu_ms, "frac_of_nominal_8TBs": achieved / 8000.0}
         line["stage_ms"] = r["stage_ms"]
     else:
