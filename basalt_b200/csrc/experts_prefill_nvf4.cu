@@ -21,6 +21,7 @@
 // rows gathered by cp.async and MMAs issued under `lane == 0`, 4.59 with bulk copies, 3.52 with the issue under elect.sync too
 // (tc5.cuh); its down product 3.80 -> 2.33 (256 instead of 128 rows an item) -> 1.87.
 // With n_ff <= 512 the down product runs as prefill_down_resident_kernel instead (the tile's rows stay in shared memory).
+#include <algorithm>
 #include <atomic>
 #include <cuda_fp16.h>
 
@@ -55,11 +56,11 @@ struct GeoQ {
     static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((uint32_t) (256 >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
 };
 
-// a 128-row tile of one expert with everything the kernels need about it (blob 0: held elsewhere)
+// a 128-row tile of one expert with everything the kernels need about it
 struct __align__(16) TileRec {
     unsigned long long blob;
     int row0, rows;
-    int64_t base;          // units (of atoms) before this tile's in the tile images, see image_block
+    int64_t base;          // units (of atoms) before this tile's in its slab's tile images, see image_block
     int64_t pad;
 };
 
@@ -68,23 +69,29 @@ struct __align__(16) TileRec {
 // codes, 128-byte swizzled], so that a stage of a tile is one bulk copy and a tile with few rows is a short one.  A tile takes
 // `units` = ceil(rows / 8) + 2 KB per (chunk, term); rows and scale words past its last row are never written (each only
 // reaches its own accumulator row, which is not stored).
+constexpr int kMaxUnits = 128 / 8 + 2;
 __host__ __device__ __forceinline__ int tile_units(int rows) { return (rows + 7) / 8 + 2; }
 __device__ __forceinline__ size_t image_block(const TileRec& r, int n_chunk, int c, int t) {
     return ((size_t) r.base * n_chunk * kTermsF + (size_t) (c * kTermsF + t) * tile_units(r.rows)) * 1024;
 }
+
 // units that cap_rows rows in cap_tiles tiles can take
 __host__ __device__ inline int64_t image_units(int64_t cap_rows, int64_t cap_tiles) { return cap_rows / 8 + 3 * cap_tiles; }
 
-// One block: the units are a running sum over the tiles.  items (optional): the tiles' rows as passes of up to pass_entries rows, for
-// the decode stream.
+// The tile list without the tiles of experts held elsewhere, cut into slabs of slab_units units: slab s is the tiles
+// slab_first[s] .. slab_first[s + 1] - 1, those whose units before them are s slabs' worth, so a slab's images end at most one tile
+// past slab_units.  One block; a scan carries units and places together.  items (optional): instead of tiles, the rows as passes of
+// up to pass_entries rows for the decode stream.  Tiles that overlap (no dispatch makes them) and exceed the room are left out and
+// set the status word.
 __global__ void __launch_bounds__(1024) tile_records_kernel(const int32_t* __restrict__ tiles, const int32_t* __restrict__ n_tiles,
                                                             const int32_t* __restrict__ off, const unsigned long long* __restrict__ blob_table,
-                                                            TileRec* __restrict__ recs, int64_t cap_tiles, int64_t cap_units, int32_t* status,
-                                                            PassRec* __restrict__ items, int* __restrict__ n_items, int pass_entries) {
+                                                            int64_t cap_tiles, TileRec* __restrict__ recs, int64_t cap_recs, int32_t* __restrict__ slab_first, int n_slabs,
+                                                            int64_t slab_units, PassRec* __restrict__ items, int* __restrict__ n_items, int64_t cap_items, int pass_entries,
+                                                            int32_t* status) {
     __shared__ unsigned long long sh[32];
+    constexpr unsigned long long kLow = (1ull << 36) - 1;               // units | places << 36
     const int64_t n = min(cap_tiles, (int64_t) *n_tiles);
-    int64_t at = 0;
-    int passes = 0;
+    int64_t at = 0, placed = 0;
     for (int64_t t0 = 0; t0 < n; t0 += 1024) {
         const int64_t t = t0 + threadIdx.x;
         TileRec r = {0ull, 0, 0, 0, 0};
@@ -92,39 +99,49 @@ __global__ void __launch_bounds__(1024) tile_records_kernel(const int32_t* __res
             const int expert = tiles[2 * t], row0 = tiles[2 * t + 1];
             r.blob = blob_table[expert];
             r.row0 = row0;
-            r.rows = min(128, off[expert + 1] - row0);
+            r.rows = r.blob != 0ull ? max(0, min(128, off[expert + 1] - row0)) : 0;
         }
         const int u = r.rows > 0 ? tile_units(r.rows) : 0;
-        const int np = items && r.rows > 0 && r.blob != 0ull ? (r.rows + pass_entries - 1) / pass_entries : 0;
+        const int places = items ? (r.rows + pass_entries - 1) / pass_entries : (r.rows > 0 ? 1 : 0);
         unsigned long long total = 0;
-        const unsigned long long before = block_excl_sum<unsigned long long>((unsigned long long) u | ((unsigned long long) np << 32), &total, sh);
-        r.base = at + (int64_t) (before & 0xFFFFFFFFull);
-        for (int p = 0; p < np; ++p) {
-            PassRec q;
-            q.blob = r.blob;
-            q.eb = r.row0 + p * pass_entries;
-            q.ntok = min(pass_entries, r.rows - p * pass_entries);
-            items[passes + (int) (before >> 32) + p] = q;
-        }
-        at += (int64_t) (total & 0xFFFFFFFFull);
-        passes += (int) (total >> 32);
-        if (t < n) {
-            if (r.rows <= 0 || r.base + u > cap_units) {      // no rows; or tiles that overlap, which no dispatch makes
-                if (r.rows > 0) atomicOr(status, 1);
-                r.blob = 0ull;
-                r.rows = 0;
+        const unsigned long long before = block_excl_sum<unsigned long long>((unsigned long long) u | ((unsigned long long) places << 36), &total, sh);
+        const int64_t units = at + (int64_t) (before & kLow), place = placed + (int64_t) (before >> 36);
+        at += (int64_t) (total & kLow);
+        placed += (int64_t) (total >> 36);
+        if (places == 0) continue;
+        if (items) {
+            for (int p = 0; p < places; ++p) {
+                PassRec q;
+                q.blob = r.blob;
+                q.eb = r.row0 + p * pass_entries;
+                q.ntok = min(pass_entries, r.rows - p * pass_entries);
+                if (place + p < cap_items) items[place + p] = q;
             }
-            recs[t] = r;
+            continue;
         }
+        const int64_t slab = units / slab_units, next = (units + u) / slab_units;
+        r.base = units - slab * slab_units;
+        if (place < cap_recs) recs[place] = r;
+        if (next > slab && next <= n_slabs) slab_first[next] = (int) min(place + 1, cap_recs);   // u <= slab_units: at most one slab begins here
     }
-    if (items && threadIdx.x == 0) *n_items = passes;
+    const int64_t room = items ? cap_items : cap_recs;
+    if (threadIdx.x == 0) {
+        if (placed > room || (!items && at > n_slabs * slab_units)) atomicOr(status, 1);
+        if (items) *n_items = (int) min(placed, room);
+        else slab_first[0] = 0;
+    }
+    if (items) return;
+    for (int64_t s = min(at / slab_units, (int64_t) n_slabs) + 1 + threadIdx.x; s <= n_slabs; s += 1024) slab_first[s] = (int) min(placed, room);
 }
+
+// The first slab's begin is not read: the image kernels, whose blocks live a few microseconds, need not wait for it before their record.
+__device__ __forceinline__ int first_tile(const int32_t* from) { return from ? *from : 0; }
 
 struct PrefillFArgs {
     bsx_expert_layout L;
-    const TileRec* recs;                     // [n_tiles]
+    const TileRec* recs;                     // every tile of the call
+    const int32_t *from, *to;                // the tiles of this launch, *from .. *to - 1 (from: null for 0)
     const int32_t* src;                      // [rows] token of each row
-    const int32_t* n_tiles;
     const uint8_t* img;                      // tile images of this product's A operand
     const float* inv;
     float* h;                                // [rows + 128][I] fp32 SwiGLU output
@@ -213,14 +230,13 @@ __global__ void __launch_bounds__(256) prefill_images_kernel(const void* __restr
 // token images -> tile images of the gate/up product.  Block = one (tile, chunk): every row's four 128-byte code runs move in
 // 16-byte pieces (eight lanes a run), the scale words are transposed through shared memory.  Bound: HBM writes of 2.25 bytes a
 // value (180,224 rows x 2048: 830 MB); the stores are streaming, so that the token images they are read from stay in L2 (247 -> 215 us).
-__global__ void __launch_bounds__(256) tile_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ n_tiles, int tile0,
+__global__ void __launch_bounds__(256) tile_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ from, const int32_t* __restrict__ to, int tile0,
                                                           const int32_t* __restrict__ src, const uint8_t* __restrict__ codes, const uint8_t* __restrict__ sfs, int64_t K,
                                                           uint8_t* __restrict__ img) {
     __shared__ __align__(16) uint32_t sf[kTermsF * kSFQ / 4];
-    const int tile = tile0 + blockIdx.y;
-    if (tile >= *n_tiles) return;
+    const int tile = first_tile(from) + tile0 + blockIdx.y;
+    if (tile >= *to) return;
     const TileRec r = recs[tile];
-    if (r.blob == 0ull) return;
     const int c = blockIdx.x, n_chunk = gridDim.x;
     uint8_t* out = img + image_block(r, n_chunk, c, 0);
     const size_t term_bytes = (size_t) tile_units(r.rows) * 1024;
@@ -260,12 +276,12 @@ __global__ void __launch_bounds__(256) tile_images_kernel(const TileRec* __restr
 // stays in registers between the row's maximum and its codes (n_ff <= 512: 205 -> 174 us for 180,224 rows of 512); 0 reads the row
 // twice (four sub-blocks in registers were slower there: 274 -> 340 us for 73,728 rows of 2048).
 template <int NIT>
-__global__ void __launch_bounds__(256) h_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ n_tiles, const float* __restrict__ h, int64_t K,
+__global__ void __launch_bounds__(256) h_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ from, const int32_t* __restrict__ to, const float* __restrict__ h, int64_t K,
                                                        uint8_t* __restrict__ img, float* __restrict__ inv) {
-    const int tile = blockIdx.x >> 4, row = (blockIdx.x & 15) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (tile >= *n_tiles) return;
+    const int tile = first_tile(from) + (int) (blockIdx.x >> 4), row = (blockIdx.x & 15) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (tile >= *to) return;
     const TileRec r = recs[tile];
-    if (r.blob == 0ull || row >= r.rows) return;
+    if (row >= r.rows) return;
     const int64_t i = r.row0 + row;
     const int n_sb = (int) (K >> 4), n_chunk = (int) (K >> 8);
     float amax = 0.f;
@@ -363,7 +379,8 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_chunk = (int) ((MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff) >> 8);
     const int n_n = (int) (MODE == QMODE_GU ? a.L.n_ff / 128 : a.L.n_embd / 256);   // items per row tile: 128 neurons, or 256 down rows
-    const int n_items = *a.n_tiles * n_n;
+    const TileRec* recs = a.recs + first_tile(a.from);
+    const int n_items = (*a.to - first_tile(a.from)) * n_n;
     const PackedGeom geo = packed_geom(a.L.n_embd, a.L.n_ff);
 
     if (threadIdx.x == 0) {
@@ -383,13 +400,14 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
     const uint32_t sbase = smem_u32(smem);
     bool ok = true;
 
-    // items of experts held elsewhere are skipped by every role alike
+    // No record in the list has a null blob.  The loaders and the epilogue test for it all the same: without these tests, which hold a role
+    // back until its record is there, the gate/up product takes 369 us instead of 330 (6000 tokens of the 2048 x 512 layer), with
+    // or without an offset in front of the list; why was not found.
     if (warp == 0) {
         // ---- MMA issuer
         if (elect_one()) {
             uint32_t kb = 0, ti = 0;
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                if (a.recs[item / n_n].blob == 0ull) continue;
                 ok = mbar_wait(acc_empty, (ti & 1u) ^ 1u);
                 if (!ok) break;
                 for (int c = 0; c < n_chunk && ok; ++c, ++kb) {
@@ -433,8 +451,8 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
             uint32_t kb = 0;
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
                 const int tile = item / n_n, n = item - tile * n_n;
-                const unsigned long long bp = a.recs[tile].blob;
-                if (bp == 0ull) continue;
+                const unsigned long long bp = recs[tile].blob;
+                if (bp == 0ull) continue;          // none is; see above
                 const uint8_t* blob = reinterpret_cast<const uint8_t*>(bp);
                 const size_t mat = (size_t) n_chunk * kBlockF;             // a 128-row block over all of K
                 const uint8_t* b0 = MODE == QMODE_GU ? blob + geo.gate + n * mat : blob + geo.down + 2 * n * mat;
@@ -460,7 +478,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
         if (elect_one()) {
             uint32_t ka = 0;
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const TileRec r = a.recs[item / n_n];
+                const TileRec r = recs[item / n_n];
                 if (r.blob == 0ull) continue;
                 const uint32_t bytes = (uint32_t) tile_units(r.rows) * 1024u;
                 const uint8_t* g = a.img + image_block(r, n_chunk, 0, 0);
@@ -485,7 +503,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
         uint32_t ti = 0;
         for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
             const int tile = item / n_n, n = item - tile * n_n;
-            const TileRec r = a.recs[tile];
+            const TileRec r = recs[tile];
             if (r.blob == 0ull) continue;
             const bool row_live = p < r.rows;
             const float* tail = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(r.blob) + geo.tail);
@@ -566,7 +584,8 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_nb = (int) (a.L.n_embd / 128);            // blocks of 128 down rows = stages per tile
-    const int n_tiles = *a.n_tiles;
+    const TileRec* recs = a.recs + first_tile(a.from);
+    const int n_tiles = *a.to - first_tile(a.from);
     const PackedGeom geo = packed_geom(a.L.n_embd, a.L.n_ff);
 
     if (threadIdx.x == 0) {
@@ -588,7 +607,6 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
         if (elect_one()) {
             uint32_t ti = 0, nbc = 0;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                if (a.recs[tile].blob == 0ull) continue;
                 ok = mbar_wait(a_full, ti & 1u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -634,9 +652,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
         if (elect_one()) {
             uint32_t nbc = 0;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                const unsigned long long bp = a.recs[tile].blob;
-                if (bp == 0ull) continue;
-                const uint8_t* down = reinterpret_cast<const uint8_t*>(bp) + geo.down;
+                const uint8_t* down = reinterpret_cast<const uint8_t*>(recs[tile].blob) + geo.down;
                 for (int nb = 0; nb < n_nb; ++nb, ++nbc) {
                     const uint32_t s = nbc & 1u;
                     ok = mbar_wait(&b_empty[s], ((nbc >> 1) & 1u) ^ 1u);
@@ -653,8 +669,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
         if (elect_one()) {
             uint32_t ti = 0;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                const TileRec r = a.recs[tile];
-                if (r.blob == 0ull) continue;
+                const TileRec r = recs[tile];
                 ok = mbar_wait(a_empty, (ti & 1u) ^ 1u);
                 if (!ok) break;
                 const uint32_t bytes = (uint32_t) tile_units(r.rows) * 1024u, bar = smem_u32(a_full);
@@ -673,8 +688,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_down_resident_kernel(Pre
         const bool wide = (reinterpret_cast<uintptr_t>(a.dm) & 31) == 0;
         uint32_t nbc = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            const TileRec r = a.recs[tile];
-            if (r.blob == 0ull) continue;
+            const TileRec r = recs[tile];
             const bool row_live = p < r.rows;
             const float* tail = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(r.blob) + geo.tail);
             const float sd = row_live ? tail[2] * a.inv[r.row0 + p] : 0.f;
@@ -741,61 +755,100 @@ int32_t launch_q(const PrefillFArgs& a, cudaStream_t st) {
 
 using namespace bsx;
 
-// Rows an expert, on average over the call, up to which the decode stream takes it.  Whole layer, stream against tiles: 2048 x 512 with
+// Rows an expert, on average over the call, up to which the decode stream takes it.  Whole layer, bf16 rows, back to back, stream against tiles: 2048 x 512 with
 // 512 + 1 experts at 1.4 rows an expert 207 : 310 us, 16.7 338 : 498, 32 443 : 547, 47 567 : 604; 5120 x 2304 with 384 + 1 at 14
 // rows 1500 : 2411, 27 2103 : 2780; 7168 x 2048 with 256 + 1 at 17.5 rows 1473 : 2203, 35 2112 : 2437.
 constexpr int64_t kShortRows = 48;
 
-// the tiles that rows of up to 1024 experts can make
-static int64_t prefill_cap_tiles(int64_t cap_rows) { return cap_rows < 1025 ? cap_rows : cap_rows / 128 + 1025; }
+// Rows of up to 1025 experts make at most this many tiles.
+static int64_t prefill_cap_tiles(int64_t cap_rows, int64_t n_expert) { return std::min(cap_rows, cap_rows / 128 + std::min<int64_t>(n_expert, 1025)); }
 
-extern "C" size_t bsx_experts_prefill_packed_scratch_bytes(const bsx_expert_layout* L, int64_t n_tokens, int64_t cap_rows) {
-    if (!L || n_tokens < 0 || cap_rows < 0 || !bsx_expert_packed_bytes(L)) return 0;
-    const size_t H = (size_t) L->n_embd, I = (size_t) L->n_ff, R = (size_t) cap_rows + 128;
-    const size_t units = (size_t) image_units(cap_rows, prefill_cap_tiles(cap_rows));
-    return al256q((size_t) n_tokens * kTermsF * H / 2) + al256q((size_t) n_tokens * kTermsF * H / 16) + al256q((size_t) n_tokens * 4) + al256q(R * I * 4) +
-           units * 1024 * kTermsF * (H / 256 + I / 256) + al256q(R * 4) + al256q(((size_t) cap_rows / 128 + 1025) * sizeof(TileRec)) + 256;
+// Where a call's buffers lie in its scratch, and the route that its numbers choose.
+struct PrefillCarve {
+    bool stream;                       // few rows an expert: the decode stream
+    int64_t cap_recs, cap_items, slab_units;
+    int n_slabs;
+    size_t xcodes, xsf, xinv, h, img, hcodes, hsf, hinv, recs, slabs, items, n_items, bytes;
+};
+// n_held of the n_expert experts have blobs here.  Where that is not all of them, the tile images have room for twice an even share
+// of the rows, and what a skewed routing sends beyond it is done in further slabs over the same room (kernels of a slab without
+// tiles return at once).
+static PrefillCarve prefill_carve(const bsx_expert_layout& L, int64_t n_tokens, int64_t cap_rows, int64_t n_expert, int64_t n_held) {
+    PrefillCarve c = {};
+    const int64_t H = L.n_embd, I = L.n_ff;
+    c.stream = cap_rows <= kShortRows * n_expert && n_tokens <= 0x7FFFFFFF;
+    c.cap_recs = prefill_cap_tiles(cap_rows, n_held);
+    c.cap_items = cap_rows / kPassEntries + c.cap_recs;
+    const int64_t all = image_units(cap_rows, c.cap_recs);
+    const int64_t share = n_held < n_expert ? std::min(cap_rows, (2 * cap_rows * n_held + n_expert - 1) / n_expert) : cap_rows;
+    c.slab_units = std::max<int64_t>(kMaxUnits, std::min(all, image_units(share, prefill_cap_tiles(share, n_held))));
+    c.n_slabs = (int) ((all + c.slab_units - 1) / c.slab_units);
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t r = at;
+        at += al256q(bytes);
+        return r;
+    };
+    c.xcodes = take((size_t) n_tokens * kTermsF * H / 2);
+    c.xsf = take((size_t) n_tokens * kTermsF * H / 16);
+    c.xinv = take((size_t) n_tokens * 4);
+    c.h = take((size_t) (cap_rows + 128) * I * 4);
+    if (c.stream) {
+        c.hcodes = take((size_t) cap_rows * kTermsF * I / 2);
+        c.hsf = take((size_t) cap_rows * kTermsF * I / 16);
+        c.items = take((size_t) c.cap_items * sizeof(PassRec));
+        c.n_items = take(4);
+    } else {
+        at = (at + 4095) & ~(size_t) 4095;
+        c.img = take((size_t) (c.slab_units + kMaxUnits) * 1024 * kTermsF * ((H + I) / 256));
+        c.recs = take((size_t) c.cap_recs * sizeof(TileRec));
+        c.slabs = take((size_t) (c.n_slabs + 1) * 4);
+    }
+    c.hinv = take((size_t) (cap_rows + 128) * 4);
+    c.bytes = at;
+    return c;
 }
 
-extern "C" int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, const unsigned long long* blob_table, const int32_t* off,
-                                              const int32_t* src, const int32_t* tiles, const int32_t* n_tiles, int64_t cap_tiles, int64_t cap_rows,
-                                              const void* x, int32_t x_kind, int64_t n_tokens, int32_t n_expert, void* scratch, float* dm, int32_t* status,
-                                              void* stream) {
+extern "C" size_t bsx_experts_prefill_packed_held_scratch_bytes(const bsx_expert_layout* L, int64_t n_tokens, int64_t cap_rows, int32_t n_expert, int32_t n_held) {
+    if (!L || n_tokens < 0 || cap_rows < 0 || n_expert < 1 || n_held < 0 || n_held > n_expert || !bsx_expert_packed_bytes(L)) return 0;
+    return prefill_carve(*L, n_tokens, cap_rows, n_expert, n_held).bytes;
+}
+
+// the most that any number of experts needs: the stream's for all of them, the tiles' for the largest number that goes to tiles
+extern "C" size_t bsx_experts_prefill_packed_scratch_bytes(const bsx_expert_layout* L, int64_t n_tokens, int64_t cap_rows) {
+    if (!L || n_tokens < 0 || cap_rows < 0 || !bsx_expert_packed_bytes(L)) return 0;
+    const int64_t many = std::max<int64_t>(1025, (cap_rows + kShortRows - 1) / kShortRows);
+    const int64_t tiled = n_tokens > 0x7FFFFFFF ? 1025 : std::min<int64_t>(1025, (cap_rows - 1) / kShortRows);
+    const size_t a = prefill_carve(*L, n_tokens, cap_rows, many, many).bytes;
+    return tiled < 1 ? a : std::max(a, prefill_carve(*L, n_tokens, cap_rows, tiled, tiled).bytes);
+}
+
+extern "C" int32_t bsx_experts_prefill_packed_held(const bsx_expert_layout* layout, const unsigned long long* blob_table, const int32_t* off,
+                                                   const int32_t* src, const int32_t* tiles, const int32_t* n_tiles, int64_t cap_tiles, int64_t cap_rows,
+                                                   const void* x, int32_t x_kind, int64_t n_tokens, int32_t n_expert, int32_t n_held, void* scratch, float* dm,
+                                                   int32_t* status, void* stream) {
     if (!stream) return BSX_E_STREAM;
     if (!layout || !blob_table || !off || !src || !tiles || !n_tiles || !aligned(x, 16) || !aligned(scratch, 256) || !aligned(dm, 16) || !status)
         return BSX_E_POINTER;
     if (!bsx_expert_packed_bytes(layout)) return BSX_E_TYPE;
     if (x_kind != BSX_X_F32 && x_kind != BSX_X_BF16) return BSX_E_GEOMETRY;
-    if (cap_tiles < 0 || cap_rows < 0 || n_tokens < 0 || n_expert < 1) return BSX_E_GEOMETRY;
-    if (cap_tiles == 0 || n_tokens == 0 || cap_rows == 0) return BSX_OK;
+    if (cap_tiles < 0 || cap_rows < 0 || n_tokens < 0 || n_expert < 1 || n_held < 0 || n_held > n_expert) return BSX_E_GEOMETRY;
+    if (cap_tiles == 0 || n_tokens == 0 || cap_rows == 0 || n_held == 0) return BSX_OK;
+    if (cap_tiles > cap_rows / 128 + 1025) return BSX_E_LIMIT;      // more tiles than rows / 128 + experts can make
     const bsx_expert_layout& L = *layout;
     const cudaStream_t st = (cudaStream_t) stream;
-    const size_t H = (size_t) L.n_embd, I = (size_t) L.n_ff, R = (size_t) cap_rows + 128;
-    uint8_t* p = static_cast<uint8_t*>(scratch);
-    uint8_t* xcodes = p;
-    p += al256q((size_t) n_tokens * kTermsF * H / 2);
-    uint8_t* xsf = p;
-    p += al256q((size_t) n_tokens * kTermsF * H / 16);
-    float* xinv = reinterpret_cast<float*>(p);
-    p += al256q((size_t) n_tokens * 4);
-    float* h = reinterpret_cast<float*>(p);
-    p += al256q(R * I * 4);
-    const int64_t units = image_units(cap_rows, prefill_cap_tiles(cap_rows));
-    uint8_t* ximg = p;
-    p += (size_t) units * 1024 * kTermsF * (H / 256);
-    uint8_t* himg = p;
-    p += (size_t) units * 1024 * kTermsF * (I / 256);
-    float* hinv = reinterpret_cast<float*>(p);
-    p += al256q(R * 4);
-    TileRec* recs = reinterpret_cast<TileRec*>(p);
-    if (cap_tiles > cap_rows / 128 + 1025) return BSX_E_LIMIT;      // more tiles than rows / 128 + experts can make
+    const int64_t H = L.n_embd, I = L.n_ff;
+    const PrefillCarve c = prefill_carve(L, n_tokens, cap_rows, n_expert, n_held);
+    uint8_t* base = static_cast<uint8_t*>(scratch);
+    uint8_t *xcodes = base + c.xcodes, *xsf = base + c.xsf;
+    float *xinv = reinterpret_cast<float*>(base + c.xinv), *h = reinterpret_cast<float*>(base + c.h), *hinv = reinterpret_cast<float*>(base + c.hinv);
     // Few rows an expert: a tile's 128 tensor-core rows would be mostly padding and cost twice what the weights' bytes do, so the rows
     // go through the decode stream instead (experts_nvf4.cu: passes of 8 or 16 rows as the MMA's narrow side, bound by the weights).
-    if (cap_rows <= kShortRows * n_expert && n_tokens <= 0x7FFFFFFF) {
+    if (c.stream) {
         const int pass_entries = cap_rows > kPassEntries / 2 * n_expert ? 2 * kPassEntries : kPassEntries;
-        int* n_items = reinterpret_cast<int*>(ximg);                 // the images' room holds the pass list: at most a pass a row
-        PassRec* items = reinterpret_cast<PassRec*>(ximg + 256);
-        tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, recs, cap_tiles, units, status, items, n_items, pass_entries);
+        PassRec* items = reinterpret_cast<PassRec*>(base + c.items);
+        int* n_items = reinterpret_cast<int*>(base + c.n_items);
+        tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, cap_tiles, nullptr, 0, nullptr, 0, 1, items, n_items, c.cap_items, pass_entries, status);
         ExpertArgs e;
         e.L = L;
         e.grp_ptr = nullptr;
@@ -812,33 +865,49 @@ extern "C" int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, c
         e.out_kind = BSX_OUT_F32;
         e.n_x_rows = (int32_t) n_tokens;
         e.grid = nullptr;
-        return experts_packed_passes(e, items, n_items, pass_entries, xcodes, xsf, xinv, himg, himg + al256q((size_t) cap_rows * kTermsF * I / 2), hinv, status, st);
+        return experts_packed_passes(e, items, n_items, pass_entries, xcodes, xsf, xinv, base + c.hcodes, base + c.hsf, hinv, status, st);
     }
-    tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, recs, cap_tiles, units, status, nullptr, nullptr, 1);
+    uint8_t *ximg = base + c.img, *himg = ximg + (size_t) (c.slab_units + kMaxUnits) * 1024 * kTermsF * (H / 256);
+    TileRec* recs = reinterpret_cast<TileRec*>(base + c.recs);
+    int32_t* slabs = reinterpret_cast<int32_t*>(base + c.slabs);
+    tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, cap_tiles, recs, c.cap_recs, slabs, c.n_slabs, c.slab_units, nullptr, nullptr, 0, 1, status);
+    if (H <= 2048) prefill_images_kernel<128><<<(unsigned) ((n_tokens + 1) / 2), 256, 0, st>>>(x, x_kind, n_tokens, H, xcodes, xsf, xinv);
+    else prefill_images_kernel<256><<<(unsigned) n_tokens, 256, 0, st>>>(x, x_kind, n_tokens, H, xcodes, xsf, xinv);
     PrefillFArgs a;
     a.L = L;
     a.recs = recs;
     a.src = src;
-    a.n_tiles = n_tiles;
     a.h = h;
     a.dm = dm;
     a.status = status;
-    if (H <= 2048) prefill_images_kernel<128><<<(unsigned) ((n_tokens + 1) / 2), 256, 0, st>>>(x, x_kind, n_tokens, (int64_t) H, xcodes, xsf, xinv);
-    else prefill_images_kernel<256><<<(unsigned) n_tokens, 256, 0, st>>>(x, x_kind, n_tokens, (int64_t) H, xcodes, xsf, xinv);
-    for (int64_t t0 = 0; t0 < cap_tiles; t0 += 65535)
-        tile_images_kernel<<<dim3((unsigned) (H / 256), (unsigned) (cap_tiles - t0 < 65535 ? cap_tiles - t0 : 65535)), 256, 0, st>>>(recs, n_tiles, (int) t0, src, xcodes,
-                                                                                                                                     xsf, (int64_t) H, ximg);
-    a.img = ximg;
-    a.inv = xinv;
-    int32_t rc = launch_q<QMODE_GU>(a, st);
-    if (rc != BSX_OK) return rc;
-    const unsigned hb = (unsigned) (cap_tiles * 16);
-    if (I <= 512) h_images_kernel<1><<<hb, 256, 0, st>>>(recs, n_tiles, h, (int64_t) I, himg, hinv);
-    else h_images_kernel<0><<<hb, 256, 0, st>>>(recs, n_tiles, h, (int64_t) I, himg, hinv);
-    a.img = himg;
-    a.inv = hinv;
-    // n_ff <= 512: the tile's rows stay in shared memory and only weights stream
-    if (I == 256) return launch_down_resident<1>(a, st);
-    if (I == 512) return launch_down_resident<2>(a, st);
-    return launch_q<QMODE_DOWN>(a, st);
+    // a tile takes three units at least, and one may begin in a slab's last unit
+    const int64_t slab_tiles = std::min(std::min(cap_tiles, c.cap_recs), c.slab_units / 3 + 1);
+    for (int s = 0; s < c.n_slabs; ++s) {
+        a.from = s ? slabs + s : nullptr;
+        a.to = slabs + s + 1;
+        for (int64_t t0 = 0; t0 < slab_tiles; t0 += 65535)
+            tile_images_kernel<<<dim3((unsigned) (H / 256), (unsigned) std::min<int64_t>(slab_tiles - t0, 65535)), 256, 0, st>>>(recs, a.from, a.to, (int) t0, src, xcodes, xsf, H,
+                                                                                                                                 ximg);
+        a.img = ximg;
+        a.inv = xinv;
+        int32_t rc = launch_q<QMODE_GU>(a, st);
+        if (rc != BSX_OK) return rc;
+        const unsigned hb = (unsigned) (slab_tiles * 16);
+        a.img = himg;
+        if (I <= 512) h_images_kernel<1><<<hb, 256, 0, st>>>(recs, a.from, a.to, h, I, himg, hinv);
+        else h_images_kernel<0><<<hb, 256, 0, st>>>(recs, a.from, a.to, h, I, himg, hinv);
+        a.inv = hinv;
+        // n_ff <= 512: the tile's rows stay in shared memory and only weights stream
+        rc = I == 256 ? launch_down_resident<1>(a, st) : I == 512 ? launch_down_resident<2>(a, st) : launch_q<QMODE_DOWN>(a, st);
+        if (rc != BSX_OK) return rc;
+    }
+    return BSX_OK;
+}
+
+extern "C" int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, const unsigned long long* blob_table, const int32_t* off,
+                                              const int32_t* src, const int32_t* tiles, const int32_t* n_tiles, int64_t cap_tiles, int64_t cap_rows,
+                                              const void* x, int32_t x_kind, int64_t n_tokens, int32_t n_expert, void* scratch, float* dm, int32_t* status,
+                                              void* stream) {
+    return bsx_experts_prefill_packed_held(layout, blob_table, off, src, tiles, n_tiles, cap_tiles, cap_rows, x, x_kind, n_tokens, n_expert, n_expert, scratch, dm,
+                                           status, stream);
 }

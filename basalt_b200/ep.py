@@ -522,8 +522,11 @@ class EPPrefillMoELayer:
         self.tiles = torch.zeros((n // 128 + n_expert_total, 2), dtype=i32, device=dev)
         self.n_tiles = torch.zeros(1, dtype=i32, device=dev)
         self.dscratch = torch.empty(lib.bsx_dispatch_scratch_bytes(n, n_expert_total), dtype=u8, device=dev)
-        scr = lib.bsx_experts_prefill_packed_scratch_bytes if packed else lib.bsx_experts_prefill_scratch_bytes
-        self.scratch = torch.empty(scr(C.byref(layout), W * T, n), dtype=u8, device=dev)
+        def scr(tokens, rows, experts, held):
+            return (lib.bsx_experts_prefill_packed_held_scratch_bytes(C.byref(layout), tokens, rows, experts, held) if packed
+                    else lib.bsx_experts_prefill_scratch_bytes(C.byref(layout), tokens, rows))
+
+        self.scratch = torch.empty(scr(W * T, n, n_expert_total, El), dtype=u8, device=dev)
         self.dm = torch.empty((n, H), dtype=f32, device=dev)
         self.status = torch.zeros(1, dtype=i32, device=dev)
         self.y_part = torch.empty((W * T, H), dtype=f32, device=dev)
@@ -538,7 +541,7 @@ class EPPrefillMoELayer:
             nt = (T + 127) // 128
             self.s_tiles = torch.stack([torch.zeros(nt, dtype=i32), torch.arange(nt, dtype=i32) * 128], dim=1).contiguous().to(dev)
             self.s_ntiles = torch.tensor([nt], dtype=i32, device=dev)
-            self.s_scratch = torch.empty(scr(C.byref(layout), T, T), dtype=u8, device=dev)
+            self.s_scratch = torch.empty(scr(T, T, 1, 1), dtype=u8, device=dev)
             self.s_dm = torch.empty((T, H), dtype=f32, device=dev)
 
     def check_status(self):
@@ -568,9 +571,9 @@ class EPPrefillMoELayer:
         capi.check("bsx_dispatch", lib.bsx_dispatch(p(self.ids_all), n, k, self.E, p(self.cnt), p(self.off), p(self.slot), p(self.src), 128,
                                                      p(self.tiles), p(self.n_tiles), p(self.dscratch), st))
         if self.packed:
-            capi.check("bsx_experts_prefill_packed", lib.bsx_experts_prefill_packed(C.byref(L), p(self.blob_table), p(self.off), p(self.src), p(self.tiles),
-                                                                                    p(self.n_tiles), self.tiles.shape[0], n, p(self.x_all), kind, W * T, self.E,
-                                                                                    p(self.scratch), p(self.dm), p(self.status), st))
+            capi.check("bsx_experts_prefill_packed_held", lib.bsx_experts_prefill_packed_held(
+                C.byref(L), p(self.blob_table), p(self.off), p(self.src), p(self.tiles), p(self.n_tiles), self.tiles.shape[0], n, p(self.x_all), kind, W * T, self.E,
+                self.hi - self.lo, p(self.scratch), p(self.dm), p(self.status), st))
         else:
             capi.check("bsx_experts_prefill", lib.bsx_experts_prefill(C.byref(L), p(self.blob_table), p(self.off), p(self.src), p(self.tiles), p(self.n_tiles),
                                                                       self.tiles.shape[0], n, p(self.x_all), kind, W * T, p(self.scratch), p(self.dm),

@@ -600,7 +600,8 @@ class PrefillMoELayer:
         self.tiles = torch.zeros((n // 128 + self.EE, 2), dtype=i32, device=dev)
         self.n_tiles = torch.zeros(1, dtype=i32, device=dev)
         self.dscratch = torch.empty(capi.lib().bsx_dispatch_scratch_bytes(n, self.EE), dtype=torch.uint8, device=dev)
-        nscr = (capi.lib().bsx_experts_prefill_packed_scratch_bytes if packed else capi.lib().bsx_experts_prefill_scratch_bytes)(C.byref(layout), T, n)
+        nscr = (capi.lib().bsx_experts_prefill_packed_held_scratch_bytes(C.byref(layout), T, n, self.EE, self.EE) if packed
+                else capi.lib().bsx_experts_prefill_scratch_bytes(C.byref(layout), T, n))
         self.scratch = torch.empty(nscr, dtype=torch.uint8, device=dev)
         self.dm = torch.empty((n, layout.n_embd), dtype=f32, device=dev)
         self.status = torch.zeros(1, dtype=i32, device=dev)

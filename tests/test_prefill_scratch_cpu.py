@@ -1,0 +1,45 @@
+"""What the packed prompt call asks its caller to allocate: the exact size for a number of experts never exceeds the one that covers any
+number, short calls hold no tile images, and a rank that holds an eighth of the experts does not hold the images of all rows."""
+import ctypes as C
+import random
+
+import pytest
+
+from basalt_b200 import capi, moe
+from oracle import oracle as O
+
+
+def sizes(H, I, tokens, rows, experts, held):
+    L = moe.native_expert_layout(O.T_NVFP4, O.T_NVFP4, H, I)
+    lb = capi.lib()
+    return (lb.bsx_experts_prefill_packed_scratch_bytes(C.byref(L), tokens, rows),
+            lb.bsx_experts_prefill_packed_held_scratch_bytes(C.byref(L), tokens, rows, experts, held))
+
+
+def test_any_number_of_experts_is_covered(lib):
+    rng = random.Random(1)
+    for _ in range(3000):
+        T, k, E = int(2 ** rng.uniform(0, 17)), rng.randint(1, 12), rng.randint(1, 1100)
+        any_number, exact = sizes(256 * rng.randint(1, 28), 256 * rng.randint(1, 9), T, T * k, E, E)
+        assert 0 < exact <= any_number, (T, k, E)
+
+
+@pytest.mark.parametrize("T", [65, 256, 1300])
+def test_short_calls_hold_rows_not_images_of_tiles(lib, T):
+    H, I, rows = 7168, 2048, 9 * T
+    _, exact = sizes(H, I, T, rows, 257, 257)
+    row_buffers = T * (2.25 * H + 4) + rows * (4 * I + 2.25 * I + 4)          # FP4 terms of x, fp32 h and its FP4 terms
+    lists = (rows + 1025) * 64 + 128 * I * 4                                  # pass and tile records; the rows past the last tile
+    assert exact <= row_buffers + lists + 16 * 256
+
+
+def test_long_call_and_a_rank_with_an_eighth(lib):
+    H, I, T, k, E = 7168, 2048, 8192, 8, 256
+    rows = 8 * T * k
+    _, whole = sizes(H, I, 8 * T, rows, E, E)
+    _, eighth = sizes(H, I, 8 * T, rows, E, E // 8)
+    fixed = 8 * T * (2.25 * H + 4) + (rows + 128) * (4 * I + 4)
+    images = (rows + E * 24) * 2.25 * (H + I)                                  # of x and of h; a tile's: up to 24 rows more than its rows
+    assert whole <= fixed + 1.3 * images
+    assert eighth <= fixed + 0.25 * 1.3 * images + (1 << 20)
+    assert sizes(H, I, T, T, 8, 9)[1] == 0 and sizes(H, I, T, T, 0, 0)[1] == 0

@@ -21,7 +21,8 @@ SHORT16 = [0, 1, 8, 9, 15, 16, 17, 0, 130, 32, 33, 0, 0, 2, 0, 0]               
 SHORT8 = [0, 1, 7, 8, 9, 0, 17, 0, 0, 0, 0, 0, 0, 1, 0, 0]                       # 3 an expert: passes of 8
 
 
-def run(H, I, shift, counts, held_elsewhere=()):
+def run(H, I, shift, counts, held_elsewhere=(), n_held=None):
+    """n_held: through the entry that is told the number of experts held here, whose scratch is exact"""
     rng = np.random.default_rng(H * 3 + I)
     E = len(counts)
     Lo, blobs = make_expert_blobs(rng, min(E, 10), O.T_NVFP4, O.T_NVFP4, H, I)
@@ -35,7 +36,9 @@ def run(H, I, shift, counts, held_elsewhere=()):
     table = packed.data_ptr() + torch.arange(E, dtype=torch.int64, device="cuda") % len(blobs) * packed.shape[1]
     table[list(held_elsewhere)] = 0
     lb = capi.lib()
-    scratch = torch.full((lb.bsx_experts_prefill_packed_scratch_bytes(C.byref(L), T, n),), 0xFF, dtype=torch.uint8, device="cuda")
+    size = (lb.bsx_experts_prefill_packed_scratch_bytes(C.byref(L), T, n) if n_held is None
+            else lb.bsx_experts_prefill_packed_held_scratch_bytes(C.byref(L), T, n, E, n_held))
+    scratch = torch.full((size + 4096,), 0xFF, dtype=torch.uint8, device="cuda")
     raw = torch.full((n * H * 4 + 256,), 0xFF, dtype=torch.uint8, device="cuda")
     dm = raw[shift:shift + n * H * 4].view(torch.float32).view(n, H)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
@@ -43,13 +46,13 @@ def run(H, I, shift, counts, held_elsewhere=()):
     stream = moe._stream(None)
     torch.cuda.synchronize()
     for _ in range(2):          # again over the scratch that the first call left
-        capi.check("prefill packed", lb.bsx_experts_prefill_packed(C.byref(L), table.data_ptr(), o.data_ptr(), s.data_ptr(), t.data_ptr(), nt.data_ptr(),
-                                                                   len(tiles), n, xd.data_ptr(), capi.X_F32, T, E, scratch.data_ptr(), dm.data_ptr(),
-                                                                   status.data_ptr(), stream))
+        args = (C.byref(L), table.data_ptr(), o.data_ptr(), s.data_ptr(), t.data_ptr(), nt.data_ptr(), len(tiles), n, xd.data_ptr(), capi.X_F32, T, E)
+        rest = (scratch.data_ptr(), dm.data_ptr(), status.data_ptr(), stream)
+        capi.check("prefill packed", lb.bsx_experts_prefill_packed(*args, *rest) if n_held is None else lb.bsx_experts_prefill_packed_held(*args, n_held, *rest))
     torch.cuda.synchronize()
     assert int(status.item()) == 0
     got = dm.cpu().numpy()
-    assert (raw[:shift] == 0xFF).all() and (raw[shift + n * H * 4:] == 0xFF).all()
+    assert (raw[:shift] == 0xFF).all() and (raw[shift + n * H * 4:] == 0xFF).all() and (scratch[size:] == 0xFF).all()
     for e in range(E):
         rows = got[off[e]:off[e + 1]]
         if e in held_elsewhere:
@@ -73,3 +76,11 @@ MANY = [130, 500, 257] * 17                                                     
                                              (512, 256, SHORT8, (1, 6, 13)), (768, 768, SHORT8, (4,)), (256, 256, SHORT8, range(16)), (256, 256, TILES, range(10))])
 def test_experts_held_elsewhere(lib, cuda, H, I, counts, away):
     run(H, I, 0, counts, tuple(away))
+
+
+@pytest.mark.parametrize("H,I,counts,here", [(256, 256, TILES, (9,)), (512, 768, TILES, (9,)), (256, 512, TILES, (7, 9)), (512, 256, TILES, range(10)), (256, 768, MANY, range(34, 51)),
+                                             (256, 512, MANY, (50,)), (256, 256, MANY, range(51)), (512, 512, SHORT16, (8,)), (768, 768, SHORT8, (6, 8)), (256, 256, [49], (0,)),
+                                             (256, 512, [1, 120], (1,))])
+def test_rounds_over_the_room_of_an_even_share(lib, cuda, H, I, counts, here):
+    """rows that crowd onto the experts held here: more than twice an even share, so that the tile images take several rounds"""
+    run(H, I, 0, counts, tuple(e for e in range(len(counts)) if e not in here), len(tuple(here)))
