@@ -189,22 +189,33 @@ __global__ void __launch_bounds__(256) x_images_kernel(const void* __restrict__ 
     fp4_image_row<TPR>(x, kind, i < n_rows ? i : 0, K, i < n_rows, i, codes, sfs, inv, shf);
 }
 
-// rows of h that a pass list names: a block takes 256 / TPR of the list's pass_entries places at a time.  (Rows of experts held
-// elsewhere are in no pass and have never been written.)
+// rows of h that a pass list and a tile list name: a block takes 256 / TPR places of a pass (of pass_entries) or a tile (of 128) at a
+// time.  (Rows of experts held elsewhere are in neither and have never been written.)
 template <int TPR>
-__global__ void __launch_bounds__(256) pass_images_kernel(const float* __restrict__ h, const PassRec* __restrict__ items, const int* __restrict__ n_items, int pass_entries,
-                                                           int64_t K, uint8_t* __restrict__ codes, uint8_t* __restrict__ sfs, float* __restrict__ inv) {
+__global__ void __launch_bounds__(256) listed_images_kernel(const float* __restrict__ h, const PassRec* __restrict__ items, const int* __restrict__ n_items, int pass_entries,
+                                                             const TileRec* __restrict__ recs, const int32_t* __restrict__ slab, int64_t K, uint8_t* __restrict__ codes,
+                                                             uint8_t* __restrict__ sfs, float* __restrict__ inv) {
     __shared__ float shf[8];
-    constexpr int kRows = 256 / TPR;          // divides pass_entries: a block's places are one pass's
+    constexpr int kRows = 256 / TPR;          // divides both lengths: a block's places are one pass's or tile's
     pdl_wait();
     pdl_launch_dependents();
-    const int64_t n = (int64_t) *n_items * pass_entries;
+    const int64_t n_pass = (int64_t) *n_items * pass_entries, n = n_pass + (int64_t) slab[1] * 128;
     for (int64_t at = (int64_t) blockIdx.x * kRows; at < n; at += (int64_t) gridDim.x * kRows) {
-        const PassRec r = items[at / pass_entries];
-        const int j0 = (int) (at % pass_entries), j = j0 + (int) threadIdx.x / TPR;
-        if (j0 >= r.ntok) continue;           // the whole block's
-        const int row = r.eb + min(j, r.ntok - 1);
-        fp4_image_row<TPR>(h, BSX_X_F32, row, K, j < r.ntok, row, codes, sfs, inv, shf);
+        int row0, rows, j0;
+        if (at < n_pass) {
+            const PassRec r = items[at / pass_entries];
+            row0 = r.eb;
+            rows = r.ntok;
+            j0 = (int) (at % pass_entries);
+        } else {
+            const TileRec r = recs[(at - n_pass) / 128];
+            row0 = r.row0;
+            rows = r.rows;
+            j0 = (int) ((at - n_pass) % 128);
+        }
+        if (j0 >= rows) continue;             // the whole block's
+        const int j = j0 + (int) threadIdx.x / TPR, row = row0 + min(j, rows - 1);
+        fp4_image_row<TPR>(h, BSX_X_F32, row, K, j < rows, row, codes, sfs, inv, shf);
         __syncthreads();                      // shf
     }
 }
@@ -650,33 +661,33 @@ int32_t experts_grouped_packed(const ExpertArgs& a, int32_t* status, cudaStream_
     return wide ? launch_stream<FMODE_DOWN, kEntWide>(sa, st) : launch_stream<FMODE_DOWN, kEntNarrow>(sa, st);
 }
 
-// The same two products over a pass list that is there already, entry e = row e: x rows ent_tok[e], output row e.  xcodes .. xinv and
-// hcodes .. hinv: room for the images of n_x_rows rows of n_embd and of a.cap_entries rows of n_ff.
-int32_t experts_packed_passes(const ExpertArgs& a, const PassRec* items, const int* n_items, int pass_entries, uint8_t* xcodes, uint8_t* xsf, float* xinv,
-                              uint8_t* hcodes, uint8_t* hsf, float* hinv, int32_t* status, cudaStream_t st) {
+// The pieces of a short prompt (experts_prefill_nvf4.cu): images of all rows of x; of the rows of h that the lists name; and one product
+// over a pass list that is there already, entry e = row e: x rows ent_tok[e], output row e.
+void packed_x_images(const void* x, int kind, int64_t rows, int64_t K, uint8_t* codes, uint8_t* sfs, float* inv, cudaStream_t st) {
+    if (K <= 512) launch_k(x_images_kernel<32>, dim3((unsigned) ((rows + 7) / 8)), dim3(256), 0, st, x, kind, (int) rows, K, codes, sfs, inv);
+    else if (K <= 2048) launch_k(x_images_kernel<128>, dim3((unsigned) ((rows + 1) / 2)), dim3(256), 0, st, x, kind, (int) rows, K, codes, sfs, inv);
+    else launch_k(x_images_kernel<256>, dim3((unsigned) rows), dim3(256), 0, st, x, kind, (int) rows, K, codes, sfs, inv);
+}
+void packed_listed_images(const float* h, const PassRec* items, const int* n_items, int pass_entries, const TileRec* recs, const int32_t* slab, int64_t K, uint8_t* codes,
+                          uint8_t* sfs, float* inv, cudaStream_t st) {
+    const dim3 grid((unsigned) (8 * sm_count()));
+    if (K <= 512) launch_k(listed_images_kernel<32>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, slab, K, codes, sfs, inv);
+    else if (K <= 2048) launch_k(listed_images_kernel<128>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, slab, K, codes, sfs, inv);
+    else launch_k(listed_images_kernel<256>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, slab, K, codes, sfs, inv);
+}
+int32_t packed_pass_product(bool down, const ExpertArgs& a, const PassRec* items, const int* n_items, int pass_entries, const uint8_t* codes, const uint8_t* sfs,
+                            const float* inv, int32_t* status, cudaStream_t st) {
     StreamArgs sa;
     sa.e = a;
     sa.items = items;
     sa.n_items = n_items;
     sa.status = status;
     sa.early_weights = 0;
-    const int64_t H = a.L.n_embd, I = a.L.n_ff, rows = a.n_x_rows;
-    if (H <= 512) launch_k(x_images_kernel<32>, dim3((unsigned) ((rows + 7) / 8)), dim3(256), 0, st, a.x, (int) a.x_kind, (int) rows, H, xcodes, xsf, xinv);
-    else if (H <= 2048) launch_k(x_images_kernel<128>, dim3((unsigned) ((rows + 1) / 2)), dim3(256), 0, st, a.x, (int) a.x_kind, (int) rows, H, xcodes, xsf, xinv);
-    else launch_k(x_images_kernel<256>, dim3((unsigned) rows), dim3(256), 0, st, a.x, (int) a.x_kind, (int) rows, H, xcodes, xsf, xinv);
-    sa.codes = xcodes;
-    sa.sfs = xsf;
-    sa.inv = xinv;
-    const int32_t rc = pass_entries == kEntWide ? launch_stream<FMODE_GU, kEntWide>(sa, st) : launch_stream<FMODE_GU, kEntNarrow>(sa, st);
-    if (rc != BSX_OK) return rc;
-    const dim3 grid((unsigned) (8 * sm_count()));
-    if (I <= 512) launch_k(pass_images_kernel<32>, grid, dim3(256), 0, st, (const float*) a.h, items, n_items, pass_entries, I, hcodes, hsf, hinv);
-    else if (I <= 2048) launch_k(pass_images_kernel<128>, grid, dim3(256), 0, st, (const float*) a.h, items, n_items, pass_entries, I, hcodes, hsf, hinv);
-    else launch_k(pass_images_kernel<256>, grid, dim3(256), 0, st, (const float*) a.h, items, n_items, pass_entries, I, hcodes, hsf, hinv);
-    sa.codes = hcodes;
-    sa.sfs = hsf;
-    sa.inv = hinv;
-    return pass_entries == kEntWide ? launch_stream<FMODE_DOWN, kEntWide>(sa, st) : launch_stream<FMODE_DOWN, kEntNarrow>(sa, st);
+    sa.codes = codes;
+    sa.sfs = sfs;
+    sa.inv = inv;
+    if (down) return pass_entries == kEntWide ? launch_stream<FMODE_DOWN, kEntWide>(sa, st) : launch_stream<FMODE_DOWN, kEntNarrow>(sa, st);
+    return pass_entries == kEntWide ? launch_stream<FMODE_GU, kEntWide>(sa, st) : launch_stream<FMODE_GU, kEntNarrow>(sa, st);
 }
 
 }  // namespace bsx

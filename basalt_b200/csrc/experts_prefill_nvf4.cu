@@ -28,13 +28,17 @@
 #include "common.cuh"
 #include "experts.cuh"
 #include "nvf4.cuh"
+#include "pdl.cuh"
 #include "plan.cuh"
 #include "tc5.cuh"
 
 namespace bsx {
 
-int32_t experts_packed_passes(const ExpertArgs& a, const PassRec* items, const int* n_items, int pass_entries, uint8_t* xcodes, uint8_t* xsf, float* xinv,
-                              uint8_t* hcodes, uint8_t* hsf, float* hinv, int32_t* status, cudaStream_t st);
+void packed_x_images(const void* x, int kind, int64_t rows, int64_t K, uint8_t* codes, uint8_t* sfs, float* inv, cudaStream_t st);
+void packed_listed_images(const float* h, const PassRec* items, const int* n_items, int pass_entries, const TileRec* recs, const int32_t* slab, int64_t K, uint8_t* codes,
+                          uint8_t* sfs, float* inv, cudaStream_t st);
+int32_t packed_pass_product(bool down, const ExpertArgs& a, const PassRec* items, const int* n_items, int pass_entries, const uint8_t* codes, const uint8_t* sfs,
+                            const float* inv, int32_t* status, cudaStream_t st);
 
 namespace {
 
@@ -56,14 +60,6 @@ struct GeoQ {
     static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((uint32_t) (256 >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
 };
 
-// a 128-row tile of one expert with everything the kernels need about it
-struct __align__(16) TileRec {
-    unsigned long long blob;
-    int row0, rows;
-    int64_t base;          // units (of atoms) before this tile's in its slab's tile images, see image_block
-    int64_t pad;
-};
-
 // Tile images.  The activation rows a tile multiplies lie in dispatch order, in the form a stage has in shared memory: for each
 // (chunk of 256 columns, FP4 term) one run of [2 KB scale words, as tcgen05.cp reads them for 128 rows | 1 KB per eight rows of
 // codes, 128-byte swizzled], so that a stage of a tile is one bulk copy and a tile with few rows is a short one.  A tile takes
@@ -80,58 +76,87 @@ __host__ __device__ inline int64_t image_units(int64_t cap_rows, int64_t cap_til
 
 // The tile list without the tiles of experts held elsewhere, cut into slabs of slab_units units: slab s is the tiles
 // slab_first[s] .. slab_first[s + 1] - 1, those whose units before them are s slabs' worth, so a slab's images end at most one tile
-// past slab_units.  One block; a scan carries units and places together.  items (optional): instead of tiles, the rows as passes of
-// up to pass_entries rows for the decode stream.  Tiles that overlap (no dispatch makes them) and exceed the room are left out and
-// set the status word.
-__global__ void __launch_bounds__(1024) tile_records_kernel(const int32_t* __restrict__ tiles, const int32_t* __restrict__ n_tiles,
-                                                            const int32_t* __restrict__ off, const unsigned long long* __restrict__ blob_table,
-                                                            int64_t cap_tiles, TileRec* __restrict__ recs, int64_t cap_recs, int32_t* __restrict__ slab_first, int n_slabs,
-                                                            int64_t slab_units, PassRec* __restrict__ items, int* __restrict__ n_items, int64_t cap_items, int pass_entries,
-                                                            int32_t* status) {
+// past slab_units.  One block; a scan carries units and places together.  Tiles that overlap (no dispatch makes them) and exceed the
+// room are left out and set the status word.
+// items (optional, a short call): the rows become passes of up to pass_entries rows for the decode stream instead.  But a call that is
+// short by its average may still send most rows to a few experts, and the stream reads an expert's weights once a pass: tiles of more
+// than kCrowdedRows rows then are one slab of tiles, provided the passes they save outweigh what the tile kernels take in the
+// whole.  A tile costs the chip about as much as three passes (5120 x 2304 with 27 rows an expert: 7.0 and 2.4 us), and the tile
+// kernels come in rounds of sm_count items, of which a call pays one more than it fills (launches, the last item's latency).
+constexpr int kCrowdedRows = 64;
+struct RecordArgs {
+    const int32_t *tiles, *n_tiles, *off;
+    const unsigned long long* blob_table;
+    int64_t cap_tiles;
+    TileRec* recs;
+    int64_t cap_recs;
+    int32_t* slab_first;
+    int n_slabs;
+    int64_t slab_units;
+    PassRec* items;
+    int* n_items;
+    int64_t cap_items;
+    int pass_entries, tile_items, sm_count;      // tile_items: items of a tile's gate/up product
+    int32_t* status;
+};
+__global__ void __launch_bounds__(1024) tile_records_kernel(RecordArgs a) {
     __shared__ unsigned long long sh[32];
-    constexpr unsigned long long kLow = (1ull << 36) - 1;               // units | places << 36
-    const int64_t n = min(cap_tiles, (int64_t) *n_tiles);
-    int64_t at = 0, placed = 0;
-    for (int64_t t0 = 0; t0 < n; t0 += 1024) {
-        const int64_t t = t0 + threadIdx.x;
+    constexpr unsigned long long kLow = (1ull << 36) - 1;               // units or passes | tiles << 36
+    pdl_wait();
+    pdl_launch_dependents();
+    const int64_t n = min(a.cap_tiles, (int64_t) *a.n_tiles);
+    auto record = [&](int64_t t) {
         TileRec r = {0ull, 0, 0, 0, 0};
         if (t < n) {
-            const int expert = tiles[2 * t], row0 = tiles[2 * t + 1];
-            r.blob = blob_table[expert];
+            const int expert = a.tiles[2 * t], row0 = a.tiles[2 * t + 1];
+            r.blob = a.blob_table[expert];
             r.row0 = row0;
-            r.rows = r.blob != 0ull ? max(0, min(128, off[expert + 1] - row0)) : 0;
+            r.rows = r.blob != 0ull ? max(0, min(128, a.off[expert + 1] - row0)) : 0;
         }
-        const int u = r.rows > 0 ? tile_units(r.rows) : 0;
-        const int places = items ? (r.rows + pass_entries - 1) / pass_entries : (r.rows > 0 ? 1 : 0);
+        return r;
+    };
+    int tile_rows = 1;                                                   // from this many rows on a tile stays one
+    if (a.items) {
+        unsigned long long v = 0, total = 0;
+        for (int64_t t = threadIdx.x; t < n; t += 1024) {
+            const int rows = record(t).rows;
+            if (rows > kCrowdedRows) v += (unsigned long long) ((rows + 15) / 16) | (1ull << 36);
+        }
+        block_excl_sum<unsigned long long>(v, &total, sh);
+        const int64_t saved = (int64_t) (total & kLow) * a.tile_items, rounds = ((int64_t) (total >> 36) * a.tile_items + a.sm_count - 1) / a.sm_count;
+        tile_rows = saved > 3 * (int64_t) a.sm_count * (rounds + 1) ? kCrowdedRows + 1 : 129;
+    }
+    int64_t low = 0, placed = 0;
+    for (int64_t t0 = 0; t0 < n; t0 += 1024) {
+        TileRec r = record(t0 + threadIdx.x);
+        const bool tile = r.rows >= tile_rows;
+        const int passes = a.items && !tile ? (r.rows + a.pass_entries - 1) / a.pass_entries : 0, u = tile ? tile_units(r.rows) : 0;
         unsigned long long total = 0;
-        const unsigned long long before = block_excl_sum<unsigned long long>((unsigned long long) u | ((unsigned long long) places << 36), &total, sh);
-        const int64_t units = at + (int64_t) (before & kLow), place = placed + (int64_t) (before >> 36);
-        at += (int64_t) (total & kLow);
+        const unsigned long long before =
+            block_excl_sum<unsigned long long>((unsigned long long) (a.items ? passes : u) | ((unsigned long long) tile << 36), &total, sh);
+        const int64_t at = low + (int64_t) (before & kLow), place = placed + (int64_t) (before >> 36);
+        low += (int64_t) (total & kLow);
         placed += (int64_t) (total >> 36);
-        if (places == 0) continue;
-        if (items) {
-            for (int p = 0; p < places; ++p) {
-                PassRec q;
-                q.blob = r.blob;
-                q.eb = r.row0 + p * pass_entries;
-                q.ntok = min(pass_entries, r.rows - p * pass_entries);
-                if (place + p < cap_items) items[place + p] = q;
-            }
-            continue;
+        for (int p = 0; p < passes; ++p) {
+            PassRec q;
+            q.blob = r.blob;
+            q.eb = r.row0 + p * a.pass_entries;
+            q.ntok = min(a.pass_entries, r.rows - p * a.pass_entries);
+            if (at + p < a.cap_items) a.items[at + p] = q;
         }
-        const int64_t slab = units / slab_units, next = (units + u) / slab_units;
-        r.base = units - slab * slab_units;
-        if (place < cap_recs) recs[place] = r;
-        if (next > slab && next <= n_slabs) slab_first[next] = (int) min(place + 1, cap_recs);   // u <= slab_units: at most one slab begins here
+        if (!tile) continue;
+        const int64_t slab = a.items ? 0 : at / a.slab_units, next = a.items ? 0 : (at + u) / a.slab_units;
+        r.base = at - slab * a.slab_units;
+        if (place < a.cap_recs) a.recs[place] = r;
+        if (next > slab && next <= a.n_slabs) a.slab_first[next] = (int) min(place + 1, a.cap_recs);   // u <= slab_units: at most one slab begins here
     }
-    const int64_t room = items ? cap_items : cap_recs;
     if (threadIdx.x == 0) {
-        if (placed > room || (!items && at > n_slabs * slab_units)) atomicOr(status, 1);
-        if (items) *n_items = (int) min(placed, room);
-        else slab_first[0] = 0;
+        if (placed > a.cap_recs || low > (a.items ? a.cap_items : a.n_slabs * a.slab_units)) atomicOr(a.status, 1);
+        if (a.items) *a.n_items = (int) min(low, a.cap_items);
+        a.slab_first[0] = 0;
     }
-    if (items) return;
-    for (int64_t s = min(at / slab_units, (int64_t) n_slabs) + 1 + threadIdx.x; s <= n_slabs; s += 1024) slab_first[s] = (int) min(placed, room);
+    for (int64_t s = (a.items ? 0 : min(low / a.slab_units, (int64_t) a.n_slabs)) + 1 + threadIdx.x; s <= a.n_slabs; s += 1024)
+        a.slab_first[s] = (int) min(placed, a.cap_recs);
 }
 
 // The first slab's begin is not read: the image kernels, whose blocks live a few microseconds, need not wait for it before their record.
@@ -142,7 +167,8 @@ struct PrefillFArgs {
     const TileRec* recs;                     // every tile of the call
     const int32_t *from, *to;                // the tiles of this launch, *from .. *to - 1 (from: null for 0)
     const int32_t* src;                      // [rows] token of each row
-    const uint8_t* img;                      // tile images of this product's A operand
+    const uint8_t* img;                      // tile images of this product's A operand; or (GATHER) its rows' images
+    const uint8_t* sfs;                      // GATHER: the rows' scales
     const float* inv;
     float* h;                                // [rows + 128][I] fp32 SwiGLU output
     float* dm;                               // [rows][H] fp32
@@ -363,7 +389,10 @@ __device__ __forceinline__ void tmem_give_q(uint32_t tmem, int warp) {
     }
 }
 
-template <int MODE>
+// GATHER: the rows come from their own images instead (two warps of cp.async, warps 2 and 3), which takes no room that grows with the
+// tiles.  For the crowded tiles of short calls: 1300 rows on nine experts of the 7168 x 2048 layer take 1.43 ms so, 2.03 through the
+// stream alone.
+template <int MODE, bool GATHER>
 __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs a) {
     using G = GeoQ;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -379,13 +408,15 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_chunk = (int) ((MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff) >> 8);
     const int n_n = (int) (MODE == QMODE_GU ? a.L.n_ff / 128 : a.L.n_embd / 256);   // items per row tile: 128 neurons, or 256 down rows
+    if (GATHER) pdl_wait();
     const TileRec* recs = a.recs + first_tile(a.from);
     const int n_items = (*a.to - first_tile(a.from)) * n_n;
+    if (GATHER && n_items == 0) return;
     const PackedGeom geo = packed_geom(a.L.n_embd, a.L.n_ff);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kASlots; ++s) {
-            mbar_init(&a_full[s], 1);
+            mbar_init(&a_full[s], GATHER ? 64 : 1);
             mbar_init(&a_empty[s], 1);
         }
         for (int s = 0; s < kBStages; ++s) {
@@ -397,6 +428,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     const uint32_t tmem = tmem_take_q(tmem_slot, warp);
+    if (GATHER) pdl_launch_dependents();          // with tensor memory in hand
     const uint32_t sbase = smem_u32(smem);
     bool ok = true;
 
@@ -473,7 +505,64 @@ __global__ void __launch_bounds__(kThreadsQ, 1) prefill_nvf4_kernel(PrefillFArgs
             }
             if (!ok) atomicOr(a.status, 1);
         }
-    } else if (warp == 2) {
+    } else if (GATHER && (warp == 2 || warp == 3)) {
+        // ---- activation loaders, 64 rows each.  Lane = (16-byte piece c8, row r4 of four): rows r4 + 4 i of the warp's 64; scale words:
+        // lane = row, a word into each K-step's block.  Rows past the tile's last are left as they are.  A lane runs up to five slots
+        // ahead of its own landed copies (of eight: the tensor core can always go on) and arrives on a slot once they are visible.
+        const int64_t K = (int64_t) n_chunk * 256;
+        const int lw = warp - 2, c8 = lane & 7, r4 = lane >> 3;
+        uint32_t dsto[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r7 = 4 * h + r4;
+            dsto[h] = (uint32_t) (kSFQ + lw * 8 * 1024 + r7 * 128 + ((c8 ^ r7) << 4));
+        }
+        uint32_t issued = 0, arrived = 0;
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            const TileRec r = recs[item / n_n];
+            auto image_row = [&](int row) -> size_t {
+                const int i = r.row0 + min(row, r.rows - 1);
+                return (size_t) (MODE == QMODE_GU ? a.src[i] : i) * kTermsF;
+            };
+            const uint8_t *crow[16], *srow[2];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) crow[i] = a.img + image_row(64 * lw + 4 * i + r4) * (size_t) (K >> 1) + c8 * 16;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) srow[j] = a.sfs + image_row(64 * lw + 32 * j + lane) * (size_t) (K >> 4);
+            const int live = (r.rows - 64 * lw - r4 + 3) >> 2;         // this lane's rows are i < live
+            for (int c = 0; c < n_chunk && ok; ++c)
+#pragma unroll 1
+                for (int t = 0; t < kTermsF; ++t) {
+                    const uint32_t s = issued % kASlots;
+                    ok = mbar_wait(&a_empty[s], ((issued / kASlots) & 1u) ^ 1u);
+                    if (!ok) break;
+                    const uint32_t slot = sbase + (uint32_t) (G::kOffA + s * kSlotQ);
+                    const size_t co = (size_t) t * (size_t) (K >> 1) + (size_t) c * 128, so = (size_t) t * (size_t) (K >> 4) + (size_t) c * 16;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (i < live) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(slot + (uint32_t) ((i >> 1) * 1024) + dsto[i & 1]), "l"(crow[i] + co) : "memory");
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        if (64 * lw + 32 * j + lane < r.rows)
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(slot + (uint32_t) (k * 512 + lane * 16 + (2 * lw + j) * 4)), "l"(srow[j] + so + 4 * k)
+                                             : "memory");
+                    asm volatile("cp.async.commit_group;\n" ::: "memory");
+                    ++issued;
+                    if (issued - arrived > 5) {
+                        asm volatile("cp.async.wait_group 5;\n" ::: "memory");
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                        mbar_arrive(&a_full[arrived % kASlots]);
+                        ++arrived;
+                    }
+                }
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        for (; arrived < issued; ++arrived) mbar_arrive(&a_full[arrived % kASlots]);
+        if (!ok) atomicOr(a.status, 1);
+    } else if (!GATHER && warp == 2) {
         // ---- activation loader: one lane, one copy a slot
         if (elect_one()) {
             uint32_t ka = 0;
@@ -736,17 +825,18 @@ int32_t launch_down_resident(const PrefillFArgs& a, cudaStream_t st) {
 
 size_t al256q(size_t v) { return (v + 255) & ~(size_t) 255; }
 
-template <int MODE>
+template <int MODE, bool GATHER>
 int32_t launch_q(const PrefillFArgs& a, cudaStream_t st) {
     static std::atomic<bool> configured[64];   // per device; threads of different devices call concurrently
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(prefill_nvf4_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GeoQ::kSmem);
+        const cudaError_t e = cudaFuncSetAttribute(prefill_nvf4_kernel<MODE, GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GeoQ::kSmem);
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
-    prefill_nvf4_kernel<MODE><<<(unsigned) sm_count(), kThreadsQ, GeoQ::kSmem, st>>>(a);
+    if (GATHER) launch_k(prefill_nvf4_kernel<MODE, GATHER>, dim3((unsigned) sm_count()), dim3(kThreadsQ), GeoQ::kSmem, st, a);
+    else prefill_nvf4_kernel<MODE, GATHER><<<(unsigned) sm_count(), kThreadsQ, GeoQ::kSmem, st>>>(a);
     return launch_status();
 }
 
@@ -782,7 +872,7 @@ static PrefillCarve prefill_carve(const bsx_expert_layout& L, int64_t n_tokens, 
     const int64_t all = image_units(cap_rows, c.cap_recs);
     const int64_t share = n_held < n_expert ? std::min(cap_rows, (2 * cap_rows * n_held + n_expert - 1) / n_expert) : cap_rows;
     c.slab_units = std::max<int64_t>(kMaxUnits, std::min(all, image_units(share, prefill_cap_tiles(share, n_held))));
-    c.n_slabs = (int) ((all + c.slab_units - 1) / c.slab_units);
+    c.n_slabs = c.stream ? 1 : (int) ((all + c.slab_units - 1) / c.slab_units);
     size_t at = 0;
     auto take = [&](size_t bytes) {
         const size_t r = at;
@@ -801,10 +891,10 @@ static PrefillCarve prefill_carve(const bsx_expert_layout& L, int64_t n_tokens, 
     } else {
         at = (at + 4095) & ~(size_t) 4095;
         c.img = take((size_t) (c.slab_units + kMaxUnits) * 1024 * kTermsF * ((H + I) / 256));
-        c.recs = take((size_t) c.cap_recs * sizeof(TileRec));
-        c.slabs = take((size_t) (c.n_slabs + 1) * 4);
     }
     c.hinv = take((size_t) (cap_rows + 128) * 4);
+    c.recs = take((size_t) c.cap_recs * sizeof(TileRec));
+    c.slabs = take((size_t) (c.n_slabs + 1) * 4);
     c.bytes = at;
     return c;
 }
@@ -842,13 +932,42 @@ extern "C" int32_t bsx_experts_prefill_packed_held(const bsx_expert_layout* layo
     uint8_t* base = static_cast<uint8_t*>(scratch);
     uint8_t *xcodes = base + c.xcodes, *xsf = base + c.xsf;
     float *xinv = reinterpret_cast<float*>(base + c.xinv), *h = reinterpret_cast<float*>(base + c.h), *hinv = reinterpret_cast<float*>(base + c.hinv);
+    RecordArgs ra;
+    ra.tiles = tiles;
+    ra.n_tiles = n_tiles;
+    ra.off = off;
+    ra.blob_table = blob_table;
+    ra.cap_tiles = cap_tiles;
+    ra.recs = reinterpret_cast<TileRec*>(base + c.recs);
+    ra.cap_recs = c.cap_recs;
+    ra.slab_first = reinterpret_cast<int32_t*>(base + c.slabs);
+    ra.n_slabs = c.n_slabs;
+    ra.slab_units = c.slab_units;
+    ra.items = nullptr;
+    ra.n_items = nullptr;
+    ra.cap_items = c.cap_items;
+    ra.pass_entries = cap_rows > kPassEntries / 2 * n_expert ? 2 * kPassEntries : kPassEntries;
+    ra.tile_items = (int) (I / 128);
+    ra.sm_count = sm_count();
+    ra.status = status;
+    PrefillFArgs a;
+    a.L = L;
+    a.recs = ra.recs;
+    a.from = nullptr;
+    a.to = ra.slab_first + 1;
+    a.src = src;
+    a.sfs = nullptr;
+    a.h = h;
+    a.dm = dm;
+    a.status = status;
     // Few rows an expert: a tile's 128 tensor-core rows would be mostly padding and cost twice what the weights' bytes do, so the rows
-    // go through the decode stream instead (experts_nvf4.cu: passes of 8 or 16 rows as the MMA's narrow side, bound by the weights).
+    // go through the decode stream instead (experts_nvf4.cu: passes of 8 or 16 rows as the MMA's narrow side, bound by the weights),
+    // crowded tiles aside (tile_records_kernel), which in most calls there are none of: their kernels then return at once.
     if (c.stream) {
-        const int pass_entries = cap_rows > kPassEntries / 2 * n_expert ? 2 * kPassEntries : kPassEntries;
-        PassRec* items = reinterpret_cast<PassRec*>(base + c.items);
-        int* n_items = reinterpret_cast<int*>(base + c.n_items);
-        tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, cap_tiles, nullptr, 0, nullptr, 0, 1, items, n_items, c.cap_items, pass_entries, status);
+        PdlScope pdl(true, 1);      // the first kernel follows the caller's work
+        ra.items = reinterpret_cast<PassRec*>(base + c.items);
+        ra.n_items = reinterpret_cast<int*>(base + c.n_items);
+        launch_k(tile_records_kernel, dim3(1), dim3(1024), 0, st, ra);
         ExpertArgs e;
         e.L = L;
         e.grp_ptr = nullptr;
@@ -865,21 +984,28 @@ extern "C" int32_t bsx_experts_prefill_packed_held(const bsx_expert_layout* layo
         e.out_kind = BSX_OUT_F32;
         e.n_x_rows = (int32_t) n_tokens;
         e.grid = nullptr;
-        return experts_packed_passes(e, items, n_items, pass_entries, xcodes, xsf, xinv, base + c.hcodes, base + c.hsf, hinv, status, st);
+        packed_x_images(x, x_kind, n_tokens, H, xcodes, xsf, xinv, st);
+        a.img = xcodes;
+        a.sfs = xsf;
+        a.inv = xinv;
+        int32_t rc = launch_q<QMODE_GU, true>(a, st);
+        if (rc == BSX_OK) rc = packed_pass_product(false, e, ra.items, ra.n_items, ra.pass_entries, xcodes, xsf, xinv, status, st);
+        if (rc != BSX_OK) return rc;
+        uint8_t *hcodes = base + c.hcodes, *hsf = base + c.hsf;
+        packed_listed_images(h, ra.items, ra.n_items, ra.pass_entries, ra.recs, ra.slab_first, I, hcodes, hsf, hinv, st);
+        a.img = hcodes;
+        a.sfs = hsf;
+        a.inv = hinv;
+        rc = launch_q<QMODE_DOWN, true>(a, st);
+        if (rc != BSX_OK) return rc;
+        return packed_pass_product(true, e, ra.items, ra.n_items, ra.pass_entries, hcodes, hsf, hinv, status, st);
     }
     uint8_t *ximg = base + c.img, *himg = ximg + (size_t) (c.slab_units + kMaxUnits) * 1024 * kTermsF * (H / 256);
-    TileRec* recs = reinterpret_cast<TileRec*>(base + c.recs);
-    int32_t* slabs = reinterpret_cast<int32_t*>(base + c.slabs);
-    tile_records_kernel<<<1, 1024, 0, st>>>(tiles, n_tiles, off, blob_table, cap_tiles, recs, c.cap_recs, slabs, c.n_slabs, c.slab_units, nullptr, nullptr, 0, 1, status);
+    const TileRec* recs = ra.recs;
+    const int32_t* slabs = ra.slab_first;
+    tile_records_kernel<<<1, 1024, 0, st>>>(ra);
     if (H <= 2048) prefill_images_kernel<128><<<(unsigned) ((n_tokens + 1) / 2), 256, 0, st>>>(x, x_kind, n_tokens, H, xcodes, xsf, xinv);
     else prefill_images_kernel<256><<<(unsigned) n_tokens, 256, 0, st>>>(x, x_kind, n_tokens, H, xcodes, xsf, xinv);
-    PrefillFArgs a;
-    a.L = L;
-    a.recs = recs;
-    a.src = src;
-    a.h = h;
-    a.dm = dm;
-    a.status = status;
     // a tile takes three units at least, and one may begin in a slab's last unit
     const int64_t slab_tiles = std::min(std::min(cap_tiles, c.cap_recs), c.slab_units / 3 + 1);
     for (int s = 0; s < c.n_slabs; ++s) {
@@ -890,7 +1016,7 @@ extern "C" int32_t bsx_experts_prefill_packed_held(const bsx_expert_layout* layo
                                                                                                                                  ximg);
         a.img = ximg;
         a.inv = xinv;
-        int32_t rc = launch_q<QMODE_GU>(a, st);
+        int32_t rc = launch_q<QMODE_GU, false>(a, st);
         if (rc != BSX_OK) return rc;
         const unsigned hb = (unsigned) (slab_tiles * 16);
         a.img = himg;
@@ -898,7 +1024,7 @@ extern "C" int32_t bsx_experts_prefill_packed_held(const bsx_expert_layout* layo
         else h_images_kernel<0><<<hb, 256, 0, st>>>(recs, a.from, a.to, h, I, himg, hinv);
         a.inv = hinv;
         // n_ff <= 512: the tile's rows stay in shared memory and only weights stream
-        rc = I == 256 ? launch_down_resident<1>(a, st) : I == 512 ? launch_down_resident<2>(a, st) : launch_q<QMODE_DOWN>(a, st);
+        rc = I == 256 ? launch_down_resident<1>(a, st) : I == 512 ? launch_down_resident<2>(a, st) : launch_q<QMODE_DOWN, false>(a, st);
         if (rc != BSX_OK) return rc;
     }
     return BSX_OK;

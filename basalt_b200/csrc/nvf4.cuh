@@ -149,5 +149,12 @@ __device__ __forceinline__ void fp4_image_row(const void* src, int kind, int64_t
     }
 }
 
+// a 128-row tile of one expert with everything the kernels need about it
+struct __align__(16) TileRec {
+    unsigned long long blob;
+    int row0, rows;
+    int64_t base;          // units (of atoms) before this tile's in its slab's tile images (experts_prefill_nvf4.cu)
+    int64_t pad;
+};
 
 }  // namespace bsx

@@ -84,3 +84,16 @@ def test_experts_held_elsewhere(lib, cuda, H, I, counts, away):
 def test_rounds_over_the_room_of_an_even_share(lib, cuda, H, I, counts, here):
     """rows that crowd onto the experts held here: more than twice an even share, so that the tile images take several rounds"""
     run(H, I, 0, counts, tuple(e for e in range(len(counts)) if e not in here), len(tuple(here)))
+
+
+# short calls by their average whose rows crowd onto few experts: full tiles and remainders above and below the 65 rows from which a
+# tile stays one, over enough items that the call takes them (22 tiles x 6 or more), with passes of 16 and of 8 beside them
+CROWD = [1000, 3, 0, 1000, 64, 65, 0, 700] + [0] * 55 + [9]
+
+
+@pytest.mark.parametrize("H,I,shift,counts,away", [(256, 768, 0, CROWD, ()), (512, 1280, 16, CROWD, ()), (768, 2304, 0, CROWD, (1, 4)), (2048, 768, 0, CROWD, ()),
+                                                   (256, 512, 16, CROWD * 2, ()), (512, 256, 0, CROWD * 5, (0, 64)), (256, 768, 0, CROWD + [0] * 700, ()),
+                                                   (256, 768, 0, CROWD, (0, 3, 7))])
+def test_crowded_short_calls(lib, cuda, H, I, shift, counts, away):
+    run(H, I, shift, counts, away)
+    run(H, I, shift, counts, away, len(counts))
