@@ -15,10 +15,10 @@
 //     are the 32 group coefficients m (8 -+ 1) <= 135 (u8) and the 32 negated group sums split as 16 hi + lo (s8 each).
 //     Everything up to the factor d / 8 is exact integer arithmetic.
 //   * Q6_K (ggml_common.h:279-285, ggml_quants.c:1048-1075): a weight is d sc (q - 32), sc an int8 per 16 weights: one
-//     m16n8k16 s8 MMA per scale group, its int32 result scaled by d sc in fp32.
+//     m16n8k16 MMA per scale group, its result times sc added up in int32, the 32 taken off by a correction like IQ1_M's.
 // Each warp owns 16 weight rows (8 gate rows with their 8 up rows, so SwiGLU stays in the thread; or 16 down rows) and
 // streams them through its own cp.async ring in chunks of 512 columns; a block's warps share the pass's activation columns.
-// Blocks are persistent and draw (pass, row block) units from a counter.
+// Blocks are persistent; each takes an equal run of the (pass, row block) sequence.
 //
 // Semantics: Basalt's native_expert_grouped (include/basalt/kernels/iq_kernels.hpp:77-92; its IQ1_M dot src/kernels/cuda/
 // iq_kernels.cu:227-257 with the grid table staged in shared memory :1516-1521), minus the single-term q8_1 rounding.
@@ -30,6 +30,7 @@
 #include "experts.cuh"
 #include "formats.cuh"
 #include "pdl.cuh"
+#include "plan.cuh"
 
 namespace bsx {
 namespace {
@@ -50,13 +51,12 @@ constexpr int64_t kMaxColsQ6K = 8192;
 // leave room for one CTA and take two blocks (7168 x 2048, 256 experts: 64 tokens 2834 us, with one block and five stages 3239).
 template <int TYPE> struct QT;
 template <int TYPE, int CB> constexpr int kRowStage = TYPE == kTypeIQ1M ? 112 : CB == 1 ? 240 : 420;
+template <int TYPE> constexpr int kCorrBytes = TYPE == kTypeIQ1M ? 64 : 32;   // correction bytes of a column and block
 template <> struct QT<kTypeIQ1M> {
-    static constexpr int kBlock = 56, kWarps = 16, kPad = 32;
-    static constexpr bool kCorr = true;
+    static constexpr int kBlock = 56, kPad = 32;
 };
 template <> struct QT<kTypeQ6K> {
-    static constexpr int kBlock = 210, kWarps = 8, kPad = 16;
-    static constexpr bool kCorr = false;
+    static constexpr int kBlock = 210, kPad = 16;
 };
 
 __device__ __forceinline__ void cpa16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory"); }
@@ -71,7 +71,12 @@ __device__ __forceinline__ void mma_u8s8_k32(int (&c)[4], uint32_t a0, uint32_t 
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// D (16 x 8, s32) = A (16 x 16, s8, row) x B (16 x 8, s8, col)
+// D (16 x 8, s32) = A (16 x 16, u8 or s8, row) x B (16 x 8, s8, col)
+__device__ __forceinline__ void mma_u8s8_k16(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};\n"
+                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(b0), "r"(0));
+}
 __device__ __forceinline__ void mma_s8_k16(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};\n"
                  : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
@@ -80,16 +85,17 @@ __device__ __forceinline__ void mma_s8_k16(int (&c)[4], uint32_t a0, uint32_t a1
 
 // ---------------------------------------------------------------- activation images
 // One warp per image row: the row as two int8 terms under one scale, x s ~ q1 + q2 / 254, s = 127 / max|x|; inv[row] = 1 / s.
-// Layout: img[row][term][K] int8 in column order.  CORR (IQ1_M): per 256 columns the 32 negated group-of-8 sums of each term as
+// Layout: img[row][term][K] int8 in column order.  Q6_K: per 256 columns the 16 negated group-of-16 sums of each term as 16 hi + lo,
+// corr[row][term][K / 256][hi 16 bytes | lo 16 bytes].  IQ1_M: per 256 columns the 32 negated group-of-8 sums of each term as
 // 16 hi + lo, corr[row][term][K / 256][hi 32 bytes | lo 32 bytes], a group at the byte its coefficient has in the A fragment:
 // group 4 u + t (u = 32-column unit, t = group inside it) -> byte 4 t + p (u < 4) or 16 + 4 t + p with p = 0, 2, 1, 3 for
 // u % 4 = 0, 1, 2, 3 (the order in which the product kernel can assemble the coefficients cheaply).
 // FROM_H = false: rows of x (row i of x when the caller gave the number of x rows, else the row of entry i); true: row e of
-// the SwiGLU output.  The last block lists the passes (up to 4 consecutive entries of a group) and zeroes the work counter.
-template <bool FROM_H, bool CORR>
+// the SwiGLU output.  The last block lists the passes (up to pass_entries consecutive entries of a group).
+template <bool FROM_H, int TYPE>
 __global__ void __launch_bounds__(256)
-kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ corr, float* __restrict__ inv, int2* __restrict__ items,
-                int* __restrict__ n_items) {
+kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ corr, float* __restrict__ inv, PassRec* __restrict__ items,
+                int* __restrict__ n_items, int pass_entries) {
     pdl_wait();
     pdl_launch_dependents();
     const int ng = min(*a.n_groups, (int) a.cap_groups);
@@ -104,7 +110,7 @@ kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ cor
             const int g = g0 + threadIdx.x;
             const int s0 = g < ng ? a.grp_start[g] : 0;
             const int cnt = g < ng ? max(0, min(a.grp_start[g + 1], (int) a.cap_entries) - s0) : 0;
-            const int np = (cnt + kEntQ - 1) / kEntQ;
+            const int np = (cnt + pass_entries - 1) / pass_entries;
             int x = np;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -115,15 +121,18 @@ kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ cor
             __syncthreads();
             int before = s_base;
             for (int w = 0; w < warp; ++w) before += sh[w];
-            for (int p = 0; p < np; ++p) items[before + x - np + p] = make_int2(g, s0 + p * kEntQ);
+            for (int p = 0; p < np; ++p) {
+                PassRec r;
+                r.blob = a.grp_ptr[g];
+                r.eb = s0 + p * pass_entries;
+                r.ntok = min(pass_entries, cnt - p * pass_entries);
+                items[before + x - np + p] = r;
+            }
             __syncthreads();
             if (threadIdx.x == 255) s_base = before + x;
             __syncthreads();
         }
-        if (threadIdx.x == 0) {
-            n_items[0] = s_base;
-            n_items[1] = 0;
-        }
+        if (threadIdx.x == 0) n_items[0] = s_base;
         return;
     }
     const int i = blockIdx.x * 8 + warp;
@@ -171,8 +180,8 @@ kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ cor
         }
         reinterpret_cast<uint4*>(q1)[sb] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
         reinterpret_cast<uint4*>(q2)[sb] = make_uint4(w2[0], w2[1], w2[2], w2[3]);
-        if (CORR) {
-            const int blk = sb >> 4;
+        const int blk = sb >> 4;
+        if constexpr (TYPE == kTypeIQ1M) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int gi = ((sb & 15) << 1) + h;               // group inside the 256-column block
@@ -183,24 +192,32 @@ kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ cor
                 for (int term = 0; term < 2; ++term) {
                     const int neg = -(term ? sum2[h] : sum1[h]);
                     const int hi = neg >> 4, lo = neg & 15;       // neg = 16 hi + lo, 0 <= lo < 16 (arithmetic shift floors)
-                    int8_t* c = corr + (((size_t) i * 2 + term) * nblk + blk) * 64;
+                    int8_t* c = corr + (((size_t) i * 2 + term) * nblk + blk) * kCorrBytes<TYPE>;
                     c[slot] = (int8_t) hi;
                     c[32 + slot] = (int8_t) lo;
                 }
+            }
+        } else {
+#pragma unroll
+            for (int term = 0; term < 2; ++term) {
+                const int neg = -(term ? sum2[0] + sum2[1] : sum1[0] + sum1[1]);
+                int8_t* c = corr + (((size_t) i * 2 + term) * nblk + blk) * kCorrBytes<TYPE>;
+                c[sb & 15] = (int8_t) (neg >> 4);
+                c[16 + (sb & 15)] = (int8_t) (neg & 15);
             }
         }
     }
 }
 
 // ---------------------------------------------------------------- block decoders
-// IQ1_M: one 256-weight block of rows g and g + 8 (raw 56-byte blocks ra, rb in shared memory, 8-byte aligned) against the 8
-// activation columns; adds d / 8-scaled... the caller scales: tot[i] += I[i] * d[row] where I is the exact integer
+// IQ1_M: one 256-weight block of rows g and g + 8 (raw 56-byte blocks ra, rb in shared memory, 8-byte aligned) against NB times 8
+// activation columns; the caller scales: tot[i] += I[i] * d[row] where I is the exact integer
 // 8 m c q - coefficient sums described at the top.  bcol: this lane's column, at the block's first byte plus 8 t;
-// ccol: the column's 64 correction bytes of this block.
+// ccol: the column's 64 correction bytes of this block; bnext / cnext: bytes to the column 8 further; wide: the pass has such columns.
 // tab: the lane's copy of the table (NC copies interleaved point by point).
-template <int NC>
+template <int NC, int NB>
 __device__ __forceinline__ void iq1m_block(const uint8_t* ra, const uint8_t* rb, const uint2* __restrict__ tab, const uint8_t* bcol,
-                                           const uint8_t* ccol, int t, float (&tot)[4]) {
+                                           const uint8_t* ccol, int bnext, int cnext, bool wide, int t, float (&tot)[NB][4]) {
     uint32_t wa[14], wb[14];
 #pragma unroll
     for (int i = 0; i < 7; ++i) {
@@ -209,9 +226,12 @@ __device__ __forceinline__ void iq1m_block(const uint8_t* ra, const uint8_t* rb,
         wb[2 * i] = vb.x; wb[2 * i + 1] = vb.y;
     }
     // words 0-7: qs (unit u = bytes 4u..4u+3), 8-11: qh (unit u = bytes 2u, 2u+1; group t = nibble t), 12-13: four scale words
-    int acc[4] = {0, 0, 0, 0};
-    const uint32_t sel = 0x4440u | (uint32_t) t;     // byte t of a word, zero-extended
+    int acc[NB][4];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0;
     const int s4 = 4 * t, s3 = 3 * (t >> 1);
+    // a point's index: byte t of the unit's qs word under the three high bits, which byte 0 (even units) or 2 of the masked qh word holds
+    const uint32_t sel0 = 0x7740u + (uint32_t) t, sel1 = 0x7760u + (uint32_t) t;
     uint32_t msum[4] = {0u, 0u, 0u, 0u};              // the groups' scales m as bytes, in the correction operand's order (below)
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -220,9 +240,8 @@ __device__ __forceinline__ void iq1m_block(const uint8_t* ra, const uint8_t* rb,
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint32_t* w = r ? wb : wa;
-            const uint32_t qsb = __byte_perm(w[u], 0u, sel);
-            const uint32_t nib = (w[8 + (u >> 1)] >> (16 * (u & 1) + s4)) & 7u;
-            const uint2 e = tab[(nib * 256u + qsb) * NC];
+            const uint32_t hi = (w[8 + (u >> 1)] >> s4) & 0x00070007u;
+            const uint2 e = tab[__byte_perm(w[u], hi, (u & 1) ? sel1 : sel0) * NC];
             const uint32_t sw = w[12 + (u >> 2)] >> s3;                                    // the thread's scale field of unit u now sits at a fixed bit
             const int fb = 16 * ((u >> 1) & 1) + 6 * (u & 1);
             const uint32_t m = fb > 0 ? (((sw >> (fb - 1)) & 14u) | 1u) : (((sw << 1) & 14u) | 1u);   // 2 s + 1
@@ -231,7 +250,14 @@ __device__ __forceinline__ void iq1m_block(const uint8_t* ra, const uint8_t* rb,
             msum[(u < 4 ? 0 : 2) + r] += m << (8 * kPos[u & 3]);
         }
         const uint2 b = *reinterpret_cast<const uint2*>(bcol + 32 * u);
-        mma_u8s8_k32(acc, a[0], a[1], a[2], a[3], b.x, b.y);
+        mma_u8s8_k32(acc[0], a[0], a[1], a[2], a[3], b.x, b.y);
+        if (NB > 1 && wide) {
+#pragma unroll
+            for (int n = 1; n < NB; ++n) {
+                const uint2 bn = *reinterpret_cast<const uint2*>(bcol + n * bnext + 32 * u);
+                mma_u8s8_k32(acc[n], a[0], a[1], a[2], a[3], bn.x, bn.y);
+            }
+        }
     }
     // the correction operand: byte = m (8 - 8 delta) = 7 m + 2 m [delta = -1/8], four groups at a time.  The delta bits of units
     // (0, 1) are bits 4t+3 and 4t+19 of qh word 0, of units (2, 3) the same bits of qh word 1: shifted and merged they land in bytes
@@ -245,13 +271,6 @@ __device__ __forceinline__ void iq1m_block(const uint8_t* ra, const uint8_t* rb,
         ca[r] = 7u * msum[r] + 2u * (msum[r] & (dlo * 0xFFu));
         ca[2 + r] = 7u * msum[2 + r] + 2u * (msum[2 + r] & (dhi * 0xFFu));
     }
-    int chi[4] = {0, 0, 0, 0}, clo[4] = {0, 0, 0, 0};
-    {
-        const uint32_t h0 = *reinterpret_cast<const uint32_t*>(ccol + 4 * t), h1 = *reinterpret_cast<const uint32_t*>(ccol + 16 + 4 * t);
-        const uint32_t l0 = *reinterpret_cast<const uint32_t*>(ccol + 32 + 4 * t), l1 = *reinterpret_cast<const uint32_t*>(ccol + 48 + 4 * t);
-        mma_u8s8_k32(chi, ca[0], ca[1], ca[2], ca[3], h0, h1);
-        mma_u8s8_k32(clo, ca[0], ca[1], ca[2], ca[3], l0, l1);
-    }
     // the fp16 super-scale: the top nibbles of the four scale words
     float d[2];
 #pragma unroll
@@ -261,76 +280,110 @@ __device__ __forceinline__ void iq1m_block(const uint8_t* ra, const uint8_t* rb,
         d[r] = __half2float(__ushort_as_half((unsigned short) bits));
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) tot[i] = fmaf((float) (8 * acc[i] + 16 * chi[i] + clo[i]), d[i >> 1], tot[i]);
+    for (int n = 0; n < NB; ++n) {
+        if (n > 0 && !wide) break;
+        const uint8_t* cc = ccol + n * cnext;
+        int chi[4] = {0, 0, 0, 0}, clo[4] = {0, 0, 0, 0};
+        const uint32_t h0 = *reinterpret_cast<const uint32_t*>(cc + 4 * t), h1 = *reinterpret_cast<const uint32_t*>(cc + 16 + 4 * t);
+        const uint32_t l0 = *reinterpret_cast<const uint32_t*>(cc + 32 + 4 * t), l1 = *reinterpret_cast<const uint32_t*>(cc + 48 + 4 * t);
+        mma_u8s8_k32(chi, ca[0], ca[1], ca[2], ca[3], h0, h1);
+        mma_u8s8_k32(clo, ca[0], ca[1], ca[2], ca[3], l0, l1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) tot[n][i] = fmaf((float) (8 * acc[n][i] + 16 * chi[i] + clo[i]), d[i >> 1], tot[n][i]);
+    }
 }
 
-// a byte of shared memory at any alignment, two bytes, four bytes (blocks of 210 bytes are only 2-byte aligned)
-__device__ __forceinline__ uint32_t ld_u16(const uint8_t* p) { return *reinterpret_cast<const uint16_t*>(p); }
-__device__ __forceinline__ uint32_t ld_u32_a2(const uint8_t* p) { return ld_u16(p) | (ld_u16(p + 2) << 16); }
+// four bytes of shared memory from an address that is a multiple of four, or two past one (every second 210-byte block)
+template <bool ODD>
+__device__ __forceinline__ uint32_t ld_word(const uint8_t* p) {
+    if (!ODD) return *reinterpret_cast<const uint32_t*>(p);
+    return __byte_perm(*reinterpret_cast<const uint32_t*>(p - 2), *reinterpret_cast<const uint32_t*>(p + 2), 0x5432);
+}
 
-// four 6-bit codes (one a byte) -> four s8 values code - 32: the low five bits stay, bits 5-7 become the sign
-__device__ __forceinline__ uint32_t q6_to_s8(uint32_t v) { return (v & 0x1F1F1F1Fu) + ((~v & 0x20202020u) * 7u); }
-
-// Q6_K: one 256-weight block of rows g and g + 8 (raw 210-byte blocks in shared memory, 2-byte aligned); bcol: this lane's
-// column at the block's first byte plus 4 t.  tot[i] += sum over the 16 scale groups of (int dot) * d * sc.
-__device__ __forceinline__ void q6k_block(const uint8_t* ra, const uint8_t* rb, const uint8_t* bcol, int t, float (&tot)[4]) {
-    const float da = __half2float(__ushort_as_half((unsigned short) ld_u16(ra + 208))), db = __half2float(__ushort_as_half((unsigned short) ld_u16(rb + 208)));
+// Q6_K: one 256-weight block of rows g and g + 8 (raw 210-byte blocks in shared memory) against NB times 8 columns; bcol: this lane's
+// column at the block's first byte plus 4 t, ccol: its 32 correction bytes of this block plus 4 t.  All of it up to d is integer: the
+// codes go in as they are (0 .. 63), a group's sum times its scale adds up in 32 bits (below 2^29), and the 32 that a code is too
+// large by comes off as one MMA pair over the block's 16 scales and the groups' negated activation sums (16 hi + lo).  What bounds the
+// kernel is instructions: with signed codes, a scale converted to fp32 for each group and half-words loaded one by one a warp spent
+// 794 on a block of 16 rows and the 64-token step of 2048 x 512, 512 experts, took 325 us; now 250.
+template <int NB, bool ODD>
+__device__ __forceinline__ void q6k_block(const uint8_t* ra, const uint8_t* rb, const uint8_t* bcol, const uint8_t* ccol, int bnext, int cnext, bool wide, int t,
+                                          float (&tot)[NB][4]) {
+    int sum[NB][4];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) sum[n][0] = sum[n][1] = sum[n][2] = sum[n][3] = 0;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            const int lo = 64 * h + 16 * j + 4 * t;
-            const uint32_t qa1 = ld_u32_a2(ra + lo), qa2 = ld_u32_a2(ra + lo + 32), qah = ld_u32_a2(ra + 128 + 32 * h + 16 * j + 4 * t);
-            const uint32_t qb1 = ld_u32_a2(rb + lo), qb2 = ld_u32_a2(rb + lo + 32), qbh = ld_u32_a2(rb + 128 + 32 * h + 16 * j + 4 * t);
+            const int lo = 64 * h + 16 * j + 4 * t, hi = 128 + 32 * h + 16 * j + 4 * t;
+            const uint32_t qa[2] = {ld_word<ODD>(ra + lo), ld_word<ODD>(ra + lo + 32)}, qah = ld_word<ODD>(ra + hi);
+            const uint32_t qb[2] = {ld_word<ODD>(rb + lo), ld_word<ODD>(rb + lo + 32)}, qbh = ld_word<ODD>(rb + hi);
 #pragma unroll
             for (int sub = 0; sub < 4; ++sub) {
-                const uint32_t la = ((((sub & 1) ? qa2 : qa1) >> (sub >= 2 ? 4 : 0)) & 0x0F0F0F0Fu) | (((qah >> (2 * sub)) & 0x03030303u) << 4);
-                const uint32_t lb = ((((sub & 1) ? qb2 : qb1) >> (sub >= 2 ? 4 : 0)) & 0x0F0F0F0Fu) | (((qbh >> (2 * sub)) & 0x03030303u) << 4);
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(bcol + 128 * h + 32 * sub + 16 * j);
-                int c[4];
-                mma_s8_k16(c, q6_to_s8(la), q6_to_s8(lb), b0);
+                const int down = sub >= 2 ? 4 : 0;
+                const uint32_t a0 = ((qa[sub & 1] >> down) & 0x0F0F0F0Fu) | ((sub < 2 ? qah << (4 - 2 * sub) : qah >> (2 * sub - 4)) & 0x30303030u);
+                const uint32_t a1 = ((qb[sub & 1] >> down) & 0x0F0F0F0Fu) | ((sub < 2 ? qbh << (4 - 2 * sub) : qbh >> (2 * sub - 4)) & 0x30303030u);
                 const int is = 8 * h + 2 * sub + j;
-                const float sa = da * (float) (int) (int8_t) ra[192 + is], sb = db * (float) (int) (int8_t) rb[192 + is];
-                tot[0] = fmaf((float) c[0], sa, tot[0]);
-                tot[1] = fmaf((float) c[1], sa, tot[1]);
-                tot[2] = fmaf((float) c[2], sb, tot[2]);
-                tot[3] = fmaf((float) c[3], sb, tot[3]);
+                const int sa = (int8_t) ra[192 + is], sb = (int8_t) rb[192 + is];
+#pragma unroll
+                for (int n = 0; n < NB; ++n) {
+                    if (n > 0 && !wide) break;
+                    int c[4];
+                    mma_u8s8_k16(c, a0, a1, *reinterpret_cast<const uint32_t*>(bcol + n * bnext + 128 * h + 32 * sub + 16 * j));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[n][i] += c[i] * (i < 2 ? sa : sb);
+                }
             }
         }
+    }
+    const float da = __half2float(*reinterpret_cast<const __half*>(ra + 208)), db = __half2float(*reinterpret_cast<const __half*>(rb + 208));
+    const uint32_t ca = ld_word<ODD>(ra + 192 + 4 * t), cb = ld_word<ODD>(rb + 192 + 4 * t);
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+        if (n > 0 && !wide) break;
+        int chi[4], clo[4];
+        mma_s8_k16(chi, ca, cb, *reinterpret_cast<const uint32_t*>(ccol + n * cnext));
+        mma_s8_k16(clo, ca, cb, *reinterpret_cast<const uint32_t*>(ccol + n * cnext + 16));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) tot[n][i] = fmaf((float) (sum[n][i] + 512 * chi[i] + 32 * clo[i]), i < 2 ? da : db, tot[n][i]);
     }
 }
 
 // ---------------------------------------------------------------- the product kernel
 // MODE GU: rows = 8 gate rows r0.. with the up rows r0..; columns = the entries' x images; writes h (fp32).
 // MODE DOWN: rows = 16 down rows; columns = the entries' h images; writes out rows through ent_dst.
-// KS > 1: KS neighbouring warps share a row tile, each a part of its columns, and their sums meet in shared memory - for calls so
-// small that whole rows would leave most SMs without a unit (a shared expert of 2048 x 512 at 5 tokens: 16 units of 148; its two
-// products took 47 of the step's 155 us, with the split the step takes 121).
-template <int TYPE, int MODE, int KS, int NC, int ST, int CB>
-__global__ void __launch_bounds__(QT<TYPE>::kWarps * 32, CB == 1 && ST == 3 ? 2 : 1)
+// NB: a pass is up to 4 NB entries, NB column blocks of the MMA over one decoded A fragment; a pass of four or fewer multiplies one block.
+// KS > 1: KS neighbouring warps share a row tile, each a part of its columns, and their sums meet in shared memory: a step of the
+// block is then W / KS tiles instead of W, so that a small call still divides evenly.
+// Work: the row blocks (W / KS tiles) of all passes in one sequence, cut into equal runs, one a block.  A run's part of one pass shares
+// its columns and its weight stream, so barriers, activation copies and first loads come once or twice a call.  (Units drawn from a
+// counter instead: IQ1_M gate/up of 7168 x 2048 at 64 tokens 765 us, with runs and a look-up index made by one byte permutation 655.)
+template <int TYPE, int MODE, int W, int OCC, int KS, int NC, int ST, int CB, int NB>
+__global__ void __launch_bounds__(W * 32, OCC)
 kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __restrict__ corr, const float* __restrict__ inv,
-              const int2* __restrict__ items, int* __restrict__ n_items, int tiles_per_warp, int n_row_blocks) {
+              const PassRec* __restrict__ items, const int* __restrict__ n_items, int n_row_blocks) {
     using Q = QT<TYPE>;
-    constexpr int kWarps = Q::kWarps, kThreads = kWarps * 32, kStages = ST;
+    constexpr int kThreads = W * 32, kStages = ST, kEntP = kEntQ * NB, kCols = kColsQ * NB, kTiles = W / KS;
     constexpr int kChunkBytes = CB * Q::kBlock, kRow = kRowStage<TYPE, CB>, kStageBytes = kRowsQ * kRow;
     extern __shared__ __align__(128) uint8_t smem[];
     const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
     const int nblk = (int) (K >> 8);
     const int cstride = (int) K + Q::kPad;                                   // bytes between activation columns
-    const int xstride = nblk * 64 + 16;                                        // ... and between their correction columns
-    uint8_t* xs = smem;                                                        // [8][cstride]
-    uint8_t* cs = xs + (size_t) kColsQ * cstride;                              // [8][xstride] (IQ1_M)
-    uint2* tab = reinterpret_cast<uint2*>(cs + (Q::kCorr ? (size_t) kColsQ * xstride : 0));   // [2048][NC] (IQ1_M)
-    uint8_t* wbase = reinterpret_cast<uint8_t*>(tab) + (Q::kCorr ? 16384 * NC : 0);
+    const int xstride = nblk * kCorrBytes<TYPE> + 16;                                        // ... and between their correction columns
+    uint8_t* xs = smem;                                                        // [kCols][cstride]
+    uint8_t* cs = xs + (size_t) kCols * cstride;                               // [kCols][xstride]
+    uint2* tab = reinterpret_cast<uint2*>(cs + (size_t) kCols * xstride);      // [2048][NC] (IQ1_M)
+    uint8_t* wbase = reinterpret_cast<uint8_t*>(tab) + (TYPE == kTypeIQ1M ? 16384 * NC : 0);
+    float2* part = reinterpret_cast<float2*>(wbase + (size_t) W * kStages * kStageBytes);     // [2][tiles][KS - 1][NB][32] (KS > 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* wring = wbase + (size_t) warp * kStages * kStageBytes;
     const uint32_t wring_s = (uint32_t) __cvta_generic_to_shared(wring);
     const uint32_t xs_s = (uint32_t) __cvta_generic_to_shared(xs), cs_s = (uint32_t) __cvta_generic_to_shared(cs);
-    __shared__ int s_ir[kEntQ];
-    __shared__ int s_work;
+    __shared__ int s_ir[kEntP];
 
-    if (Q::kCorr) {
+    if (TYPE == kTypeIQ1M) {
         // the codebook as 8 bytes per point, coordinate i's code c = g + 1 in byte i: the two words are the two MMA operand
         // registers of an 8-weight group.  The look-ups are the kernel's scarce resource (16 data-dependent 8-byte reads a lane and
         // block), and what they cost is bank conflicts.  NC copies, interleaved so that a lane's copy (lane % NC) lives in 1 / NC of the
@@ -353,31 +406,31 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
 
     const int64_t n_rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd;
     constexpr int kTileRows = MODE == QMODE_GU ? 8 : 16;
-    static_assert(kWarps % KS == 0, "");
-    constexpr int tile_stride = kWarps / KS * kTileRows;
+    static_assert(W % KS == 0, "");
+    constexpr int kStepRows = kTiles * kTileRows;
     const int n_chunks = nblk / CB / KS, chunk0 = (warp % KS) * n_chunks;      // this warp's part of a row
     const size_t row_bytes = MODE == QMODE_GU ? (size_t) a.L.gu_row : (size_t) a.L.d_row;
 
-    const int n_work = n_items[0] * n_row_blocks;
-    // the next unit is drawn while this one streams: the counter's round trip is off the path from unit to unit
-    int drawn = threadIdx.x == 0 ? atomicAdd(&n_items[1], 1) : 0;
-    for (;;) {
-        if (threadIdx.x == 0) s_work = drawn;
-        __syncthreads();   // the previous unit is done with xs, cs and s_ir
-        const int work = s_work;
-        if (work >= n_work) break;
-        if (threadIdx.x == 0) drawn = atomicAdd(&n_items[1], 1);
+    const int64_t n_work = (int64_t) n_items[0] * n_row_blocks;
+    int work = (int) (n_work * blockIdx.x / gridDim.x);
+    const int work_end = (int) (n_work * (blockIdx.x + 1) / gridDim.x);
+    PassRec next{0ull, 0, 0};
+    if (work < work_end) next = items[work / n_row_blocks];
+    while (work < work_end) {
+        const PassRec pass = next;
         const int item = work / n_row_blocks, rb = work - item * n_row_blocks;
-        const int64_t r0 = (int64_t) rb * tiles_per_warp * tile_stride + warp / KS * kTileRows;
+        const int steps = min(work_end - work, n_row_blocks - rb);
+        work += steps;
+        if (work < work_end) next = items[item + 1];      // rides under this pass
+        const int64_t r0 = (int64_t) rb * kStepRows + warp / KS * kTileRows;
         int live_tiles = 0;
-        while (live_tiles < tiles_per_warp && r0 + (int64_t) live_tiles * tile_stride < n_rows) ++live_tiles;
+        if (r0 < n_rows) live_tiles = (int) min((int64_t) steps, (n_rows - r0 + kStepRows - 1) / kStepRows);
         const int n_units = live_tiles * n_chunks;
-        const int2 it = items[item];
-        const int grp = it.x, eb = it.y;
-        const uint8_t* blob = reinterpret_cast<const uint8_t*>(a.grp_ptr[grp]);
-        const int e1 = min(a.grp_start[grp + 1], (int) a.cap_entries);
-        const int ntok = min(kEntQ, e1 - eb);
+        const uint8_t* blob = reinterpret_cast<const uint8_t*>(pass.blob);
+        const int eb = pass.eb, ntok = pass.ntok;
         const int ncol = 2 * ntok;
+        const bool wide = NB > 1 && ntok > kEntQ;
+        __syncthreads();   // the previous pass is done with xs, cs and s_ir
         if (threadIdx.x < ntok) s_ir[threadIdx.x] = (MODE == QMODE_GU && a.n_x_rows > 0) ? a.ent_tok[eb + threadIdx.x] : eb + (int) threadIdx.x;
         __syncthreads();
         // the pass's activation columns (and their correction bytes): column c = 2 entry + term.  Columns beyond ncol keep
@@ -388,12 +441,10 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
                 const int c = i / per_col, q = i - c * per_col;
                 cpa16(xs_s + (uint32_t) (c * cstride + q * 16), img + ((size_t) s_ir[c >> 1] * 2 + (c & 1)) * K + (size_t) q * 16);
             }
-            if (Q::kCorr) {
-                const int per_cc = nblk * 4;
-                for (int i = threadIdx.x; i < ncol * per_cc; i += kThreads) {
-                    const int c = i / per_cc, q = i - c * per_cc;
-                    cpa16(cs_s + (uint32_t) (c * xstride + q * 16), corr + ((size_t) s_ir[c >> 1] * 2 + (c & 1)) * nblk * 64 + (size_t) q * 16);
-                }
+            const int per_cc = nblk * (kCorrBytes<TYPE> / 16);
+            for (int i = threadIdx.x; i < ncol * per_cc; i += kThreads) {
+                const int c = i / per_cc, q = i - c * per_cc;
+                cpa16(cs_s + (uint32_t) (c * xstride + q * 16), corr + ((size_t) s_ir[c >> 1] * 2 + (c & 1)) * nblk * kCorrBytes<TYPE> + (size_t) q * 16);
             }
             cpa_commit();
         }
@@ -401,7 +452,7 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
         const uint8_t* row0 = MODE == QMODE_GU ? blob + (size_t) r0 * a.L.gu_row : blob + a.L.down_off + (size_t) r0 * a.L.d_row;
         const size_t pitch0 = row_bytes, pitch1 = MODE == QMODE_GU ? (size_t) a.L.up_row : row_bytes;
         const size_t half = MODE == QMODE_GU ? (size_t) a.L.up_off + (size_t) r0 * (a.L.up_row - a.L.gu_row) : 8 * row_bytes;
-        const size_t tile_bytes = (size_t) tile_stride * row_bytes;
+        const size_t tile_bytes = (size_t) kStepRows * row_bytes;
         int iss_unit = 0, iss_chunk = 0;
         size_t iss_tile = 0;
         auto issue = [&]() {
@@ -450,16 +501,24 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
         cpa_wait<kStages - 1>();   // the activation group (the oldest) has landed
         __syncthreads();
 
-        // epilogue constants of this thread's entry (columns 2 t, 2 t + 1)
-        float f = 0.f;
-        int64_t orow = 0;
-        if (t < ntok) {
-            f = inv[s_ir[t]] * (Q::kCorr ? 0.125f : 1.f);
-            orow = MODE == QMODE_GU ? (int64_t) (eb + t) * a.L.n_ff : (int64_t) a.ent_dst[eb + t] * a.L.n_embd;
+        // epilogue constants of this thread's entries (columns 2 t, 2 t + 1 of each column block)
+        float f[NB];
+        int64_t orow[NB];
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+            const int j = kEntQ * n + t;
+            f[n] = 0.f;
+            orow[n] = 0;
+            if (j < ntok) {
+                f[n] = inv[s_ir[j]] * (TYPE == kTypeIQ1M ? 0.125f : 1.f);
+                orow[n] = MODE == QMODE_GU ? (int64_t) (eb + j) * a.L.n_ff : (int64_t) a.ent_dst[eb + j] * a.L.n_embd;
+            }
         }
-        float tot[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint8_t* bcol = xs + (size_t) g * cstride + (Q::kCorr ? 8 * t : 4 * t);
-        const uint8_t* ccol = cs + (size_t) g * xstride;
+        float tot[NB][4];
+#pragma unroll
+        for (int n = 0; n < NB; ++n) tot[n][0] = tot[n][1] = tot[n][2] = tot[n][3] = 0.f;
+        const uint8_t* bcol = xs + (size_t) g * cstride + (TYPE == kTypeIQ1M ? 8 * t : 4 * t);
+        const uint8_t* ccol = cs + (size_t) g * xstride + (TYPE == kTypeIQ1M ? 0 : 4 * t);
         int tile = 0, chunk = 0;
         for (int unit = 0; unit < n_units; ++unit) {
             issue();
@@ -472,116 +531,163 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
                 const int at = CB == 2 ? b * Q::kBlock : 2 * ((chunk0 + chunk) & 1);
                 const uint8_t* ra = st + g * kRow + at;
                 const uint8_t* rbp = st + (g + 8) * kRow + at;
-                if constexpr (Q::kCorr) iq1m_block<NC>(ra, rbp, tab + (lane & (NC - 1)), bcol + 256 * blk, ccol + 64 * blk, t, tot);
-                else q6k_block(ra, rbp, bcol + 256 * blk, t, tot);
+                const uint8_t *bc = bcol + 256 * blk, *cc = ccol + kCorrBytes<TYPE> * blk;
+                if constexpr (TYPE == kTypeIQ1M) iq1m_block<NC, NB>(ra, rbp, tab + (lane & (NC - 1)), bc, cc, kColsQ * cstride, kColsQ * xstride, wide, t, tot);
+                else if (blk & 1) q6k_block<NB, true>(ra, rbp, bc, cc, kColsQ * cstride, kColsQ * xstride, wide, t, tot);
+                else q6k_block<NB, false>(ra, rbp, bc, cc, kColsQ * cstride, kColsQ * xstride, wide, t, tot);
             }
             __syncwarp();   // every lane is done with this stage before a later issue overwrites it
             if (++chunk != n_chunks) continue;
-            if constexpr (KS > 1) break;       // one tile a unit: the parts are put together below
-            const int64_t rt = r0 + (int64_t) tile * tile_stride;
+            const int64_t rt = r0 + (int64_t) tile * kStepRows;
             chunk = 0;
-            ++tile;
-            const float v0 = (tot[0] + tot[1] * kTerm2) * f, v1 = (tot[2] + tot[3] * kTerm2) * f;
-            tot[0] = tot[1] = tot[2] = tot[3] = 0.f;
-            if (t < ntok) {
-                if (MODE == QMODE_GU) {
-                    a.h[orow + rt + g] = swiglu(v0, v1, a.L);
-                } else {
-                    store_out(a.out, a.out_kind, orow + rt + g, v0);
-                    store_out(a.out, a.out_kind, orow + rt + g + 8, v1);
-                }
-            }
-        }
-        if constexpr (KS > 1) {
-            __shared__ float4 part[kWarps][32];
-            if (n_units > 0) part[warp][lane] = make_float4(tot[0], tot[1], tot[2], tot[3]);
-            __syncthreads();
-            if (n_units > 0 && warp % KS == 0 && t < ntok) {
-                float4 v = part[warp][lane];
+            float2 v[NB];
 #pragma unroll
-                for (int k = 1; k < KS; ++k) {
-                    const float4 o = part[warp + k][lane];
-                    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-                }
-                const float v0 = (v.x + v.y * kTerm2) * f, v1 = (v.z + v.w * kTerm2) * f;
-                if (MODE == QMODE_GU) {
-                    a.h[orow + r0 + g] = swiglu(v0, v1, a.L);
-                } else {
-                    store_out(a.out, a.out_kind, orow + r0 + g, v0);
-                    store_out(a.out, a.out_kind, orow + r0 + g + 8, v1);
+            for (int n = 0; n < NB; ++n) {
+                v[n] = make_float2(tot[n][0] + tot[n][1] * kTerm2, tot[n][2] + tot[n][3] * kTerm2);
+                tot[n][0] = tot[n][1] = tot[n][2] = tot[n][3] = 0.f;
+            }
+            if constexpr (KS > 1) {
+                // the tile's other warps hand their sums to its first; two buffers, so one barrier of the tile's warps is enough: a
+                // buffer is written again only after the barrier of the tile in between, which its reader has passed
+                float2* buf = part + ((size_t) (tile & 1) * kTiles + warp / KS) * (KS - 1) * NB * 32 + lane;
+                if (warp % KS != 0)
+#pragma unroll
+                    for (int n = 0; n < NB; ++n) buf[((warp % KS - 1) * NB + n) * 32] = v[n];
+                asm volatile("bar.sync %0, %1;\n" ::"r"(1 + warp / KS), "n"(KS * 32) : "memory");
+                if (warp % KS == 0)
+#pragma unroll
+                    for (int n = 0; n < NB; ++n)
+#pragma unroll
+                        for (int k = 0; k < KS - 1; ++k) {
+                            const float2 o = buf[(k * NB + n) * 32];
+                            v[n].x += o.x;
+                            v[n].y += o.y;
+                        }
+            }
+            ++tile;
+            if (KS == 1 || warp % KS == 0) {
+#pragma unroll
+                for (int n = 0; n < NB; ++n) {
+                    if (kEntQ * n + t < ntok) {
+                        if (MODE == QMODE_GU) {
+                            a.h[orow[n] + rt + g] = swiglu(v[n].x * f[n], v[n].y * f[n], a.L);
+                        } else {
+                            store_out(a.out, a.out_kind, orow[n] + rt + g, v[n].x * f[n]);
+                            store_out(a.out, a.out_kind, orow[n] + rt + g + 8, v[n].y * f[n]);
+                        }
+                    }
                 }
             }
         }
         cpa_wait<0>();
     }
-    cpa_wait<0>();
 }
 
 size_t al256q(size_t v) { return (v + 255) & ~(size_t) 255; }
 
+// shared memory that a block may ask for, alone on its SM or one of two (227 and 113 KB less the static words)
+constexpr size_t kSmemOne = 232448 - 256, kSmemTwo = 115712 - 256;
+
 template <int TYPE>
-size_t kq_smem(int64_t K, int copies = 2, int stages = 3, int cb = 2) {
+size_t kq_smem(int64_t K, int W, int KS, int NC, int ST, int CB, int NB) {
     using Q = QT<TYPE>;
-    return (size_t) kColsQ * (K + Q::kPad) + (Q::kCorr ? (size_t) kColsQ * ((K >> 8) * 64 + 16) + (size_t) 16384 * copies : 0) +
-           (size_t) Q::kWarps * stages * kRowsQ * (cb == 1 ? kRowStage<TYPE, 1> : kRowStage<TYPE, 2>) + 128;
+    return (size_t) kColsQ * NB * (K + Q::kPad) + (size_t) kColsQ * NB * ((K >> 8) * kCorrBytes<TYPE> + 16) + (TYPE == kTypeIQ1M ? (size_t) 16384 * NC : 0) +
+           (size_t) W * ST * kRowsQ * (CB == 1 ? kRowStage<TYPE, 1> : kRowStage<TYPE, 2>) + (size_t) W / KS * (KS - 1) * NB * 512 + 128;
 }
 
-template <int TYPE, int MODE, int KS, int NC, int ST, int CB>
-int32_t kq_launch_split(const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const int2* items, int* n_items, int tpw, cudaStream_t st) {
-    using Q = QT<TYPE>;
-    const size_t smem = kq_smem<TYPE>(MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff, NC, ST, CB);
+template <int TYPE, int MODE, int W, int OCC, int KS, int NC, int ST, int CB, int NB>
+int32_t kq_launch_as(const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const PassRec* items, const int* n_items, cudaStream_t st) {
+    const size_t smem = kq_smem<TYPE>(MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff, W, KS, NC, ST, CB, NB);
     static std::atomic<bool> configured[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(kq_mma_kernel<TYPE, MODE, KS, NC, ST, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, KS > 1 ? 220 * 1024 : 225 * 1024);
+        const cudaError_t e = cudaFuncSetAttribute(kq_mma_kernel<TYPE, MODE, W, OCC, KS, NC, ST, CB, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int) (OCC == 2 ? kSmemTwo : kSmemOne));
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
-    const int64_t rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd, tile_rows = (MODE == QMODE_GU ? 8 : 16) * Q::kWarps / KS;
-    const int64_t n_tiles = (rows + tile_rows - 1) / tile_rows;
-    const int n_row_blocks = (int) ((n_tiles + tpw - 1) / tpw);
-    const int per_sm = CB == 1 && ST == 3 ? 2 : 1;
-    launch_k(kq_mma_kernel<TYPE, MODE, KS, NC, ST, CB>, dim3((unsigned) (per_sm * sm_count())), dim3(Q::kWarps * 32), smem, st, a, img, corr, inv, items, n_items, tpw,
-             n_row_blocks);
+    const int64_t rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd, step_rows = (MODE == QMODE_GU ? 8 : 16) * W / KS;
+    launch_k(kq_mma_kernel<TYPE, MODE, W, OCC, KS, NC, ST, CB, NB>, dim3((unsigned) (OCC * sm_count())), dim3(W * 32), smem, st, a, img, corr, inv, items, n_items,
+             (int) ((rows + step_rows - 1) / step_rows));
     return launch_status();
 }
 
-template <int TYPE, int MODE>
-int32_t kq_launch(const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const int2* items, int* n_items, cudaStream_t st) {
-    using Q = QT<TYPE>;
-    const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
-    const int64_t rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd;
-    const int64_t row_bytes = K / 256 * Q::kBlock;
-    const int64_t tile_bytes = (int64_t) Q::kWarps * kRowsQ * row_bytes;                 // one row tile of every warp
-    const int64_t tile_rows = (MODE == QMODE_GU ? 8 : 16) * Q::kWarps;
-    const int64_t n_tiles = (rows + tile_rows - 1) / tile_rows;
-    int64_t tpw0 = (384 * 1024 + tile_bytes - 1) / tile_bytes;                           // a unit streams ~400 KB
-    tpw0 = tpw0 < 1 ? 1 : tpw0 > 8 ? 8 : tpw0;
-    const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
-    const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
-    if constexpr (TYPE == kTypeQ6K) {
-        // Where even one row tile a warp and unit cannot reach every SM (at most a pass per group and one per four entries), the columns
-        // are split too.  cap_groups and cap_entries bound the passes on the host.
-        const int64_t passes = a.cap_groups + a.cap_entries / kEntQ, units = passes * n_tiles, chunks = K / 256;
-        if (kq_smem<TYPE>(K, 0, 3, 1) <= 108 * 1024) {                                   // two blocks an SM
-            if (units >= sm_count()) {
-                // two tiles where one is less than 64 KB (down rows of 512 columns) and the units still go round the SMs four times:
-                // 2048 x 512, 512 experts, 64 tokens 331 us against 342 with one; at 32 tokens 226 against 230
-                const int two = tile_bytes < 64 * 1024 && units >= 2 * 4 * 2 * (int64_t) sm_count() ? 2 : 1;
-                return kq_launch_split<TYPE, MODE, 1, 1, 3, 1>(a, img, corr, inv, items, n_items, two, st);
-            }
-            if (chunks % 8 == 0) return kq_launch_split<TYPE, MODE, 8, 1, 3, 1>(a, img, corr, inv, items, n_items, 1, st);
-            if (chunks % 4 == 0) return kq_launch_split<TYPE, MODE, 4, 1, 3, 1>(a, img, corr, inv, items, n_items, 1, st);
-            return kq_launch_split<TYPE, MODE, 2, 1, 3, 1>(a, img, corr, inv, items, n_items, 1, st);      // whole 512-column rows
-        }
-        if (units < sm_count() && chunks % 4 == 0) return kq_launch_split<TYPE, MODE, 4, 1, 5, 1>(a, img, corr, inv, items, n_items, 1, st);
-        return kq_launch_split<TYPE, MODE, 1, 1, 3, 2>(a, img, corr, inv, items, n_items, tpw, st);
+// The shape of a product's launch: OCC blocks an SM, KS warps to a row tile, NB column blocks (4 NB entries) a pass.  Q6_K: two blocks of
+// eight warps where shared memory holds two (K up to about 5000), which hide each other's first loads (2048 x 512, 512 experts, 64 tokens:
+// one block of 16 warps 365 us, two of eight 312); wider rows one block of 16 warps (7168 x 2048: 2178 us, of eight 2668).  Two column
+// blocks where they fit, for a pass of four or fewer entries multiplies one; four, or two and twelve warps, only where the groups are deep
+// (a shared expert of 64 tokens, 7168 x 2048: gate/up 113 us with one, 76 with two).
+struct KqShape { int OCC, KS, NB; };
+
+// cap_groups and cap_entries bound the passes on the host.
+template <int TYPE>
+KqShape kq_shape(const ExpertArgs& a, bool gu) {
+    const int64_t K = gu ? a.L.n_embd : a.L.n_ff, rows = gu ? a.L.n_ff : a.L.n_embd;
+    const bool deep = a.cap_entries >= 8 * a.cap_groups;
+    KqShape s{1, 1, 1};
+    int W = 16, most = 2;
+    if (TYPE == kTypeIQ1M) {
+        if (kq_smem<TYPE>(K, 16, 2, 4, 3, 2, 2) <= kSmemOne) s.NB = 2;
     } else {
-        // four copies of the codebook where they fit beside the columns and the stages (K up to 7680), else two
-        if (kq_smem<TYPE>(K, 4) <= 225 * 1024) return kq_launch_split<TYPE, MODE, 1, 4, 3, 2>(a, img, corr, inv, items, n_items, tpw, st);
-        return kq_launch_split<TYPE, MODE, 1, 2, 3, 2>(a, img, corr, inv, items, n_items, tpw, st);
+        W = 8;
+        if (deep && kq_smem<TYPE>(K, 8, 2, 1, 2, 1, 4) <= kSmemTwo) { s.OCC = 2; s.NB = 4; }
+        else if (kq_smem<TYPE>(K, 8, 8, 1, 2, 1, 2) <= kSmemTwo) { s.OCC = 2; s.NB = 2; most = 8; }
+        else if (!deep && kq_smem<TYPE>(K, 8, 4, 1, 2, 1, 1) <= kSmemTwo) { s.OCC = 2; most = 4; }
+        else {
+            s.NB = deep && kq_smem<TYPE>(K, 12, 4, 1, 2, 1, 2) <= kSmemOne ? 2 : 1;
+            W = s.NB == 2 ? 12 : 16;
+            most = 4;
+        }
     }
+    // Columns are split where whole rows would leave a block few steps, so that the last, partial one weighs little
+    const int64_t chunks = K / (TYPE == kTypeIQ1M ? 512 : 256), step_rows = (gu ? 8 : 16) * W;
+    const int64_t steps = (a.cap_groups + a.cap_entries / (kEntQ * s.NB)) * ((rows + step_rows - 1) / step_rows);
+    while (s.KS < most && chunks % (2 * s.KS) == 0 && steps * s.KS < 8 * (int64_t) s.OCC * sm_count()) s.KS *= 2;
+    return s;
+}
+
+template <int TYPE, int MODE>
+int32_t kq_launch(const KqShape& s, const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const PassRec* items, const int* n_items, cudaStream_t st) {
+    const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
+#define KQ_AS(W, OCC, KS, NC, ST, CB, NB) return kq_launch_as<TYPE, MODE, W, OCC, KS, NC, ST, CB, NB>(a, img, corr, inv, items, n_items, st)
+    if constexpr (TYPE == kTypeQ6K) {
+        if (s.OCC == 2 && s.NB == 4) {
+            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 1, 4);
+            KQ_AS(8, 2, 1, 1, 2, 1, 4);
+        }
+        if (s.OCC == 2 && s.NB == 2) {
+            if (s.KS == 8) KQ_AS(8, 2, 8, 1, 2, 1, 2);
+            if (s.KS == 4) KQ_AS(8, 2, 4, 1, 2, 1, 2);
+            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 1, 2);
+            KQ_AS(8, 2, 1, 1, 2, 1, 2);
+        }
+        if (s.OCC == 2) {
+            if (s.KS == 4) KQ_AS(8, 2, 4, 1, 2, 1, 1);
+            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 1, 1);
+            KQ_AS(8, 2, 1, 1, 2, 1, 1);
+        }
+        if (s.NB == 2) {
+            if (s.KS == 4) KQ_AS(12, 1, 4, 1, 2, 1, 2);
+            if (s.KS == 2) KQ_AS(12, 1, 2, 1, 2, 1, 2);
+            KQ_AS(12, 1, 1, 1, 2, 1, 2);
+        }
+        if (s.KS == 4) KQ_AS(16, 1, 4, 1, 2, 1, 1);
+        if (s.KS == 2) KQ_AS(16, 1, 2, 1, 2, 1, 1);
+        KQ_AS(16, 1, 1, 1, 2, 1, 1);
+    } else {
+        if (s.NB == 2) {
+            if (s.KS == 2) KQ_AS(16, 1, 2, 4, 3, 2, 2);
+            KQ_AS(16, 1, 1, 4, 3, 2, 2);
+        }
+        // four copies of the codebook where they fit beside the columns and the stages (K up to 7680), else two
+        if (kq_smem<TYPE>(K, 16, 2, 4, 3, 2, 1) <= kSmemOne) {
+            if (s.KS == 2) KQ_AS(16, 1, 2, 4, 3, 2, 1);
+            KQ_AS(16, 1, 1, 4, 3, 2, 1);
+        }
+        KQ_AS(16, 1, 1, 2, 3, 2, 1);
+    }
+#undef KQ_AS
 }
 
 bool kq_type(int t) { return t == kTypeIQ1M || t == kTypeQ6K; }
@@ -598,15 +704,15 @@ bool kq_dim_ok(int type, int64_t K, int64_t rows) {
 // scratch beyond the SwiGLU buffer: x images, h images (2 int8 terms each), their correction bytes, inverse scales, pass list
 size_t experts_kq_scratch_bytes(int64_t cap, int64_t H, int64_t I) {
     return al256q((size_t) cap * 2 * H) + al256q((size_t) cap * 2 * I) + al256q((size_t) cap * 2 * (H / 256) * 64) + al256q((size_t) cap * 2 * (I / 256 + 1) * 64) +
-           2 * al256q((size_t) cap * 4) + al256q((size_t) (cap + 1) * 8 + 16);
+           2 * al256q((size_t) cap * 4) + al256q((size_t) (cap + 1) * 16 + 16);
 }
 
 int32_t experts_grouped_kq(const ExpertArgs& a, cudaStream_t st) {
     const bsx_expert_layout& L = a.L;
     if (!kq_type(L.gu_type) || L.up_type != L.gu_type || !kq_type(L.d_type)) return BSX_E_TYPE;
     if (!kq_dim_ok(L.gu_type, L.n_embd, L.n_ff) || !kq_dim_ok(L.d_type, L.n_ff, L.n_embd) || L.n_embd % 16) return BSX_E_TYPE;
-    if (L.gu_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_embd) > 225 * 1024 : L.n_embd > kMaxColsQ6K) return BSX_E_TYPE;
-    if (L.d_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_ff) > 225 * 1024 : L.n_ff > kMaxColsQ6K) return BSX_E_TYPE;
+    if (L.gu_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_embd, 16, 1, 2, 3, 2, 1) > kSmemOne : L.n_embd > kMaxColsQ6K) return BSX_E_TYPE;
+    if (L.d_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_ff, 16, 1, 2, 3, 2, 1) > kSmemOne : L.n_ff > kMaxColsQ6K) return BSX_E_TYPE;
     const int64_t cap = a.cap_entries, H = L.n_embd, I = L.n_ff;
     uint8_t* p = reinterpret_cast<uint8_t*>(a.h) + al256q((size_t) cap * I * 4);
     int8_t* ximg = reinterpret_cast<int8_t*>(p);
@@ -622,27 +728,29 @@ int32_t experts_grouped_kq(const ExpertArgs& a, cudaStream_t st) {
     float* hinv = reinterpret_cast<float*>(p);
     p += al256q((size_t) cap * 4);
     int* n_items = reinterpret_cast<int*>(p);
-    int2* items = reinterpret_cast<int2*>(n_items + 4);
+    PassRec* items = reinterpret_cast<PassRec*>(n_items + 4);
     const int phase = experts_phase(a.L);
     const int64_t x_rows = a.n_x_rows > 0 ? a.n_x_rows : cap;
     const unsigned nbx = (unsigned) ((x_rows + 7) / 8 + 1), nbh = (unsigned) ((cap + 7) / 8 + 1);
     int32_t rc = BSX_OK;
+    const KqShape gu = L.gu_type == kTypeIQ1M ? kq_shape<kTypeIQ1M>(a, true) : kq_shape<kTypeQ6K>(a, true);
+    const KqShape dn = L.d_type == kTypeIQ1M ? kq_shape<kTypeIQ1M>(a, false) : kq_shape<kTypeQ6K>(a, false);
     if (phase != 2) {
         if (L.gu_type == kTypeIQ1M) {
-            launch_k(kq_image_kernel<false, true>, dim3(nbx), dim3(256), 0, st, a, ximg, xcorr, xinv, items, n_items);
-            rc = kq_launch<kTypeIQ1M, QMODE_GU>(a, ximg, xcorr, xinv, items, n_items, st);
+            launch_k(kq_image_kernel<false, kTypeIQ1M>, dim3(nbx), dim3(256), 0, st, a, ximg, xcorr, xinv, items, n_items, kEntQ * gu.NB);
+            rc = kq_launch<kTypeIQ1M, QMODE_GU>(gu, a, ximg, xcorr, xinv, items, n_items, st);
         } else {
-            launch_k(kq_image_kernel<false, false>, dim3(nbx), dim3(256), 0, st, a, ximg, xcorr, xinv, items, n_items);
-            rc = kq_launch<kTypeQ6K, QMODE_GU>(a, ximg, xcorr, xinv, items, n_items, st);
+            launch_k(kq_image_kernel<false, kTypeQ6K>, dim3(nbx), dim3(256), 0, st, a, ximg, xcorr, xinv, items, n_items, kEntQ * gu.NB);
+            rc = kq_launch<kTypeQ6K, QMODE_GU>(gu, a, ximg, xcorr, xinv, items, n_items, st);
         }
     }
     if (rc != BSX_OK || phase == 1) return rc;
     if (L.d_type == kTypeIQ1M) {
-        launch_k(kq_image_kernel<true, true>, dim3(nbh), dim3(256), 0, st, a, himg, hcorr, hinv, items, n_items);
-        return kq_launch<kTypeIQ1M, QMODE_DOWN>(a, himg, hcorr, hinv, items, n_items, st);
+        launch_k(kq_image_kernel<true, kTypeIQ1M>, dim3(nbh), dim3(256), 0, st, a, himg, hcorr, hinv, items, n_items, kEntQ * dn.NB);
+        return kq_launch<kTypeIQ1M, QMODE_DOWN>(dn, a, himg, hcorr, hinv, items, n_items, st);
     }
-    launch_k(kq_image_kernel<true, false>, dim3(nbh), dim3(256), 0, st, a, himg, hcorr, hinv, items, n_items);
-    return kq_launch<kTypeQ6K, QMODE_DOWN>(a, himg, hcorr, hinv, items, n_items, st);
+    launch_k(kq_image_kernel<true, kTypeQ6K>, dim3(nbh), dim3(256), 0, st, a, himg, hcorr, hinv, items, n_items, kEntQ * dn.NB);
+    return kq_launch<kTypeQ6K, QMODE_DOWN>(dn, a, himg, hcorr, hinv, items, n_items, st);
 }
 
 }  // namespace bsx

@@ -39,3 +39,27 @@ def test_rows_beyond_the_integer_kernel_keep_their_24_bits(lib, cuda, H, I):
     x = rng.standard_normal((3, H)).astype(np.float32)
     out = run_grouped(L, dev(stack_blobs(blobs)), [0], [[0, 1, 2]], dev(x), 3).cpu().numpy()
     assert rel_l2(out, O.expert_forward(Lo, blobs[0], x, dtype=np.float64)) < 1e-5
+
+
+@pytest.mark.parametrize("t,H,I", [(O.T_Q6_K, 512, 512), (O.T_Q6_K, 1536, 1024), (O.T_Q6_K, 5632, 1024), (O.T_Q6_K, 7168, 512), (O.T_Q6_K, 512, 8192),
+                                   (O.T_IQ1_M, 2048, 512), (O.T_IQ1_M, 7168, 512), (O.T_IQ1_M, 512, 5120)])
+@pytest.mark.parametrize("sizes", [[41], [1, 4, 5, 8, 9], [3] * 33], ids=["deep", "ragged", "many"])
+def test_column_blocks_and_runs(lib, cuda, t, H, I, sizes):
+    """One, two and four column blocks a pass, full and ragged; one or two blocks an SM; rows split over warps or not; runs of row blocks
+    that end inside a pass, and row blocks that the rows do not fill (512 over the three tiles of twelve warps)."""
+    rng = np.random.default_rng(H + I + len(sizes))
+    Lo, blobs = make_expert_blobs(rng, 2, t, t, H, I)
+    L = moe.native_expert_layout(t, t, H, I)
+    xd = dev(rng.standard_normal((41, H)).astype(np.float32))
+    x = xd.cpu().numpy()
+    groups, at = [], 0
+    for n in sizes:
+        groups.append([(at + j) % 41 for j in range(n)])
+        at += n
+    ids = [i % 2 for i in range(len(groups))]
+    out = run_grouped(L, dev(stack_blobs(blobs)), ids, groups, xd, at).cpu().numpy()
+    want = {e: O.expert_forward(Lo, blobs[e], x, dtype=np.float64) for e in set(ids)}
+    at = 0
+    for e, toks in zip(ids, groups):
+        assert rel_l2(out[at:at + len(toks)], want[e][toks]) < 4e-4, (e, toks, rel_l2(out[at:at + len(toks)], want[e][toks]))
+        at += len(toks)
