@@ -3,8 +3,8 @@
 //
 // Shape of the work (HBM-bound): every touched expert's gate, up and down rows are read exactly once per pass of up to 8
 // activation columns.  Each warp owns 16 weight rows (8 gate rows paired with the 8 matching up rows, or 16 down rows) and
-// streams them in 256-column chunks (144 bytes a row) through its own 4-stage cp.async ring, so no block-wide barrier sits
-// in the stream and ~110 KB a SM is in flight.  A row's E2M1 codes go to fp16 pairs with cvt.rn.f16x2.e2m1x2 (one ALU-pipe
+// streams them in 256-column chunks (144 bytes a row) through its own cp.async ring of two or three stages, so no block-wide barrier
+// sits in the stream.  A row's E2M1 codes go to fp16 pairs with cvt.rn.f16x2.e2m1x2 (one ALU-pipe
 // instruction per byte, the scarce resource here: the ALU pipe issues at half rate), are multiplied by the block's UE4M3
 // scale as fp16 (the product has at most 5 significant bits: exact; the scale comes from a 256-entry shared-memory table)
 // and feed mma.sync.m16n8k16 with fp32 accumulation.  Each of a row group's four threads owns one 16-value sub-block, so it
@@ -14,8 +14,11 @@
 // accumulators, so SwiGLU is fused; a second small kernel turns the SwiGLU output into the down product's fp16 image.
 //
 // IQ3_S rows take the same stream with another decoder (iq3s_16): codebook points as four fp16 magnitudes in shared memory, signs
-// and the odd scales applied in packed fp16, exactly.  Bound by the decode's integer work and look-ups.  5 tokens through 512
-// experts of 2048 x 512, top-10: the layer's step took 315 us with the warp-per-row fp32 kernels and 155 with this one.
+// and the odd scales applied in packed fp16, exactly.  Bound by the decode's integer work and look-ups.
+//
+// What the launch shape is worth (equal runs of row blocks, sixteen warps an SM, whole-row or split tiles: launch() below), 2048 x 512 unless
+// said: IQ3_S, 512 experts, 5 tokens 125 -> 99 us, 64 tokens 420 -> 305; NVFP4, 1 token 52 -> 34, 64 tokens 169 -> 154, 27 tokens of
+// 2560 x 640 223 -> 175.
 //
 // Semantics: Basalt's native_expert_grouped (include/basalt/kernels/iq_kernels.hpp:77-92; kernels src/kernels/cuda/iq_kernels.cu:
 // 1605-1658 gate/up, :2512-2524 SwiGLU, :2140-2164 down), NVFP4 decoding per src/kernels/cpu/ggml/ggml_quants.c:1397-1422,
@@ -27,13 +30,11 @@
 #include "experts.cuh"
 #include "formats.cuh"
 #include "pdl.cuh"
+#include "plan.cuh"
 
 namespace bsx {
 namespace {
 
-constexpr int kWarps = 8;
-constexpr int kThreads = kWarps * 32;
-constexpr int kStages = 4;
 constexpr int kRows = 16;                      // weight rows per warp
 constexpr int kCols = 8;                       // MMA n: activation columns per pass
 
@@ -91,6 +92,12 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void mma_f16_zero(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 // UE4M3 scale byte -> fp16 pair {d, d} with d = scale / 2^8: (byte & 0x7F) << 7 puts E4M3's exponent and mantissa where
 // fp16 keeps them (value 2^(e-15) (1 + m/8), subnormals included) while the scale itself is 2^(e-7) (1 + m/8) (ggml halves
 // it only because its E2M1 table is doubled; the cvt above yields undoubled values), so the epilogue multiplies the sums
@@ -104,7 +111,9 @@ __device__ __forceinline__ uint32_t scale_pair_bits(uint32_t byte) {
 // IQ3_S (include/basalt/ggml/ggml_common.h block_iq3_s: fp16 d, qs[64], qh[8], signs[32], scales[4]; decode rule
 // src/kernels/cpu/ggml/ggml_quants.c:1200-1239): a weight is d (2 s + 1) x +-(2 c + 1), c a 3-bit coordinate of a 512-point
 // codebook.  One thread decodes the 16 values [16 t, 16 t + 16) of granule `gr` (64 columns) of a row's block: four points, 16 sign
-// bits, one scale.  Magnitude x scale is an integer up to 465, exact in fp16; d stays outside the sums.  q[i]: values i and i + 8.
+// bits, one scale.  Magnitude x scale is an integer up to 465, exact in fp16; d stays outside the sums.  q[i]: values 2 i and 2 i + 1,
+// as a point holds them.  points: the lane's copy of the codebook, NC copies interleaved point by point.
+template <int NC>
 __device__ __forceinline__ void iq3s_16(const uint8_t* blk, int gr, int t, const uint2* __restrict__ points, uint32_t (&q)[8]) {
     const int ib = 2 * gr + (t >> 1), half = t & 1;
     const uint16_t* qs = reinterpret_cast<const uint16_t*>(blk + 2 + 8 * ib + 4 * half);
@@ -116,37 +125,18 @@ __device__ __forceinline__ void iq3s_16(const uint8_t* blk, int gr, int t, const
     const __half2 m = __hsub2(__halves2half2(__ushort_as_half((unsigned short) (0x6400u + 2u * s + 1u)), __ushort_as_half((unsigned short) (0x6400u + 2u * s + 1u))),
                               __float2half2_rn(1024.f));
     const uint32_t mm = *reinterpret_cast<const uint32_t*>(&m);
-    const uint2 p0 = points[(q01 & 0xFFu) | ((qh & 1u) << 8)], p1 = points[(q01 >> 8) | ((qh & 2u) << 7)];
-    const uint2 p2 = points[(q23 & 0xFFu) | ((qh & 4u) << 6)], p3 = points[(q23 >> 8) | ((qh & 8u) << 5)];
-    const uint32_t sw = __byte_perm(sg, 0u, 0x4140);                             // signs of values 0-7 low, of 8-15 high half
-    q[0] = __byte_perm(p0.x, p2.x, 0x5410);
-    q[1] = __byte_perm(p0.x, p2.x, 0x7632);
-    q[2] = __byte_perm(p0.y, p2.y, 0x5410);
-    q[3] = __byte_perm(p0.y, p2.y, 0x7632);
-    q[4] = __byte_perm(p1.x, p3.x, 0x5410);
-    q[5] = __byte_perm(p1.x, p3.x, 0x7632);
-    q[6] = __byte_perm(p1.y, p3.y, 0x5410);
-    q[7] = __byte_perm(p1.y, p3.y, 0x7632);
+    const uint2 p0 = points[((q01 & 0xFFu) | ((qh & 1u) << 8)) * NC], p1 = points[((q01 >> 8) | ((qh & 2u) << 7)) * NC];
+    const uint2 p2 = points[((q23 & 0xFFu) | ((qh & 4u) << 6)) * NC], p3 = points[((q23 >> 8) | ((qh & 8u) << 5)) * NC];
+    const uint32_t sw = sg | (sg << 15);                                         // signs 2 i at bit 2 i, signs 2 i + 1 sixteen above
+    const uint32_t v[8] = {p0.x, p0.y, p1.x, p1.y, p2.x, p2.y, p3.x, p3.y};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = hmul2_bits(q[i] ^ ((sw << (15 - i)) & 0x80008000u), mm);
+    for (int i = 0; i < 8; ++i) q[i] = hmul2_bits(v[i] ^ ((sw << (15 - 2 * i)) & 0x80008000u), mm);
 }
 
-// Where column c of an activation row sits in its fp16 image, which is laid out so that a thread's B fragments are two
-// 16-byte pieces per 64 columns: piece (gran, h, t) holds, for sub-block t of granule gran, the values the thread with
-// id-in-group t needs for MMA steps 2h and 2h + 1.  Step s takes code bytes 2s and 2s + 1 of the sub-block's 8 bytes; byte b
-// holds values b (low nibble -> k slot 2t) and b + 8 (high nibble -> k slot 2t + 1), bytes 2s + 1 go to slots 2t + 8, 2t + 9.
-__device__ __forceinline__ int image_index(int c) {
-    const int gran = c >> 6, t = (c >> 4) & 3, jj = c & 15, b = jj & 7, half = jj >> 3;
-    const int step = b >> 1, reg = b & 1;
-    return (((gran * 2 + (step >> 1)) * 4 + t) << 3) + 4 * (step & 1) + 2 * reg + half;
-}
-
-__device__ __forceinline__ float load_x(const void* x, int kind, int64_t row, int64_t K, int c) {
-    if (kind == BSX_X_F32) return static_cast<const float*>(x)[row * K + c];
-    if (kind == BSX_X_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(x)[row * K + c]);
-    const uint8_t* b = static_cast<const uint8_t*>(x) + (row * (K / 32) + (c >> 5)) * 36;
-    return __half2float(*reinterpret_cast<const __half*>(b)) * (float) (int8_t) b[4 + (c & 31)];
-}
+// An activation row's fp16 image is laid out so that a thread's B fragments are two 16-byte pieces per 64 columns: piece (gran, h, t)
+// holds, for sub-block t of granule gran, the values the thread with id-in-group t needs for MMA steps 2h and 2h + 1.  NVFP4: step s
+// takes code bytes 2s and 2s + 1 of the sub-block's 8 bytes; byte b holds values b (low nibble -> k slot 2t) and b + 8 (high nibble ->
+// k slot 2t + 1), bytes 2s + 1 go to slots 2t + 8, 2t + 9.  IQ3_S: the values in order (points hold neighbours).
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     return (uint32_t) __half_as_ushort(__float2half_rn(lo)) | ((uint32_t) __half_as_ushort(__float2half_rn(hi)) << 16);
@@ -161,10 +151,10 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 // FROM_H = false: rows of x (kind x_kind, width n_embd) - row i of x when the caller gave the number of x rows, else the
 // row of entry i; true: row e of the SwiGLU output h (fp32, width n_ff).
 // The last block lists the passes of the product that follows: a pass is up to 8 / TERMS consecutive entries of one group,
-// items[i] = {group, first entry}, so that kernel's blocks take one pass each however the entries are spread.
-template <bool FROM_H, int TERMS>
+// items[i] = {blob, first entry, entries}, so that kernel's blocks take passes however the entries are spread.
+template <int FMT, bool FROM_H, int TERMS>
 __global__ void __launch_bounds__(256)
-prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ inv, int2* __restrict__ items, int* __restrict__ n_items) {
+prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ inv, PassRec* __restrict__ items, int* __restrict__ n_items) {
     pdl_wait();
     pdl_launch_dependents();
     const int ng = min(*a.n_groups, (int) a.cap_groups);
@@ -191,15 +181,18 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
             __syncthreads();
             int before = s_base;
             for (int w = 0; w < warp; ++w) before += sh[w];
-            for (int p = 0; p < np; ++p) items[before + x - np + p] = make_int2(g, s0 + p * NTOK);
+            for (int p = 0; p < np; ++p) {
+                PassRec r;
+                r.blob = a.grp_ptr[g];
+                r.eb = s0 + p * NTOK;
+                r.ntok = min(NTOK, cnt - p * NTOK);
+                items[before + x - np + p] = r;
+            }
             __syncthreads();
             if (threadIdx.x == 255) s_base = before + x;
             __syncthreads();
         }
-        if (threadIdx.x == 0) {
-            n_items[0] = s_base;
-            n_items[1] = 0;      // the work counter of the product kernel that follows
-        }
+        if (threadIdx.x == 0) n_items[0] = s_base;
         return;
     }
     const int i = blockIdx.x * 8 + warp;   // image row
@@ -231,17 +224,21 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
         load16(src, kind, row, K, sb, v);
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = v[j] * s * s_rest;
-        // pieces (gran, 0, t) and (gran, 1, t): values {0,8,1,9,2,10,3,11} and {4,12,5,13,6,14,7,15}
+        // pieces (gran, 0, t) and (gran, 1, t): values {0,8,1,9,2,10,3,11} and {4,12,5,13,6,14,7,15}, or {0,...,7} and {8,...,15}
         const int piece = ((sb >> 2) * 2) * 4 + (sb & 3);
-        out[piece] = make_uint4(pack_half2(v[0], v[8]), pack_half2(v[1], v[9]), pack_half2(v[2], v[10]), pack_half2(v[3], v[11]));
-        out[piece + 4] = make_uint4(pack_half2(v[4], v[12]), pack_half2(v[5], v[13]), pack_half2(v[6], v[14]), pack_half2(v[7], v[15]));
+        auto store = [&](uint4* o, const float (&w)[16]) {
+            uint32_t u[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) u[j] = FMT == FMT_IQ3S ? pack_half2(w[2 * j], w[2 * j + 1]) : pack_half2(w[j], w[j + 8]);
+            o[piece] = make_uint4(u[0], u[1], u[2], u[3]);
+            o[piece + 4] = make_uint4(u[4], u[5], u[6], u[7]);
+        };
+        store(out, v);
         if (TERMS == 2) {
             float r[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) r[j] = isinf(v[j]) ? 0.f : v[j] - __half2float(__float2half_rn(v[j]));
-            uint4* lo = out + (K >> 3);
-            lo[piece] = make_uint4(pack_half2(r[0], r[8]), pack_half2(r[1], r[9]), pack_half2(r[2], r[10]), pack_half2(r[3], r[11]));
-            lo[piece + 4] = make_uint4(pack_half2(r[4], r[12]), pack_half2(r[5], r[13]), pack_half2(r[6], r[14]), pack_half2(r[7], r[15]));
+            store(out + (K >> 3), r);
         }
     }
 }
@@ -257,33 +254,38 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
 // 8 MMAs 2.9e-7, 179 us; 4 (a block of 64 columns) 2.1e-7, 186 us; 2 1.8e-7, 189 us; 1 1.7e-7, 192 us; the fp32 kernel 2.6e-7.
 // Four where no layout needs better.  IQ3_S and NVFP4 with ragged down rows, which the fp32 kernel had before, take one: with four,
 // bf16 rows would be further off than there (1.75e-7 against 1.6e-7 at 2560 x 640).
-template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN>
-__global__ void __launch_bounds__(kThreads, 2)
-blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __restrict__ inv, const int2* __restrict__ items,
-               int* __restrict__ n_items, int tiles_per_warp, int n_row_blocks) {
+// KS > 1: KS neighbouring warps share a row tile, each a part of its chunks; their sums meet in shared memory.
+// Work: the row blocks (W / KS tiles) of all passes in one sequence, cut into equal runs, one a block; a run's part of one pass shares
+// its columns and its weight stream.
+// W, OCC, NC: warps a block, blocks an SM, copies of the IQ3_S codebook (blk_shape).
+template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN, int W, int OCC, int ST, int NC, int KS>
+__global__ void __launch_bounds__(W * 32, OCC)
+blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __restrict__ inv, const PassRec* __restrict__ items,
+               const int* __restrict__ n_items, int n_row_blocks) {
     extern __shared__ __align__(128) uint8_t smem[];
+    constexpr int kThreads = W * 32, kStages = ST, kTiles = W / KS;
     const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff;
     const int n_gran = (int) (K >> 6);                       // 64-column granules
     __half* xs = reinterpret_cast<__half*>(smem);            // [n_gran][2][8 cols][4][8]
     using F = Fmt<FMT>;
     constexpr int kRowBytes = F::kRowBytes, kStageB = kStageBytes<FMT>;
     uint32_t* lut = reinterpret_cast<uint32_t*>(smem + (size_t) K * kCols * 2);     // the format's table
-    uint4* zero = reinterpret_cast<uint4*>(smem + (size_t) K * kCols * 2 + F::kTable);   // 64 zero bytes: the B fragments of unused columns
-    uint8_t* wbase = smem + (size_t) K * kCols * 2 + F::kTable + 128;
+    uint4* zero = reinterpret_cast<uint4*>(smem + (size_t) K * kCols * 2 + F::kTable * NC);   // 64 zero bytes: the B fragments of unused columns
+    uint8_t* wbase = smem + (size_t) K * kCols * 2 + F::kTable * NC + 128;
+    float4* part = reinterpret_cast<float4*>(wbase + (size_t) W * kStages * kStageB);         // [2][tiles][KS - 1][32] (KS > 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* wring = wbase + (size_t) warp * kStages * kStageB;
     const uint32_t wring_s = (uint32_t) __cvta_generic_to_shared(wring);
     const uint32_t xs_s = (uint32_t) __cvta_generic_to_shared(xs);
-    constexpr int NTOK = kCols / TERMS;
 
     __shared__ int s_ir[kCols];                        // image row of each entry of the pass
-    // 256 threads; the first barrier below publishes the table
+    // the first barrier below publishes the table
     if constexpr (FMT == FMT_NVFP4) {
-        lut[threadIdx.x] = scale_pair_bits(threadIdx.x);
+        if (threadIdx.x < 256) lut[threadIdx.x] = scale_pair_bits(threadIdx.x);
     } else {
-        for (int i = threadIdx.x; i < 512; i += kThreads) {
-            const uint32_t pt = a.grid[kGridIQ3S + i];
+        for (int i = threadIdx.x; i < 512 * NC; i += kThreads) {
+            const uint32_t pt = a.grid[kGridIQ3S + i / NC];
             const __half2 lo = __floats2half2_rn((float) (2u * (pt & 7u) + 1u), (float) (2u * ((pt >> 3) & 7u) + 1u));
             const __half2 hi = __floats2half2_rn((float) (2u * ((pt >> 6) & 7u) + 1u), (float) (2u * ((pt >> 9) & 7u) + 1u));
             reinterpret_cast<uint2*>(lut)[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
@@ -292,14 +294,11 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
     if (threadIdx.x < 4) zero[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
 
     const int64_t n_rows = MODE == MODE_GU ? a.L.n_ff : a.L.n_embd;      // neurons (pairs) or down rows
-    // A work unit is (pass, row block): a row block covers tiles_per_warp row tiles per warp; tile j of warp w starts at row (or
-    // neuron) r0 + j * tile_stride.  The blocks are persistent and draw work units from a counter in global memory (zeroed by
-    // the image kernel that runs before this one), so no block idles while another still has several units queued.
     constexpr int kTileRows = MODE == MODE_GU ? 8 : 16;
-    constexpr int tile_stride = kWarps * kTileRows;
-    __shared__ int s_work;
-    const int n_chunks = (n_gran + F::kGranules - 1) / F::kGranules;
-    const int last_bytes = FMT == FMT_IQ3S || PIECE == 16 ? kRowBytes : (n_gran - 4 * (n_chunks - 1)) * 36;   // bytes of a row in the last chunk
+    constexpr int kStepRows = kTiles * kTileRows;
+    const int row_chunks = (n_gran + F::kGranules - 1) / F::kGranules;
+    const int chunk0 = row_chunks * (warp % KS) / KS, n_chunks = row_chunks * (warp % KS + 1) / KS - chunk0;      // this warp's part of a row
+    const int last_bytes = FMT == FMT_IQ3S || PIECE == 16 ? kRowBytes : (n_gran - 4 * (row_chunks - 1)) * 36;   // bytes of a row in its last chunk
     const int pieces_per_col = (int) (K >> 3);               // 16-byte pieces of one image
 
     // this lane's copy duty inside a stage: pieces lane, lane + 32, ...; row = piece / kRowPieces
@@ -318,23 +317,23 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
 
     pdl_wait();      // the table does not depend on earlier kernels; everything below does
     pdl_launch_dependents();
-    const int n_work = n_items[0] * n_row_blocks;
-    for (;;) {
-        __syncthreads();   // the previous unit is done with xs and s_work
-        if (threadIdx.x == 0) s_work = atomicAdd(&n_items[1], 1);
-        __syncthreads();
-        const int work = s_work;
-        if (work >= n_work) break;
+    const int64_t n_work = (int64_t) n_items[0] * n_row_blocks;
+    int work = (int) (n_work * blockIdx.x / gridDim.x);
+    const int work_end = (int) (n_work * (blockIdx.x + 1) / gridDim.x);
+    PassRec next{0ull, 0, 0};
+    if (work < work_end) next = items[work / n_row_blocks];
+    while (work < work_end) {
+        const PassRec pass = next;
         const int item = work / n_row_blocks, rb = work - item * n_row_blocks;
-        const int64_t r0 = (int64_t) rb * tiles_per_warp * tile_stride + warp * kTileRows;
+        const int steps = min(work_end - work, n_row_blocks - rb);
+        work += steps;
+        if (work < work_end) next = items[item + 1];         // rides under this pass
+        const int64_t r0 = (int64_t) rb * kStepRows + warp / KS * kTileRows;
         int live_tiles = 0;
-        while (live_tiles < tiles_per_warp && r0 + (int64_t) live_tiles * tile_stride < n_rows) ++live_tiles;
-        const int n_units = live_tiles * n_chunks;               // (tile, chunk) stages this warp streams for this unit
-        const int2 it = items[item];
-        const int grp = it.x;
-        const uint8_t* blob = reinterpret_cast<const uint8_t*>(a.grp_ptr[grp]);
+        if (r0 < n_rows) live_tiles = (int) min((int64_t) steps, (n_rows - r0 + kStepRows - 1) / kStepRows);
+        const int n_units = live_tiles * n_chunks;               // (tile, chunk) stages this warp streams for this part of the run
+        const uint8_t* blob = reinterpret_cast<const uint8_t*>(pass.blob);
         const float* tail = reinterpret_cast<const float*>(blob + a.L.bytes - 16);
-        const int e1 = min(a.grp_start[grp + 1], (int) a.cap_entries);
         // global address of this lane's pieces at chunk 0
         const uint8_t* src[kCopies];
 #pragma unroll
@@ -345,19 +344,19 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                 rp = row < 8 ? blob + (size_t) (r0 + row) * a.L.gu_row : blob + a.L.up_off + (size_t) (r0 + row - 8) * a.L.up_row;
             else
                 rp = blob + a.L.down_off + (size_t) (r0 + row) * a.L.d_row;
-            src[j] = rp + cp_off[j];
+            src[j] = rp + cp_off[j] + (size_t) chunk0 * kRowBytes;
         }
         // row 8's distance from row 0 (the first up row from the first gate row), and a row's from the one before it in each half
         const size_t row8 = MODE == MODE_GU ? (size_t) a.L.up_off + (size_t) r0 * (a.L.up_row - a.L.gu_row) : 8 * (size_t) a.L.d_row;
         const size_t pitch0 = MODE == MODE_GU ? (size_t) a.L.gu_row : (size_t) a.L.d_row, pitch1 = MODE == MODE_GU ? (size_t) a.L.up_row : (size_t) a.L.d_row;
-        const size_t tile_bytes = (size_t) tile_stride * (MODE == MODE_GU ? a.L.gu_row : a.L.d_row);
+        const size_t tile_bytes = (size_t) kStepRows * (MODE == MODE_GU ? a.L.gu_row : a.L.d_row);
         // the next (tile, chunk) unit to request and its global byte offset from the tile-0, chunk-0 addresses
         int iss_unit = 0, iss_chunk = 0;
         size_t iss_off = 0;
         auto issue = [&]() {
             if (iss_unit < n_units) {
-                const uint32_t dst = wring_s + (uint32_t) (iss_unit & (kStages - 1)) * kStageB;
-                const int row_bytes = iss_chunk + 1 < n_chunks ? kRowBytes : last_bytes;
+                const uint32_t dst = wring_s + (uint32_t) (iss_unit % kStages) * kStageB;
+                const int row_bytes = chunk0 + iss_chunk + 1 < row_chunks ? kRowBytes : last_bytes;
                 if constexpr (kByRow) {
 #pragma unroll
                     for (int row = 0; row < kRows; ++row) {
@@ -382,9 +381,9 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
             cp_async_commit();
         };
         {
-            const int eb = it.y;
-            const int ntok = min(NTOK, e1 - eb);
+            const int eb = pass.eb, ntok = pass.ntok;
             const int ncol = ntok * TERMS;
+            __syncthreads();   // the previous pass is done with xs and s_ir
             if (threadIdx.x < ntok)
                 s_ir[threadIdx.x] = (MODE == MODE_GU && a.n_x_rows > 0) ? a.ent_tok[eb + threadIdx.x] : eb + (int) threadIdx.x;
             __syncthreads();
@@ -434,39 +433,39 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                 issue();
                 cp_async_wait<kStages - 1>();
                 __syncwarp();
-                const uint8_t* st = wring + (size_t) (unit & (kStages - 1)) * kStageB;
+                const uint8_t* st = wring + (size_t) (unit % kStages) * kStageB;
                 const uint32_t* ra = reinterpret_cast<const uint32_t*>(st + g * kRowBytes);          // row g
                 const uint32_t* rb = reinterpret_cast<const uint32_t*>(st + (g + 8) * kRowBytes);    // row g + 8
-                const uint4* bp = bcol + (size_t) chunk * F::kGranules * bstep;
+                const uint4* bp = bcol + (size_t) (chunk0 + chunk) * F::kGranules * bstep;
                 if constexpr (FMT == FMT_IQ3S) {
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
                         const uint8_t* ba = reinterpret_cast<const uint8_t*>(ra) + 110 * b;
                         const uint8_t* bb = reinterpret_cast<const uint8_t*>(rb) + 110 * b;
-                        float part[4] = {0.f, 0.f, 0.f, 0.f};
+                        float sum[4] = {0.f, 0.f, 0.f, 0.f};
                         const float da = __half2float(*reinterpret_cast<const __half*>(ba)), db = __half2float(*reinterpret_cast<const __half*>(bb));
 #pragma unroll
                         for (int gr = 0; gr < 4; ++gr) {
                             const uint4 b0 = bp[(4 * b + gr) * bstep], b1 = bp[(4 * b + gr) * bstep + bhalf];
                             uint32_t qa[8], qb[8];
-                            iq3s_16(ba, gr, t, reinterpret_cast<const uint2*>(lut), qa);
-                            iq3s_16(bb, gr, t, reinterpret_cast<const uint2*>(lut), qb);
-                            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f}, s3[4] = {0.f, 0.f, 0.f, 0.f};
-                            mma_f16(s0, qa[0], qb[0], qa[1], qb[1], b0.x, b0.y);
-                            mma_f16(s1, qa[2], qb[2], qa[3], qb[3], b0.z, b0.w);
-                            mma_f16(s2, qa[4], qb[4], qa[5], qb[5], b1.x, b1.y);
-                            mma_f16(s3, qa[6], qb[6], qa[7], qb[7], b1.z, b1.w);
+                            iq3s_16<NC>(ba, gr, t, reinterpret_cast<const uint2*>(lut) + (lane & (NC - 1)), qa);
+                            iq3s_16<NC>(bb, gr, t, reinterpret_cast<const uint2*>(lut) + (lane & (NC - 1)), qb);
+                            float s0[4], s1[4], s2[4], s3[4];
+                            mma_f16_zero(s0, qa[0], qb[0], qa[1], qb[1], b0.x, b0.y);
+                            mma_f16_zero(s1, qa[2], qb[2], qa[3], qb[3], b0.z, b0.w);
+                            mma_f16_zero(s2, qa[4], qb[4], qa[5], qb[5], b1.x, b1.y);
+                            mma_f16_zero(s3, qa[6], qb[6], qa[7], qb[7], b1.z, b1.w);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) part[i] += (s0[i] + s1[i]) + (s2[i] + s3[i]);
+                            for (int i = 0; i < 4; ++i) sum[i] += (s0[i] + s1[i]) + (s2[i] + s3[i]);
                         }
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) acc[i] = fmaf(part[i], i < 2 ? da : db, acc[i]);
+                        for (int i = 0; i < 4; ++i) acc[i] = fmaf(sum[i], i < 2 ? da : db, acc[i]);
                     }
                 } else {
-                    float part[4] = {0.f, 0.f, 0.f, 0.f};      // a chunk's sum, so that the row's is a short chain
+                    float sum[4] = {0.f, 0.f, 0.f, 0.f};       // a chunk's sum, so that the row's is a short chain
 #pragma unroll
                     for (int blk = 0; blk < 4; ++blk) {
-                        if (PIECE != 16 && 4 * chunk + blk >= n_gran) break;   // past the row's last block
+                        if (PIECE != 16 && 4 * (chunk0 + chunk) + blk >= n_gran) break;   // past the row's last block
                         const uint4 b0 = bp[blk * bstep], b1 = bp[blk * bstep + bhalf];
                         const uint32_t sa = lut[reinterpret_cast<const uint8_t*>(ra)[36 * blk + t]];
                         const uint32_t sb = lut[reinterpret_cast<const uint8_t*>(rb)[36 * blk + t]];
@@ -482,26 +481,47 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                             qb0[i] = hmul2_bits(qb0[i], sb);
                             qb1[i] = hmul2_bits(qb1[i], sb);
                         }
-                        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f}, s3[4] = {0.f, 0.f, 0.f, 0.f};
-                        constexpr bool kOne = CHAIN == 1;
-                        mma_f16(s0, qa0[0], qb0[0], qa0[1], qb0[1], b0.x, b0.y);
-                        mma_f16(kOne ? s1 : s0, qa0[2], qb0[2], qa0[3], qb0[3], b0.z, b0.w);
-                        mma_f16(kOne ? s2 : s0, qa1[0], qb1[0], qa1[1], qb1[1], b1.x, b1.y);
-                        mma_f16(kOne ? s3 : s0, qa1[2], qb1[2], qa1[3], qb1[3], b1.z, b1.w);
+                        float s0[4], s1[4], s2[4], s3[4];
+                        mma_f16_zero(s0, qa0[0], qb0[0], qa0[1], qb0[1], b0.x, b0.y);
+                        if constexpr (CHAIN == 1) {
+                            mma_f16_zero(s1, qa0[2], qb0[2], qa0[3], qb0[3], b0.z, b0.w);
+                            mma_f16_zero(s2, qa1[0], qb1[0], qa1[1], qb1[1], b1.x, b1.y);
+                            mma_f16_zero(s3, qa1[2], qb1[2], qa1[3], qb1[3], b1.z, b1.w);
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) part[i] += kOne ? (s0[i] + s1[i]) + (s2[i] + s3[i]) : s0[i];
+                            for (int i = 0; i < 4; ++i) sum[i] += (s0[i] + s1[i]) + (s2[i] + s3[i]);
+                        } else {
+                            mma_f16(s0, qa0[2], qb0[2], qa0[3], qb0[3], b0.z, b0.w);
+                            mma_f16(s0, qa1[0], qb1[0], qa1[1], qb1[1], b1.x, b1.y);
+                            mma_f16(s0, qa1[2], qb1[2], qa1[3], qb1[3], b1.z, b1.w);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) sum[i] += s0[i];
+                        }
                     }
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[i] += part[i];
+                    for (int i = 0; i < 4; ++i) acc[i] += sum[i];
                 }
                 __syncwarp();   // every lane is done with this stage before a later issue overwrites it
                 if (++chunk != n_chunks) continue;
                 // the tile is complete: undo the row scale and the 2^-8 of the fp16 block scales, apply the tail scales
-                const int64_t rt = r0 + (int64_t) tile * tile_stride;
+                const int64_t rt = r0 + (int64_t) tile * kStepRows;
                 chunk = 0;
+                if constexpr (KS > 1) {
+                    // the tile's other warps hand their sums to its first; two buffers, so one barrier of the tile's warps is enough: a
+                    // buffer is written again only after the barrier of the tile in between, which its reader has passed
+                    float4* buf = part + ((size_t) (tile & 1) * kTiles + warp / KS) * (KS - 1) * 32 + lane;
+                    if (warp % KS != 0) buf[(warp % KS - 1) * 32] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                    asm volatile("bar.sync %0, %1;\n" ::"r"(1 + warp / KS), "n"(KS * 32) : "memory");
+                    if (warp % KS == 0)
+#pragma unroll
+                        for (int k = 0; k < KS - 1; ++k) {
+                            const float4 o = buf[k * 32];
+                            acc[0] += o.x; acc[1] += o.y; acc[2] += o.z; acc[3] += o.w;
+                        }
+                }
                 ++tile;
                 const float c0 = acc[0], c1 = acc[1], c2 = acc[2], c3 = acc[3];
                 acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+                if (KS > 1 && warp % KS != 0) continue;
                 if (MODE == MODE_GU) {
                     if (TERMS == 1) {
                         if (2 * t < ntok) a.h[o0 + rt + g] = swiglu(c0 * f0 * sg, c2 * f0 * su, a.L);
@@ -531,44 +551,75 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
     cp_async_wait<0>();
 }
 
+// shared memory that a block may ask for, alone on its SM or one of two (227 and 113 KB less the static words)
+constexpr size_t kSmemOne = 232448 - 256, kSmemTwo = 115712 - 256;
+
 template <int FMT>
-size_t smem_bytes(int64_t K) { return (size_t) K * kCols * 2 + Fmt<FMT>::kTable + 128 + (size_t) kWarps * kStages * kStageBytes<FMT>; }
+size_t smem_bytes(int64_t K, int W, int ST, int NC, int KS) {
+    return (size_t) K * kCols * 2 + (size_t) Fmt<FMT>::kTable * NC + 128 + (size_t) W * ST * kStageBytes<FMT> + (size_t) 2 * (W / KS) * (KS - 1) * 512;
+}
+// the widest rows: those whose columns leave room for a ring (what this kernel has taken from the start)
+template <int FMT>
+bool fits(int64_t K) { return (size_t) K * kCols * 2 + Fmt<FMT>::kTable + 128 + 32 * kStageBytes<FMT> <= 200 * 1024; }
 size_t align256(size_t v) { return (v + 255) & ~(size_t) 255; }
 
-template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN>
-int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const int2* items, int* n_items, cudaStream_t st) {
-    const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff;
-    const size_t smem = smem_bytes<FMT>(K);
+template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN, int W, int OCC, int ST, int NC, int KS>
+int32_t launch_as(const ExpertArgs& a, const __half* img, const float* inv, const PassRec* items, const int* n_items, cudaStream_t st) {
+    const size_t smem = smem_bytes<FMT>(MODE == MODE_GU ? a.L.n_embd : a.L.n_ff, W, ST, NC, KS);
     static std::atomic<bool> configured[64];   // per device; threads of different devices call concurrently
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(blk_mma_kernel<FMT, MODE, TERMS, PIECE, CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        const cudaError_t e = cudaFuncSetAttribute(blk_mma_kernel<FMT, MODE, TERMS, PIECE, CHAIN, W, OCC, ST, NC, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int) (OCC == 2 ? kSmemTwo : kSmemOne));
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
-    const int64_t rows = MODE == MODE_GU ? a.L.n_ff : a.L.n_embd;
-    // a work unit streams ~150 KB of weights (enough to hide its start-up: activation copy, first loads); the row tiles of an
-    // expert are dealt evenly over the units
-    const int64_t tile_bytes = (int64_t) kWarps * 16 * (FMT == FMT_IQ3S ? K / 256 * 110 : K / 64 * 36);
-    const int64_t tile_rows = MODE == MODE_GU ? kWarps * 8 : kWarps * 16;
-    const int64_t n_tiles = (rows + tile_rows - 1) / tile_rows;
-    int64_t tpw0 = (150 * 1024 + tile_bytes - 1) / tile_bytes;
-    tpw0 = tpw0 < 1 ? 1 : tpw0 > 8 ? 8 : tpw0;
-    const int64_t n_blocks = (n_tiles + tpw0 - 1) / tpw0;
-    const int tpw = (int) ((n_tiles + n_blocks - 1) / n_blocks);
-    const int n_row_blocks = (int) ((n_tiles + tpw - 1) / tpw);
-    launch_k(blk_mma_kernel<FMT, MODE, TERMS, PIECE, CHAIN>, dim3((unsigned) (2 * sm_count())), dim3(kThreads), smem, st, a, img, inv, items, n_items, tpw, n_row_blocks);
+    const int64_t rows = MODE == MODE_GU ? a.L.n_ff : a.L.n_embd, step_rows = (MODE == MODE_GU ? 8 : 16) * (W / KS);
+    launch_k(blk_mma_kernel<FMT, MODE, TERMS, PIECE, CHAIN, W, OCC, ST, NC, KS>, dim3((unsigned) (OCC * sm_count())), dim3(W * 32), smem, st, a, img, inv, items, n_items,
+             (int) ((rows + step_rows - 1) / step_rows));
     return launch_status();
+}
+
+// Sixteen warps an SM either way: two blocks of eight where shared memory holds two, which hide each other's first loads, else one of
+// sixteen.  (Four stages a warp left one block of eight: 2560-column NVFP4 rows and every IQ3_S row.)  IQ3_S is bound by its look-ups,
+// eight bytes at 32 unrelated points: sixteen copies of the codebook, a lane's own in two banks of its own, take the bank conflicts away
+// (4 passes over the banks a look-up on average without them), which one block of sixteen warps has room for.
+template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN>
+int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const PassRec* items, const int* n_items, cudaStream_t st) {
+    const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff, rows = MODE == MODE_GU ? a.L.n_ff : a.L.n_embd;
+    const bool two = FMT == FMT_NVFP4 && smem_bytes<FMT>(K, 8, 3, 1, 4) <= kSmemTwo;
+    const bool copies = FMT == FMT_IQ3S && smem_bytes<FMT>(K, 16, 2, 16, 4) <= kSmemOne;
+    // columns are split where whole rows would leave a block few steps, so that the last, partial one weighs little: IQ3_S up to eight
+    // steps (24 tokens of 2048 x 512, 512 experts, 7.4 steps: 202 us whole, 193 split in two), NVFP4, whose decode costs less beside the
+    // sums' exchange, up to four (16 tokens of 2560 x 640, 6.2 steps: 123 whole, 130 split).  cap_groups and cap_entries bound the passes
+    // on the host
+    const int64_t chunks = FMT == FMT_IQ3S ? K / 512 : (K + 255) / 256, step_rows = (MODE == MODE_GU ? 8 : 16) * (two ? 8 : 16);
+    const int64_t steps = (a.cap_groups + a.cap_entries / (kCols / TERMS)) * ((rows + step_rows - 1) / step_rows);
+    int ks = 1;
+    while (ks < 4 && chunks >= 2 * ks && steps * ks < (FMT == FMT_IQ3S ? 8 : 4) * (int64_t) sm_count() * (two ? 2 : 1)) ks *= 2;
+#define BLK_AS(W, OCC, ST, NC) \
+    do { \
+        if (ks == 4) return launch_as<FMT, MODE, TERMS, PIECE, CHAIN, W, OCC, ST, NC, 4>(a, img, inv, items, n_items, st); \
+        if (ks == 2) return launch_as<FMT, MODE, TERMS, PIECE, CHAIN, W, OCC, ST, NC, 2>(a, img, inv, items, n_items, st); \
+        return launch_as<FMT, MODE, TERMS, PIECE, CHAIN, W, OCC, ST, NC, 1>(a, img, inv, items, n_items, st); \
+    } while (0)
+    if constexpr (FMT == FMT_NVFP4) {
+        if (two) BLK_AS(8, 2, 3, 1);
+    } else {
+        if (copies) BLK_AS(16, 1, 2, 16);
+    }
+    BLK_AS(16, 1, 2, 1);
+#undef BLK_AS
 }
 
 }  // namespace
 
 // scratch beyond the SwiGLU buffer: the x images (up to two fp16 terms), the h images (two terms), the inverse row scales
 size_t experts_mma_scratch_bytes(int64_t cap_entries, int64_t n_embd, int64_t n_ff) {
-    // the pass list: at most one pass per entry, 8 bytes each, plus its count
+    // the pass list: at most one pass per entry, 16 bytes each, plus its count
     return align256((size_t) cap_entries * n_embd * 4) + align256((size_t) cap_entries * n_ff * 4) + 2 * align256((size_t) cap_entries * 4) +
-           align256((size_t) (cap_entries + 1) * 8 + 16);
+           align256((size_t) (cap_entries + 1) * 16 + 16);
 }
 
 int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
@@ -581,10 +632,10 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     if ((L.gu_type != kTypeNVFP4 && L.gu_type != kTypeIQ3S) || L.up_type != L.gu_type || L.d_type != L.gu_type) return BSX_E_TYPE;
     if (fmt == FMT_NVFP4) {
         if (L.n_embd % 256 || L.n_ff % 64) return BSX_E_TYPE;
-        if (smem_bytes<FMT_NVFP4>(L.n_embd) > 200 * 1024 || smem_bytes<FMT_NVFP4>(L.n_ff) > 200 * 1024) return BSX_E_TYPE;
+        if (!fits<FMT_NVFP4>(L.n_embd) || !fits<FMT_NVFP4>(L.n_ff)) return BSX_E_TYPE;
     } else {
         if (L.n_embd % 512 || L.n_ff % 512) return BSX_E_TYPE;
-        if (smem_bytes<FMT_IQ3S>(L.n_embd) > 200 * 1024 || smem_bytes<FMT_IQ3S>(L.n_ff) > 200 * 1024) return BSX_E_TYPE;
+        if (!fits<FMT_IQ3S>(L.n_embd) || !fits<FMT_IQ3S>(L.n_ff)) return BSX_E_TYPE;
     }
     // scratch: [h fp32][x images][h images][x inverse scales][h inverse scales]
     uint8_t* p = reinterpret_cast<uint8_t*>(a.h) + align256((size_t) a.cap_entries * L.n_ff * 4);
@@ -595,7 +646,7 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     float* xinv = reinterpret_cast<float*>(p);
     float* hinv = xinv + align256((size_t) a.cap_entries * 4) / 4;
     int* n_items = reinterpret_cast<int*>(hinv + align256((size_t) a.cap_entries * 4) / 4);
-    int2* items = reinterpret_cast<int2*>(n_items + 4);
+    PassRec* items = reinterpret_cast<PassRec*>(n_items + 4);
     const int phase = experts_phase(a.L);
     // a warp per image row, 8 a block, plus the block that lists the passes
     const int64_t x_rows = a.n_x_rows > 0 ? a.n_x_rows : a.cap_entries;
@@ -603,19 +654,19 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     int32_t rc = BSX_OK;
     if (phase != 2) {
         if (a.x_kind == BSX_X_BF16) {
-            launch_k(prep_image_kernel<false, 1>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
+            launch_k(fmt == FMT_IQ3S ? prep_image_kernel<FMT_IQ3S, false, 1> : prep_image_kernel<FMT_NVFP4, false, 1>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
             rc = fmt == FMT_IQ3S ? launch<FMT_IQ3S, MODE_GU, 1, 4, 1>(a, ximg, xinv, items, n_items, st)
                  : whole         ? launch<FMT_NVFP4, MODE_GU, 1, 16, 4>(a, ximg, xinv, items, n_items, st)
                                  : launch<FMT_NVFP4, MODE_GU, 1, 16, 1>(a, ximg, xinv, items, n_items, st);
         } else {
-            launch_k(prep_image_kernel<false, 2>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
+            launch_k(fmt == FMT_IQ3S ? prep_image_kernel<FMT_IQ3S, false, 2> : prep_image_kernel<FMT_NVFP4, false, 2>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
             rc = fmt == FMT_IQ3S ? launch<FMT_IQ3S, MODE_GU, 2, 4, 1>(a, ximg, xinv, items, n_items, st)
                  : whole         ? launch<FMT_NVFP4, MODE_GU, 2, 16, 4>(a, ximg, xinv, items, n_items, st)
                                  : launch<FMT_NVFP4, MODE_GU, 2, 16, 1>(a, ximg, xinv, items, n_items, st);
         }
     }
     if (rc != BSX_OK || phase == 1) return rc;
-    launch_k(prep_image_kernel<true, 2>, dim3(nbh), dim3(256), 0, st, a, himg, hinv, items, n_items);
+    launch_k(fmt == FMT_IQ3S ? prep_image_kernel<FMT_IQ3S, true, 2> : prep_image_kernel<FMT_NVFP4, true, 2>, dim3(nbh), dim3(256), 0, st, a, himg, hinv, items, n_items);
     if (fmt == FMT_IQ3S) return launch<FMT_IQ3S, MODE_DOWN, 2, 4, 1>(a, himg, hinv, items, n_items, st);
     // Down rows of n_ff columns: the copies' width is what their start is aligned to.  An n_ff that is not whole 256-column chunks
     // went to the warp-per-row kernels before (2 % of the copy bandwidth: fp32 decode and FMA for every weight and entry); here
