@@ -10,41 +10,82 @@
 // (bsx_router_select) is unchanged and reads these logits; ids can differ from the decode path's only where two scores tie
 // to that precision.
 //
-// One CTA per (128 tokens, 256 experts) tile: warp 0 allocates 256 TMEM columns and its lane 0 issues the MMAs; warp 1
-// loads activation rows, warps 2-3 gate rows (cp.async into 128-byte-swizzled stages, 4-stage mbarrier ring, every wait
-// time-bounded); warps 4-7 are the epilogue (thread = TMEM lane = token).
+// One CTA per (128 tokens, N experts) tile, N = 256, or less where that leaves SMs idle (the sums of a logit stay in the same order:
+// splitting the columns instead would turn near-ties): warp 0 allocates N TMEM columns and one of its lanes issues the MMAs; the next
+// three to six warps load token and gate rows (cp.async into 128-byte-swizzled stages of 128 columns, a mbarrier ring, every wait
+// time-bounded); the last four are the epilogue (thread = TMEM lane = token).
 #include <atomic>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "experts.cuh"
 #include "tc5.cuh"
 
 namespace bsx {
 namespace {
 
-constexpr int kTM = 128, kTN = 256, kBK = 64, kStg = 4;
-constexpr int kThreadsR = 256;
-constexpr int kABytesR = kTM * kBK * 2, kBBytesR = kTN * kBK * 2, kStageR = kABytesR + kBBytesR;
-constexpr size_t kSmemR = 1024 + (size_t) kStg * kStageR + 128 + kTN * 4 + 64;
-constexpr uint32_t kIdescR = instr_desc_f16(kTM, kTN);
+constexpr int kTM = 128, kBK = 64;             // a stage holds two k-blocks of kBK columns
+template <int N>
+struct RG {
+    static constexpr int kRowsWarp = N >= 128 ? 64 : 32;                         // operand rows a loader warp copies
+    static constexpr int kLoaders = (kTM + N) / kRowsWarp, kThreads = 32 * (1 + kLoaders + 4);
+    static constexpr int kBlock = (kTM + N) * kBK * 2, kStage = 2 * kBlock;      // [k-block: token rows | gate rows] twice
+    static constexpr int kStg = N == 256 ? 2 : N == 128 ? 3 : N == 64 ? 4 : 5;
+    static constexpr size_t kSmem = 1024 + (size_t) kStg * kStage + 128 + N * 4 + 64;
+    static constexpr uint32_t kIdesc = instr_desc_f16(kTM, N), kTmem = N;
+    static_assert(kSmem <= 227 * 1024 && kTM % kRowsWarp == 0 && N % kRowsWarp == 0, "stage geometry");
+};
 
 size_t al256(size_t v) { return (v + 255) & ~(size_t) 255; }
 
 // rows [R][H] (fp32 or bf16) -> `terms` fp16 planes [terms][R][H], each row scaled by a power of two so its largest magnitude
 // lands in [2^13, 2^14), k-permuted inside 16-column groups; inv[r] undoes the scale.  Plane 1 holds the rounding residual
-// of plane 0.  One warp per row.
-__global__ void __launch_bounds__(256) rows_to_fp16_planes_kernel(const void* __restrict__ x, int kind, int64_t R, int64_t H, int terms,
-                                                                  __half* __restrict__ img, float* __restrict__ inv) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t r = (int64_t) blockIdx.x * 8 + warp;
-    if (r >= R) return;
-    auto ld = [&](int64_t c) {
-        return kind == BSX_X_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(x)[r * H + c]) : static_cast<const float*>(x)[r * H + c];
-    };
+// of plane 0.
+struct PlaneRows {
+    const void* x;
+    int kind, terms;
+    int64_t R;
+    __half* img;
+    float* inv;
+};
+
+// The rows of both operands in one launch: TPR threads a row, each with up to two of its 16-column groups in registers (a row is read
+// once up to 32 TPR columns) and stored as two 16-byte pieces.  Bound by HBM.  With a warp a row, single values loaded and stored and a
+// launch for each operand, 8192 bf16 rows of 7168 columns and 256 gate rows took 94 + 42 us and 777 fp32 rows of 5120 columns and 384 gate
+// rows 28 + 26.
+template <int TPR>
+__global__ void __launch_bounds__(256) rows_to_fp16_planes_kernel(PlaneRows x, PlaneRows gate, int64_t H) {
+    constexpr int kRows = 256 / TPR, kKeep = 2;
+    __shared__ float s_max[8];
+    const unsigned x_blocks = (unsigned) ((x.R + kRows - 1) / kRows);
+    const bool is_x = blockIdx.x < x_blocks;
+    const PlaneRows& a = is_x ? x : gate;
+    const int64_t r = (int64_t) (is_x ? blockIdx.x : blockIdx.x - x_blocks) * kRows + threadIdx.x / TPR;
+    const int tr = threadIdx.x % TPR, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool live = r < a.R;
+    const int n_sb = live ? (int) (H >> 4) : 0;
+    float v[kKeep][16];
     float amax = 0.f;
-    for (int64_t c = lane; c < H; c += 32) amax = fmaxf(amax, fabsf(ld(c)));
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) {
+        if (tr + i * TPR < n_sb) {
+            load16(a.x, a.kind, r, H, tr + i * TPR, v[i]);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[i][j]));
+        }
+    }
+    for (int sb = tr + kKeep * TPR; sb < n_sb; sb += TPR) {
+        float w[16];
+        load16(a.x, a.kind, r, H, sb, w);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(w[j]));
+    }
     amax = warp_max_xor(amax);
+    if (lane == 0) s_max[warp] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TPR / 32; ++i) amax = fmaxf(amax, s_max[warp / (TPR / 32) * (TPR / 32) + i]);
     int ex = 0;
     float s = 1.f, iv = 1.f;
     if (amax > 0.f && amax <= 3.0e38f) {
@@ -53,13 +94,32 @@ __global__ void __launch_bounds__(256) rows_to_fp16_planes_kernel(const void* __
         s = ldexpf(1.f, ex);
         iv = ldexpf(1.f, -ex);
     }
-    if (lane == 0) inv[r] = iv;
-    for (int64_t c = lane; c < H; c += 32) {
-        const float v = ld(c) * s;
-        const __half hi = __float2half_rn(v);
-        const int64_t o = r * H + (c & ~(int64_t) 15) + perm16((int) (c & 15));
-        img[o] = hi;
-        if (terms > 1) img[R * H + o] = __float2half_rn(v - __half2float(hi));
+    if (live && tr == 0) a.inv[r] = iv;
+    auto store = [&](int sb, const float (&w)[16]) {
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {       // positions 2 i and 2 i + 1 of the permuted order: columns i and i + 8
+            const float p = w[i] * s, q = w[i + 8] * s;
+            const __half hp = __float2half_rn(p), hq = __float2half_rn(q);
+            hi[i] = (uint32_t) __half_as_ushort(hp) | ((uint32_t) __half_as_ushort(hq) << 16);
+            lo[i] = (uint32_t) __half_as_ushort(__float2half_rn(p - __half2float(hp))) | ((uint32_t) __half_as_ushort(__float2half_rn(q - __half2float(hq))) << 16);
+        }
+        uint4* o = reinterpret_cast<uint4*>(a.img + r * H + 16 * sb);
+        o[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        o[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+        if (a.terms > 1) {
+            o = reinterpret_cast<uint4*>(a.img + (a.R + r) * H + 16 * sb);
+            o[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            o[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i)
+        if (tr + i * TPR < n_sb) store(tr + i * TPR, v[i]);
+    for (int sb = tr + kKeep * TPR; sb < n_sb; sb += TPR) {
+        float w[16];
+        load16(a.x, a.kind, r, H, sb, w);
+        store(sb, w);
     }
 }
 
@@ -74,27 +134,30 @@ struct LogitsArgs {
     int E, H, x_terms;
 };
 
-__global__ void __launch_bounds__(kThreadsR, 1) router_logits_tc_kernel(LogitsArgs a) {
+template <int N>
+__global__ void __launch_bounds__(RG<N>::kThreads, 1) router_logits_tc_kernel(LogitsArgs a) {
+    using G = RG<N>;
+    constexpr int kStg = G::kStg;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStg * kStageR);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStg * G::kStage);
     uint64_t* empty = full + kStg;
     uint64_t* accum = empty + kStg;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
-    float* s_ginv = reinterpret_cast<float*>(smem + kStg * kStageR + 128);
+    float* s_ginv = reinterpret_cast<float*>(smem + kStg * G::kStage + 128);
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
-    const int e0 = blockIdx.x * kTN;
+    const int e0 = blockIdx.x * N;
     const int64_t t0 = (int64_t) blockIdx.y * kTM;
     const int nkb = a.H / kBK;
     // the products summed into the accumulator: (x hi, gate hi), (x hi, gate lo) and, for two x terms, (x lo, gate hi)
     const int n_prod = a.x_terms > 1 ? 3 : 2;
-    const int n_it = n_prod * nkb;
+    const int n_blk = n_prod * nkb, n_it = (n_blk + 1) / 2;
 
-    for (int i = threadIdx.x; i < kTN; i += kThreadsR) s_ginv[i] = a.ginv[min(e0 + i, a.E - 1)];
+    for (int i = threadIdx.x; i < N; i += G::kThreads) s_ginv[i] = a.ginv[min(e0 + i, a.E - 1)];
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStg; ++s) {
-            mbar_init(&full[s], 96);      // three loader warps
+            mbar_init(&full[s], 32 * G::kLoaders);
             mbar_init(&empty[s], 1);
         }
         mbar_init(accum, 1);
@@ -102,7 +165,7 @@ __global__ void __launch_bounds__(kThreadsR, 1) router_logits_tc_kernel(LogitsAr
     }
     if (warp == 0) {
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t) kTN) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(G::kTmem) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -118,28 +181,31 @@ __global__ void __launch_bounds__(kThreadsR, 1) router_logits_tc_kernel(LogitsAr
                 ok = mbar_wait(&full[s], ((uint32_t) it / kStg) & 1u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t sa = smem_u32(smem + s * kStageR), sb = sa + kABytesR;
-                const uint64_t ad = smem_desc_sw128(sa), bd = smem_desc_sw128(sb);          // addresses in 16 bytes: 2 a step
+                const uint32_t st = smem_u32(smem + s * G::kStage);
 #pragma unroll
-                for (int k = 0; k < kBK / 16; ++k) umma_f16(tmem, ad + 2 * k, bd + 2 * k, kIdescR, (it | k) ? 1u : 0u);
+                for (int b = 0; b < 2; ++b) {
+                    if (2 * it + b == n_blk) break;
+                    const uint64_t ad = smem_desc_sw128(st + b * G::kBlock), bd = smem_desc_sw128(st + b * G::kBlock + kTM * kBK * 2);    // addresses in 16 bytes: 2 a step
+#pragma unroll
+                    for (int k = 0; k < kBK / 16; ++k) umma_f16(tmem, ad + 2 * k, bd + 2 * k, G::kIdesc, (it | b | k) ? 1u : 0u);
+                }
                 umma_commit(&empty[s]);
             }
             umma_commit(accum);
             if (!ok) atomicOr(a.status, 1);
         }
-    } else if (warp <= 3) {
-        // ---- loaders: warp 1 the 128 token rows, warps 2 and 3 128 expert rows each.  Lane l copies 16-byte chunk l % 8 of
+    } else if (warp <= G::kLoaders) {
+        // ---- loaders: warp w copies operand rows kRowsWarp (w - 1) ... (token rows, then gate rows).  Lane l copies 16-byte chunk l % 8 of
         // rows l / 8 + 4 i.  Rows past the end of the matrix read its last row (their results are never stored).
-        const int c = lane & 7, r4 = lane >> 3;
-        const bool is_x = warp == 1;
+        const int c = lane & 7, r4 = lane >> 3, row0 = (warp - 1) * G::kRowsWarp;
+        const bool is_x = row0 < kTM;
         const int64_t n_rows = is_x ? a.T : (int64_t) a.E;
-        const int64_t first = is_x ? t0 : (int64_t) e0 + (warp - 2) * 128;
-        const uint32_t tile_off = is_x ? 0u : (uint32_t) (kABytesR + (warp - 2) * 16 * 1024);
+        const int64_t first = is_x ? t0 + row0 : (int64_t) e0 + row0 - kTM;
         const size_t plane = (size_t) n_rows * a.H * 2;          // bytes of one term's image
         const uint8_t* base = reinterpret_cast<const uint8_t*>(is_x ? a.ximg : a.gimg);
-        uint32_t roff[32];   // row starts in 16-byte units
+        uint32_t roff[G::kRowsWarp / 4];   // row starts in 16-byte units
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        for (int i = 0; i < G::kRowsWarp / 4; ++i) {
             const int64_t r = first + 4 * i + r4;
             roff[i] = (uint32_t) ((r < n_rows ? r : n_rows - 1) * (a.H >> 3)) + (uint32_t) c;
         }
@@ -147,26 +213,35 @@ __global__ void __launch_bounds__(kThreadsR, 1) router_logits_tc_kernel(LogitsAr
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int r7 = 4 * h + r4;
-            dsto[h] = tile_off + (uint32_t) (r7 * 128 + ((c ^ r7) << 4));
+            dsto[h] = (uint32_t) (row0 * 128 + r7 * 128 + ((c ^ r7) << 4));
         }
+        constexpr int kAhead = kStg - 1;      // stages requested before the oldest is waited for
         uint32_t issued = 0, arrived = 0;
+        int prod = 0, kb = 0;
         for (int it = 0; it < n_it; ++it) {
-            const int prod = it / nkb, kb = it - prod * nkb;
-            const int term = is_x ? (prod == 2 ? 1 : 0) : (prod == 1 ? 1 : 0);
             const uint32_t s = issued % kStg;
             ok = mbar_wait(&empty[s], ((issued / kStg) & 1u) ^ 1u);
             if (!ok) break;
-            const uint32_t dst = smem_u32(smem + s * kStageR);
-            const uint8_t* src = base + (size_t) term * plane + (size_t) kb * 128;
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (uint32_t) ((i >> 1) * 1024) + dsto[i & 1]),
-                             "l"(src + (size_t) roff[i] * 16)
-                             : "memory");
+            for (int b = 0; b < 2; ++b) {
+                if (2 * it + b == n_blk) break;
+                const int term = is_x ? (prod == 2 ? 1 : 0) : (prod == 1 ? 1 : 0);
+                const uint32_t dst = smem_u32(smem + s * G::kStage + b * G::kBlock);
+                const uint8_t* src = base + (size_t) term * plane + (size_t) kb * 128;
+#pragma unroll
+                for (int i = 0; i < G::kRowsWarp / 4; ++i)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (uint32_t) ((i >> 1) * 1024) + dsto[i & 1]),
+                                 "l"(src + (size_t) roff[i] * 16)
+                                 : "memory");
+                if (++kb == nkb) {
+                    kb = 0;
+                    ++prod;
+                }
+            }
             asm volatile("cp.async.commit_group;\n" ::: "memory");
             ++issued;
-            if (issued - arrived > 2) {
-                asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+            if (issued - arrived > kAhead) {
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(kAhead) : "memory");
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 mbar_arrive(&full[arrived % kStg]);
                 ++arrived;
@@ -187,7 +262,7 @@ __global__ void __launch_bounds__(kThreadsR, 1) router_logits_tc_kernel(LogitsAr
             float* out = a.logits + (size_t) (t0 + p) * a.E + e0;
             const uint32_t tbase = tmem + ((uint32_t) ((warp & 3) * 32) << 16);
 #pragma unroll 1
-            for (int c0 = 0; c0 < kTN; c0 += 32) {
+            for (int c0 = 0; c0 < N; c0 += 32) {
                 uint32_t d[32];
                 tmem_ld32(tbase + (uint32_t) c0, d);
                 if (live && e0 + c0 < a.E) {
@@ -207,8 +282,23 @@ __global__ void __launch_bounds__(kThreadsR, 1) router_logits_tc_kernel(LogitsAr
     if (warp == 0) {
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t) kTN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(G::kTmem) : "memory");
     }
+}
+
+template <int N>
+int32_t launch_logits(const LogitsArgs& a, cudaStream_t st) {
+    static std::atomic<bool> configured[64];   // per device; threads of different devices call concurrently
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
+    if (!configured[dev].load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(router_logits_tc_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) RG<N>::kSmem);
+        if (e != cudaSuccess) return (int32_t) e;
+        configured[dev].store(true, std::memory_order_release);
+    }
+    const dim3 grid((unsigned) ((a.E + N - 1) / N), (unsigned) ((a.T + kTM - 1) / kTM));
+    router_logits_tc_kernel<N><<<grid, RG<N>::kThreads, RG<N>::kSmem, st>>>(a);
+    return launch_status();
 }
 
 }  // namespace
@@ -248,17 +338,16 @@ extern "C" int32_t bsx_router_logits_prefill(const void* x, int32_t x_kind, cons
     a.E = E;
     a.H = H;
     a.x_terms = x_kind == BSX_X_BF16 ? 1 : 2;
-    static std::atomic<bool> configured[64];   // per device; threads of different devices call concurrently
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
-    if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(router_logits_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemR);
-        if (e != cudaSuccess) return (int32_t) e;
-        configured[dev].store(true, std::memory_order_release);
-    }
-    rows_to_fp16_planes_kernel<<<(unsigned) ((T + 7) / 8), 256, 0, st>>>(x, x_kind, T, H, a.x_terms, ximg, xinv);
-    rows_to_fp16_planes_kernel<<<(unsigned) ((E + 7) / 8), 256, 0, st>>>(gate, BSX_X_F32, E, H, 2, gimg, ginv);
-    const dim3 grid((unsigned) ((E + kTN - 1) / kTN), (unsigned) ((T + kTM - 1) / kTM));
-    router_logits_tc_kernel<<<grid, kThreadsR, kSmemR, st>>>(a);
-    return launch_status();
+    const PlaneRows xr{x, x_kind, a.x_terms, T, ximg, xinv}, gr{gate, BSX_X_F32, 2, E, gimg, ginv};
+    if (H <= 4096) rows_to_fp16_planes_kernel<128><<<(unsigned) ((T + 1) / 2 + (E + 1) / 2), 256, 0, st>>>(xr, gr, H);
+    else rows_to_fp16_planes_kernel<256><<<(unsigned) (T + E), 256, 0, st>>>(xr, gr, H);
+    const int32_t rc = launch_status();
+    if (rc != BSX_OK) return rc;
+    // the widest tile that still gives two thirds of the SMs one: a narrower one reads the token rows again for each of its neighbours
+    auto tiles = [&](int n) { return (int64_t) ((E + n - 1) / n) * ((T + kTM - 1) / kTM); };
+    const int64_t want = 2 * (int64_t) sm_count() / 3;
+    if (tiles(256) >= want) return launch_logits<256>(a, st);
+    if (tiles(128) >= want) return launch_logits<128>(a, st);
+    if (tiles(64) >= want) return launch_logits<64>(a, st);
+    return launch_logits<32>(a, st);
 }
