@@ -12,7 +12,7 @@
 //
 // One CTA per (128 tokens, N experts) tile, N = 256, or less where that leaves SMs idle (the sums of a logit stay in the same order:
 // splitting the columns instead would turn near-ties): warp 0 allocates N TMEM columns and one of its lanes issues the MMAs; the next
-// three to six warps load token and gate rows (cp.async into 128-byte-swizzled stages of 128 columns, a mbarrier ring, every wait
+// three to six warps load token and gate rows (cp.async into 128-byte-swizzled stages, a mbarrier ring, every wait
 // time-bounded); the last four are the epilogue (thread = TMEM lane = token).
 #include <atomic>
 #include <cuda_bf16.h>
@@ -25,13 +25,16 @@
 namespace bsx {
 namespace {
 
-constexpr int kTM = 128, kBK = 64;             // a stage holds two k-blocks of kBK columns
+constexpr int kTM = 128, kBK = 64;             // a stage holds one or two k-blocks of kBK columns
 template <int N>
 struct RG {
     static constexpr int kRowsWarp = N >= 128 ? 64 : 32;                         // operand rows a loader warp copies
     static constexpr int kLoaders = (kTM + N) / kRowsWarp, kThreads = 32 * (1 + kLoaders + 4);
-    static constexpr int kBlock = (kTM + N) * kBK * 2, kStage = 2 * kBlock;      // [k-block: token rows | gate rows] twice
-    static constexpr int kStg = N == 256 ? 2 : N == 128 ? 3 : N == 64 ? 4 : 5;
+    static constexpr int kSub = N == 256 ? 1 : 2;                                // k-blocks a stage
+    static constexpr int kBlock = (kTM + N) * kBK * 2, kStage = kSub * kBlock;   // [k-block: token rows | gate rows] each
+    static constexpr int kStg = N == 256 || N == 64 ? 4 : N == 128 ? 3 : 5;
+    // stages requested before the oldest is waited for: one less than could be, or the tensor core would wait for its own last stage
+    static constexpr int kAhead = kStg - 2;
     static constexpr size_t kSmem = 1024 + (size_t) kStg * kStage + 128 + N * 4 + 64;
     static constexpr uint32_t kIdesc = instr_desc_f16(kTM, N), kTmem = N;
     static_assert(kSmem <= 227 * 1024 && kTM % kRowsWarp == 0 && N % kRowsWarp == 0, "stage geometry");
@@ -152,7 +155,7 @@ __global__ void __launch_bounds__(RG<N>::kThreads, 1) router_logits_tc_kernel(Lo
     const int nkb = a.H / kBK;
     // the products summed into the accumulator: (x hi, gate hi), (x hi, gate lo) and, for two x terms, (x lo, gate hi)
     const int n_prod = a.x_terms > 1 ? 3 : 2;
-    const int n_blk = n_prod * nkb, n_it = (n_blk + 1) / 2;
+    const int n_blk = n_prod * nkb, n_it = (n_blk + G::kSub - 1) / G::kSub;
 
     for (int i = threadIdx.x; i < N; i += G::kThreads) s_ginv[i] = a.ginv[min(e0 + i, a.E - 1)];
     if (threadIdx.x == 0) {
@@ -183,8 +186,8 @@ __global__ void __launch_bounds__(RG<N>::kThreads, 1) router_logits_tc_kernel(Lo
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t st = smem_u32(smem + s * G::kStage);
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    if (2 * it + b == n_blk) break;
+                for (int b = 0; b < G::kSub; ++b) {
+                    if (G::kSub * it + b == n_blk) break;
                     const uint64_t ad = smem_desc_sw128(st + b * G::kBlock), bd = smem_desc_sw128(st + b * G::kBlock + kTM * kBK * 2);    // addresses in 16 bytes: 2 a step
 #pragma unroll
                     for (int k = 0; k < kBK / 16; ++k) umma_f16(tmem, ad + 2 * k, bd + 2 * k, G::kIdesc, (it | b | k) ? 1u : 0u);
@@ -215,7 +218,6 @@ __global__ void __launch_bounds__(RG<N>::kThreads, 1) router_logits_tc_kernel(Lo
             const int r7 = 4 * h + r4;
             dsto[h] = (uint32_t) (row0 * 128 + r7 * 128 + ((c ^ r7) << 4));
         }
-        constexpr int kAhead = kStg - 1;      // stages requested before the oldest is waited for
         uint32_t issued = 0, arrived = 0;
         int prod = 0, kb = 0;
         for (int it = 0; it < n_it; ++it) {
@@ -223,8 +225,8 @@ __global__ void __launch_bounds__(RG<N>::kThreads, 1) router_logits_tc_kernel(Lo
             ok = mbar_wait(&empty[s], ((issued / kStg) & 1u) ^ 1u);
             if (!ok) break;
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                if (2 * it + b == n_blk) break;
+            for (int b = 0; b < G::kSub; ++b) {
+                if (G::kSub * it + b == n_blk) break;
                 const int term = is_x ? (prod == 2 ? 1 : 0) : (prod == 1 ? 1 : 0);
                 const uint32_t dst = smem_u32(smem + s * G::kStage + b * G::kBlock);
                 const uint8_t* src = base + (size_t) term * plane + (size_t) kb * 128;
@@ -240,8 +242,8 @@ __global__ void __launch_bounds__(RG<N>::kThreads, 1) router_logits_tc_kernel(Lo
             }
             asm volatile("cp.async.commit_group;\n" ::: "memory");
             ++issued;
-            if (issued - arrived > kAhead) {
-                asm volatile("cp.async.wait_group %0;\n" ::"n"(kAhead) : "memory");
+            if (issued - arrived > G::kAhead) {
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(G::kAhead) : "memory");
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 mbar_arrive(&full[arrived % kStg]);
                 ++arrived;
