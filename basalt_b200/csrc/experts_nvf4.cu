@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const uint8_t* __restrict__ i
 // power of two (largest magnitude into [2^7, 2^8), so block scales sit well inside UE4M3's range) as kTermsF FP4 terms.
 // Term t of a sub-block: scale = the smallest UE4M3 value s with 6 s >= the largest residual, codes = rn(residual / s),
 // residual -= code value x s.  Layout: codes [row][term][K / 2] bytes with ggml's nibble order (byte b of a sub-block =
-// values b and b + 8), scales [row][term][K / 16] bytes, inv[row].  FROM_H = false: rows of x (kind x_kind) - row i of x
+// values b and b + 8), scales [row][K / 256][term][16] bytes, inv[row].  FROM_H = false: rows of x (kind x_kind) - row i of x
 // when the caller gave the number of x rows, else the row of entry i; true: row e of the SwiGLU output h.  The last block
 // lists the passes (up to pass_entries consecutive entries of one group).
 template <bool FROM_H, int TPR>
@@ -189,17 +189,17 @@ __global__ void __launch_bounds__(256) x_images_kernel(const void* __restrict__ 
     fp4_image_row<TPR>(x, kind, i < n_rows ? i : 0, K, i < n_rows, i, codes, sfs, inv, shf);
 }
 
-// rows of h that a pass list and a tile list name: a block takes 256 / TPR places of a pass (of pass_entries) or a tile (of 128) at a
-// time.  (Rows of experts held elsewhere are in neither and have never been written.)
+// rows of h that a pass list (or none) and a tile list name: a block takes 256 / TPR places of a pass (of pass_entries) or a tile (of 128)
+// at a time.  (Rows of experts held elsewhere are in neither and have never been written.)
 template <int TPR>
 __global__ void __launch_bounds__(256) listed_images_kernel(const float* __restrict__ h, const PassRec* __restrict__ items, const int* __restrict__ n_items, int pass_entries,
-                                                             const TileRec* __restrict__ recs, const int32_t* __restrict__ slab, int64_t K, uint8_t* __restrict__ codes,
+                                                             const TileRec* __restrict__ recs, const int32_t* __restrict__ n_recs, int64_t K, uint8_t* __restrict__ codes,
                                                              uint8_t* __restrict__ sfs, float* __restrict__ inv) {
     __shared__ float shf[8];
     constexpr int kRows = 256 / TPR;          // divides both lengths: a block's places are one pass's or tile's
     pdl_wait();
     pdl_launch_dependents();
-    const int64_t n_pass = (int64_t) *n_items * pass_entries, n = n_pass + (int64_t) slab[1] * 128;
+    const int64_t n_pass = items ? (int64_t) *n_items * pass_entries : 0, n = n_pass + (int64_t) *n_recs * 128;
     for (int64_t at = (int64_t) blockIdx.x * kRows; at < n; at += (int64_t) gridDim.x * kRows) {
         int row0, rows, j0;
         if (at < n_pass) {
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) nvf4_stream_kernel(StreamArgs sa
                 const int j = 8 * h + (lane >> 2);
                 const int e = u.eb + (j < u.ntok ? j : 0);
                 const int ir = (MODE == FMODE_GU && a.n_x_rows > 0) ? a.ent_tok[e] : e;
-                srow[h] = sa.sfs + ((size_t) ir * kTermsF + (lane & 3)) * (size_t) (K >> 4);
+                srow[h] = sa.sfs + (size_t) ir * (size_t) (K >> 2) + (lane & 3) * 16;
             }
             for (int rb = rb0; rb < rb1 && ok; ++rb) {
                 for (int c = 0; c < n_chunk; ++c) {
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) nvf4_stream_kernel(StreamArgs sa
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(st + (uint32_t) kOffSFB + k * 512 + lane * 16 + h * 4),
-                                         "l"(srow[h] + (size_t) c * 16 + 4 * k)
+                                         "l"(srow[h] + (size_t) c * kSFChunk + 4 * k)
                                          : "memory");
                     asm volatile("cp.async.commit_group;\n" ::: "memory");
                     ++issued;
@@ -668,12 +668,12 @@ void packed_x_images(const void* x, int kind, int64_t rows, int64_t K, uint8_t* 
     else if (K <= 2048) launch_k(x_images_kernel<128>, dim3((unsigned) ((rows + 1) / 2)), dim3(256), 0, st, x, kind, (int) rows, K, codes, sfs, inv);
     else launch_k(x_images_kernel<256>, dim3((unsigned) rows), dim3(256), 0, st, x, kind, (int) rows, K, codes, sfs, inv);
 }
-void packed_listed_images(const float* h, const PassRec* items, const int* n_items, int pass_entries, const TileRec* recs, const int32_t* slab, int64_t K, uint8_t* codes,
+void packed_listed_images(const float* h, const PassRec* items, const int* n_items, int pass_entries, const TileRec* recs, const int32_t* n_recs, int64_t K, uint8_t* codes,
                           uint8_t* sfs, float* inv, cudaStream_t st) {
     const dim3 grid((unsigned) (8 * sm_count()));
-    if (K <= 512) launch_k(listed_images_kernel<32>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, slab, K, codes, sfs, inv);
-    else if (K <= 2048) launch_k(listed_images_kernel<128>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, slab, K, codes, sfs, inv);
-    else launch_k(listed_images_kernel<256>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, slab, K, codes, sfs, inv);
+    if (K <= 512) launch_k(listed_images_kernel<32>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, n_recs, K, codes, sfs, inv);
+    else if (K <= 2048) launch_k(listed_images_kernel<128>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, n_recs, K, codes, sfs, inv);
+    else launch_k(listed_images_kernel<256>, grid, dim3(256), 0, st, h, items, n_items, pass_entries, recs, n_recs, K, codes, sfs, inv);
 }
 int32_t packed_pass_product(bool down, const ExpertArgs& a, const PassRec* items, const int* n_items, int pass_entries, const uint8_t* codes, const uint8_t* sfs,
                             const float* inv, int32_t* status, cudaStream_t st) {

@@ -9,6 +9,7 @@
 namespace bsx {
 
 constexpr int kTermsF = 4;                 // FP4 terms per activation row
+constexpr int kSFChunk = kTermsF * 16;     // scale bytes of a row image's 256 columns, the terms side by side: two whole sectors
 
 // A matrix of R rows x K columns becomes (R / 128) x (K / 256) blocks of kBlockF bytes, row tile major: the block of
 // (tile, chunk) holds that tile's 128 rows x 256 columns of codes as the 16 KB image a stage wants in shared memory
@@ -105,7 +106,7 @@ __device__ __forceinline__ uint32_t fp4_term(float (&v)[16], uint32_t& w0, uint3
 // TPR threads per activation row (32, 128 or 256: a thread per 16-value sub-block where the row allows), 256 / TPR rows a
 // block; every thread of the block must call (the row maximum is reduced through `shf`, 8 floats of shared memory).
 // The scaled row becomes kTermsF FP4 terms, term t of a sub-block from the residual of the ones before.  Layout: codes [image row][term][K / 2] bytes with ggml's nibble order
-// (byte b of a sub-block = values b and b + 8), scales [image row][term][K / 16] bytes, inv[image row] undoes the power of two.
+// (byte b of a sub-block = values b and b + 8), scales [image row][K / 256][term][16] bytes, inv[image row] undoes the power of two.
 template <int TPR>
 __device__ __forceinline__ void fp4_image_row(const void* src, int kind, int64_t row, int64_t K, bool live, int i, uint8_t* __restrict__ codes,
                                               uint8_t* __restrict__ sfs, float* __restrict__ inv, float* shf) {
@@ -144,7 +145,7 @@ __device__ __forceinline__ void fp4_image_row(const void* src, int kind, int64_t
             const uint32_t sb8 = fp4_term(v, w0, w1);
             const size_t r4 = (size_t) i * kTermsF + t;
             *reinterpret_cast<uint2*>(codes + r4 * (K / 2) + (size_t) sb * 8) = make_uint2(w0, w1);
-            sfs[r4 * (K / 16) + sb] = (uint8_t) sb8;
+            sfs[(size_t) i * (K >> 2) + (sb >> 4) * kSFChunk + t * 16 + (sb & 15)] = (uint8_t) sb8;
         }
     }
 }
@@ -153,7 +154,7 @@ __device__ __forceinline__ void fp4_image_row(const void* src, int kind, int64_t
 struct __align__(16) TileRec {
     unsigned long long blob;
     int row0, rows;
-    int64_t base;          // units (of atoms) before this tile's in its slab's tile images (experts_prefill_nvf4.cu)
+    int64_t base;          // units before this tile's in the tile images of its SwiGLU rows, where there are such (experts_prefill_nvf4.cu)
     int64_t pad;
 };
 

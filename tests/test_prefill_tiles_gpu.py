@@ -97,3 +97,15 @@ CROWD = [1000, 3, 0, 1000, 64, 65, 0, 700] + [0] * 55 + [9]
 def test_crowded_short_calls(lib, cuda, H, I, shift, counts, away):
     run(H, I, shift, counts, away)
     run(H, I, shift, counts, away, len(counts))
+
+
+# 34 rows an expert: tiles whose SwiGLU rows are gathered from row images
+MID = [40, 1, 16, 17, 33, 129, 8, 64, 0, 31]
+
+
+@pytest.mark.parametrize("H,I,shift,counts,away", [(256, 256, 0, MID, ()), (768, 512, 16, MID, ()), (512, 1280, 0, MID, (0, 5)), (2048, 2304, 0, MID, ()), (256, 512, 0, MID * 12, ()),
+                                                   (768, 256, 0, TILES * 12, ()), (1280, 768, 0, TILES, (1, 9))])
+def test_tiles_of_gathered_rows(lib, cuda, H, I, shift, counts, away):
+    """Every number of columns modulo 16 on either side of a pair's halves, one and two accumulators an item, few and many items a pair."""
+    run(H, I, shift, counts, away)
+    run(H, I, shift, counts, away, len(counts))
