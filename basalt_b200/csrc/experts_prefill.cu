@@ -22,11 +22,13 @@
 // a sub-block's values in - so no shuffling is needed: the activation image (made by a small kernel here) and the SwiGLU
 // output are simply written in that order.
 #include <atomic>
+#include <type_traits>
 #include <cuda_fp16.h>
 
 #include "common.cuh"
 #include "experts.cuh"
 #include "formats.cuh"
+#include "iq1m.cuh"
 #include "tc5.cuh"
 
 namespace bsx {
@@ -66,38 +68,17 @@ __device__ __forceinline__ uint32_t scale_pair_bits(uint32_t byte) {
     return v | (v << 16);
 }
 
-__device__ __forceinline__ uint32_t hadd2_bits(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-
-// IQ1_M weights as fp16(16 w), packed arithmetic throughout.  A weight is d m (g + delta), g = c - 1 with c the codebook's 2-bit
-// code, m = 2 s + 1 <= 15, delta = +-1/8.  8 m (g + delta) is an integer of at most 135 and exact in fp16 at every step below; the
-// product with 2 d rounds once, so the stored value is the same fp16 the fp32 product would round to.
-// A code becomes its value by masking it where it lies in the codebook word and or-ing in an exponent that makes its place worth
-// one: bits 4-5 under 2^6, 6-7 under 2^4, 8-9 under 2^2 (the constants -(2^E + 1) +- 1/8 stay within fp16's 11 bits only there), so
-// two shifts bring all eight pairs into place and a pair costs one logic and three fp16x2 operations.
-// q16: the two index bytes of 16 values; h8: their high bits and delta signs; s3: the scale field; d2: 2 d twice.
-// out[i] = values i (low half) and i + 8 (high half): the k order both operands are stored in.
+// IQ1_M weights as fp16(16 w): the exact 8 w / d of iq1m.cuh times 2 d, rounded once, so the stored value is the same fp16 the fp32
+// product would round to.  d2: 2 d twice.  out[i] = values i (low half) and i + 8 (high half): the k order both operands are stored in.
 __device__ __forceinline__ void iq1m_16(uint32_t q16, uint32_t h8, uint32_t s3, uint32_t d2, const uint16_t* grid, uint32_t (&out)[8]) {
-    const uint32_t ia = (q16 & 0xFFu) | ((h8 & 7u) << 8), ib = (q16 >> 8) | ((h8 & 0x70u) << 4);
-    const uint32_t x = (uint32_t) grid[ia] | ((uint32_t) grid[ib] << 16);
-    const uint32_t delta = 0x30003000u | ((h8 & 8u) << 12) | ((h8 & 0x80u) << 24);       // +-0.125 each
-    const uint32_t k2 = hadd2_bits(delta, 0xC500C500u), k4 = hadd2_bits(delta, 0xCC40CC40u), k6 = hadd2_bits(delta, 0xD410D410u);   // -5, -17, -65
-    const uint32_t m8 = hadd2_bits((0x6408u | (s3 << 4)) * 0x10001u, 0xE400E400u);       // 1024 + 16 s + 8 - 1024
-    const uint32_t y = x << 4, z = x >> 6;
-    const uint32_t v[8] = {hadd2_bits((y & 0x00300030u) | 0x54005400u, k6), hadd2_bits((y & 0x00C000C0u) | 0x4C004C00u, k4),
-                           hadd2_bits((x & 0x00300030u) | 0x54005400u, k6), hadd2_bits((x & 0x00C000C0u) | 0x4C004C00u, k4),
-                           hadd2_bits((x & 0x03000300u) | 0x44004400u, k2), hadd2_bits((z & 0x00300030u) | 0x54005400u, k6),
-                           hadd2_bits((z & 0x00C000C0u) | 0x4C004C00u, k4), hadd2_bits((z & 0x03000300u) | 0x44004400u, k2)};
+    iq1m_units_16(q16, h8, s3, grid, out);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) out[i] = hmul2_bits(hmul2_bits(v[i], m8), d2);
+    for (int i = 0; i < 8; ++i) out[i] = hmul2_bits(out[i], d2);
 }
-// the block's fp16 super-scale, from the top nibbles of its four scale words, times two, in both halves
+// the block's fp16 super-scale times two, in both halves
 __device__ __forceinline__ uint32_t iq1m_twice_d(uint2 sc) {
-    const uint32_t d = (((sc.x >> 12) & 0x000Fu) | ((sc.x >> 24) & 0x00F0u) | ((sc.y >> 4) & 0x0F00u) | ((sc.y >> 16) & 0xF000u)) * 0x10001u;
-    return hadd2_bits(d, d);
+    const uint32_t d = iq1m_d_bits(sc) * 0x10001u;
+    return iq1m_add2(d, d);
 }
 
 struct PrefillArgs {
@@ -139,16 +120,23 @@ __global__ void __launch_bounds__(256) prefill_prep_x_kernel(const void* __restr
     for (int64_t c = lane; c < H; c += 32) xh[t * H + (c & ~(int64_t) 15) + perm16((int) (c & 15))] = __float2half_rn(ld(c) * s);
 }
 
+// Stages: Q6_K gives one up for the raw words of the two decoder groups, half a block of 256 rows each.
+template <int WT> constexpr int kStagesOf = WT == WT_Q6K ? kStagesP - 1 : kStagesP;
+constexpr int kRawPitch = 31, kRawWords = 256 * kRawPitch;      // 30 words a row; an odd pitch, so that 32 rows' words meet no bank twice
+template <int WT>
+constexpr size_t kSmemOf = 1024 + kStagesOf<WT> * (kTileM * kBlockK * 2 + kTileN * kBlockK * 2) + 256 + 1024 + 4096 + 64 + (WT == WT_Q6K ? 2 * kRawWords * 4 : 0);
+static_assert(kSmemOf<WT_Q6K> <= 227 * 1024 && kSmemOf<WT_NVFP4> <= 227 * 1024, "one CTA per SM");
+
 template <int MODE, bool ALIGNED, int WT>
 __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // 1024-byte aligned operand stages: A then B per stage
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
-    constexpr int kABytes = kTileM * kBlockK * 2, kBBytes = kTileN * kBlockK * 2, kStage = kABytes + kBBytes;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStagesP * kStage);
+    constexpr int kABytes = kTileM * kBlockK * 2, kBBytes = kTileN * kBlockK * 2, kStage = kABytes + kBBytes, kStg = kStagesOf<WT>;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStg * kStage);
     uint64_t* full = bars;                        // [S] loader lanes + one decoder group arrive
-    uint64_t* empty = bars + kStagesP;            // [S] tcgen05.commit arrives
-    uint64_t* acc_full = bars + 2 * kStagesP;     // [2] tcgen05.commit after a tile's last MMA
+    uint64_t* empty = bars + kStg;            // [S] tcgen05.commit arrives
+    uint64_t* acc_full = bars + 2 * kStg;     // [2] tcgen05.commit after a tile's last MMA
     uint64_t* acc_empty = acc_full + 2;           // [2] the 128 epilogue threads arrive
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     uint32_t* lut = tmem_slot + 2;                // [256] fp16 scale pairs
@@ -167,7 +155,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
     if (WT == WT_IQ1M)
         for (int i = threadIdx.x; i < 2048; i += kThreadsP) s_grid[i] = a.grid[i];
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStagesP; ++s) {
+        for (int s = 0; s < kStg; ++s) {
             mbar_init(&full[s], kGroupThreads + 32 * kLoaderWarps);
             mbar_init(&empty[s], 1);
         }
@@ -215,8 +203,8 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 for (int kb = 0; kb < nkb; ++kb, ++kc) {
-                    const uint32_t s = kc % kStagesP;
-                    ok = mbar_wait(&full[s], (kc / kStagesP) & 1u);
+                    const uint32_t s = kc % kStg;
+                    ok = mbar_wait(&full[s], (kc / kStg) & 1u);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     const uint32_t sa = smem_u32(smem + s * kStage), sb = sa + kABytes;
@@ -255,8 +243,8 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                 aoff[i] = grow * (uint32_t) (K >> 3) + (uint32_t) c;
             }
             for (int kb = 0; kb < nkb; ++kb) {
-                const uint32_t s = issued % kStagesP;
-                ok = mbar_wait(&empty[s], ((issued / kStagesP) & 1u) ^ 1u);
+                const uint32_t s = issued % kStg;
+                ok = mbar_wait(&empty[s], ((issued / kStg) & 1u) ^ 1u);
                 if (!ok) break;
                 const uint32_t dst = smem_u32(smem + s * kStage);
 #pragma unroll
@@ -266,17 +254,17 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                 }
                 asm volatile("cp.async.commit_group;\n" ::: "memory");
                 ++issued;
-                if (issued - arrived > 2) {
-                    asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+                if (issued - arrived > kStg - 2) {      // one less than could be requested, or the tensor core would wait for its own last stage
+                    asm volatile("cp.async.wait_group %0;\n" ::"n"(kStg - 2) : "memory");
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    mbar_arrive(&full[arrived % kStagesP]);
+                    mbar_arrive(&full[arrived % kStg]);
                     ++arrived;
                 }
             }
         }
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        for (; arrived < issued; ++arrived) mbar_arrive(&full[arrived % kStagesP]);
+        for (; arrived < issued; ++arrived) mbar_arrive(&full[arrived % kStg]);
         if (!ok) atomicOr(a.status, kStatusTimeout);
     } else if (warp <= kLoaderWarps + kDecoderWarps) {
         // ---- weight decoders: thread (group, row r) turns the NVFP4 blocks of weight row r of the tile into fp16 B-tile rows
@@ -361,8 +349,8 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                     for (int j = 0; j < 2; ++j) {
                         const int kb = 2 * q + j;
                         if (kb < nkb && ok) {
-                            const uint32_t kk = kc + (uint32_t) kb, s = kk % kStagesP;
-                            ok = mbar_wait(&empty[s], ((kk / kStagesP) & 1u) ^ 1u);
+                            const uint32_t kk = kc + (uint32_t) kb, s = kk % kStg;
+                            ok = mbar_wait(&empty[s], ((kk / kStg) & 1u) ^ 1u);
                             if (ok) {
                                 store_b(s, &wc[9 * j]);
                                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> visible to the tensor core
@@ -412,8 +400,8 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
 #pragma unroll
                         for (int sub = 0; sub < 4; ++sub)
                             iq1m_16((qs[2 * j + (sub >> 1)] >> (16 * (sub & 1))) & 0xFFFFu, (qh[j] >> (8 * sub)) & 0xFFu, (scw >> (16 * j + 3 * sub)) & 7u, d2, s_grid, p[sub]);
-                        const uint32_t kk = kc + (uint32_t) kb, s = kk % kStagesP;
-                        ok = mbar_wait(&empty[s], ((kk / kStagesP) & 1u) ^ 1u);
+                        const uint32_t kk = kc + (uint32_t) kb, s = kk % kStg;
+                        ok = mbar_wait(&empty[s], ((kk / kStg) & 1u) ^ 1u);
                         if (!ok) break;
                         uint4* brow = reinterpret_cast<uint4*>(smem + s * kStage + row_off);
 #pragma unroll
@@ -430,43 +418,77 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                 it = itn;
             }
         } else {
-            // Q6_K rows (210 bytes per 256 values): the thread decodes its row's 64 values of a k-block exactly (formats.cuh), stores
-            // them as fp16(16 w) - the rounding, 2^-11 relative, is the only one - in the permuted k order, and hands the stage over.
+            // Q6_K rows (210 bytes per 256 values, on 2 bytes): a pair of k-blocks is half a block - 64 bytes of low bits, 32 of high bits, 8
+            // scales, d - as the 30 words that cover it, which the group's warps fetch row by row (a row's words side by side, where a
+            // thread reading its own row touches 32 lines a load) into shared memory.  A thread then decodes its row: codes four at a
+            // time, each to fp32 by its byte under the exponent of 2^23, times 16 d sc, pairs rounded to fp16 - the only rounding, 2^-11
+            // relative.  4096 rows of 2048 x 512, 512 experts, whole layer: byte by byte from global memory 28.4 ms, so 1.94.
+            // A wait that gave up does not end the loop: the other threads of the group wait for this one at its barriers.
+            uint32_t* raw = reinterpret_cast<uint32_t*>(s_grid + 2048) + grp * kRawWords;
+            const uint32_t* mine = raw + r * kRawPitch;
+            const int warp_g = td >> 5 & 7;
+            const int seg = lane < 17 ? 0 : lane < 26 ? 1 : lane < 29 ? 2 : 3, seg_word = lane - (seg == 0 ? 0 : seg == 1 ? 17 : seg == 2 ? 26 : 29);
             uint32_t kc = 0;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
                 Item it;
                 if (!get_item(item, it)) continue;
-                const uint8_t* wrow = weight_row(it);
-                for (int q = grp; q < npair && ok; q += 2) {
-#pragma unroll 1
+                auto row_at = [&](int row) -> const uint8_t* {
+                    if (MODE == PMODE_GU) {
+                        const int n = min(it.n0 + (row & 127), n_out - 1);
+                        return row < 128 ? it.blob + (size_t) n * a.L.gu_row : it.blob + a.L.up_off + (size_t) n * a.L.up_row;
+                    }
+                    return it.blob + a.L.down_off + (size_t) min(it.n0 + row, n_out - 1) * a.L.d_row;
+                };
+                const bool own_odd = (reinterpret_cast<uintptr_t>(row_at(r)) & 2) != 0;
+                for (int q = grp; q < npair; q += 2) {
+                    const size_t blk = (size_t) (q >> 1) * 210;
+                    const int hb = q & 1;
+                    const size_t off = blk + (seg == 0 ? 64 * hb : seg == 1 ? 128 + 32 * hb : seg == 2 ? 192 + 8 * hb : 208);
+                    asm volatile("bar.sync %0, 256;\n" ::"r"(1 + grp) : "memory");            // everyone is done with the words of the pair before
+#pragma unroll 4
+                    for (int i = 0; i < 32; ++i) {
+                        const int row = 32 * warp_g + i;
+                        const uintptr_t src = (reinterpret_cast<uintptr_t>(row_at(row) + off) & ~(uintptr_t) 3) + 4 * seg_word;
+                        if (lane < 30)
+                            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(raw + row * kRawPitch + lane)), "l"(src) : "memory");
+                    }
+                    asm volatile("cp.async.wait_all;\n" ::: "memory");
+                    asm volatile("bar.sync %0, 256;\n" ::"r"(1 + grp) : "memory");
+                    const bool odd = own_odd != ((q >> 1) & 1);
+                    auto word = [&](int first, int k) { return odd ? __funnelshift_r(mine[first + k], mine[first + k + 1], 16) : mine[first + k]; };
+                    const uint32_t dw = mine[29];
+                    const float d16 = __half2float(__ushort_as_half((unsigned short) (odd ? dw >> 16 : dw & 0xFFFFu))) * kWScaleKQ;
+                    const uint32_t sc[2] = {word(26, 0), word(26, 1)};
+#pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        const int kb = 2 * q + j;
-                        if (kb >= nkb || !ok) continue;
-                        float v[64];
-                        const uint8_t* blk = wrow + (size_t) (kb >> 2) * 210;
-                        const int u0 = 2 * (kb & 3);
-                        decode_q6k_32(blk, u0, v);
-                        decode_q6k_32(blk, u0 + 1, v + 32);
-                        const uint32_t kk = kc + (uint32_t) kb, s = kk % kStagesP;
-                        ok = mbar_wait(&empty[s], ((kk / kStagesP) & 1u) ^ 1u);
-                        if (!ok) break;
+                        const uint32_t kk = kc + (uint32_t) (2 * q + j), s = kk % kStg;
+                        if (ok) ok = mbar_wait(&empty[s], ((kk / kStg) & 1u) ^ 1u);
                         uint4* brow = reinterpret_cast<uint4*>(smem + s * kStage + row_off);
 #pragma unroll
                         for (int sub = 0; sub < 4; ++sub) {
-                            const float* w = v + 16 * sub;
-                            uint32_t p0[4], p1[4];
+                            const int g4 = 4 * j + sub, from = g4 >> 1, l16 = g4 & 1;             // 32 values `from` of the half, 16 of them
+                            const float scale = d16 * (float) (int8_t) (sc[g4 >> 2] >> (8 * (g4 & 3)));
+                            uint32_t c[4];
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
-                                const __half2 a2 = __floats2half2_rn(w[i] * kWScaleKQ, w[i + 8] * kWScaleKQ);
-                                const __half2 b2 = __floats2half2_rn(w[4 + i] * kWScaleKQ, w[12 + i] * kWScaleKQ);
-                                p0[i] = *reinterpret_cast<const uint32_t*>(&a2);
-                                p1[i] = *reinterpret_cast<const uint32_t*>(&b2);
+                                const uint32_t lo = word(0, (from & 1) * 8 + 4 * l16 + i), hi = word(17, 4 * l16 + i);
+                                c[i] = ((from >= 2 ? lo >> 4 : lo) & 0x0F0F0F0Fu) | (((hi >> (2 * from)) & 0x03030303u) << 4);
                             }
-                            brow[(2 * sub) ^ swz] = make_uint4(p0[0], p0[1], p0[2], p0[3]);
-                            brow[(2 * sub + 1) ^ swz] = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+                            uint32_t p[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {       // values i and i + 8: the k order both operands are stored in
+                                const float u = __uint_as_float(__byte_perm(c[i >> 2], 0x4B000000u, 0x7440 + (i & 3))) - 8388640.f;
+                                const float v = __uint_as_float(__byte_perm(c[2 + (i >> 2)], 0x4B000000u, 0x7440 + (i & 3))) - 8388640.f;
+                                const __half2 h2 = __floats2half2_rn(u * scale, v * scale);
+                                p[i] = *reinterpret_cast<const uint32_t*>(&h2);
+                            }
+                            if (ok) {
+                                brow[(2 * sub) ^ swz] = make_uint4(p[0], p[1], p[2], p[3]);
+                                brow[(2 * sub + 1) ^ swz] = make_uint4(p[4], p[5], p[6], p[7]);
+                            }
                         }
                         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                        mbar_arrive(&full[s]);
+                        if (ok) mbar_arrive(&full[s]);
                     }
                 }
                 kc += (uint32_t) nkb;
@@ -478,6 +500,7 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
         // TMEM lanes 32 (warp % 4) .. + 31.  tcgen05.ld is warp-wide: every lane runs the loads; only the stores are predicated.
         const int p = (warp & 3) * 32 + lane;
         const uint32_t lane_base = (uint32_t) ((warp & 3) * 32) << 16;
+        const int form = swiglu_form(a.L);
         uint32_t ti = 0;
         for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
             Item it;
@@ -503,11 +526,16 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                     tmem_ld16(tbase + (uint32_t) c0, g);
                     tmem_ld16(tbase + (uint32_t) (kTileN / 2 + c0), u);
                     __half out[16];
+                    auto work = [&](auto act) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float hv = swiglu(__uint_as_float(g[j]) * sg, __uint_as_float(u[j]) * su, a.L) * kHScale;
-                        out[perm16(j)] = __float2half_rn(fminf(fmaxf(hv, -65504.f), 65504.f));
-                    }
+                        for (int j = 0; j < 16; ++j) {
+                            const float hv = swiglu_as<decltype(act)::value>(__uint_as_float(g[j]) * sg, __uint_as_float(u[j]) * su, a.L) * kHScale;
+                            out[perm16(j)] = __float2half_rn(fminf(fmaxf(hv, -65504.f), 65504.f));
+                        }
+                    };
+                    if (form == SWIGLU_PLAIN) work(std::integral_constant<int, SWIGLU_PLAIN>{});
+                    else if (form == SWIGLU_LIMIT) work(std::integral_constant<int, SWIGLU_LIMIT>{});
+                    else work(std::integral_constant<int, SWIGLU_CAP>{});
                     if (row_live && it.n0 + c0 < n_out) {
                         reinterpret_cast<uint4*>(hrow + c0)[0] = reinterpret_cast<const uint4*>(out)[0];
                         reinterpret_cast<uint4*>(hrow + c0)[1] = reinterpret_cast<const uint4*>(out)[1];
@@ -545,22 +573,21 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
 }
 
 size_t align256p(size_t v) { return (v + 255) & ~(size_t) 255; }
-constexpr size_t kSmemP = 1024 + kStagesP * (kTileM * kBlockK * 2 + kTileN * kBlockK * 2) + 256 + 1024 + 4096 + 64;   // 203,136 bytes: one CTA per SM
 
 int wt_of(int type) { return type == kTypeNVFP4 ? WT_NVFP4 : type == kTypeQ6K ? WT_Q6K : type == kTypeIQ1M ? WT_IQ1M : -1; }
 
 template <int MODE, bool ALIGNED, int WT>
-cudaError_t configure_one() { return cudaFuncSetAttribute(prefill_gemm_kernel<MODE, ALIGNED, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemP); }
+cudaError_t configure_one() { return cudaFuncSetAttribute(prefill_gemm_kernel<MODE, ALIGNED, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemOf<WT>); }
 
 template <int MODE>
 void launch_mode(int wt, bool aligned16, unsigned grid, const PrefillArgs& a, cudaStream_t st) {
     if (wt == WT_NVFP4) {
-        if (aligned16) prefill_gemm_kernel<MODE, true, WT_NVFP4><<<grid, kThreadsP, kSmemP, st>>>(a);
-        else prefill_gemm_kernel<MODE, false, WT_NVFP4><<<grid, kThreadsP, kSmemP, st>>>(a);
+        if (aligned16) prefill_gemm_kernel<MODE, true, WT_NVFP4><<<grid, kThreadsP, kSmemOf<WT_NVFP4>, st>>>(a);
+        else prefill_gemm_kernel<MODE, false, WT_NVFP4><<<grid, kThreadsP, kSmemOf<WT_NVFP4>, st>>>(a);
     } else if (wt == WT_Q6K) {
-        prefill_gemm_kernel<MODE, false, WT_Q6K><<<grid, kThreadsP, kSmemP, st>>>(a);
+        prefill_gemm_kernel<MODE, false, WT_Q6K><<<grid, kThreadsP, kSmemOf<WT_Q6K>, st>>>(a);
     } else {
-        prefill_gemm_kernel<MODE, false, WT_IQ1M><<<grid, kThreadsP, kSmemP, st>>>(a);
+        prefill_gemm_kernel<MODE, false, WT_IQ1M><<<grid, kThreadsP, kSmemOf<WT_IQ1M>, st>>>(a);
     }
 }
 
