@@ -265,9 +265,11 @@ static int32_t experts_grouped_impl(int32_t n_x_rows, const bsx_expert_layout* l
     if (!a.grid) return (int32_t) cudaErrorInvalidSymbol;
     const cudaStream_t st = (cudaStream_t) stream;
     if (!(a.L.options & BSX_EXPERT_PLAIN)) {
-        int32_t rc = experts_grouped_mma(a, st);      // NVFP4 and IQ3_S blobs: fp16 images, mma.sync
+        int32_t rc = experts_grouped_mma(a, false, st);      // NVFP4 and IQ3_S blobs: fp16 images, mma.sync
         if (rc != BSX_E_TYPE) return rc;
-        rc = experts_grouped_kq(a, st);               // Q6_K / IQ1_M blobs: int8 images, integer mma.sync
+        rc = experts_grouped_kq(a, st);                      // Q6_K / IQ1_M blobs: int8 images, integer mma.sync
+        if (rc != BSX_E_TYPE) return rc;
+        rc = experts_grouped_mma(a, true, st);               // IQ1_M blobs of other widths: as the first
         if (rc != BSX_E_TYPE) return rc;
     }
     return experts_grouped_simple(a, st);

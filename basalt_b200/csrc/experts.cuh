@@ -95,7 +95,8 @@ inline int experts_phase(const bsx_expert_layout& L) { return L.options & BSX_EX
 
 int32_t experts_grouped_simple(const ExpertArgs& a, cudaStream_t st);
 // returns BSX_E_TYPE when the fast path does not cover the layout (the caller then runs the plain kernels)
-int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st);
+// (iq1m: take IQ1_M too, where the integer kernel does not)
+int32_t experts_grouped_mma(const ExpertArgs& a, bool iq1m, cudaStream_t st);
 // the same call over blobs repacked by bsx_expert_pack (experts_nvf4.cu): block-scaled FP4 MMAs straight on the NVFP4 codes
 // pass_list_ready: the pass list (plan.cuh) already sits in the scratch (the fused selection + plan kernel wrote it)
 struct PassRec;

@@ -20,6 +20,9 @@
 // said: IQ3_S, 512 experts, 5 tokens 125 -> 99 us, 64 tokens 420 -> 305; NVFP4, 1 token 52 -> 34, 64 tokens 169 -> 154, 27 tokens of
 // 2560 x 640 223 -> 175.
 //
+// IQ1_M rows take it where the integer kernel (experts_kq.cu) does not: widths of an odd number of 256-column blocks, which the
+// warp-per-row fp32 kernels had before, so they keep fp32-class results.  Weights are 8 w / d, exact in fp16 (iq1m.cuh).
+//
 // Semantics: Basalt's native_expert_grouped (include/basalt/kernels/iq_kernels.hpp:77-92; kernels src/kernels/cuda/iq_kernels.cu:
 // 1605-1658 gate/up, :2512-2524 SwiGLU, :2140-2164 down), NVFP4 decoding per src/kernels/cpu/ggml/ggml_quants.c:1397-1422,
 // tail scales per iq_kernels.cu:683-701 - but without the int8 rounding of x and h the reference applies.
@@ -29,6 +32,7 @@
 #include "common.cuh"
 #include "experts.cuh"
 #include "formats.cuh"
+#include "iq1m.cuh"
 #include "pdl.cuh"
 #include "plan.cuh"
 
@@ -38,9 +42,10 @@ namespace {
 constexpr int kRows = 16;                      // weight rows per warp
 constexpr int kCols = 8;                       // MMA n: activation columns per pass
 
-// The formats.  A chunk of a row is what a stage holds: 4 NVFP4 blocks of 64 columns, or 2 IQ3_S blocks of 256 (110 bytes, so every
-// second one starts on 4 bytes).  kTable: the shared-memory table, 256 fp16 scale pairs or 512 points of four fp16 magnitudes.
-enum { FMT_NVFP4 = 0, FMT_IQ3S = 1 };
+// The formats.  A chunk of a row is what a stage holds: 4 NVFP4 blocks of 64 columns, 2 IQ3_S blocks of 256 (110 bytes, so every
+// second one starts on 4 bytes) or 2 IQ1_M blocks of 256 (56 bytes; a row may end in one).  kTable: the shared-memory table, 256 fp16 scale
+// pairs, 512 points of four fp16 magnitudes or the 2048 points of the IQ1 codebook as they are.
+enum { FMT_NVFP4 = 0, FMT_IQ3S = 1, FMT_IQ1M = 2 };
 template <int FMT> struct Fmt;
 template <> struct Fmt<FMT_NVFP4> {
     static constexpr int kRowBytes = 144, kGranules = 4, kTable = 1024;
@@ -49,6 +54,10 @@ template <> struct Fmt<FMT_NVFP4> {
 template <> struct Fmt<FMT_IQ3S> {
     static constexpr int kRowBytes = 220, kGranules = 8, kTable = 4096;
     static constexpr float kUnscale = 1.f;
+};
+template <> struct Fmt<FMT_IQ1M> {
+    static constexpr int kRowBytes = 112, kGranules = 8, kTable = 4096;
+    static constexpr float kUnscale = 0.125f;          // weights enter as 8 w / d
 };
 template <int FMT> constexpr int kStageBytes = kRows * Fmt<FMT>::kRowBytes;
 
@@ -283,6 +292,8 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
     // the first barrier below publishes the table
     if constexpr (FMT == FMT_NVFP4) {
         if (threadIdx.x < 256) lut[threadIdx.x] = scale_pair_bits(threadIdx.x);
+    } else if constexpr (FMT == FMT_IQ1M) {
+        for (int i = threadIdx.x; i < 1024; i += kThreads) lut[i] = reinterpret_cast<const uint32_t*>(a.grid)[i];
     } else {
         for (int i = threadIdx.x; i < 512 * NC; i += kThreads) {
             const uint32_t pt = a.grid[kGridIQ3S + i / NC];
@@ -298,7 +309,8 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
     constexpr int kStepRows = kTiles * kTileRows;
     const int row_chunks = (n_gran + F::kGranules - 1) / F::kGranules;
     const int chunk0 = row_chunks * (warp % KS) / KS, n_chunks = row_chunks * (warp % KS + 1) / KS - chunk0;      // this warp's part of a row
-    const int last_bytes = FMT == FMT_IQ3S || PIECE == 16 ? kRowBytes : (n_gran - 4 * (row_chunks - 1)) * 36;   // bytes of a row in its last chunk
+    const int last_bytes = FMT == FMT_IQ1M ? (n_gran - 8 * (row_chunks - 1)) / 4 * 56       // bytes of a row in its last chunk
+                         : FMT == FMT_IQ3S || PIECE == 16 ? kRowBytes : (n_gran - 4 * (row_chunks - 1)) * 36;
     const int pieces_per_col = (int) (K >> 3);               // 16-byte pieces of one image
 
     // this lane's copy duty inside a stage: pieces lane, lane + 32, ...; row = piece / kRowPieces
@@ -437,19 +449,37 @@ blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __rest
                 const uint32_t* ra = reinterpret_cast<const uint32_t*>(st + g * kRowBytes);          // row g
                 const uint32_t* rb = reinterpret_cast<const uint32_t*>(st + (g + 8) * kRowBytes);    // row g + 8
                 const uint4* bp = bcol + (size_t) (chunk0 + chunk) * F::kGranules * bstep;
-                if constexpr (FMT == FMT_IQ3S) {
+                if constexpr (FMT != FMT_NVFP4) {
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
-                        const uint8_t* ba = reinterpret_cast<const uint8_t*>(ra) + 110 * b;
-                        const uint8_t* bb = reinterpret_cast<const uint8_t*>(rb) + 110 * b;
+                        if (FMT == FMT_IQ1M && 8 * (chunk0 + chunk) + 4 * b >= n_gran) break;       // past the row's last block
+                        const uint8_t* ba = reinterpret_cast<const uint8_t*>(ra) + kRowBytes / 2 * b;
+                        const uint8_t* bb = reinterpret_cast<const uint8_t*>(rb) + kRowBytes / 2 * b;
                         float sum[4] = {0.f, 0.f, 0.f, 0.f};
-                        const float da = __half2float(*reinterpret_cast<const __half*>(ba)), db = __half2float(*reinterpret_cast<const __half*>(bb));
+                        float da, db;
+                        if constexpr (FMT == FMT_IQ1M) {
+                            da = __half2float(__ushort_as_half((unsigned short) iq1m_d_bits(*reinterpret_cast<const uint2*>(ba + 48))));
+                            db = __half2float(__ushort_as_half((unsigned short) iq1m_d_bits(*reinterpret_cast<const uint2*>(bb + 48))));
+                        } else {
+                            da = __half2float(*reinterpret_cast<const __half*>(ba));
+                            db = __half2float(*reinterpret_cast<const __half*>(bb));
+                        }
 #pragma unroll
                         for (int gr = 0; gr < 4; ++gr) {
                             const uint4 b0 = bp[(4 * b + gr) * bstep], b1 = bp[(4 * b + gr) * bstep + bhalf];
                             uint32_t qa[8], qb[8];
-                            iq3s_16<NC>(ba, gr, t, reinterpret_cast<const uint2*>(lut) + (lane & (NC - 1)), qa);
-                            iq3s_16<NC>(bb, gr, t, reinterpret_cast<const uint2*>(lut) + (lane & (NC - 1)), qb);
+                            if constexpr (FMT == FMT_IQ1M) {
+                                // the sub-block's two index bytes, its byte of high bits, its 3 bits of the granule's scale word
+                                auto units = [&](const uint8_t* blk, uint32_t (&q)[8]) {
+                                    iq1m_units_16(*reinterpret_cast<const uint16_t*>(blk + 8 * gr + 2 * t), blk[32 + 4 * gr + t],
+                                                  (*reinterpret_cast<const uint16_t*>(blk + 48 + 2 * gr) >> (3 * t)) & 7u, reinterpret_cast<const uint16_t*>(lut), q);
+                                };
+                                units(ba, qa);
+                                units(bb, qb);
+                            } else {
+                                iq3s_16<NC>(ba, gr, t, reinterpret_cast<const uint2*>(lut) + (lane & (NC - 1)), qa);
+                                iq3s_16<NC>(bb, gr, t, reinterpret_cast<const uint2*>(lut) + (lane & (NC - 1)), qb);
+                            }
                             float s0[4], s1[4], s2[4], s3[4];
                             mma_f16_zero(s0, qa[0], qb[0], qa[1], qb[1], b0.x, b0.y);
                             mma_f16_zero(s1, qa[2], qb[2], qa[3], qb[3], b0.z, b0.w);
@@ -588,23 +618,23 @@ int32_t launch_as(const ExpertArgs& a, const __half* img, const float* inv, cons
 template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN>
 int32_t launch(const ExpertArgs& a, const __half* img, const float* inv, const PassRec* items, const int* n_items, cudaStream_t st) {
     const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff, rows = MODE == MODE_GU ? a.L.n_ff : a.L.n_embd;
-    const bool two = FMT == FMT_NVFP4 && smem_bytes<FMT>(K, 8, 3, 1, 4) <= kSmemTwo;
+    const bool two = FMT != FMT_IQ3S && smem_bytes<FMT>(K, 8, 3, 1, 4) <= kSmemTwo;
     const bool copies = FMT == FMT_IQ3S && smem_bytes<FMT>(K, 16, 2, 16, 4) <= kSmemOne;
     // columns are split where whole rows would leave a block few steps, so that the last, partial one weighs little: IQ3_S up to eight
     // steps (24 tokens of 2048 x 512, 512 experts, 7.4 steps: 202 us whole, 193 split in two), NVFP4, whose decode costs less beside the
     // sums' exchange, up to four (16 tokens of 2560 x 640, 6.2 steps: 123 whole, 130 split).  cap_groups and cap_entries bound the passes
     // on the host
-    const int64_t chunks = FMT == FMT_IQ3S ? K / 512 : (K + 255) / 256, step_rows = (MODE == MODE_GU ? 8 : 16) * (two ? 8 : 16);
+    const int64_t chunks = FMT == FMT_NVFP4 ? (K + 255) / 256 : (K + 511) / 512, step_rows = (MODE == MODE_GU ? 8 : 16) * (two ? 8 : 16);
     const int64_t steps = (a.cap_groups + a.cap_entries / (kCols / TERMS)) * ((rows + step_rows - 1) / step_rows);
     int ks = 1;
-    while (ks < 4 && chunks >= 2 * ks && steps * ks < (FMT == FMT_IQ3S ? 8 : 4) * (int64_t) sm_count() * (two ? 2 : 1)) ks *= 2;
+    while (ks < 4 && chunks >= 2 * ks && steps * ks < (FMT == FMT_NVFP4 ? 4 : 8) * (int64_t) sm_count() * (two ? 2 : 1)) ks *= 2;
 #define BLK_AS(W, OCC, ST, NC) \
     do { \
         if (ks == 4) return launch_as<FMT, MODE, TERMS, PIECE, CHAIN, W, OCC, ST, NC, 4>(a, img, inv, items, n_items, st); \
         if (ks == 2) return launch_as<FMT, MODE, TERMS, PIECE, CHAIN, W, OCC, ST, NC, 2>(a, img, inv, items, n_items, st); \
         return launch_as<FMT, MODE, TERMS, PIECE, CHAIN, W, OCC, ST, NC, 1>(a, img, inv, items, n_items, st); \
     } while (0)
-    if constexpr (FMT == FMT_NVFP4) {
+    if constexpr (FMT != FMT_IQ3S) {
         if (two) BLK_AS(8, 2, 3, 1);
     } else {
         if (copies) BLK_AS(16, 1, 2, 16);
@@ -622,20 +652,23 @@ size_t experts_mma_scratch_bytes(int64_t cap_entries, int64_t n_embd, int64_t n_
            align256((size_t) (cap_entries + 1) * 16 + 16);
 }
 
-int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
+int32_t experts_grouped_mma(const ExpertArgs& a, bool iq1m, cudaStream_t st) {
     const bsx_expert_layout& L = a.L;
     // NVFP4: gate and up rows are whole 256-column chunks (n_embd % 256 == 0 in every layout), down rows whole 64-column blocks.
-    // IQ3_S: rows of whole 512-column chunks (every other 110-byte block starts on 4 bytes, what the copies need).  The activation
-    // image must fit shared memory.
-    const int fmt = L.gu_type == kTypeNVFP4 ? FMT_NVFP4 : FMT_IQ3S;
+    // IQ3_S: rows of whole 512-column chunks (every other 110-byte block starts on 4 bytes, what the copies need).  IQ1_M: whole blocks of
+    // 256 columns.  The activation image must fit shared memory.
+    const int fmt = L.gu_type == kTypeNVFP4 ? FMT_NVFP4 : L.gu_type == kTypeIQ3S ? FMT_IQ3S : FMT_IQ1M;
     const bool whole = L.n_ff % 256 == 0;
-    if ((L.gu_type != kTypeNVFP4 && L.gu_type != kTypeIQ3S) || L.up_type != L.gu_type || L.d_type != L.gu_type) return BSX_E_TYPE;
+    if ((L.gu_type != kTypeNVFP4 && L.gu_type != kTypeIQ3S && !(iq1m && L.gu_type == kTypeIQ1M)) || L.up_type != L.gu_type || L.d_type != L.gu_type) return BSX_E_TYPE;
     if (fmt == FMT_NVFP4) {
         if (L.n_embd % 256 || L.n_ff % 64) return BSX_E_TYPE;
         if (!fits<FMT_NVFP4>(L.n_embd) || !fits<FMT_NVFP4>(L.n_ff)) return BSX_E_TYPE;
-    } else {
+    } else if (fmt == FMT_IQ3S) {
         if (L.n_embd % 512 || L.n_ff % 512) return BSX_E_TYPE;
         if (!fits<FMT_IQ3S>(L.n_embd) || !fits<FMT_IQ3S>(L.n_ff)) return BSX_E_TYPE;
+    } else {
+        if (L.n_embd % 256 || L.n_ff % 256) return BSX_E_TYPE;
+        if (!fits<FMT_IQ1M>(L.n_embd) || !fits<FMT_IQ1M>(L.n_ff)) return BSX_E_TYPE;
     }
     // scratch: [h fp32][x images][h images][x inverse scales][h inverse scales]
     uint8_t* p = reinterpret_cast<uint8_t*>(a.h) + align256((size_t) a.cap_entries * L.n_ff * 4);
@@ -656,11 +689,13 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
         if (a.x_kind == BSX_X_BF16) {
             launch_k(fmt == FMT_IQ3S ? prep_image_kernel<FMT_IQ3S, false, 1> : prep_image_kernel<FMT_NVFP4, false, 1>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
             rc = fmt == FMT_IQ3S ? launch<FMT_IQ3S, MODE_GU, 1, 4, 1>(a, ximg, xinv, items, n_items, st)
+                 : fmt == FMT_IQ1M ? launch<FMT_IQ1M, MODE_GU, 1, 8, 1>(a, ximg, xinv, items, n_items, st)
                  : whole         ? launch<FMT_NVFP4, MODE_GU, 1, 16, 4>(a, ximg, xinv, items, n_items, st)
                                  : launch<FMT_NVFP4, MODE_GU, 1, 16, 1>(a, ximg, xinv, items, n_items, st);
         } else {
             launch_k(fmt == FMT_IQ3S ? prep_image_kernel<FMT_IQ3S, false, 2> : prep_image_kernel<FMT_NVFP4, false, 2>, dim3(nbx), dim3(256), 0, st, a, ximg, xinv, items, n_items);
             rc = fmt == FMT_IQ3S ? launch<FMT_IQ3S, MODE_GU, 2, 4, 1>(a, ximg, xinv, items, n_items, st)
+                 : fmt == FMT_IQ1M ? launch<FMT_IQ1M, MODE_GU, 2, 8, 1>(a, ximg, xinv, items, n_items, st)
                  : whole         ? launch<FMT_NVFP4, MODE_GU, 2, 16, 4>(a, ximg, xinv, items, n_items, st)
                                  : launch<FMT_NVFP4, MODE_GU, 2, 16, 1>(a, ximg, xinv, items, n_items, st);
         }
@@ -668,6 +703,7 @@ int32_t experts_grouped_mma(const ExpertArgs& a, cudaStream_t st) {
     if (rc != BSX_OK || phase == 1) return rc;
     launch_k(fmt == FMT_IQ3S ? prep_image_kernel<FMT_IQ3S, true, 2> : prep_image_kernel<FMT_NVFP4, true, 2>, dim3(nbh), dim3(256), 0, st, a, himg, hinv, items, n_items);
     if (fmt == FMT_IQ3S) return launch<FMT_IQ3S, MODE_DOWN, 2, 4, 1>(a, himg, hinv, items, n_items, st);
+    if (fmt == FMT_IQ1M) return launch<FMT_IQ1M, MODE_DOWN, 2, 8, 1>(a, himg, hinv, items, n_items, st);
     // Down rows of n_ff columns: the copies' width is what their start is aligned to.  An n_ff that is not whole 256-column chunks
     // went to the warp-per-row kernels before (2 % of the copy bandwidth: fp32 decode and FMA for every weight and entry); here
     // the same 27-token step (2560 x 640, 512 + 1 experts, top-10) takes 217 us instead of 3648.

@@ -1,4 +1,4 @@
-"""NVFP4 and IQ3_S experts in place where the streaming kernel's launch shape changes: rows split over four, two or no warps (few, some and
+"""NVFP4, IQ3_S and (odd numbers of 256-column blocks) IQ1_M experts in place where the streaming kernel's launch shape changes: rows split over four, two or no warps (few, some and
 many groups), one block of sixteen warps or two of eight (narrow and wide rows), one codebook copy or sixteen, runs of row blocks that
 end inside a pass.  Bound 1e-5, as for the same kernel's other tests: fp16 hi + lo rows (22 bits), fp32 sums over at most 5120 columns."""
 import numpy as np
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("t,H,I", [(O.T_NVFP4, 2048, 512), (O.T_NVFP4, 4096, 320), (O.T_NVFP4, 512, 3584), (O.T_IQ3_S, 2048, 512), (O.T_IQ3_S, 3072, 512),
-                                   (O.T_IQ3_S, 512, 5120)])
+                                   (O.T_IQ3_S, 512, 5120), (O.T_IQ1_M, 768, 256), (O.T_IQ1_M, 2560, 1280), (O.T_IQ1_M, 256, 3840), (O.T_IQ1_M, 5120, 768)])
 @pytest.mark.parametrize("n_groups", [2, 40, 300])
 def test_runs_of_row_blocks(lib, cuda, t, H, I, n_groups):
     rng = np.random.default_rng(H + I + n_groups)
