@@ -330,21 +330,25 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
             // the stream of own pairs runs across items: the first pair of the next item is requested while the last pair of this
             // one is decoded, so a tile switch does not expose a load
             uint32_t wc[18], wn[18];
+            // The groups take turns across items too (an item may have an odd number of pairs): a group that left out more k-blocks than there
+            // are stages could take an earlier phase of a stage's barrier for the one it waits for.
             uint32_t kc = 0;
+            int first = grp;
             int item = blockIdx.x;
             Item it;
             while (item < n_items && !get_item(item, it)) item += gridDim.x;
-            if (item < n_items && grp < npair) load_pair(weight_row(it), grp, wn);
+            if (item < n_items && first < npair) load_pair(weight_row(it), first, wn);
             while (item < n_items && ok) {
                 const uint8_t* wrow = weight_row(it);
                 int nxt = item + gridDim.x;
                 Item itn;
                 while (nxt < n_items && !get_item(nxt, itn)) nxt += gridDim.x;
-                for (int q = grp; q < npair && ok; q += 2) {
+                const int first_next = first ^ (npair & 1);
+                for (int q = first; q < npair && ok; q += 2) {
 #pragma unroll
                     for (int i = 0; i < 18; ++i) wc[i] = wn[i];
                     if (q + 2 < npair) load_pair(wrow, q + 2, wn);
-                    else if (nxt < n_items) load_pair(weight_row(itn), grp, wn);
+                    else if (nxt < n_items && first_next < npair) load_pair(weight_row(itn), first_next, wn);
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         const int kb = 2 * q + j;
@@ -359,6 +363,8 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_gemm_kernel(PrefillArgs 
                         }
                     }
                 }
+                if (first >= npair && nxt < n_items && first_next < npair) load_pair(weight_row(itn), first_next, wn);      // this item had no pair for the group
+                first = first_next;
                 kc += (uint32_t) nkb;
                 item = nxt;
                 it = itn;
