@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "experts.cuh"
 #include "formats.cuh"
+#include "fp16_rows.cuh"
 #include "iq1m.cuh"
 #include "tc5.cuh"
 
@@ -95,30 +96,6 @@ struct PrefillArgs {
     float* dm;                               // [rows][H] fp32
     int32_t* status;                         // sticky error word (0 = ok)
 };
-
-// x [T][H] (fp32 or bf16) -> fp16 rows scaled by a power of two into fp16's range, k-permuted inside 16-column groups
-__global__ void __launch_bounds__(256) prefill_prep_x_kernel(const void* __restrict__ x, int kind, int64_t T, int64_t H, __half* __restrict__ xh,
-                                                             float* __restrict__ xinv) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t t = (int64_t) blockIdx.x * 8 + warp;
-    if (t >= T) return;
-    auto ld = [&](int64_t c) {
-        return kind == BSX_X_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(x)[t * H + c]) : static_cast<const float*>(x)[t * H + c];
-    };
-    float amax = 0.f;
-    for (int64_t c = lane; c < H; c += 32) amax = fmaxf(amax, fabsf(ld(c)));
-    amax = warp_max_xor(amax);
-    int ex = 0;
-    float s = 1.f, iv = 1.f;
-    if (amax > 0.f && amax <= 3.0e38f) {
-        frexpf(amax, &ex);
-        ex = max(-100, min(100, 14 - ex));
-        s = ldexpf(1.f, ex);
-        iv = ldexpf(1.f, -ex);
-    }
-    if (lane == 0) xinv[t] = iv;
-    for (int64_t c = lane; c < H; c += 32) xh[t * H + (c & ~(int64_t) 15) + perm16((int) (c & 15))] = __float2half_rn(ld(c) * s);
-}
 
 // Stages: Q6_K gives one up for the raw words of the two decoder groups, half a block of 256 rows each.
 template <int WT> constexpr int kStagesOf = WT == WT_Q6K ? kStagesP - 1 : kStagesP;
@@ -656,7 +633,9 @@ extern "C" int32_t bsx_experts_prefill(const bsx_expert_layout* layout, const un
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
-    prefill_prep_x_kernel<<<(unsigned) ((n_tokens + 7) / 8), 256, 0, st>>>(x, x_kind, n_tokens, L.n_embd, xh, xinv);
+    const PlaneRows xr{x, x_kind, 1, n_tokens, xh, xinv}, none{x, x_kind, 1, 0, xh, xinv};
+    if (L.n_embd <= 4096) rows_to_fp16_planes_kernel<128><<<(unsigned) ((n_tokens + 1) / 2), 256, 0, st>>>(xr, none, L.n_embd);
+    else rows_to_fp16_planes_kernel<256><<<(unsigned) n_tokens, 256, 0, st>>>(xr, none, L.n_embd);
     // persistent CTAs, one per SM; rows that are whole 144-byte chunks (K % 256 == 0) take the variant with 16-byte weight loads
     const unsigned grid = (unsigned) sm_count();
     launch_mode<PMODE_GU>(wt_gu, L.n_embd % 256 == 0, grid, a, st);
