@@ -334,9 +334,10 @@ __device__ __forceinline__ float gate_score(float x, int gate) {
 
 // One warp per token; lane l holds experts l, l+32, ...  The selection is the reference's rank rule (higher s + bias first,
 // the lower index on a tie; src/kernels/cuda/router.cu:170-217) made as k warp-wide argmax passes, which yield the ids in rank
-// order directly; lane 0 adds the chosen unbiased scores in that order, as the reference's thread 0 does.
+// order directly; every lane adds the chosen unbiased scores in that order, as the reference's thread 0 does.  Returns the id of rank
+// `lane` (lane < k), or -1.
 template <int REGT>
-__device__ __forceinline__ void select_token(const float* __restrict__ lg, const float* __restrict__ bias, int E, int k, float scale, int gate,
+__device__ __forceinline__ int select_token(const float* __restrict__ lg, const float* __restrict__ bias, int E, int k, float scale, int gate,
                                              int n_group, int topk_group, float prior, const HeldTabs& held, int32_t* __restrict__ ids,
                                              float* __restrict__ weights) {
     constexpr int MAXR = REGT > 0 ? REGT : 32;
@@ -390,6 +391,7 @@ __device__ __forceinline__ void select_token(const float* __restrict__ lg, const
             if (i < reg && !((live >> ((lane + i * 32) / gs)) & 1u)) dead |= 1u << i;
     }
     float my_sel = 0.f, sum = 0.f;
+    int my_id = -1;
     for (int r = 0; r < k; ++r) {
         // every index into s[] / b[] is a compile-time constant (a runtime index would move the arrays to local memory): the scan
         // carries the candidate's unbiased score along, and taken experts are remembered in the `dead` mask
@@ -411,11 +413,17 @@ __device__ __forceinline__ void select_token(const float* __restrict__ lg, const
         }
         sv = __shfl_sync(kFull, sv, ex == INT_MAX ? 0 : (ex & 31));
         sum += sv;
-        if (lane == r) my_sel = sv;
-        if (lane == 0) ids[r] = ex == INT_MAX ? -1 : ex;
+        if (lane == r) {
+            my_sel = sv;
+            my_id = ex == INT_MAX ? -1 : ex;
+        }
     }
     const float denom = sum + 1e-20f;
-    if (lane < k) weights[lane] = my_sel / denom * scale;
+    if (lane < k) {
+        ids[lane] = my_id;
+        weights[lane] = my_sel / denom * scale;
+    }
+    return my_id;
 }
 
 template <int REGT>
@@ -530,15 +538,19 @@ route_tail_skip_kernel(int32_t* __restrict__ ids, float* __restrict__ w, HeldTab
 // The experts' blob addresses, which are constants, are read before the wait for the logits.
 // With items / n_items the pass list of the packed expert kernels is written as well.
 constexpr int kRoutePlanThreads = 512;     // 16 warps: the window's tokens
+constexpr int kRoutePlanMaxTokens = 16;
+// keys and plan tables of the largest window fit the 48 KB of a launch without an opt-in
+static_assert(kRoutePlanMaxTokens * 16 * 33 * 4 + 24 * 512 + 8 + kRoutePlanMaxTokens * 32 * 4 <= kPlanSmemMax, "16 values a lane are the most");
 
 template <int REGT>
-__global__ void __launch_bounds__(kRoutePlanThreads)
+__global__ void __launch_bounds__(kRoutePlanThreads, 1)
 route_plan_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E, int k, float scale, int gate, int n_group,
                   int topk_group, float prior, HeldTabs held, const unsigned long long* __restrict__ blobs, unsigned long long shared_blob,
                   int32_t* ids, float* weights, unsigned long long* __restrict__ ptr, int32_t* __restrict__ start,
                   int32_t* __restrict__ n_groups, int32_t* __restrict__ dst, int32_t* __restrict__ tok, PassRec* __restrict__ items,
                   int* __restrict__ n_items) {
     extern __shared__ unsigned long long smb[];
+    __shared__ uint32_t keys[kRoutePlanMaxTokens][REGT > 0 ? REGT * 33 : 1];
     const PlanSmem ps = plan_smem(smb, E, true);
     plan_load_blobs(ps, blobs, E);
     __syncthreads();
@@ -549,10 +561,9 @@ route_plan_kernel(const float* __restrict__ logits, const float* __restrict__ bi
         const int t = warp;
         int32_t* it = ids + (size_t) t * k;
         float* wt = weights + (size_t) t * k;
-        if (gate == BSX_GATE_SOFTMAX) softmax_topk_token<REGT>(logits + (size_t) t * E, it, wt, E, k);
-        else select_token<REGT>(logits + (size_t) t * E, bias, E, k, scale, gate, n_group, topk_group, prior, held, it, wt);
-        __syncwarp();                    // lane 0's ids are visible to the warp
-        if (lane < k) plan_note_pair(ps, t * k + lane, t, it[lane], E);
+        const int id = gate == BSX_GATE_SOFTMAX ? softmax_topk_token<REGT>(logits + (size_t) t * E, it, wt, E, k, keys[warp])
+                                                : select_token<REGT>(logits + (size_t) t * E, bias, E, k, scale, gate, n_group, topk_group, prior, held, it, wt);
+        if (lane < k) plan_note_pair(ps, t * k + lane, t, id, E);
     }
     __syncthreads();
     plan_finish(ps, T * k, k, E, shared_blob, shared_blob != 0ull ? T : 0, ptr, start, n_groups, dst, tok, items, n_items);
@@ -707,7 +718,6 @@ int32_t moe_plan_with_passes(const int32_t* ids, int32_t T, int32_t k, int32_t E
                              unsigned long long* ptr, int32_t* start, int32_t* n_groups, int32_t* dst, int32_t* tok, PassRec* items, int* n_items,
                              cudaStream_t st);
 
-constexpr int kRoutePlanMaxTokens = 16;
 
 // selection + plan (+ the packed kernels' pass list when items is given); BSX_E_TYPE: a gate kind the fused kernel does not cover
 int32_t route_plan_launch(const float* logits, const float* bias, int32_t T, int32_t E, int32_t k, int32_t gate_kind, float weight_scale,

@@ -16,9 +16,10 @@
 
 namespace bsx {
 
-// one token by one warp: lg = the token's E logits; ids / wout = its k outputs
+// one token by one warp: lg = the token's E logits; ids / wout = its k outputs; keys: 33 REGT words of the warp's own (unused for REGT = 0).
+// Returns the id of rank `lane` (lane < k).
 template <int REGT>
-__device__ __forceinline__ void BSX_SOFTMAX_TOKEN(const float* __restrict__ lg, int32_t* __restrict__ ids, float* __restrict__ wout, int E, int k) {
+__device__ __forceinline__ int BSX_SOFTMAX_TOKEN(const float* __restrict__ lg, int32_t* __restrict__ ids, float* __restrict__ wout, int E, int k, uint32_t* keys) {
     constexpr int MAXR = REGT > 0 ? REGT : 32;
     const int lane = threadIdx.x & 31;
     const int reg = REGT > 0 ? REGT : (E >> 5);
@@ -61,20 +62,54 @@ __device__ __forceinline__ void BSX_SOFTMAX_TOKEN(const float* __restrict__ lg, 
             if (i < reg && !((taken >> i) & 1u) && kv[i] > lmax) { lmax = kv[i]; lidx = i; }
     };
     rescan();
-    for (int rank = 0; rank < k; ++rank) {
-        const uint32_t gmax = __reduce_max_sync(kFull, lmax);
-        const int ex = (int) __reduce_min_sync(kFull, lmax == gmax ? (unsigned) (lane + lidx * 32) : 0xFFFFFFFFu);
-        float best = 0.f;
-        if ((ex & 31) == lane) {
-            best = unkey(lmax);
-            taken |= 1u << lidx;
-            selected_sum += best;
-            rescan();
+    int my_id = 0;
+    if constexpr (REGT > 0) {
+        // A rank is a chain of dependent steps, so the rescan of the winning lane's values (64 instructions with one lane active) is
+        // shared out: value i of every lane also lies in row i of `keys`, which lane i alone reads and writes.
+        // Selection + plan of one token, 512 experts, top 10, after the logits: 5.1 us -> 4.3; of 8 tokens 8.2 -> 6.6 (with the ids kept in
+        // registers instead of read back).
+#pragma unroll
+        for (int i = 0; i < REGT; ++i) keys[i * 33 + lane] = kv[i];
+        __syncwarp();
+        for (int rank = 0; rank < k; ++rank) {
+            const uint32_t gmax = __reduce_max_sync(kFull, lmax);
+            const int ex = (int) __reduce_min_sync(kFull, lmax == gmax ? (unsigned) (lane + lidx * 32) : 0xFFFFFFFFu);
+            const int wl = ex & 31;
+            uint32_t q = 0u;
+            if (lane < REGT) {
+                q = keys[lane * 33 + wl];
+                if (lane == (ex >> 5)) keys[lane * 33 + wl] = q = 0u;
+            }
+            const uint32_t next = __reduce_max_sync(kFull, q);
+            const int at = __ffs(__ballot_sync(kFull, q == next)) - 1;      // the lowest index holding it (0 when none is left: never chosen)
+            const float best = unkey(gmax);
+            if (wl == lane) {
+                selected_sum += best;
+                lmax = next;
+                lidx = at;
+            }
+            if (rank == lane) {
+                selected = best;
+                my_id = ex;
+            }
         }
-        best = __shfl_sync(kFull, best, ex & 31);
-        if (lane == 0) ids[rank] = ex;
-        if (rank == lane) selected = best;
+    } else {
+        for (int rank = 0; rank < k; ++rank) {
+            const uint32_t gmax = __reduce_max_sync(kFull, lmax);
+            const int ex = (int) __reduce_min_sync(kFull, lmax == gmax ? (unsigned) (lane + lidx * 32) : 0xFFFFFFFFu);
+            const float best = unkey(gmax);
+            if ((ex & 31) == lane) {
+                taken |= 1u << lidx;
+                selected_sum += best;
+                rescan();
+            }
+            if (rank == lane) {
+                selected = best;
+                my_id = ex;
+            }
+        }
     }
+    if (lane < k) ids[lane] = my_id;
     selected_sum = fmaxf(warp_sum_xor(selected_sum), 6.103515625e-5f);
 #if BSX_SOFTMAX_RECIPROCAL
     const float inv = 1.0f / selected_sum;
@@ -82,16 +117,18 @@ __device__ __forceinline__ void BSX_SOFTMAX_TOKEN(const float* __restrict__ lg, 
 #else
     if (lane < k) wout[lane] = selected / selected_sum;
 #endif
+    return my_id;
 }
 
 template <int REGT>
 __global__ void __launch_bounds__(256) BSX_SOFTMAX_KERNEL(const float* __restrict__ logits, int32_t* __restrict__ ids,
                                                          float* __restrict__ wout, int64_t T, int E, int k) {
+    __shared__ uint32_t keys[8][REGT > 0 ? REGT * 33 : 1];
     pdl_wait();
     pdl_launch_dependents();
     const int64_t t = (int64_t) blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= T) return;
-    BSX_SOFTMAX_TOKEN<REGT>(logits + t * E, ids + t * k, wout + t * k, E, k);
+    BSX_SOFTMAX_TOKEN<REGT>(logits + t * E, ids + t * k, wout + t * k, E, k, keys[threadIdx.x >> 5]);
 }
 
 static inline int32_t BSX_SOFTMAX_LAUNCH(const float* logits, int64_t T, int E, int k, int32_t* ids, float* w, cudaStream_t st) {
