@@ -29,6 +29,7 @@
 //
 // Semantics: Basalt's native_expert_grouped (include/basalt/kernels/iq_kernels.hpp:77-92) without its int8 rounding of x, h.
 #include <atomic>
+#include <climits>
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(256) prep_fp4_kernel(ExpertArgs a, uint8_t* __
 
 // rows 0 .. n_rows - 1 of x alone (no plan needed): for a caller that makes the images beside the routing
 template <int TPR>
-__global__ void __launch_bounds__(256) x_images_kernel(const void* __restrict__ x, int kind, int n_rows, int64_t K, uint8_t* __restrict__ codes,
+__global__ void __launch_bounds__(256, 4) x_images_kernel(const void* __restrict__ x, int kind, int n_rows, int64_t K, uint8_t* __restrict__ codes,
                                                         uint8_t* __restrict__ sfs, float* __restrict__ inv) {
     __shared__ float shf[8];
     pdl_wait();
@@ -570,6 +571,285 @@ int32_t launch_stream(const StreamArgs& sa, cudaStream_t st) {
     return launch_status();
 }
 
+// ---------------------------------------------------------------- the down product straight from the SwiGLU rows
+// For n_ff of one or two chunks and passes of 8.  Such rows are short, so eight warps turn them into FP4 terms in shared memory
+// themselves (a warp a row, a lane a 16-value sub-block) while the unit's weights are on their way.  The kernel that made the images,
+// its launch and the rows' way through memory go, and a unit's rows are fetched once instead of once per row block.  Weights, MMAs and
+// epilogue as above; the stages hold weights only.  Experts of 2048 x 512, top-10 of 256: the step of one token 31.9 -> 29.2 us, of 8
+// tokens 57.3 -> 54.1, of 64 tokens 115.4 -> 112.8, the same bits.  Longer rows keep the images: at 8 chunks a unit's rows take as long
+// to convert as its weights to arrive, two buffers of them 96 KB of the stages, and the launch is under 1 % of such a step.
+template <int KC>
+struct FD {
+    static constexpr int kStages = 5, kStage = 2 * kBlockF;
+    static constexpr int kRowsB = kTermsF * kEntNarrow * 128;                          // a chunk's codes: column n = 4 entry + term
+    static constexpr int kBuf = KC * (kRowsB + kSFTile), kOffBuf = kStages * kStage;    // two buffers: [chunk codes][chunk scales]
+    static constexpr int kBars = kOffBuf + 2 * kBuf;
+    static constexpr size_t kSmem = 1024 + (size_t) kBars + 256 + 4 * kEntNarrow * sizeof(float);
+    // tensor memory: two accumulator sets of 2 x 32 columns, 32 scale columns a stage, 16 a chunk of each buffer
+    static constexpr uint32_t kCols = kTermsF * kEntNarrow, kTmemSFA = 4 * kCols, kTmemSFB = kTmemSFA + 32 * kStages;
+    static constexpr uint32_t kIdesc = FG<kEntNarrow>::kIdesc;
+    static_assert(kBuf % 1024 == 0 && kSmem <= 227 * 1024 && kTmemSFB + 2 * 16 * KC <= kTmemCols, "geometry");
+};
+constexpr int kThreadsD = 32 * 14;       // MMA issuer, weight loader, four epilogue warps (2-5: one a lane quadrant), eight row warps (6-13)
+
+template <int KC>
+__global__ void __launch_bounds__(kThreadsD, 1) nvf4_down_rows_kernel(StreamArgs sa) {
+    using G = FD<KC>;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + G::kBars);
+    uint64_t* empty = full + G::kStages;
+    uint64_t* b_full = empty + G::kStages;
+    uint64_t* b_empty = b_full + 2;
+    uint64_t* acc_full = b_empty + 2;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    // inverse row scales of the last four units: unit u + 4 writes over u only after the MMAs of u + 2, which wait for the epilogue of u
+    float* s_inv = reinterpret_cast<float*>(smem + G::kBars + 256);
+
+    const ExpertArgs& a = sa.e;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const int n_rb = (int) ((a.L.n_embd + 255) / 256);                  // row blocks: 256 down rows
+    const PackedGeom geo = packed_geom(a.L.n_embd, a.L.n_ff);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < G::kStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&b_full[s], kEntNarrow);
+            mbar_init(&b_empty[s], 1);
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], 128);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 0) {
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+    const uint32_t sbase = smem_u32(smem);
+    bool ok = true;
+    if (!(sa.early_weights && warp == 1)) pdl_wait();     // as in nvf4_stream_kernel
+    pdl_launch_dependents();
+    const int n_pass = sa.n_items[0];
+    // Row blocks a unit: the SMs go round the units as often as the fullest one has them, and a round takes as long as the unit's weights
+    // (0.8 us a chunk and row block) or the conversion of its rows (2 us), whichever is longer.  A window of one token takes one row
+    // block a unit, of 8 or 64 tokens two (against one: 47.1 -> 44.9 and 111.0 -> 106.9 us).
+    int n_sub = 1, best = INT_MAX;
+    for (int n = 1; n <= 8 && n <= n_rb; n <<= 1) {
+        const int rounds = (n_pass * ((n_rb + n - 1) / n) + (int) gridDim.x - 1) / (int) gridDim.x, cost = rounds * max(4 * n * KC, 10);
+        if (cost < best) {
+            best = cost;
+            n_sub = n;
+        }
+    }
+    const int n_upp = (n_rb + n_sub - 1) / n_sub;
+    const int n_units = n_pass * n_upp;
+
+    if (warp == 0) {
+        // ---- MMA issuer
+        if (elect_one()) {
+            uint32_t kc = 0, ti = 0, ui = 0;
+            for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ++ui) {
+                const int pass = unit / n_upp, rb0 = (unit - pass * n_upp) * n_sub, rb1 = min(n_rb, rb0 + n_sub);
+                const uint32_t buf = ui & 1u, bst = sbase + (uint32_t) G::kOffBuf + buf * G::kBuf, tsfb = tmem + G::kTmemSFB + buf * (16 * KC);
+                ok = mbar_wait(&b_full[buf], (ui >> 1) & 1u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+                for (int q = 0; q < 4 * KC; ++q)
+                    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsfb + 4 * q), "l"(sf_desc(bst + (uint32_t) (KC * G::kRowsB + q * 512))) : "memory");
+                for (int rb = rb0; rb < rb1 && ok; ++rb) {
+                    const uint32_t acc = ti & 1u;
+                    ok = mbar_wait(&acc_empty[acc], ((ti >> 1) & 1u) ^ 1u);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    const uint32_t d0 = tmem + acc * 2 * G::kCols, d1 = d0 + G::kCols;
+                    for (int c = 0; c < KC; ++c, ++kc) {
+                        const uint32_t s = kc % G::kStages;
+                        ok = mbar_wait(&full[s], (kc / G::kStages) & 1u);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                        const uint32_t st = sbase + s * G::kStage, tsfa = tmem + G::kTmemSFA + s * 32;
+                        const uint64_t a0 = smem_desc_sw128(st), a1 = smem_desc_sw128(st + kBlockF), bd = smem_desc_sw128(bst + (uint32_t) (c * G::kRowsB));
+                        const uint64_t f0 = sf_desc(st + kATile), f1 = sf_desc(st + kBlockF + kATile);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsfa + 4 * k), "l"(f0 + 32 * k) : "memory");
+                            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n" ::"r"(tsfa + 16 + 4 * k), "l"(f1 + 32 * k) : "memory");
+                            const uint32_t accum = (c | k) ? 1u : 0u;
+                            asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
+                                         "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(d0),
+                                         "l"(a0 + 2 * k), "l"(bd + 2 * k), "r"(G::kIdesc), "r"(tsfa + 4 * k), "r"(tsfb + 16 * c + 4 * k), "r"(accum)
+                                         : "memory");
+                            asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
+                                         "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(d1),
+                                         "l"(a1 + 2 * k), "l"(bd + 2 * k), "r"(G::kIdesc), "r"(tsfa + 16 + 4 * k), "r"(tsfb + 16 * c + 4 * k), "r"(accum)
+                                         : "memory");
+                        }
+                        umma_commit(&empty[s]);
+                    }
+                    if (!ok) break;
+                    if (rb == rb1 - 1) umma_commit(&b_empty[buf]);      // before the last accumulator's commit, which the epilogue outlasts
+                    umma_commit(&acc_full[acc]);
+                    ++ti;
+                }
+            }
+            if (!ok) atomicOr(sa.status, 1);
+        }
+    } else if (warp == 1) {
+        // ---- weight loader: a stage is two packed blocks of down rows
+        if (elect_one()) {
+            uint32_t issued = 0;
+            for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+                const int pass = unit / n_upp, rb0 = (unit - pass * n_upp) * n_sub, rb1 = min(n_rb, rb0 + n_sub);
+                const uint8_t* down = reinterpret_cast<const uint8_t*>(sa.items[pass].blob) + geo.down;
+                for (int rb = rb0; rb < rb1 && ok; ++rb) {
+                    const uint8_t* b0 = down + (size_t) (2 * rb) * KC * kBlockF;
+                    for (int c = 0; c < KC; ++c, ++issued) {
+                        const uint32_t s = issued % G::kStages;
+                        ok = mbar_wait(&empty[s], ((issued / G::kStages) & 1u) ^ 1u);
+                        if (!ok) break;
+                        const uint32_t st = sbase + s * G::kStage, bar = smem_u32(&full[s]);
+                        asm volatile("{\n.reg .b64 t;\nmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n}\n" ::"r"(bar), "r"(2u * kBlockF) : "memory");
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(st + (uint32_t) (h * kBlockF)),
+                                         "l"(b0 + (size_t) (h * KC + c) * kBlockF), "r"((uint32_t) kBlockF), "r"(bar)
+                                         : "memory");
+                    }
+                }
+            }
+            if (!ok) atomicOr(sa.status, 1);
+        }
+    } else if (warp < 6) {
+        // ---- epilogue: thread = TMEM lane = weight row of both tiles; lane j holds entry j's output row
+        const int q = warp & 3, rl = q * 32 + lane;
+        const uint32_t lane_base = (uint32_t) (q * 32) << 16;
+        uint32_t ti = 0, ui = 0;
+        PassRec nxt;
+        nxt.blob = 0ull; nxt.eb = 0; nxt.ntok = 0;
+        if ((int) blockIdx.x < n_units) nxt = sa.items[blockIdx.x / n_upp];
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ++ui) {
+            const int rb0 = (unit % n_upp) * n_sub, rb1 = min(n_rb, rb0 + n_sub);
+            const PassRec u = nxt;
+            if (unit + (int) gridDim.x < n_units) nxt = sa.items[(unit + gridDim.x) / n_upp];
+            const float sd = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(u.blob) + geo.tail)[2];
+            int row_lane = 0;
+            if (lane < u.ntok) row_lane = a.ent_dst ? a.ent_dst[u.eb + lane] : u.eb + lane;
+            for (int rb = rb0; rb < rb1; ++rb) {
+                const uint32_t acc = ti & 1u;
+                ok = __all_sync(kFull, mbar_wait(&acc_full[acc], (ti >> 1) & 1u));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                uint32_t d0[32], d1[32];
+                tmem_ld32(tmem + lane_base + acc * 2 * G::kCols, d0);
+                tmem_ld32(tmem + lane_base + acc * 2 * G::kCols + G::kCols, d1);
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                const float f_lane = s_inv[(ui & 3u) * kEntNarrow + (lane & 7)];
+                mbar_arrive(&acc_empty[acc]);
+                ++ti;
+#pragma unroll
+                for (int j = 0; j < kEntNarrow; ++j) {
+                    if (j < u.ntok) {
+                        const float f = __shfl_sync(kFull, f_lane, j);
+                        const int64_t o = (int64_t) __shfl_sync(kFull, row_lane, j) * a.L.n_embd + rb * 256 + rl;
+                        const float v0 = ((__uint_as_float(d0[4 * j]) + __uint_as_float(d0[4 * j + 1])) + __uint_as_float(d0[4 * j + 2])) + __uint_as_float(d0[4 * j + 3]);
+                        const float v1 = ((__uint_as_float(d1[4 * j]) + __uint_as_float(d1[4 * j + 1])) + __uint_as_float(d1[4 * j + 2])) + __uint_as_float(d1[4 * j + 3]);
+                        store_out(a.out, a.out_kind, o, v0 * f * sd);
+                        store_out(a.out, a.out_kind, o + 128, v1 * f * sd);
+                    }
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicOr(sa.status, 1);
+    } else if (warp < 6 + kEntNarrow) {
+        // ---- rows: warp = entry of the pass, lane = sub-block (fp4_image_row's arithmetic); columns of entries that the pass does not have keep
+        // what they held, which only reaches their own results
+        // The next unit's row is requested while this one's is converted, and a row is stored once the MMAs of two units ago are done.
+        const int j = warp - 6, c = lane >> 4, q = lane & 15;
+        uint32_t ui = 0;
+        PassRec u, nxt;
+        nxt.blob = 0ull; nxt.eb = 0; nxt.ntok = 0;
+        u = nxt;
+        float v[16], vn[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) vn[e] = 0.f;
+        auto request = [&](const PassRec& p) {
+            if (j < p.ntok && lane < 16 * KC) load16(a.h, BSX_X_F32, p.eb + j, a.L.n_ff, lane, vn);
+        };
+        if ((int) blockIdx.x < n_units) u = sa.items[blockIdx.x / n_upp];
+        request(u);
+        if ((int) (blockIdx.x + gridDim.x) < n_units) nxt = sa.items[(blockIdx.x + gridDim.x) / n_upp];
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ++ui) {
+            const uint32_t buf = ui & 1u;
+            const bool mine = j < u.ntok && lane < 16 * KC;
+            float amax = 0.f;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                v[e] = vn[e];
+                if (mine) amax = fmaxf(amax, fabsf(v[e]));
+            }
+            u = nxt;
+            if (unit + (int) gridDim.x < n_units) request(nxt);
+            if (unit + 2 * (int) gridDim.x < n_units) nxt = sa.items[(unit + 2 * gridDim.x) / n_upp];
+            amax = warp_max_xor(amax);
+            const Pow2Scale ps = fp4_row_scale(amax);
+            uint32_t w[kTermsF][2], sb8[kTermsF];
+            if (mine) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) v[e] *= ps.s;
+#pragma unroll
+                for (int t = 0; t < kTermsF; ++t) sb8[t] = fp4_term(v, w[t][0], w[t][1]);
+            }
+            ok = __all_sync(kFull, mbar_wait(&b_empty[buf], ((ui >> 1) & 1u) ^ 1u));
+            if (!ok) break;
+            if (mine) {
+                if (lane == 0) s_inv[(ui & 3u) * kEntNarrow + j] = ps.inv;
+                uint8_t* b = smem + G::kOffBuf + buf * G::kBuf;
+#pragma unroll
+                for (int t = 0; t < kTermsF; ++t) {
+                    const int n = kTermsF * j + t;
+                    *reinterpret_cast<uint2*>(b + c * G::kRowsB + (n >> 3) * 1024 + (n & 7) * 128 + (((q >> 1) ^ (n & 7)) << 4) + (q & 1) * 8) = make_uint2(w[t][0], w[t][1]);
+                    b[KC * G::kRowsB + c * kSFTile + (q >> 2) * 512 + n * 16 + (q & 3)] = (uint8_t) sb8[t];
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&b_full[buf]);
+        }
+        if (!ok && lane == 0) atomicOr(sa.status, 1);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmemCols) : "memory");
+    }
+}
+
+template <int KC>
+int32_t launch_down_rows(const StreamArgs& sa, cudaStream_t st) {
+    static std::atomic<bool> configured[64];   // per device; threads of different devices call concurrently
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
+    if (!configured[dev].load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(nvf4_down_rows_kernel<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) FD<KC>::kSmem);
+        if (e != cudaSuccess) return (int32_t) e;
+        configured[dev].store(true, std::memory_order_release);
+    }
+    launch_k(nvf4_down_rows_kernel<KC>, dim3((unsigned) sm_count()), dim3(kThreadsD), FD<KC>::kSmem, st, sa);
+    return launch_status();
+}
+
 }  // namespace
 
 // scratch beyond the SwiGLU buffer: x images (codes, scales), h images, inverse row scales, the pass list
@@ -653,11 +933,14 @@ int32_t experts_grouped_packed(const ExpertArgs& a, int32_t* status, cudaStream_
         rc = wide ? launch_stream<FMODE_GU, kEntWide>(sa, st) : launch_stream<FMODE_GU, kEntNarrow>(sa, st);
     }
     if (rc != BSX_OK || phase == 1) return rc;
-    launch_prep<true>(a, cap, I, hcodes, hsf, hinv, items, n_items, 0, st);   // the pass list is the gate/up stage's
+    // The pass list is the gate/up stage's.  Where this call launched that stage, the list was complete before it began, and the down
+    // kernel's weight loader may run ahead of it.
+    sa.early_weights = phase == 0;
+    if (!wide && I <= 512) return I == 256 ? launch_down_rows<1>(sa, st) : launch_down_rows<2>(sa, st);
+    launch_prep<true>(a, cap, I, hcodes, hsf, hinv, items, n_items, 0, st);
     sa.codes = hcodes;
     sa.sfs = hsf;
     sa.inv = hinv;
-    sa.early_weights = 1;
     return wide ? launch_stream<FMODE_DOWN, kEntWide>(sa, st) : launch_stream<FMODE_DOWN, kEntNarrow>(sa, st);
 }
 
