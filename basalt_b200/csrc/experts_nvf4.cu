@@ -575,8 +575,8 @@ int32_t launch_stream(const StreamArgs& sa, cudaStream_t st) {
 // For n_ff of one or two chunks and passes of 8.  Such rows are short, so eight warps turn them into FP4 terms in shared memory
 // themselves (a warp a row, a lane a 16-value sub-block) while the unit's weights are on their way.  The kernel that made the images,
 // its launch and the rows' way through memory go, and a unit's rows are fetched once instead of once per row block.  Weights, MMAs and
-// epilogue as above; the stages hold weights only.  Experts of 2048 x 512, top-10 of 256: the step of one token 31.9 -> 29.2 us, of 8
-// tokens 57.3 -> 54.1, of 64 tokens 115.4 -> 112.8, the same bits.  Longer rows keep the images: at 8 chunks a unit's rows take as long
+// epilogue as above; the stages hold weights only.  Experts of 2048 x 512, top-10 of 512: the step of one token 31.9 -> 29.2 us, of 8
+// tokens 57.3 -> 54.1, of 64 tokens 115.4 -> 112.8, the same bits; after the gate/up product one token 7.7 -> 4.8 us, 8 tokens 16.7 -> 9.7.  Longer rows keep the images: at 8 chunks a unit's rows take as long
 // to convert as its weights to arrive, two buffers of them 96 KB of the stages, and the launch is under 1 % of such a step.
 template <int KC>
 struct FD {
@@ -636,7 +636,8 @@ __global__ void __launch_bounds__(kThreadsD, 1) nvf4_down_rows_kernel(StreamArgs
     const uint32_t tmem = *tmem_slot;
     const uint32_t sbase = smem_u32(smem);
     bool ok = true;
-    if (!(sa.early_weights && warp == 1)) pdl_wait();     // as in nvf4_stream_kernel
+    // The pass list and the blobs are there before the gate/up stage runs (early_weights): only who reads its rows or writes results waits for it
+    if (!sa.early_weights) pdl_wait();
     pdl_launch_dependents();
     const int n_pass = sa.n_items[0];
     // Row blocks a unit: the SMs go round the units as often as the fullest one has them, and a round takes as long as the unit's weights
@@ -737,6 +738,7 @@ __global__ void __launch_bounds__(kThreadsD, 1) nvf4_down_rows_kernel(StreamArgs
         PassRec nxt;
         nxt.blob = 0ull; nxt.eb = 0; nxt.ntok = 0;
         if ((int) blockIdx.x < n_units) nxt = sa.items[blockIdx.x / n_upp];
+        pdl_wait();
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ++ui) {
             const int rb0 = (unit % n_upp) * n_sub, rb1 = min(n_rb, rb0 + n_sub);
             const PassRec u = nxt;
@@ -786,8 +788,9 @@ __global__ void __launch_bounds__(kThreadsD, 1) nvf4_down_rows_kernel(StreamArgs
             if (j < p.ntok && lane < 16 * KC) load16(a.h, BSX_X_F32, p.eb + j, a.L.n_ff, lane, vn);
         };
         if ((int) blockIdx.x < n_units) u = sa.items[blockIdx.x / n_upp];
-        request(u);
         if ((int) (blockIdx.x + gridDim.x) < n_units) nxt = sa.items[(blockIdx.x + gridDim.x) / n_upp];
+        pdl_wait();
+        request(u);
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ++ui) {
             const uint32_t buf = ui & 1u;
             const bool mine = j < u.ntok && lane < 16 * KC;
