@@ -15,7 +15,7 @@
 // warps 1-2 load the tile's activation rows (cp.async gather through `src`); warps 3-18 decode NVFP4 weight rows to fp16
 // straight into 128-byte-swizzled shared memory (two groups of 256 threads, a thread per weight row, the groups taking
 // alternate pairs of 64-column k-blocks); warps 19-22 are the epilogue (thread = TMEM lane = output row), which drains one
-// accumulator while the tensor core fills the other.  K-blocks move through a 4-stage ring guarded by mbarriers; every wait
+// accumulator while the tensor core fills the other.  K-blocks move through a ring of four stages (Q6_K three) guarded by mbarriers; every wait
 // is bounded and reports through a status word instead of hanging.
 //
 // Both operands use the SAME permutation of k inside each 16-column group, (0,8,1,9,...,7,15) - the order cvt.e2m1x2 emits

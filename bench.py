@@ -410,7 +410,9 @@ def run_decode(w: Weights, T, steps, warmup, copies, dev, kind="native", experts
     L = w.L
     blob = L.bytes - 16
     out["bytes_step"] = (out["experts_touched"] + 1) * blob + E * H * 4 + T * H * (xs[0].element_size() + 4) + T * k * 8
-    out["launches"] = ({"none": 7, "fused": 7, "separate": 8}[input_norm] if kind == "native" else {"none": 8, "fused": 8, "separate": 9}[input_norm])
+    # images (or norm + images), logits, selection and plan (one launch up to 16 tokens), gate/up, down, combine; images of the SwiGLU rows where the
+    # down kernel does not make them itself; call by call the pass list; the norm where it is a launch of its own
+    out["launches"] = 5 + (1 if T <= 16 else 2) + (0 if experts == "packed" and L.n_ff <= 512 else 1) + (0 if kind == "native" else 1) + (1 if input_norm == "separate" else 0)
     del layers
     torch.cuda.empty_cache()
     return out
@@ -597,7 +599,7 @@ def run_decode_codebook(args, dev, sh, steps=None, warmup=None, copies=None):
                        expert_kernels=("ggml blobs in place, warp-per-row fp32 kernels (experts_simple.cu)" if getattr(args, "plain_experts", False)
                                        else "ggml blobs in place, integer tensor-core kernels (experts_kq.cu)")),
         "e2e": {"value": T / (ms_e2e * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": T * H * 2, "d2h_bytes_per_step": T * H * 4},
-        "gpu_launches": 11 * steps,   # logits, selection + plan, 2 x (images, product) routed, shared plan, 2 x (images, product) shared... combine
+        "gpu_launches": (13 if T > 16 else 12) * steps,   # logits, selection + plan (two launches above 16 tokens), 2 x (images, product) routed, shared plan, 2 x (images, product) shared, combine
         "roofline": {"bound": "hbm", "kernel": "whole step (kq_mma_kernel<IQ1_M> gate/up and down dominate)", "achieved": gbs, "peak": pk["hbm"], "unit": "GB/s",
                      "frac": gbs / pk["hbm"], "peak_source": pk["source"], "traffic": None, "algorithmic_bytes": bytes_step, "experts_touched": touched},
         "clocks": clocks.summary(),
@@ -668,7 +670,7 @@ def run_prefill_codebook(args, dev, sh, tokens=4096, steps=3, warmup=3):
                        intermediate=I, top_k=K_TOP, router=sh["router"], expert_format="IQ1_M (56 B / 256 values)", activations="bf16", tokens_per_step=tokens,
                        l2_policy="every step reads every touched expert blob", parallelism="single GPU"),
         "e2e": {"value": tokens / (ms_e2e * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": tokens * H * 2, "d2h_bytes_per_step": tokens * H * 4},
-        "gpu_launches": 10 * steps,
+        "gpu_launches": 11 * steps,   # operand images, gate GEMM, selection, 4 dispatch, activation images, gate/up, down, combine
         "roofline": {"bound": "tensor", "kernel": "prefill_gemm_kernel<IQ1_M> gate/up + down", "achieved": achieved, "peak": pk["bf16"], "unit": "TFLOP/s",
                      "frac": achieved / pk["bf16"], "peak_source": pk["source"], "traffic": None, "algorithmic_flops_per_launch": flops,
                      "kernel_ms": stage_ms["experts"]},
@@ -799,7 +801,7 @@ def run_prefill(args, dev, rank=0, world=1, shape=None, tokens=None, steps=None,
     exp_ms = stage_ms["experts"] if world == 1 else ms_step
     achieved = flops / world / (exp_ms * 1e-3) / 1e12
     blob_b = touched * (L.bytes - 16)
-    roof = {"bound": "tensor", "kernel": (("prefill_nvf4_kernel" if use_packed else "prefill_gemm_kernel") + "<gate/up> + <down> (+ activation images)") if world == 1 else "whole step per GPU (experts + collectives)",
+    roof = {"bound": "tensor", "kernel": (("prefill_pair_kernel" if use_packed else "prefill_gemm_kernel") + "<gate/up> + <down> (+ activation images)") if world == 1 else "whole step per GPU (experts + collectives)",
             "achieved": achieved, "peak": pk["bf16"], "unit": "TFLOP/s", "frac": achieved / pk["bf16"],
             "peak_source": pk["source"] + ": the bf16 burst figure, because an activation row enters as four FP4 terms, so a K-step costs four FP4 MMAs = the tensor time of one fp16 MMA",
             "frac_of_fp4_peak": achieved / (4.0 * pk["bf16"]), "fp4_peak_assumed": "4 x the measured bf16 burst peak (no FP4 figure is measured on this pool)",
@@ -818,7 +820,7 @@ def run_prefill(args, dev, rank=0, world=1, shape=None, tokens=None, steps=None,
                        l2_policy=f"every step reads all touched expert blobs ({blob_b / 1e9:.2f} GB per GPU): larger than L2",
                        parallelism="single GPU" if world == 1 else f"ep{world}: {El} routed experts per GPU; all-gather of bf16 rows and routing, reduce-scatter of fp32 partial sums"),
         "e2e": {"value": Tn * world / (ms_e2e * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": Tn * Hs * 2 * world, "d2h_bytes_per_step": Tn * Hs * 4 * world},
-        "gpu_launches": (12 if world == 1 else 16) * steps,   # image prep x2, gate GEMM, selection, 3 dispatch, activation prep, gate/up, down, combine (+ shared expert's three and the partial combine with N > 1)
+        "gpu_launches": ((13 if use_packed else 11) + (0 if world == 1 else 4)) * steps,   # operand images, gate GEMM, selection, 4 dispatch, (tile records,) activation images, gate/up, (SwiGLU images,) down, combine (+ shared expert's three and the partial combine with N > 1)
         "roofline": roof, "stage_ms": stage_ms, "clocks": clocks.summary(),
     }
     return line
