@@ -37,6 +37,7 @@ namespace {
 
 constexpr int kLogitThreads = 256;   // the summation order is defined over 256 column-strided chains
 constexpr int kTokTile = 8;
+constexpr int kRoutePlanMaxTokens = 16;   // windows up to here choose and plan in one block (route_plan_kernel)
 
 // G gate rows a block, NV float4 a thread and row.  Each (row, token) sum runs exactly as
 // src/kernels/cuda/router.cu:49-88 defines it: thread i owns float4 columns i, i + 256, ... as one fmaf chain, the warp's 32
@@ -105,7 +106,13 @@ router_logits_kernel(const void* __restrict__ x, const float* __restrict__ gate,
     // late_wait: x was complete before the kernel ahead of this one started (that kernel makes the expert kernels' images of x),
     // so this grid runs beside it and only orders itself after it before exiting
     if (!late_wait) pdl_wait();
-    pdl_launch_dependents();
+    // When the next kernel may be scheduled.  Up to 16 tokens that is one block, which has tables to load: at once.  A wider window's
+    // selection is a small block for every two tokens and nothing to do ahead of the logits.  Scheduled now, while this grid holds most SMs'
+    // registers, its blocks pile up where there is room (36 of 64 tokens on one SM) and then take turns there: 64 bf16 tokens of 7168
+    // columns, 256 experts in 8 groups, 24.1 us from the last logit to the selection's end, 32 tokens 19.6; scheduled as this grid's blocks end,
+    // 11.8 both.
+    const bool next_early = n_tokens <= kRoutePlanMaxTokens;
+    if (next_early) pdl_launch_dependents();
     const int t_begin = blockIdx.y * tok_per_block;
     const int t_end = min(n_tokens, t_begin + tok_per_block);
     for (int t0 = t_begin; t0 < t_end; t0 += kTokTile) {
@@ -166,6 +173,7 @@ router_logits_kernel(const void* __restrict__ x, const float* __restrict__ gate,
         }
         __syncthreads();
     }
+    if (!next_early) pdl_launch_dependents();
     if (late_wait) pdl_wait();
 }
 
@@ -542,8 +550,7 @@ route_tail_skip_kernel(int32_t* __restrict__ ids, float* __restrict__ w, HeldTab
 // the block goes straight on to the plan - one launch and one round trip through global memory fewer in a step that is latency-bound.
 // The experts' blob addresses, which are constants, are read before the wait for the logits.
 // With items / n_items the pass list of the packed expert kernels is written as well.
-constexpr int kRoutePlanThreads = 512;     // 16 warps: the window's tokens
-constexpr int kRoutePlanMaxTokens = 16;
+constexpr int kRoutePlanThreads = 32 * kRoutePlanMaxTokens;
 // keys and plan tables of the largest window fit the 48 KB of a launch without an opt-in
 static_assert(kRoutePlanMaxTokens * 16 * 33 * 4 + 24 * 512 + 8 + kRoutePlanMaxTokens * 32 * 4 <= kPlanSmemMax, "16 values a lane are the most");
 
