@@ -426,9 +426,10 @@ __device__ __forceinline__ int select_token(const float* __restrict__ lg, const 
         }
         sv = __shfl_sync(kFull, sv, ex == INT_MAX ? 0 : (ex & 31));
         sum += sv;
+        const int chosen = __shfl_sync(kFull, ex, 0);     // NaN scores compare false either way round and lanes may differ: lane 0's stands
         if (lane == r) {
             my_sel = sv;
-            my_id = ex == INT_MAX ? -1 : ex;
+            my_id = chosen == INT_MAX ? -1 : chosen;
         }
     }
     const float denom = sum + 1e-20f;
