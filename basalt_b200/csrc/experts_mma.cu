@@ -21,7 +21,11 @@
 // 2560 x 640 223 -> 175.
 //
 // IQ1_M rows take it where the integer kernel (experts_kq.cu) does not: widths of an odd number of 256-column blocks, which the
-// warp-per-row fp32 kernels had before, so they keep fp32-class results.  Weights are 8 w / d, exact in fp16 (iq1m.cuh).
+// warp-per-row fp32 kernels had before, so the results may be no further off than theirs.  Weights are 8 w / d, exact in fp16 (iq1m.cuh);
+// a row is two fp16 terms, which costs one rounding of 2^-24 a value and what lies below 2^-38 of the row's largest, against the fp32
+// kernels' longer chains.  A row's distance to 64-bit sums (root mean square over rows), fp32 kernels and this one: 5120 x 2304 normal fp32
+// rows 3.8e-7 and 1.9e-7, bf16 3.8e-7 and 1.5e-7, rows of a few large values (lognormal, sigma 4) 3.1e-7 and 2.0e-7; 1280 x 1280 2.4e-7 and
+// 1.7e-7, 2.4e-7 and 1.4e-7, 2.1e-7 and 1.9e-7; the narrowest, 256 x 256, 2.1e-7 and 1.6e-7, 2.1e-7 and 1.3e-7, 1.78e-7 and 1.82e-7.
 //
 // Semantics: Basalt's native_expert_grouped (include/basalt/kernels/iq_kernels.hpp:77-92; kernels src/kernels/cuda/iq_kernels.cu:
 // 1605-1658 gate/up, :2512-2524 SwiGLU, :2140-2164 down), NVFP4 decoding per src/kernels/cpu/ggml/ggml_quants.c:1397-1422,

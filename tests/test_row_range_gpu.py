@@ -12,7 +12,8 @@ from tests.test_experts_gpu import dev
 
 pytestmark = pytest.mark.gpu
 STAGE_GU, STAGE_DOWN, PLAIN = 1, 2, 4
-SHAPES = [(O.T_IQ3_S, 512, 512), (O.T_IQ3_S, 512, 1024), (O.T_NVFP4, 512, 320), (O.T_NVFP4, 1280, 192), (O.T_NVFP4, 512, 512)]
+SHAPES = [(O.T_IQ3_S, 512, 512), (O.T_IQ3_S, 512, 1024), (O.T_NVFP4, 512, 320), (O.T_NVFP4, 1280, 192), (O.T_NVFP4, 512, 512),
+          (O.T_IQ1_M, 1280, 1280), (O.T_IQ1_M, 2048, 768)]
 
 
 def rows(rng, K, names):

@@ -1,6 +1,7 @@
 """NVFP4, IQ3_S and (odd numbers of 256-column blocks) IQ1_M experts in place where the streaming kernel's launch shape changes: rows split over four, two or no warps (few, some and
 many groups), one block of sixteen warps or two of eight (narrow and wide rows), one codebook copy or sixteen, runs of row blocks that
-end inside a pass.  Bound 1e-5, as for the same kernel's other tests: fp16 hi + lo rows (22 bits), fp32 sums over at most 5120 columns."""
+end inside a pass.  Bound 1e-5, as for the same kernel's other tests: fp16 hi + lo rows (22 bits), fp32 sums over at most 5120 columns.  IQ1_M,
+which the fp32 kernels had before: 8e-7, four times the measured 1.9e-7."""
 import numpy as np
 import pytest
 
@@ -27,5 +28,5 @@ def test_runs_of_row_blocks(lib, cuda, t, H, I, n_groups):
     want = [O.expert_forward(Lo, b, x, dtype=np.float64) for b in blobs]
     at = 0
     for e, toks in zip(ids, groups):
-        assert rel_l2(out[at:at + len(toks)], want[e][toks]) < 1e-5, (e, toks, rel_l2(out[at:at + len(toks)], want[e][toks]))
+        assert rel_l2(out[at:at + len(toks)], want[e][toks]) < (8e-7 if t == O.T_IQ1_M else 1e-5), (e, toks, rel_l2(out[at:at + len(toks)], want[e][toks]))
         at += len(toks)
