@@ -13,10 +13,11 @@ namespace bsx {
 namespace {
 
 // every codebook in one table: the IQ1 points, then the IQ2 and IQ3 points (offsets kGrid* of formats.cuh)
-__device__ const uint16_t g_iq1_grid[kGridWords] = {
+__device__ __align__(16) const uint16_t g_iq1_grid[kGridWords] = {
 #include "iq1_grid_u16.inc"
 #include "iq_grids_u16.inc"
 };
+static_assert(__alignof__(g_iq1_grid) >= 4, "experts_mma.cu reads the IQ1 points two at a time");
 const uint16_t h_iq1_grid[kGridWords] = {
 #include "iq1_grid_u16.inc"
 #include "iq_grids_u16.inc"
