@@ -44,19 +44,16 @@ enum { QMODE_GU = 0, QMODE_DOWN = 1 };
 // Q6_K rows beyond this go to the fp32 kernels: the images hold 15 bits of a row's largest value, not its 24
 constexpr int64_t kMaxColsQ6K = 8192;
 
-// CB 256-column blocks of a row are a stage.  IQ1_M: two blocks (112 bytes), copied in 16-byte pieces.  Q6_K: one 210-byte
-// block as the 53 words that cover it (every second block starts on 2 bytes, so its copy starts 2 bytes early; none reaches past its
-// row), rows 60 words apart, which keeps a quarter-warp's reads in different banks; or two blocks as 105 words.  One block a stage lets
-// any power-of-two part of a row be a warp's own (KS below) and, up to 2048 columns, two CTAs of eight warps share an SM; wider rows
-// leave room for one CTA and take two blocks (7168 x 2048, 256 experts: 64 tokens 2834 us, with one block and five stages 3239).
+// What a stage holds of a row: kCB blocks of 256 columns, kRow bytes apart.  IQ1_M: two blocks (112 bytes), copied in 16-byte pieces.  Q6_K:
+// one 210-byte block as the 53 words that cover it (every second block starts on 2 bytes, so its copy starts 2 bytes early; none reaches
+// past its row), rows 60 words apart, which keeps a quarter-warp's reads in different banks.  One block a stage lets any power-of-two part
+// of a row be a warp's own (KS below) and, up to about 5000 columns, two CTAs of eight warps share an SM.
 template <int TYPE> struct QT;
-template <int TYPE, int CB> constexpr int kRowStage = TYPE == kTypeIQ1M ? 112 : CB == 1 ? 240 : 420;
-template <int TYPE> constexpr int kCorrBytes = TYPE == kTypeIQ1M ? 64 : 32;   // correction bytes of a column and block
 template <> struct QT<kTypeIQ1M> {
-    static constexpr int kBlock = 56, kPad = 32;
+    static constexpr int kBlock = 56, kPad = 32, kCB = 2, kRow = 112, kCorr = 64;      // kCorr: correction bytes of a column and block
 };
 template <> struct QT<kTypeQ6K> {
-    static constexpr int kBlock = 210, kPad = 16;
+    static constexpr int kBlock = 210, kPad = 16, kCB = 1, kRow = 240, kCorr = 32;
 };
 
 __device__ __forceinline__ void cpa16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory"); }
@@ -192,7 +189,7 @@ kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ cor
                 for (int term = 0; term < 2; ++term) {
                     const int neg = -(term ? sum2[h] : sum1[h]);
                     const int hi = neg >> 4, lo = neg & 15;       // neg = 16 hi + lo, 0 <= lo < 16 (arithmetic shift floors)
-                    int8_t* c = corr + (((size_t) i * 2 + term) * nblk + blk) * kCorrBytes<TYPE>;
+                    int8_t* c = corr + (((size_t) i * 2 + term) * nblk + blk) * QT<TYPE>::kCorr;
                     c[slot] = (int8_t) hi;
                     c[32 + slot] = (int8_t) lo;
                 }
@@ -201,7 +198,7 @@ kq_image_kernel(ExpertArgs a, int8_t* __restrict__ img, int8_t* __restrict__ cor
 #pragma unroll
             for (int term = 0; term < 2; ++term) {
                 const int neg = -(term ? sum2[0] + sum2[1] : sum1[0] + sum1[1]);
-                int8_t* c = corr + (((size_t) i * 2 + term) * nblk + blk) * kCorrBytes<TYPE>;
+                int8_t* c = corr + (((size_t) i * 2 + term) * nblk + blk) * QT<TYPE>::kCorr;
                 c[sb & 15] = (int8_t) (neg >> 4);
                 c[16 + (sb & 15)] = (int8_t) (neg & 15);
             }
@@ -359,18 +356,18 @@ __device__ __forceinline__ void q6k_block(const uint8_t* ra, const uint8_t* rb, 
 // Work: the row blocks (W / KS tiles) of all passes in one sequence, cut into equal runs, one a block.  A run's part of one pass shares
 // its columns and its weight stream, so barriers, activation copies and first loads come once or twice a call.  (Units drawn from a
 // counter instead: IQ1_M gate/up of 7168 x 2048 at 64 tokens 765 us, with runs and a look-up index made by one byte permutation 655.)
-template <int TYPE, int MODE, int W, int OCC, int KS, int NC, int ST, int CB, int NB>
+template <int TYPE, int MODE, int W, int OCC, int KS, int NC, int ST, int NB>
 __global__ void __launch_bounds__(W * 32, OCC)
 kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __restrict__ corr, const float* __restrict__ inv,
               const PassRec* __restrict__ items, const int* __restrict__ n_items, int n_row_blocks) {
     using Q = QT<TYPE>;
-    constexpr int kThreads = W * 32, kStages = ST, kEntP = kEntQ * NB, kCols = kColsQ * NB, kTiles = W / KS;
-    constexpr int kChunkBytes = CB * Q::kBlock, kRow = kRowStage<TYPE, CB>, kStageBytes = kRowsQ * kRow;
+    constexpr int kThreads = W * 32, kStages = ST, kEntP = kEntQ * NB, kCols = kColsQ * NB, kTiles = W / KS, CB = Q::kCB;
+    constexpr int kChunkBytes = CB * Q::kBlock, kRow = Q::kRow, kStageBytes = kRowsQ * kRow;
     extern __shared__ __align__(128) uint8_t smem[];
     const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
     const int nblk = (int) (K >> 8);
     const int cstride = (int) K + Q::kPad;                                   // bytes between activation columns
-    const int xstride = nblk * kCorrBytes<TYPE> + 16;                                        // ... and between their correction columns
+    const int xstride = nblk * Q::kCorr + 16;                                // ... and between their correction columns
     uint8_t* xs = smem;                                                        // [kCols][cstride]
     uint8_t* cs = xs + (size_t) kCols * cstride;                               // [kCols][xstride]
     uint2* tab = reinterpret_cast<uint2*>(cs + (size_t) kCols * xstride);      // [2048][NC] (IQ1_M)
@@ -441,10 +438,10 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
                 const int c = i / per_col, q = i - c * per_col;
                 cpa16(xs_s + (uint32_t) (c * cstride + q * 16), img + ((size_t) s_ir[c >> 1] * 2 + (c & 1)) * K + (size_t) q * 16);
             }
-            const int per_cc = nblk * (kCorrBytes<TYPE> / 16);
+            const int per_cc = nblk * (QT<TYPE>::kCorr / 16);
             for (int i = threadIdx.x; i < ncol * per_cc; i += kThreads) {
                 const int c = i / per_cc, q = i - c * per_cc;
-                cpa16(cs_s + (uint32_t) (c * xstride + q * 16), corr + ((size_t) s_ir[c >> 1] * 2 + (c & 1)) * nblk * kCorrBytes<TYPE> + (size_t) q * 16);
+                cpa16(cs_s + (uint32_t) (c * xstride + q * 16), corr + ((size_t) s_ir[c >> 1] * 2 + (c & 1)) * nblk * QT<TYPE>::kCorr + (size_t) q * 16);
             }
             cpa_commit();
         }
@@ -466,26 +463,13 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
                         if (p < 112) cpa16(dst + (uint32_t) (row * kRow + off), src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1) + off);
                     }
                 } else {
-                    const uint8_t* src = row0 + iss_tile + (size_t) (chunk0 + iss_chunk) * kChunkBytes - (CB == 1 ? 2 * ((chunk0 + iss_chunk) & 1) : 0) + 4 * lane;
-                    auto row_at = [&](int row) { return src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1); };
-                    if constexpr (CB == 1) {
+                    const uint8_t* src = row0 + iss_tile + (size_t) (chunk0 + iss_chunk) * kChunkBytes - 2 * ((chunk0 + iss_chunk) & 1) + 4 * lane;
 #pragma unroll
-                        for (int row = 0; row < kRowsQ; ++row) {
-                            const uint8_t* r = row_at(row);
-                            const uint32_t d = dst + (uint32_t) (row * kRow + 4 * lane);
-                            cpa4(d, r);
-                            if (lane < 53 - 32) cpa4(d + 128, r + 128);
-                        }
-                    } else {
-                        // two rows as one run of 210 words: seven copies instead of four a row
-#pragma unroll
-                        for (int row = 0; row < kRowsQ; row += 2) {
-                            const uint8_t *ra = row_at(row), *rb = row_at(row + 1) - kRow;
-                            const uint32_t d = dst + (uint32_t) (row * kRow + 4 * lane);
-#pragma unroll
-                            for (int i = 0; i < 7; ++i)
-                                if (i < 6 || lane < 210 - 192) cpa4(d + 128 * i, (i > 3 || (i == 3 && lane >= 105 - 96) ? rb : ra) + 128 * i);
-                        }
+                    for (int row = 0; row < kRowsQ; ++row) {
+                        const uint8_t* r = src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1);
+                        const uint32_t d = dst + (uint32_t) (row * kRow + 4 * lane);
+                        cpa4(d, r);
+                        if (lane < 53 - 32) cpa4(d + 128, r + 128);
                     }
                 }
                 ++iss_unit;
@@ -528,10 +512,10 @@ kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __rest
 #pragma unroll
             for (int b = 0; b < CB; ++b) {
                 const int blk = (chunk0 + chunk) * CB + b;
-                const int at = CB == 2 ? b * Q::kBlock : 2 * ((chunk0 + chunk) & 1);
+                const int at = TYPE == kTypeIQ1M ? b * Q::kBlock : 2 * (blk & 1);
                 const uint8_t* ra = st + g * kRow + at;
                 const uint8_t* rbp = st + (g + 8) * kRow + at;
-                const uint8_t *bc = bcol + 256 * blk, *cc = ccol + kCorrBytes<TYPE> * blk;
+                const uint8_t *bc = bcol + 256 * blk, *cc = ccol + QT<TYPE>::kCorr * blk;
                 if constexpr (TYPE == kTypeIQ1M) iq1m_block<NC, NB>(ra, rbp, tab + (lane & (NC - 1)), bc, cc, kColsQ * cstride, kColsQ * xstride, wide, t, tot);
                 else if (blk & 1) q6k_block<NB, true>(ra, rbp, bc, cc, kColsQ * cstride, kColsQ * xstride, wide, t, tot);
                 else q6k_block<NB, false>(ra, rbp, bc, cc, kColsQ * cstride, kColsQ * xstride, wide, t, tot);
@@ -589,26 +573,26 @@ size_t al256q(size_t v) { return (v + 255) & ~(size_t) 255; }
 constexpr size_t kSmemOne = 232448 - 256, kSmemTwo = 115712 - 256;
 
 template <int TYPE>
-size_t kq_smem(int64_t K, int W, int KS, int NC, int ST, int CB, int NB) {
+size_t kq_smem(int64_t K, int W, int KS, int NC, int ST, int NB) {
     using Q = QT<TYPE>;
-    return (size_t) kColsQ * NB * (K + Q::kPad) + (size_t) kColsQ * NB * ((K >> 8) * kCorrBytes<TYPE> + 16) + (TYPE == kTypeIQ1M ? (size_t) 16384 * NC : 0) +
-           (size_t) W * ST * kRowsQ * (CB == 1 ? kRowStage<TYPE, 1> : kRowStage<TYPE, 2>) + (size_t) W / KS * (KS - 1) * NB * 512 + 128;
+    return (size_t) kColsQ * NB * (K + Q::kPad) + (size_t) kColsQ * NB * ((K >> 8) * QT<TYPE>::kCorr + 16) + (TYPE == kTypeIQ1M ? (size_t) 16384 * NC : 0) +
+           (size_t) W * ST * kRowsQ * Q::kRow + (size_t) W / KS * (KS - 1) * NB * 512 + 128;
 }
 
-template <int TYPE, int MODE, int W, int OCC, int KS, int NC, int ST, int CB, int NB>
+template <int TYPE, int MODE, int W, int OCC, int KS, int NC, int ST, int NB>
 int32_t kq_launch_as(const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const PassRec* items, const int* n_items, cudaStream_t st) {
-    const size_t smem = kq_smem<TYPE>(MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff, W, KS, NC, ST, CB, NB);
+    const size_t smem = kq_smem<TYPE>(MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff, W, KS, NC, ST, NB);
     static std::atomic<bool> configured[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int32_t) cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(kq_mma_kernel<TYPE, MODE, W, OCC, KS, NC, ST, CB, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const cudaError_t e = cudaFuncSetAttribute(kq_mma_kernel<TYPE, MODE, W, OCC, KS, NC, ST, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int) (OCC == 2 ? kSmemTwo : kSmemOne));
         if (e != cudaSuccess) return (int32_t) e;
         configured[dev].store(true, std::memory_order_release);
     }
     const int64_t rows = MODE == QMODE_GU ? a.L.n_ff : a.L.n_embd, step_rows = (MODE == QMODE_GU ? 8 : 16) * W / KS;
-    launch_k(kq_mma_kernel<TYPE, MODE, W, OCC, KS, NC, ST, CB, NB>, dim3((unsigned) (OCC * sm_count())), dim3(W * 32), smem, st, a, img, corr, inv, items, n_items,
+    launch_k(kq_mma_kernel<TYPE, MODE, W, OCC, KS, NC, ST, NB>, dim3((unsigned) (OCC * sm_count())), dim3(W * 32), smem, st, a, img, corr, inv, items, n_items,
              (int) ((rows + step_rows - 1) / step_rows));
     return launch_status();
 }
@@ -628,14 +612,14 @@ KqShape kq_shape(const ExpertArgs& a, bool gu) {
     KqShape s{1, 1, 1};
     int W = 16, most = 2;
     if (TYPE == kTypeIQ1M) {
-        if (kq_smem<TYPE>(K, 16, 2, 4, 3, 2, 2) <= kSmemOne) s.NB = 2;
+        if (kq_smem<TYPE>(K, 16, 2, 4, 3, 2) <= kSmemOne) s.NB = 2;
     } else {
         W = 8;
-        if (deep && kq_smem<TYPE>(K, 8, 2, 1, 2, 1, 4) <= kSmemTwo) { s.OCC = 2; s.NB = 4; }
-        else if (kq_smem<TYPE>(K, 8, 8, 1, 2, 1, 2) <= kSmemTwo) { s.OCC = 2; s.NB = 2; most = 8; }
-        else if (!deep && kq_smem<TYPE>(K, 8, 4, 1, 2, 1, 1) <= kSmemTwo) { s.OCC = 2; most = 4; }
+        if (deep && kq_smem<TYPE>(K, 8, 2, 1, 2, 4) <= kSmemTwo) { s.OCC = 2; s.NB = 4; }
+        else if (kq_smem<TYPE>(K, 8, 8, 1, 2, 2) <= kSmemTwo) { s.OCC = 2; s.NB = 2; most = 8; }
+        else if (!deep && kq_smem<TYPE>(K, 8, 4, 1, 2, 1) <= kSmemTwo) { s.OCC = 2; most = 4; }
         else {
-            s.NB = deep && kq_smem<TYPE>(K, 12, 4, 1, 2, 1, 2) <= kSmemOne ? 2 : 1;
+            s.NB = deep && kq_smem<TYPE>(K, 12, 4, 1, 2, 2) <= kSmemOne ? 2 : 1;
             W = s.NB == 2 ? 12 : 16;
             most = 4;
         }
@@ -654,42 +638,42 @@ KqShape kq_shape(const ExpertArgs& a, bool gu) {
 template <int TYPE, int MODE>
 int32_t kq_launch(const KqShape& s, const ExpertArgs& a, const int8_t* img, const int8_t* corr, const float* inv, const PassRec* items, const int* n_items, cudaStream_t st) {
     const int64_t K = MODE == QMODE_GU ? a.L.n_embd : a.L.n_ff;
-#define KQ_AS(W, OCC, KS, NC, ST, CB, NB) return kq_launch_as<TYPE, MODE, W, OCC, KS, NC, ST, CB, NB>(a, img, corr, inv, items, n_items, st)
+#define KQ_AS(W, OCC, KS, NC, ST, NB) return kq_launch_as<TYPE, MODE, W, OCC, KS, NC, ST, NB>(a, img, corr, inv, items, n_items, st)
     if constexpr (TYPE == kTypeQ6K) {
         if (s.OCC == 2 && s.NB == 4) {
-            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 1, 4);
-            KQ_AS(8, 2, 1, 1, 2, 1, 4);
+            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 4);
+            KQ_AS(8, 2, 1, 1, 2, 4);
         }
         if (s.OCC == 2 && s.NB == 2) {
-            if (s.KS == 8) KQ_AS(8, 2, 8, 1, 2, 1, 2);
-            if (s.KS == 4) KQ_AS(8, 2, 4, 1, 2, 1, 2);
-            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 1, 2);
-            KQ_AS(8, 2, 1, 1, 2, 1, 2);
+            if (s.KS == 8) KQ_AS(8, 2, 8, 1, 2, 2);
+            if (s.KS == 4) KQ_AS(8, 2, 4, 1, 2, 2);
+            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 2);
+            KQ_AS(8, 2, 1, 1, 2, 2);
         }
         if (s.OCC == 2) {
-            if (s.KS == 4) KQ_AS(8, 2, 4, 1, 2, 1, 1);
-            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 1, 1);
-            KQ_AS(8, 2, 1, 1, 2, 1, 1);
+            if (s.KS == 4) KQ_AS(8, 2, 4, 1, 2, 1);
+            if (s.KS == 2) KQ_AS(8, 2, 2, 1, 2, 1);
+            KQ_AS(8, 2, 1, 1, 2, 1);
         }
         if (s.NB == 2) {
-            if (s.KS == 4) KQ_AS(12, 1, 4, 1, 2, 1, 2);
-            if (s.KS == 2) KQ_AS(12, 1, 2, 1, 2, 1, 2);
-            KQ_AS(12, 1, 1, 1, 2, 1, 2);
+            if (s.KS == 4) KQ_AS(12, 1, 4, 1, 2, 2);
+            if (s.KS == 2) KQ_AS(12, 1, 2, 1, 2, 2);
+            KQ_AS(12, 1, 1, 1, 2, 2);
         }
-        if (s.KS == 4) KQ_AS(16, 1, 4, 1, 2, 1, 1);
-        if (s.KS == 2) KQ_AS(16, 1, 2, 1, 2, 1, 1);
-        KQ_AS(16, 1, 1, 1, 2, 1, 1);
+        if (s.KS == 4) KQ_AS(16, 1, 4, 1, 2, 1);
+        if (s.KS == 2) KQ_AS(16, 1, 2, 1, 2, 1);
+        KQ_AS(16, 1, 1, 1, 2, 1);
     } else {
         if (s.NB == 2) {
-            if (s.KS == 2) KQ_AS(16, 1, 2, 4, 3, 2, 2);
-            KQ_AS(16, 1, 1, 4, 3, 2, 2);
+            if (s.KS == 2) KQ_AS(16, 1, 2, 4, 3, 2);
+            KQ_AS(16, 1, 1, 4, 3, 2);
         }
         // four copies of the codebook where they fit beside the columns and the stages (K up to 7680), else two
-        if (kq_smem<TYPE>(K, 16, 2, 4, 3, 2, 1) <= kSmemOne) {
-            if (s.KS == 2) KQ_AS(16, 1, 2, 4, 3, 2, 1);
-            KQ_AS(16, 1, 1, 4, 3, 2, 1);
+        if (kq_smem<TYPE>(K, 16, 2, 4, 3, 1) <= kSmemOne) {
+            if (s.KS == 2) KQ_AS(16, 1, 2, 4, 3, 1);
+            KQ_AS(16, 1, 1, 4, 3, 1);
         }
-        KQ_AS(16, 1, 1, 2, 3, 2, 1);
+        KQ_AS(16, 1, 1, 2, 3, 1);
     }
 #undef KQ_AS
 }
@@ -715,8 +699,8 @@ int32_t experts_grouped_kq(const ExpertArgs& a, cudaStream_t st) {
     const bsx_expert_layout& L = a.L;
     if (!kq_type(L.gu_type) || L.up_type != L.gu_type || !kq_type(L.d_type)) return BSX_E_TYPE;
     if (!kq_dim_ok(L.gu_type, L.n_embd, L.n_ff) || !kq_dim_ok(L.d_type, L.n_ff, L.n_embd) || L.n_embd % 16) return BSX_E_TYPE;
-    if (L.gu_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_embd, 16, 1, 2, 3, 2, 1) > kSmemOne : L.n_embd > kMaxColsQ6K) return BSX_E_TYPE;
-    if (L.d_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_ff, 16, 1, 2, 3, 2, 1) > kSmemOne : L.n_ff > kMaxColsQ6K) return BSX_E_TYPE;
+    if (L.gu_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_embd, 16, 1, 2, 3, 1) > kSmemOne : L.n_embd > kMaxColsQ6K) return BSX_E_TYPE;
+    if (L.d_type == kTypeIQ1M ? kq_smem<kTypeIQ1M>(L.n_ff, 16, 1, 2, 3, 1) > kSmemOne : L.n_ff > kMaxColsQ6K) return BSX_E_TYPE;
     const int64_t cap = a.cap_entries, H = L.n_embd, I = L.n_ff;
     uint8_t* p = reinterpret_cast<uint8_t*>(a.h) + al256q((size_t) cap * I * 4);
     int8_t* ximg = reinterpret_cast<int8_t*>(p);
