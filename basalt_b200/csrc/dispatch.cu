@@ -155,7 +155,7 @@ dispatch_place_kernel(const int32_t* __restrict__ ids, int64_t n, int k, int E, 
 // ---------------------------------------------------------------------------------------------- decode-window plan
 // One block of 1024 threads, everything in shared memory (plan.cuh).
 __global__ void __launch_bounds__(1024)
-moe_plan_kernel(const int32_t* __restrict__ ids, int n, int k, int E, const unsigned long long* __restrict__ blobs,
+moe_plan_kernel(const int32_t* ids, int n, int k, int E, const unsigned long long* __restrict__ blobs,
                 unsigned long long shared_blob, int n_tok, unsigned long long* __restrict__ ptr, int32_t* __restrict__ start,
                 int32_t* __restrict__ n_groups, int32_t* __restrict__ dst, int32_t* __restrict__ tok, PassRec* __restrict__ items,
                 int* __restrict__ n_items) {
@@ -179,7 +179,7 @@ moe_plan_kernel(const int32_t* __restrict__ ids, int n, int k, int E, const unsi
 // replicated (optional, [E] bytes): experts every rank holds a copy of (hot experts); a pair naming one is computed by the
 // rank that owns the pair's TOKEN (pairs own_lo .. own_lo + own_n - 1), so each pair still has exactly one rank.
 __global__ void __launch_bounds__(1024)
-ep_plan_kernel(const int32_t* __restrict__ ids, int n, int k, int blk, int blk_stride, int E, const unsigned long long* __restrict__ blobs,
+ep_plan_kernel(const int32_t* ids, int n, int k, int blk, int blk_stride, int E, const unsigned long long* __restrict__ blobs,
                unsigned long long shared_blob, int tok_lo, int tok_n, unsigned long long* __restrict__ ptr, int32_t* __restrict__ start,
                int32_t* __restrict__ n_groups, int32_t* __restrict__ dst, int32_t* __restrict__ tok, const uint8_t* __restrict__ replicated,
                int own_lo, int own_n) {

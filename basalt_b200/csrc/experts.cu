@@ -70,9 +70,8 @@ __global__ void __launch_bounds__(256) quantize_q8_1_kernel(const float* __restr
 // y[t] = fma chain over the k rows in order, then the shared expert: src/models/qwen4exp/kernels/native_moe.cu:36-50 and
 // src/models/qwen4exp/prefill/kernels.cu:438-449 (bit-equal forms).  A thread owns 4 consecutive columns.
 __global__ void __launch_bounds__(128)
-combine_kernel(const float* __restrict__ rows, const int32_t* __restrict__ slot, const float* __restrict__ w,
-               const float* __restrict__ shared, const float* __restrict__ sg, const float* __restrict__ resid, int k, int H, int pair0,
-               const int32_t* __restrict__ ids, int e_lo, int e_hi, float* __restrict__ y, int blk_tok, int blk_stride, int sh_lo, int sh_n,
+combine_kernel(const float* rows, const int32_t* slot, const float* w, const float* shared, const float* sg, const float* resid, int k, int H, int pair0,
+               const int32_t* ids, int e_lo, int e_hi, float* y, int blk_tok, int blk_stride, int sh_lo, int sh_n,
                const uint8_t* __restrict__ replicated) {
     __shared__ int s_row[64];
     __shared__ float s_w[64];

@@ -358,8 +358,7 @@ __device__ __forceinline__ void q6k_block(const uint8_t* ra, const uint8_t* rb, 
 // counter instead: IQ1_M gate/up of 7168 x 2048 at 64 tokens 765 us, with runs and a look-up index made by one byte permutation 655.)
 template <int TYPE, int MODE, int W, int OCC, int KS, int NC, int ST, int NB>
 __global__ void __launch_bounds__(W * 32, OCC)
-kq_mma_kernel(ExpertArgs a, const int8_t* __restrict__ img, const int8_t* __restrict__ corr, const float* __restrict__ inv,
-              const PassRec* __restrict__ items, const int* __restrict__ n_items, int n_row_blocks) {
+kq_mma_kernel(ExpertArgs a, const int8_t* img, const int8_t* corr, const float* inv, const PassRec* items, const int* n_items, int n_row_blocks) {
     using Q = QT<TYPE>;
     constexpr int kThreads = W * 32, kStages = ST, kEntP = kEntQ * NB, kCols = kColsQ * NB, kTiles = W / KS, CB = Q::kCB;
     constexpr int kChunkBytes = CB * Q::kBlock, kRow = Q::kRow, kStageBytes = kRowsQ * kRow;

@@ -273,8 +273,7 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
 // W, OCC, NC: warps a block, blocks an SM, copies of the IQ3_S codebook (blk_shape).
 template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN, int W, int OCC, int ST, int NC, int KS>
 __global__ void __launch_bounds__(W * 32, OCC)
-blk_mma_kernel(ExpertArgs a, const __half* __restrict__ img, const float* __restrict__ inv, const PassRec* __restrict__ items,
-               const int* __restrict__ n_items, int n_row_blocks) {
+blk_mma_kernel(ExpertArgs a, const __half* img, const float* inv, const PassRec* items, const int* n_items, int n_row_blocks) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int kThreads = W * 32, kStages = ST, kTiles = W / KS;
     const int64_t K = MODE == MODE_GU ? a.L.n_embd : a.L.n_ff;

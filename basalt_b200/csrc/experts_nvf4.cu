@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(256) prep_fp4_kernel(ExpertArgs a, uint8_t* __
 
 // rows 0 .. n_rows - 1 of x alone (no plan needed): for a caller that makes the images beside the routing
 template <int TPR>
-__global__ void __launch_bounds__(256, 4) x_images_kernel(const void* __restrict__ x, int kind, int n_rows, int64_t K, uint8_t* __restrict__ codes,
+__global__ void __launch_bounds__(256, 4) x_images_kernel(const void* x, int kind, int n_rows, int64_t K, uint8_t* __restrict__ codes,
                                                         uint8_t* __restrict__ sfs, float* __restrict__ inv) {
     __shared__ float shf[8];
     pdl_wait();
@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(256, 4) x_images_kernel(const void* __restrict
 // rows of h that a pass list (or none) and a tile list name: a block takes 256 / TPR places of a pass (of pass_entries) or a tile (of 128)
 // at a time.  (Rows of experts held elsewhere are in neither and have never been written.)
 template <int TPR>
-__global__ void __launch_bounds__(256) listed_images_kernel(const float* __restrict__ h, const PassRec* __restrict__ items, const int* __restrict__ n_items, int pass_entries,
-                                                             const TileRec* __restrict__ recs, const int32_t* __restrict__ n_recs, int64_t K, uint8_t* __restrict__ codes,
+__global__ void __launch_bounds__(256) listed_images_kernel(const float* h, const PassRec* items, const int* n_items, int pass_entries,
+                                                             const TileRec* recs, const int32_t* n_recs, int64_t K, uint8_t* __restrict__ codes,
                                                              uint8_t* __restrict__ sfs, float* __restrict__ inv) {
     __shared__ float shf[8];
     constexpr int kRows = 256 / TPR;          // divides both lengths: a block's places are one pass's or tile's
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) listed_images_kernel(const float* __restr
 // row, one launch: the block reads back the fp32 row it has just written (still in L1 / L2) instead of a second kernel
 // fetching it from HBM.
 template <bool BF16>
-__global__ void __launch_bounds__(kNormThreads) norm_images_kernel(const void* __restrict__ x, const float* __restrict__ w, float eps, int64_t K,
+__global__ void __launch_bounds__(kNormThreads) norm_images_kernel(const void* x, const float* __restrict__ w, float eps, int64_t K,
                                                                    uint16_t* act, float* xn, uint8_t* __restrict__ codes,
                                                                    uint8_t* __restrict__ sfs, float* __restrict__ inv) {
     __shared__ float red[kNormThreads / 32];

@@ -160,7 +160,7 @@ constexpr uint64_t kStepCode = 2;                  // descriptors count addresse
 // stays in registers between the row's maximum and its codes (n_ff <= 512: 205 -> 174 us for 180,224 rows of 512); 0 reads the row
 // twice (four sub-blocks in registers were slower there: 274 -> 340 us for 73,728 rows of 2048).
 template <int NIT>
-__global__ void __launch_bounds__(256) h_images_kernel(const TileRec* __restrict__ recs, const int32_t* __restrict__ n_recs, const float* __restrict__ h, int64_t K,
+__global__ void __launch_bounds__(256) h_images_kernel(const TileRec* recs, const int32_t* n_recs, const float* h, int64_t K,
                                                        uint8_t* __restrict__ img, float* __restrict__ inv) {
     pdl_wait();
     pdl_launch_dependents();

@@ -38,7 +38,7 @@ __device__ __forceinline__ float block_sum_warp_order(float v, float* scratch) {
 // of up to 8192 values is read once); columns past those are read again.  Squares enter the chain in column order either way,
 // and a column past the row's end adds fmaf(0, 0, s) = s, so no bounds test sits inside the chain.
 template <bool BF16>
-__device__ __forceinline__ void norm_row(const void* __restrict__ x, const float* __restrict__ w, float eps, int64_t K, int64_t row,
+__device__ __forceinline__ void norm_row(const void* x, const float* __restrict__ w, float eps, int64_t K, int64_t row,
                                          uint16_t* __restrict__ act, float* __restrict__ xn, float* red) {
     constexpr int kKeep = 16;
     const int64_t first = row * K;

@@ -8,7 +8,7 @@ namespace bsx {
 namespace {
 
 template <bool BF16>
-__global__ void __launch_bounds__(kNormThreads) norm_pack_kernel(const void* __restrict__ x, const float* __restrict__ w, float eps, int64_t K,
+__global__ void __launch_bounds__(kNormThreads) norm_pack_kernel(const void* x, const float* __restrict__ w, float eps, int64_t K,
                                                                  uint16_t* __restrict__ act, float* __restrict__ xn) {
     __shared__ float red[kNormThreads / 32];
     norm_row<BF16>(x, w, eps, K, blockIdx.x, act, xn, red);

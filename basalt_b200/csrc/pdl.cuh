@@ -7,6 +7,10 @@
 // kernel launched this way calls pdl_wait() before it reads anything an earlier kernel wrote and before it writes
 // anything; pdl_wait() returns once the earlier kernels have completed and their writes are visible, so results are those
 // of plain launches.  Outside a scope launch_k is the plain <<<>>> launch and pdl_wait() returns at once.
+//
+// What an earlier kernel writes is never a `const T* __restrict__` parameter of a kernel with a pdl_wait(): such loads may be taken for
+// loads of memory that nothing changes while the kernel runs and be moved ahead of the wait, which the predecessor's writes then race
+// with.  The qualifier is left to constants (weights, tables of blob addresses).
 #pragma once
 #include <cuda_runtime.h>
 

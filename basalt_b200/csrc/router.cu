@@ -85,7 +85,7 @@ __device__ __forceinline__ int merged_butterfly(float (&acc)[G], int lane) {
 
 template <int NV, int G, bool BF16>
 __global__ void __launch_bounds__(kLogitThreads, (NV <= 4 ? 2 : 1))
-router_logits_kernel(const void* __restrict__ x, const float* __restrict__ gate, int n_embd, int n_expert, int n_tokens,
+router_logits_kernel(const void* x, const float* __restrict__ gate, int n_embd, int n_expert, int n_tokens,
                      int tok_per_block, float* __restrict__ logits, int late_wait) {
     __shared__ float red[G][kTokTile][kLogitThreads / 32];
     // what the 128 registers of two blocks an SM hold beside the gate rows; wider rows keep one token ahead
@@ -186,7 +186,7 @@ router_logits_kernel(const void* __restrict__ x, const float* __restrict__ gate,
 // tile needs one block barrier.
 template <int NV, int G, bool BF16>
 __global__ void __launch_bounds__(kLogitThreads, 2)
-router_logits_staged_kernel(const void* __restrict__ x, const float* __restrict__ gate, int n_embd, int n_expert, int n_tokens,
+router_logits_staged_kernel(const void* x, const float* __restrict__ gate, int n_embd, int n_expert, int n_tokens,
                             int tok_per_block, float* __restrict__ logits, int late_wait) {
     extern __shared__ __align__(16) uint8_t xsm[];
     __shared__ float red[2][G][kTokTile][kLogitThreads / 32];
@@ -350,7 +350,7 @@ __device__ __forceinline__ float gate_score(float x, int gate) {
 // order directly; every lane adds the chosen unbiased scores in that order, as the reference's thread 0 does.  Returns the id of rank
 // `lane` (lane < k), or -1.
 template <int REGT>
-__device__ __forceinline__ int select_token(const float* __restrict__ lg, const float* __restrict__ bias, int E, int k, float scale, int gate,
+__device__ __forceinline__ int select_token(const float* lg, const float* __restrict__ bias, int E, int k, float scale, int gate,
                                              int n_group, int topk_group, float prior, const HeldTabs& held, int32_t* __restrict__ ids,
                                              float* __restrict__ weights) {
     constexpr int MAXR = REGT > 0 ? REGT : 32;
@@ -442,7 +442,7 @@ __device__ __forceinline__ int select_token(const float* __restrict__ lg, const 
 
 template <int REGT>
 __global__ void __launch_bounds__(256)
-router_select_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int64_t T, int E, int k, float scale,
+router_select_kernel(const float* logits, const float* __restrict__ bias, int64_t T, int E, int k, float scale,
                      int gate, int n_group, int topk_group, float prior, HeldTabs held, int32_t* __restrict__ ids,
                      float* __restrict__ weights) {
     pdl_wait();
@@ -557,7 +557,7 @@ static_assert(kRoutePlanMaxTokens * 16 * 33 * 4 + 24 * 512 + 8 + kRoutePlanMaxTo
 
 template <int REGT>
 __global__ void __launch_bounds__(kRoutePlanThreads, 1)
-route_plan_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E, int k, float scale, int gate, int n_group,
+route_plan_kernel(const float* logits, const float* __restrict__ bias, int T, int E, int k, float scale, int gate, int n_group,
                   int topk_group, float prior, HeldTabs held, const unsigned long long* __restrict__ blobs, unsigned long long shared_blob,
                   int32_t* ids, float* weights, unsigned long long* __restrict__ ptr, int32_t* __restrict__ start,
                   int32_t* __restrict__ n_groups, int32_t* __restrict__ dst, int32_t* __restrict__ tok, PassRec* __restrict__ items,

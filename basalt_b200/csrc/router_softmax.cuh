@@ -19,7 +19,7 @@ namespace bsx {
 // one token by one warp: lg = the token's E logits; ids / wout = its k outputs; keys: 33 REGT words of the warp's own (unused for REGT = 0).
 // Returns the id of rank `lane` (lane < k).
 template <int REGT>
-__device__ __forceinline__ int BSX_SOFTMAX_TOKEN(const float* __restrict__ lg, int32_t* __restrict__ ids, float* __restrict__ wout, int E, int k, uint32_t* keys) {
+__device__ __forceinline__ int BSX_SOFTMAX_TOKEN(const float* lg, int32_t* __restrict__ ids, float* __restrict__ wout, int E, int k, uint32_t* keys) {
     constexpr int MAXR = REGT > 0 ? REGT : 32;
     const int lane = threadIdx.x & 31;
     const int reg = REGT > 0 ? REGT : (E >> 5);
@@ -121,7 +121,7 @@ __device__ __forceinline__ int BSX_SOFTMAX_TOKEN(const float* __restrict__ lg, i
 }
 
 template <int REGT>
-__global__ void __launch_bounds__(256) BSX_SOFTMAX_KERNEL(const float* __restrict__ logits, int32_t* __restrict__ ids,
+__global__ void __launch_bounds__(256) BSX_SOFTMAX_KERNEL(const float* logits, int32_t* __restrict__ ids,
                                                          float* __restrict__ wout, int64_t T, int E, int k) {
     __shared__ uint32_t keys[8][REGT > 0 ? REGT * 33 : 1];
     pdl_wait();
