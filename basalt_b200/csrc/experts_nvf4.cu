@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) nvf4_stream_kernel(StreamArgs sa
                             const float v0 = ((__uint_as_float(d0[4 * jj]) + __uint_as_float(d0[4 * jj + 1])) + __uint_as_float(d0[4 * jj + 2])) + __uint_as_float(d0[4 * jj + 3]);
                             const float v1 = ((__uint_as_float(d1[4 * jj]) + __uint_as_float(d1[4 * jj + 1])) + __uint_as_float(d1[4 * jj + 2])) + __uint_as_float(d1[4 * jj + 3]);
                             if (MODE == FMODE_GU) {
-                                a.h[orow[j] + r0 + rl] = swiglu(v0 * f[j] * sg, v1 * f[j] * su, a.L);
+                                a.h[orow[j] + r0 + rl] = swiglu_short(v0 * f[j] * sg, v1 * f[j] * su, a.L);
                             } else {
                                 store_out(a.out, a.out_kind, orow[j] + r0 + rl, v0 * f[j] * sd);
                                 store_out(a.out, a.out_kind, orow[j] + r0 + 128 + rl, v1 * f[j] * sd);

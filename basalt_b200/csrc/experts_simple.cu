@@ -151,7 +151,7 @@ gu_simple_kernel(ExpertArgs a) {
 #pragma unroll
             for (int t = 0; t < kTok; ++t) {
                 const float gs = warp_sum_xor(ag[t]), us = warp_sum_xor(au[t]);
-                if (lane == 0 && t < nt) a.h[(size_t) (eb + t) * a.L.n_ff + r] = swiglu(gs * sg, us * su, a.L);
+                if (lane == 0 && t < nt) a.h[(size_t) (eb + t) * a.L.n_ff + r] = swiglu_short(gs * sg, us * su, a.L);
             }
         }
     }
