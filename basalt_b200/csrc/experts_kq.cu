@@ -463,9 +463,10 @@ kq_mma_kernel(ExpertArgs a, const int8_t* img, const int8_t* corr, const float* 
                     }
                 } else {
                     const uint8_t* src = row0 + iss_tile + (size_t) (chunk0 + iss_chunk) * kChunkBytes - 2 * ((chunk0 + iss_chunk) & 1) + 4 * lane;
+                    auto row_at = [&](int row) { return src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1); };
 #pragma unroll
                     for (int row = 0; row < kRowsQ; ++row) {
-                        const uint8_t* r = src + (row < 8 ? row * pitch0 : half + (row - 8) * pitch1);
+                        const uint8_t* r = row_at(row);
                         const uint32_t d = dst + (uint32_t) (row * kRow + 4 * lane);
                         cpa4(d, r);
                         if (lane < 53 - 32) cpa4(d + 128, r + 128);
