@@ -734,10 +734,12 @@ int32_t experts_grouped_kq(const ExpertArgs& a, cudaStream_t st) {
     }
     if (rc != BSX_OK || phase == 1) return rc;
     if (L.d_type == kTypeIQ1M) {
-        launch_k(kq_image_kernel<true, kTypeIQ1M>, dim3(nbh), dim3(256), 0, st, a, himg, hcorr, hinv, items, n_items, kEntQ * dn.NB);
+        rc = launch_spread<kq_image_kernel<true, kTypeIQ1M>>(nbh, st, a, himg, hcorr, hinv, items, n_items, kEntQ * dn.NB);
+        if (rc != BSX_OK) return rc;
         return kq_launch<kTypeIQ1M, QMODE_DOWN>(dn, a, himg, hcorr, hinv, items, n_items, st);
     }
-    launch_k(kq_image_kernel<true, kTypeQ6K>, dim3(nbh), dim3(256), 0, st, a, himg, hcorr, hinv, items, n_items, kEntQ * dn.NB);
+    rc = launch_spread<kq_image_kernel<true, kTypeQ6K>>(nbh, st, a, himg, hcorr, hinv, items, n_items, kEntQ * dn.NB);
+    if (rc != BSX_OK) return rc;
     return kq_launch<kTypeQ6K, QMODE_DOWN>(dn, a, himg, hcorr, hinv, items, n_items, st);
 }
 

@@ -704,7 +704,9 @@ int32_t experts_grouped_mma(const ExpertArgs& a, bool iq1m, cudaStream_t st) {
         }
     }
     if (rc != BSX_OK || phase == 1) return rc;
-    launch_k(fmt == FMT_IQ3S ? prep_image_kernel<FMT_IQ3S, true, 2> : prep_image_kernel<FMT_NVFP4, true, 2>, dim3(nbh), dim3(256), 0, st, a, himg, hinv, items, n_items);
+    rc = fmt == FMT_IQ3S ? launch_spread<prep_image_kernel<FMT_IQ3S, true, 2>>(nbh, st, a, himg, hinv, items, n_items)
+                         : launch_spread<prep_image_kernel<FMT_NVFP4, true, 2>>(nbh, st, a, himg, hinv, items, n_items);
+    if (rc != BSX_OK) return rc;
     if (fmt == FMT_IQ3S) return launch<FMT_IQ3S, MODE_DOWN, 2, 4, 1>(a, himg, hinv, items, n_items, st);
     if (fmt == FMT_IQ1M) return launch<FMT_IQ1M, MODE_DOWN, 2, 8, 1>(a, himg, hinv, items, n_items, st);
     // Down rows of n_ff columns: the copies' width is what their start is aligned to.  An n_ff that is not whole 256-column chunks
