@@ -56,8 +56,10 @@ __host__ __device__ inline int64_t image_units(int64_t cap_rows, int64_t cap_til
 // items (optional, a short call): the rows become passes of up to pass_entries rows for the decode stream instead.  But a call that is
 // short by its average may still send most rows to a few experts, and the stream reads an expert's weights once a pass: tiles of more
 // than kCrowdedRows rows then stay tiles, provided the passes they save outweigh what the tile kernels take in the whole.  A tile costs
-// the chip about as much as three passes (5120 x 2304 with 27 rows an expert: 7.0 and 2.4 us), and the tile kernels come in rounds
-// of sm_count items, of which a call pays one more than it fills (launches, the last item's latency).
+// the chip three to four passes (5120 x 2304: 5.5 us of 64 rows, 7.5 of 128, a pass of 16 rows 2.0), and the tile kernels come in rounds of
+// items, one a pair of SMs, of which a call pays one more than it fills (launches, the last item's latency).  A third of the rows on a few
+// of 385 experts, 16 rows an expert on average, all passes against this rule: on 64 experts 1440 : 1409 us, on 16 1425 : 1357, but on 4
+// 1434 : 1503 and on one 1408 : 1556, where it is too willing.
 constexpr int kCrowdedRows = 64;
 struct RecordArgs {
     const int32_t *tiles, *n_tiles, *off;
@@ -70,7 +72,7 @@ struct RecordArgs {
     PassRec* items;
     int* n_items;
     int64_t cap_items;
-    int pass_entries, tile_items, sm_count;      // tile_items: items of a tile's gate/up product
+    int pass_entries, tile_items, sm_count;      // tile_items: SMs that a tile's gate/up product keeps for an item's time (two an item of 256 neurons)
     int32_t* status;
 };
 __global__ void __launch_bounds__(1024) tile_records_kernel(RecordArgs a) {
@@ -715,11 +717,13 @@ size_t al256q(size_t v) { return (v + 255) & ~(size_t) 255; }
 
 using namespace bsx;
 
-// Rows an expert, on average over the call, up to which the decode stream takes it.  Whole layer, bf16 rows, back to back, stream against tiles
-// (these with tile images, 20 to 40 us above gathered rows): 2048 x 512 with 512 + 1 experts at 6.4 rows an expert 242 : 310 us, 21
-// 339 : 383, 34 477 : 431; 5120 x 2304 with 384 + 1 at 14 rows 1437 : 1581, 27 1877 : 1818, 45 2489 : 2201; 7168 x 2048 with 256 + 1 at 17.5
-// rows 1335 : 1424, 35 1794 : 1648.
-constexpr int64_t kShortRows = 26;
+// Rows an expert, on average over the call, up to which the decode stream takes it: from there on its second and third passes over an expert's
+// weights outweigh what tiles cost beside the rows.  Expert stage, rows dealt at random, stream against tiles, us: 2048 x 512 with 513 experts
+// at 26 rows an expert 279 : 298, 28 286 : 305, 30 301 : 316, 32 320 : 320; 5120 x 2304 with 385 at 26 1828 : 1948, 28 1920 : 1974, 30
+// 1999 : 1985, 32 2109 : 2028; 7168 x 2048 with 257 at 26 1503 : 1599, 28 1556 : 1613, 30 1650 : 1620.  An n_ff of 256 leaves a down item one
+// chunk, which its epilogue outlasts: 2048 x 256 with 513 experts at 30 202 : 232, 38 248 : 255; 4096 x 256 at 34 373 : 373; 7168 x 256 with 257 at
+// 38 350 : 358, 42 372 : 366.
+static int64_t short_rows(const bsx_expert_layout& L) { return L.n_ff == 256 ? 38 : 29; }
 // Rows an expert from which the SwiGLU rows are laid out as tile images: these hold up to 23 rows more a tile than there are.
 constexpr int64_t kTileImageRows = 48;
 
@@ -736,7 +740,7 @@ struct PrefillCarve {
 static PrefillCarve prefill_carve(const bsx_expert_layout& L, int64_t n_tokens, int64_t cap_rows, int64_t n_expert, int64_t n_held) {
     PrefillCarve c = {};
     const int64_t H = L.n_embd, I = L.n_ff;
-    c.stream = cap_rows <= kShortRows * n_expert && n_tokens <= 0x7FFFFFFF;
+    c.stream = cap_rows <= short_rows(L) * n_expert && n_tokens <= 0x7FFFFFFF;
     c.cap_recs = prefill_cap_tiles(cap_rows, n_held);
     c.cap_items = c.stream ? cap_rows / kPassEntries + c.cap_recs : 0;
     if (c.stream) c.cap_recs = std::min(c.cap_recs, cap_rows / (kCrowdedRows + 1) + 1);        // the crowded tiles
@@ -775,7 +779,7 @@ extern "C" size_t bsx_experts_prefill_packed_held_scratch_bytes(const bsx_expert
 // the most that any number of experts needs: of each route, for the largest number that takes it
 extern "C" size_t bsx_experts_prefill_packed_scratch_bytes(const bsx_expert_layout* L, int64_t n_tokens, int64_t cap_rows) {
     if (!L || n_tokens < 0 || cap_rows < 0 || !bsx_expert_packed_bytes(L)) return 0;
-    const int64_t number[3] = {std::max<int64_t>(1025, (cap_rows + kShortRows - 1) / kShortRows), (cap_rows - 1) / kShortRows, (cap_rows - 1) / kTileImageRows};
+    const int64_t few = short_rows(*L), number[3] = {std::max<int64_t>(1025, (cap_rows + few - 1) / few), (cap_rows - 1) / few, (cap_rows - 1) / kTileImageRows};
     size_t most = 0;
     for (int64_t n : number)
         if (n >= 1) most = std::max(most, prefill_carve(*L, n_tokens, cap_rows, n, n).bytes);

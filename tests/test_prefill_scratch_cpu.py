@@ -43,3 +43,18 @@ def test_long_call_and_a_rank_with_an_eighth(lib):
     assert whole <= fixed + 1.3 * images
     assert eighth <= fixed + 0.25 * 1.3 * images + (1 << 20)
     assert sizes(H, I, T, T, 8, 9)[1] == 0 and sizes(H, I, T, T, 0, 0)[1] == 0
+
+
+@pytest.mark.parametrize("I,most", [(256, 38), (512, 29), (2304, 29)])
+def test_rows_an_expert_up_to_which_a_call_is_short(lib, I, most):
+    """A short call's scratch has pass records and few tile records, a longer one's tile records alone."""
+    H, E = 2048, 64
+    up = lambda n: (n + 255) // 256 * 256
+
+    def size(T, rows, recs, passes):
+        return sum(map(up, (T * 2 * H, T * H // 4, T * 4, (rows + 128) * I * 4, rows * 2 * I, rows * I // 4, (rows + 128) * 4, recs * 32, 12, passes * 16, 4)))
+    for per, short in ((most, True), (most + 1, False)):
+        rows = per * E
+        tiles = rows // 128 + E
+        want = size(rows, rows, min(tiles, rows // 65 + 1), rows // 8 + tiles) if short else size(rows, rows, tiles, 0)
+        assert sizes(H, I, rows, rows, E, E)[1] == want, (per, want)

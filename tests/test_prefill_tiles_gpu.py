@@ -101,10 +101,11 @@ def test_crowded_short_calls(lib, cuda, H, I, shift, counts, away):
 
 # 34 rows an expert: tiles whose SwiGLU rows are gathered from row images
 MID = [40, 1, 16, 17, 33, 129, 8, 64, 0, 31]
+MID256 = [40, 1, 16, 17, 33, 129, 8, 64, 0, 120]                                 # 43 an expert: n_ff 256 is short up to 38
 
 
 @pytest.mark.parametrize("H,I,shift,counts,away", [(256, 256, 0, MID, ()), (768, 512, 16, MID, ()), (512, 1280, 0, MID, (0, 5)), (2048, 2304, 0, MID, ()), (256, 512, 0, MID * 12, ()),
-                                                   (768, 256, 0, TILES * 12, ()), (1280, 768, 0, TILES, (1, 9))])
+                                                   (768, 256, 0, TILES * 12, ()), (1280, 768, 0, TILES, (1, 9)), (256, 256, 0, MID256, ()), (2048, 256, 16, MID256 * 12, (3,))])
 def test_tiles_of_gathered_rows(lib, cuda, H, I, shift, counts, away):
     """Every number of columns modulo 16 on either side of a pair's halves, one and two accumulators an item, few and many items a pair."""
     run(H, I, shift, counts, away)
