@@ -263,14 +263,14 @@ prep_image_kernel(ExpertArgs a, __half* __restrict__ img, float* __restrict__ in
 // 64-column NVFP4 blocks, 36 bytes each) starts on 8 bytes (K % 128 == 0) or 4, and its last chunk holds fewer than four blocks:
 // those pieces are not requested and those blocks not multiplied.
 // CHAIN: MMAs that add up in one accumulator.  The tensor core truncates where it adds to an accumulator, fp32 arithmetic rounds to
-// nearest; distance to 64-bit sums of the 2048 x 512 layer's fp32 rows, and its 64-token step: a whole row chained 1.64e-6, 177 us;
-// 8 MMAs 2.9e-7, 179 us; 4 (a block of 64 columns) 2.1e-7, 186 us; 2 1.8e-7, 189 us; 1 1.7e-7, 192 us; the fp32 kernel 2.6e-7.
+// nearest.  Distance to 64-bit sums of the 2048 x 512 layer's fp32 rows: a whole row chained 1.64e-6, 8 MMAs 2.9e-7, 4 (a block of 64
+// columns) 2.1e-7, 2 1.8e-7, 1 1.7e-7; the fp32 kernel 2.6e-7.  Its 64-token step, one layer again and again: with four 95 us, with one 98.6.
 // Four where no layout needs better.  IQ3_S and NVFP4 with ragged down rows, which the fp32 kernel had before, take one: with four,
 // bf16 rows would be further off than there (1.75e-7 against 1.6e-7 at 2560 x 640).
 // KS > 1: KS neighbouring warps share a row tile, each a part of its chunks; their sums meet in shared memory.
 // Work: the row blocks (W / KS tiles) of all passes in one sequence, cut into equal runs, one a block; a run's part of one pass shares
 // its columns and its weight stream.
-// W, OCC, NC: warps a block, blocks an SM, copies of the IQ3_S codebook (blk_shape).
+// W, OCC, ST, NC: warps a block, blocks an SM, stages a warp, copies of the IQ3_S codebook (launch() below).
 template <int FMT, int MODE, int TERMS, int PIECE, int CHAIN, int W, int OCC, int ST, int NC, int KS>
 __global__ void __launch_bounds__(W * 32, OCC)
 blk_mma_kernel(ExpertArgs a, const __half* img, const float* inv, const PassRec* items, const int* n_items, int n_row_blocks) {
@@ -711,7 +711,7 @@ int32_t experts_grouped_mma(const ExpertArgs& a, bool iq1m, cudaStream_t st) {
     if (fmt == FMT_IQ1M) return launch<FMT_IQ1M, MODE_DOWN, 2, 8, 1>(a, himg, hinv, items, n_items, st);
     // Down rows of n_ff columns: the copies' width is what their start is aligned to.  An n_ff that is not whole 256-column chunks
     // went to the warp-per-row kernels before (2 % of the copy bandwidth: fp32 decode and FMA for every weight and entry); here
-    // the same 27-token step (2560 x 640, 512 + 1 experts, top-10) takes 217 us instead of 3648.
+    // the same 27-token step (2560 x 640, 512 + 1 experts, top-10) takes 170 us instead of 3648.
     if (whole) return launch<FMT_NVFP4, MODE_DOWN, 2, 16, 4>(a, himg, hinv, items, n_items, st);
     if (L.n_ff % 128 == 0) return launch<FMT_NVFP4, MODE_DOWN, 2, 8, 1>(a, himg, hinv, items, n_items, st);
     return launch<FMT_NVFP4, MODE_DOWN, 2, 4, 1>(a, himg, hinv, items, n_items, st);

@@ -455,222 +455,222 @@ __global__ void __launch_bounds__(kThreadsP, 1) prefill_pair_kernel(PrefillFArgs
         }
         if (!ok && lane == 0) atomicOr(a.status, 1);
     } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n");
-    if (warp == 0) {
-        // ---- MMA issuer
-        if (rank == 0 && elect_one()) {
-            uint32_t kb = 0, ka = 0;
-            for (uint32_t ti = 0; ok; ++ti) {
-                const int item = next_item(ti);
-                if (item < 0) break;
-                const int tile = item / n_n, n = item - tile * n_n;
-                const uint32_t idesc = G::kIdesc | ((uint32_t) ((recs[tile].rows + 15) >> 4) << 18);
-                const bool two = both(n);
-                ok = mbar_wait(acc_empty, (ti & 1u) ^ 1u);
-                if (!ok) break;
-                for (int c = 0; c < n_chunk && ok; ++c, ++kb) {
-                    const uint32_t sb = kb % G::kBStages, bst = sbase + sb * G::kBStage, tsfa = tmem + G::kTmemSFA + sb * 32;
-                    const uint64_t ad0 = smem_desc_sw128(bst), ad1 = smem_desc_sw128(bst + kBlockF);
-                    ok = mbar_wait(&ready[sb], (kb / G::kBStages) & 1u);
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n");
+        if (warp == 0) {
+            // ---- MMA issuer
+            if (rank == 0 && elect_one()) {
+                uint32_t kb = 0, ka = 0;
+                for (uint32_t ti = 0; ok; ++ti) {
+                    const int item = next_item(ti);
+                    if (item < 0) break;
+                    const int tile = item / n_n, n = item - tile * n_n;
+                    const uint32_t idesc = G::kIdesc | ((uint32_t) ((recs[tile].rows + 15) >> 4) << 18);
+                    const bool two = both(n);
+                    ok = mbar_wait(acc_empty, (ti & 1u) ^ 1u);
                     if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    for (int c = 0; c < n_chunk && ok; ++c, ++kb) {
+                        const uint32_t sb = kb % G::kBStages, bst = sbase + sb * G::kBStage, tsfa = tmem + G::kTmemSFA + sb * 32;
+                        const uint64_t ad0 = smem_desc_sw128(bst), ad1 = smem_desc_sw128(bst + kBlockF);
+                        ok = mbar_wait(&ready[sb], (kb / G::kBStages) & 1u);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll 1
-                    for (int t = 0; t < kTermsF; ++t, ++ka) {
-                        const uint32_t sa = ka % G::kASlots;
-                        const uint64_t bd = smem_desc_sw128(sbase + G::kOffA + sa * G::kSlot);
-                        const uint32_t tsfb = tmem + G::kTmemSFB + sa * 16;
+                        for (int t = 0; t < kTermsF; ++t, ++ka) {
+                            const uint32_t sa = ka % G::kASlots;
+                            const uint64_t bd = smem_desc_sw128(sbase + G::kOffA + sa * G::kSlot);
+                            const uint32_t tsfb = tmem + G::kTmemSFB + sa * 16;
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const uint32_t accum = (c | t | k) ? 1u : 0u;
-                            mma_nvf4_pair(tmem, ad0 + k * kStepCode, bd + k * kStepCode, idesc, tsfa + 4 * k, tsfb + 4 * k, accum);
-                            if (two) mma_nvf4_pair(tmem + 128, ad1 + k * kStepCode, bd + k * kStepCode, idesc, tsfa + 16 + 4 * k, tsfb + 4 * k, accum);
+                            for (int k = 0; k < 4; ++k) {
+                                const uint32_t accum = (c | t | k) ? 1u : 0u;
+                                mma_nvf4_pair(tmem, ad0 + k * kStepCode, bd + k * kStepCode, idesc, tsfa + 4 * k, tsfb + 4 * k, accum);
+                                if (two) mma_nvf4_pair(tmem + 128, ad1 + k * kStepCode, bd + k * kStepCode, idesc, tsfa + 16 + 4 * k, tsfb + 4 * k, accum);
+                            }
+                            commit_pair(&a_empty[sa]);
                         }
-                        commit_pair(&a_empty[sa]);
+                        commit_pair(&b_empty[sb]);
                     }
-                    commit_pair(&b_empty[sb]);
-                }
-                if (!ok) break;
-                commit_pair(acc_full);
-            }
-            if (!ok) atomicOr(a.status, 1);
-        }
-    } else if (warp == 1) {
-        // ---- weight loader: a stage is two packed blocks
-        if (elect_one()) {
-            uint32_t kb = 0;
-            for (uint32_t ti = 0; ok; ++ti) {
-                const int item = next_item(ti);
-                if (item < 0) break;
-                const int tile = item / n_n, n = item - tile * n_n;
-                const uint8_t* blob = reinterpret_cast<const uint8_t*>(recs[tile].blob);
-                const size_t mat = (size_t) n_chunk * kBlockF;             // a 128-row block over all of K
-                const uint8_t* b0 = MODE == QMODE_GU ? blob + geo.gate + (2 * n + rank) * mat : blob + geo.down + (4 * n + rank) * mat;
-                const uint8_t* b1 = MODE == QMODE_GU ? blob + geo.up + (2 * n + rank) * mat : b0 + 2 * mat;
-                const bool two = both(n);
-                for (int c = 0; c < n_chunk; ++c, ++kb) {
-                    const uint32_t s = kb % G::kBStages;
-                    ok = mbar_wait(&b_empty[s], ((kb / G::kBStages) & 1u) ^ 1u);
                     if (!ok) break;
-                    const uint32_t st = sbase + s * G::kBStage, bar = smem_u32(&b_full[s]);
-                    expect_bytes_q(bar, two ? 2 * kBlockF : kBlockF);
-                    bulk_copy_q(st, b0 + (size_t) c * kBlockF, kBlockF, bar);
-                    if (two) bulk_copy_q(st + kBlockF, b1 + (size_t) c * kBlockF, kBlockF, bar);
+                    commit_pair(acc_full);
                 }
+                if (!ok) atomicOr(a.status, 1);
             }
-            if (!ok) atomicOr(a.status, 1);
-        }
-    } else if (GATHER && warp >= 8) {
-        // ---- row loaders, from the rows' images.  Codes: lane = (16-byte piece c8, row r4 of four) of this CTA's half of the tile's columns,
-        // rows r4 + 4 i.  Scales, with a chunk's first term: of the whole tile, four lanes a row, the terms' pieces swizzled so that the warps
-        // that read a term of 32 rows meet no bank twice.  Rows past the tile's last are left as they are (a column reaches its own
-        // results only).  The barriers count the copies as they land, so ten slots' worth are in flight.
-        const uint32_t K = (uint32_t) n_chunk * 256u, term = K / 32, c8 = lane & 7, r4 = lane >> 3;       // image offsets in 16 bytes
-        const uint32_t dst0 = r4 * 128 + ((c8 ^ r4) << 4), dst1 = (4 + r4) * 128 + ((c8 ^ (4 + r4)) << 4);
-        const uint32_t st = lane & 3, sr = lane >> 2, sdst = sr * kSFChunk + ((st ^ ((sr >> 1) & 3)) << 4);
-        const int lw = warp - 8;
-        uint32_t issued = 0, kb = 0;
-        // arrives once this lane's copies so far have landed, without the lane waiting for it
-        auto land = [&](uint64_t* bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory"); };
-        for (uint32_t ti = 0; ok; ++ti) {
-            const int item = next_item_warp(ti);
-            if (item < 0) break;
-            const TileRec r = recs[item / n_n];
-            auto image_row = [&](int row) { return (uint32_t) (MODE == QMODE_GU ? a.src[r.row0 + row] : r.row0 + row); };
-            const int per = (r.rows + 15) >> 4, row0 = rank * per * 8, live = (min(r.rows - row0, per * 8) - (int) r4 + 3) >> 2;
-            uint32_t off[4], soff[4];          // groups 4 lw .. + 3 of the sixteen of each kind
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                off[i] = image_row(min(row0 + 4 * (4 * lw + i) + (int) r4, r.rows - 1)) * (kTermsF * term) + c8;
-                soff[i] = image_row(min(8 * (4 * lw + i) + (int) sr, r.rows - 1)) * (K / 64) + st;
-            }
-            for (int c = 0; c < n_chunk && ok; ++c, ++kb)
-#pragma unroll 1
-                for (int t = 0; t < kTermsF; ++t) {
-                    const uint32_t s = issued % G::kASlots, sb = kb % G::kBStages;
-                    ok = mbar_wait(&a_empty[s], ((issued / G::kASlots) & 1u) ^ 1u);
-                    if (t == 0) ok = ok && mbar_wait(&b_empty[sb], ((kb / G::kBStages) & 1u) ^ 1u);
-                    ok = __all_sync(kFull, ok);
-                    if (!ok) break;
-                    const uint32_t slot = sbase + (uint32_t) (G::kOffA + s * G::kSlot);
-                    const uint8_t* g = a.img + (size_t) (t * term + c * 8) * 16;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (4 * lw + i < live)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(slot + (uint32_t) ((2 * lw + (i >> 1)) * 1024) + ((i & 1) ? dst1 : dst0)), "l"(g + (size_t) off[i] * 16) : "memory");
-                    if (t == 0) {
-                        const uint32_t sf = sbase + (uint32_t) (G::kOffSF + sb * G::kSFStage) + sdst;
-                        const uint8_t* gs = a.sfs + (size_t) c * kSFChunk;
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (8 * (4 * lw + i) + (int) sr < r.rows)
-                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sf + (uint32_t) ((4 * lw + i) * 8 * kSFChunk)), "l"(gs + (size_t) soff[i] * 16) : "memory");
+        } else if (warp == 1) {
+            // ---- weight loader: a stage is two packed blocks
+            if (elect_one()) {
+                uint32_t kb = 0;
+                for (uint32_t ti = 0; ok; ++ti) {
+                    const int item = next_item(ti);
+                    if (item < 0) break;
+                    const int tile = item / n_n, n = item - tile * n_n;
+                    const uint8_t* blob = reinterpret_cast<const uint8_t*>(recs[tile].blob);
+                    const size_t mat = (size_t) n_chunk * kBlockF;             // a 128-row block over all of K
+                    const uint8_t* b0 = MODE == QMODE_GU ? blob + geo.gate + (2 * n + rank) * mat : blob + geo.down + (4 * n + rank) * mat;
+                    const uint8_t* b1 = MODE == QMODE_GU ? blob + geo.up + (2 * n + rank) * mat : b0 + 2 * mat;
+                    const bool two = both(n);
+                    for (int c = 0; c < n_chunk; ++c, ++kb) {
+                        const uint32_t s = kb % G::kBStages;
+                        ok = mbar_wait(&b_empty[s], ((kb / G::kBStages) & 1u) ^ 1u);
+                        if (!ok) break;
+                        const uint32_t st = sbase + s * G::kBStage, bar = smem_u32(&b_full[s]);
+                        expect_bytes_q(bar, two ? 2 * kBlockF : kBlockF);
+                        bulk_copy_q(st, b0 + (size_t) c * kBlockF, kBlockF, bar);
+                        if (two) bulk_copy_q(st + kBlockF, b1 + (size_t) c * kBlockF, kBlockF, bar);
                     }
-                    if (t == 0) land(&b_full[sb]);
-                    land(&a_full[s]);
-                    ++issued;
                 }
-        }
-        asm volatile("cp.async.wait_all;\n" ::: "memory");
-        if (!ok && lane == 0) atomicOr(a.status, 1);
-    } else if (!GATHER && warp >= 8) {
-        // ---- row loader, from the tile images: the scale words of the whole tile and this CTA's half of its columns, as far as there are rows
-        if (warp == 8 && elect_one()) {
-            uint32_t ka = 0, kb = 0;
+                if (!ok) atomicOr(a.status, 1);
+            }
+        } else if (GATHER && warp >= 8) {
+            // ---- row loaders, from the rows' images.  Codes: lane = (16-byte piece c8, row r4 of four) of this CTA's half of the tile's columns,
+            // rows r4 + 4 i.  Scales, with a chunk's first term: of the whole tile, four lanes a row, the terms' pieces swizzled so that the warps
+            // that read a term of 32 rows meet no bank twice.  Rows past the tile's last are left as they are (a column reaches its own
+            // results only).  The barriers count the copies as they land, so ten slots' worth are in flight.
+            const uint32_t K = (uint32_t) n_chunk * 256u, term = K / 32, c8 = lane & 7, r4 = lane >> 3;       // image offsets in 16 bytes
+            const uint32_t dst0 = r4 * 128 + ((c8 ^ r4) << 4), dst1 = (4 + r4) * 128 + ((c8 ^ (4 + r4)) << 4);
+            const uint32_t st = lane & 3, sr = lane >> 2, sdst = sr * kSFChunk + ((st ^ ((sr >> 1) & 3)) << 4);
+            const int lw = warp - 8;
+            uint32_t issued = 0, kb = 0;
+            // arrives once this lane's copies so far have landed, without the lane waiting for it
+            auto land = [&](uint64_t* bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory"); };
             for (uint32_t ti = 0; ok; ++ti) {
-                const int item = next_item(ti);
+                const int item = next_item_warp(ti);
                 if (item < 0) break;
                 const TileRec r = recs[item / n_n];
-                const uint32_t bytes = (uint32_t) tile_units(r.rows) * 1024u, atoms = (uint32_t) (r.rows + 7) >> 3, per = (uint32_t) (r.rows + 15) >> 4;
-                const uint32_t off = kSFQ + (rank ? per * 1024u : 0u), mine = (rank ? atoms - per : per) * 1024u;
-                const uint8_t* g = a.img + image_block(r, n_chunk, 0, 0);
-                for (int c = 0; c < n_chunk && ok; ++c, ++kb) {
-                    const uint32_t sb = kb % G::kBStages, sbar = smem_u32(&b_full[sb]);
+                auto image_row = [&](int row) { return (uint32_t) (MODE == QMODE_GU ? a.src[r.row0 + row] : r.row0 + row); };
+                const int per = (r.rows + 15) >> 4, row0 = rank * per * 8, live = (min(r.rows - row0, per * 8) - (int) r4 + 3) >> 2;
+                uint32_t off[4], soff[4];          // groups 4 lw .. + 3 of the sixteen of each kind
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    off[i] = image_row(min(row0 + 4 * (4 * lw + i) + (int) r4, r.rows - 1)) * (kTermsF * term) + c8;
+                    soff[i] = image_row(min(8 * (4 * lw + i) + (int) sr, r.rows - 1)) * (K / 64) + st;
+                }
+                for (int c = 0; c < n_chunk && ok; ++c, ++kb)
 #pragma unroll 1
-                    for (int t = 0; t < kTermsF; ++t, ++ka, g += bytes) {
-                        const uint32_t s = ka % G::kASlots;
-                        ok = mbar_wait(&a_empty[s], ((ka / G::kASlots) & 1u) ^ 1u);
+                    for (int t = 0; t < kTermsF; ++t) {
+                        const uint32_t s = issued % G::kASlots, sb = kb % G::kBStages;
+                        ok = mbar_wait(&a_empty[s], ((issued / G::kASlots) & 1u) ^ 1u);
                         if (t == 0) ok = ok && mbar_wait(&b_empty[sb], ((kb / G::kBStages) & 1u) ^ 1u);
+                        ok = __all_sync(kFull, ok);
                         if (!ok) break;
-                        if (t == 0) expect_bytes_q(sbar, kTermsF * kSFQ);
-                        bulk_copy_q(sbase + (uint32_t) (G::kOffSF + sb * G::kSFStage + t * kSFQ), g, kSFQ, sbar);
-                        const uint32_t bar = smem_u32(&a_full[s]);
-                        expect_bytes_q(bar, mine);
-                        if (mine) bulk_copy_q(sbase + (uint32_t) (G::kOffA + s * G::kSlot), g + off, mine, bar);
+                        const uint32_t slot = sbase + (uint32_t) (G::kOffA + s * G::kSlot);
+                        const uint8_t* g = a.img + (size_t) (t * term + c * 8) * 16;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (4 * lw + i < live)
+                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(slot + (uint32_t) ((2 * lw + (i >> 1)) * 1024) + ((i & 1) ? dst1 : dst0)), "l"(g + (size_t) off[i] * 16) : "memory");
+                        if (t == 0) {
+                            const uint32_t sf = sbase + (uint32_t) (G::kOffSF + sb * G::kSFStage) + sdst;
+                            const uint8_t* gs = a.sfs + (size_t) c * kSFChunk;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (8 * (4 * lw + i) + (int) sr < r.rows)
+                                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sf + (uint32_t) ((4 * lw + i) * 8 * kSFChunk)), "l"(gs + (size_t) soff[i] * 16) : "memory");
+                        }
+                        if (t == 0) land(&b_full[sb]);
+                        land(&a_full[s]);
+                        ++issued;
+                    }
+            }
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            if (!ok && lane == 0) atomicOr(a.status, 1);
+        } else if (!GATHER && warp >= 8) {
+            // ---- row loader, from the tile images: the scale words of the whole tile and this CTA's half of its columns, as far as there are rows
+            if (warp == 8 && elect_one()) {
+                uint32_t ka = 0, kb = 0;
+                for (uint32_t ti = 0; ok; ++ti) {
+                    const int item = next_item(ti);
+                    if (item < 0) break;
+                    const TileRec r = recs[item / n_n];
+                    const uint32_t bytes = (uint32_t) tile_units(r.rows) * 1024u, atoms = (uint32_t) (r.rows + 7) >> 3, per = (uint32_t) (r.rows + 15) >> 4;
+                    const uint32_t off = kSFQ + (rank ? per * 1024u : 0u), mine = (rank ? atoms - per : per) * 1024u;
+                    const uint8_t* g = a.img + image_block(r, n_chunk, 0, 0);
+                    for (int c = 0; c < n_chunk && ok; ++c, ++kb) {
+                        const uint32_t sb = kb % G::kBStages, sbar = smem_u32(&b_full[sb]);
+#pragma unroll 1
+                        for (int t = 0; t < kTermsF; ++t, ++ka, g += bytes) {
+                            const uint32_t s = ka % G::kASlots;
+                            ok = mbar_wait(&a_empty[s], ((ka / G::kASlots) & 1u) ^ 1u);
+                            if (t == 0) ok = ok && mbar_wait(&b_empty[sb], ((kb / G::kBStages) & 1u) ^ 1u);
+                            if (!ok) break;
+                            if (t == 0) expect_bytes_q(sbar, kTermsF * kSFQ);
+                            bulk_copy_q(sbase + (uint32_t) (G::kOffSF + sb * G::kSFStage + t * kSFQ), g, kSFQ, sbar);
+                            const uint32_t bar = smem_u32(&a_full[s]);
+                            expect_bytes_q(bar, mine);
+                            if (mine) bulk_copy_q(sbase + (uint32_t) (G::kOffA + s * G::kSlot), g + off, mine, bar);
+                        }
                     }
                 }
+                if (!ok) atomicOr(a.status, 1);
             }
-            if (!ok) atomicOr(a.status, 1);
-        }
-    } else if (warp == 2) {
-        // ---- items: the pair's own number first, then from the launch's counter, a few ahead of the roles.  Tiles differ in their rows, so
-        // items dealt in turn would leave the fullest pair 4 to 20 % behind the average.
-        if (rank == 0 && elect_one()) {
-            int item = pair;
-            for (uint32_t it = 0; ok; ++it) {
-                const uint32_t s = it % G::kRing;
-                ok = mbar_wait(&item_empty[s], ((it / G::kRing) & 1u) ^ 1u);
-                if (!ok) break;
-                const int v = item < n_items ? item : -1;
-                send_word(ring + s, v, &item_full[s], 1);
-                send_word(ring + s, v, &item_full[s], 0);
-                if (v < 0) break;
-                item = n_pairs + atomicAdd(a.counter, 1);
+        } else if (warp == 2) {
+            // ---- items: the pair's own number first, then from the launch's counter, a few ahead of the roles.  Tiles differ in their rows, so
+            // items dealt in turn would leave the fullest pair 4 to 20 % behind the average.
+            if (rank == 0 && elect_one()) {
+                int item = pair;
+                for (uint32_t it = 0; ok; ++it) {
+                    const uint32_t s = it % G::kRing;
+                    ok = mbar_wait(&item_empty[s], ((it / G::kRing) & 1u) ^ 1u);
+                    if (!ok) break;
+                    const int v = item < n_items ? item : -1;
+                    send_word(ring + s, v, &item_full[s], 1);
+                    send_word(ring + s, v, &item_full[s], 0);
+                    if (v < 0) break;
+                    item = n_pairs + atomicAdd(a.counter, 1);
+                }
+                if (!ok) atomicOr(a.status, 1);
             }
-            if (!ok) atomicOr(a.status, 1);
-        }
-    } else if (warp >= 4) {
-        // ---- scale words, shared -> tensor memory: lane l of each quadrant takes the words of rows l, l + 32, l + 64, l + 96 of a K-step
-        const uint32_t quad = (uint32_t) ((warp & 3) * 32) << 16;
-        auto fetch = [&](uint32_t from, uint32_t step, uint4 (&w)[4]) {
+        } else if (warp >= 4) {
+            // ---- scale words, shared -> tensor memory: lane l of each quadrant takes the words of rows l, l + 32, l + 64, l + 96 of a K-step
+            const uint32_t quad = (uint32_t) ((warp & 3) * 32) << 16;
+            auto fetch = [&](uint32_t from, uint32_t step, uint4 (&w)[4]) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(w[i].x), "=r"(w[i].y), "=r"(w[i].z), "=r"(w[i].w) : "r"(from + i * step) : "memory");
-        };
-        uint32_t kb = 0, ka = 0;
-        for (uint32_t ti = 0; ok; ++ti) {
-            const int item = next_item_warp(ti);
-            if (item < 0) break;
-            const bool two = both(item % n_n);
-            for (int c = 0; c < n_chunk; ++c, ++kb) {
-                // a chunk at a time: one wait for the stores, one arrival (a slot at a time the loop's latency held the tensor core back)
-                const uint32_t sb = kb % G::kBStages, bst = sbase + sb * G::kBStage + kATileQ + lane * 16, tsfa = tmem + quad + G::kTmemSFA + sb * 32;
-                const uint32_t sf = sbase + (uint32_t) (G::kOffSF + sb * G::kSFStage) + lane * (GATHER ? kSFChunk : 16);
-                ok = __all_sync(kFull, mbar_wait(&b_full[sb], (kb / G::kBStages) & 1u));
-                if (!ok) break;
-                __syncwarp();
-                uint4 w0[4], w1[4];
-                fetch(bst, 512, w0);                       // weights: a K-step's words of four rows a lane lie together
-                if (two) fetch(bst + kBlockF, 512, w1);
-                tmem_st16(tsfa, w0);
-                if (two) tmem_st16(tsfa + 16, w1);
-#pragma unroll
-                for (int t = 0; t < kTermsF; t += 2, ka += 2) {
-                    const uint32_t s0 = ka % G::kASlots, s1 = (ka + 1) % G::kASlots;
-                    ok = ok && mbar_wait(&a_full[s0], (ka / G::kASlots) & 1u) && mbar_wait(&a_full[s1], ((ka + 1) / G::kASlots) & 1u);
+                for (int i = 0; i < 4; ++i)
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(w[i].x), "=r"(w[i].y), "=r"(w[i].z), "=r"(w[i].w) : "r"(from + i * step) : "memory");
+            };
+            uint32_t kb = 0, ka = 0;
+            for (uint32_t ti = 0; ok; ++ti) {
+                const int item = next_item_warp(ti);
+                if (item < 0) break;
+                const bool two = both(item % n_n);
+                for (int c = 0; c < n_chunk; ++c, ++kb) {
+                    // a chunk at a time: one wait for the stores, one arrival (a slot at a time the loop's latency held the tensor core back)
+                    const uint32_t sb = kb % G::kBStages, bst = sbase + sb * G::kBStage + kATileQ + lane * 16, tsfa = tmem + quad + G::kTmemSFA + sb * 32;
+                    const uint32_t sf = sbase + (uint32_t) (G::kOffSF + sb * G::kSFStage) + lane * (GATHER ? kSFChunk : 16);
+                    ok = __all_sync(kFull, mbar_wait(&b_full[sb], (kb / G::kBStages) & 1u));
+                    if (!ok) break;
                     __syncwarp();
-                    if (GATHER) {                          // a row's words of four K-steps lie together
-                        fetch(sf + ((t ^ ((lane >> 1) & 3)) << 4), 32 * kSFChunk, w0);
-                        fetch(sf + (((t + 1) ^ ((lane >> 1) & 3)) << 4), 32 * kSFChunk, w1);
-                        tmem_st16t(tmem + quad + G::kTmemSFB + s0 * 16, w0);
-                        tmem_st16t(tmem + quad + G::kTmemSFB + s1 * 16, w1);
-                    } else {
-                        fetch(sf + t * kSFQ, 512, w0);
-                        fetch(sf + (t + 1) * kSFQ, 512, w1);
-                        tmem_st16(tmem + quad + G::kTmemSFB + s0 * 16, w0);
-                        tmem_st16(tmem + quad + G::kTmemSFB + s1 * 16, w1);
+                    uint4 w0[4], w1[4];
+                    fetch(bst, 512, w0);                       // weights: a K-step's words of four rows a lane lie together
+                    if (two) fetch(bst + kBlockF, 512, w1);
+                    tmem_st16(tsfa, w0);
+                    if (two) tmem_st16(tsfa + 16, w1);
+#pragma unroll
+                    for (int t = 0; t < kTermsF; t += 2, ka += 2) {
+                        const uint32_t s0 = ka % G::kASlots, s1 = (ka + 1) % G::kASlots;
+                        ok = ok && mbar_wait(&a_full[s0], (ka / G::kASlots) & 1u) && mbar_wait(&a_full[s1], ((ka + 1) / G::kASlots) & 1u);
+                        __syncwarp();
+                        if (GATHER) {                          // a row's words of four K-steps lie together
+                            fetch(sf + ((t ^ ((lane >> 1) & 3)) << 4), 32 * kSFChunk, w0);
+                            fetch(sf + (((t + 1) ^ ((lane >> 1) & 3)) << 4), 32 * kSFChunk, w1);
+                            tmem_st16t(tmem + quad + G::kTmemSFB + s0 * 16, w0);
+                            tmem_st16t(tmem + quad + G::kTmemSFB + s1 * 16, w1);
+                        } else {
+                            fetch(sf + t * kSFQ, 512, w0);
+                            fetch(sf + (t + 1) * kSFQ, 512, w1);
+                            tmem_st16(tmem + quad + G::kTmemSFB + s0 * 16, w0);
+                            tmem_st16(tmem + quad + G::kTmemSFB + s1 * 16, w1);
+                        }
                     }
+                    ok = __all_sync(kFull, ok);
+                    if (!ok) break;
+                    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                    if (GATHER) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");        // the rows' codes, which cp.async wrote, to the tensor core
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) arrive_first(&ready[sb]);
                 }
-                ok = __all_sync(kFull, ok);
-                if (!ok) break;
-                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-                if (GATHER) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");        // the rows' codes, which cp.async wrote, to the tensor core
-                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-                __syncwarp();
-                if (lane == 0) arrive_first(&ready[sb]);
             }
+            if (!ok && lane == 0) atomicOr(a.status, 1);
         }
-        if (!ok && lane == 0) atomicOr(a.status, 1);
-    }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();

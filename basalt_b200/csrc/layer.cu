@@ -209,8 +209,9 @@ extern "C" int32_t bsx_moe_layer(const bsx_moe_layer_desc* d, const void* x, int
         if (rc != BSX_OK) return rc;
         // A shared expert sees every token.  From 16 tokens on, an NVFP4 one goes through the prompt-sized kernel (one pass over the
         // blob for the whole window; the decode kernels take 4 or 8 entries a pass and would stream it several times).  Q6_K blobs
-        // stay on the decode kernels, where a shared expert is faster at 64 tokens too: the prompt kernel reads that format byte
-        // by byte.  I-quant ones stay with them; that kernel's IQ1_M decoder has not been timed on a single blob.
+        // stay on the integer decode kernels: the step of 7168 x 2048, 64 tokens 1253 us with them and 1411 with the prompt kernel, 16 tokens
+        // 565 and 793; of 2048 x 512, 64 tokens 299 and 382.  (Widths that those kernels do not take pay for it: 5120 x 2304, 64 tokens 2910 and
+        // 1490.)  I-quant ones stay too; that kernel's IQ1_M decoder has not been timed on a single blob.
         rc = BSX_E_TYPE;
         if (T >= 16 && status != nullptr && d->shared_layout.gu_type == kTypeNVFP4 && bsx_experts_prefill_group_scratch_bytes(&d->shared_layout, T, T) != 0) {
             const void* blob1[1] = {reinterpret_cast<const void*>((uintptr_t) d->shared_blob)};

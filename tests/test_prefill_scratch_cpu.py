@@ -1,5 +1,6 @@
 """What the packed prompt call asks its caller to allocate: the exact size for a number of experts never exceeds the one that covers any
-number, short calls hold no tile images, and a rank that holds an eighth of the experts does not hold the images of all rows."""
+number, short calls hold no tile images, and long ones the images of the SwiGLU rows alone, as tiles (a rank that holds an eighth of the
+experts too: its call may get every row)."""
 import ctypes as C
 import random
 
@@ -38,10 +39,11 @@ def test_long_call_and_a_rank_with_an_eighth(lib):
     rows = 8 * T * k
     _, whole = sizes(H, I, 8 * T, rows, E, E)
     _, eighth = sizes(H, I, 8 * T, rows, E, E // 8)
-    fixed = 8 * T * (2.25 * H + 4) + (rows + 128) * (4 * I + 4)
-    images = (rows + E * 24) * 2.25 * (H + I)                                  # of x and of h; a tile's: up to 24 rows more than its rows
-    assert whole <= fixed + 1.3 * images
-    assert eighth <= fixed + 0.25 * 1.3 * images + (1 << 20)
+    fixed = 8 * T * (2.25 * H + 4) + (rows + 128) * (4 * I + 8)                # FP4 terms of x, fp32 h
+    images = 2.25 * I                                                          # of a SwiGLU row; a tile's: up to 24 rows more than its rows
+    lists = (rows // 128 + E) * 32 + 16 * 256
+    assert whole <= fixed + (rows + 24 * (rows // 128 + E)) * images + lists
+    assert eighth <= fixed + (rows + 24 * (rows // 128 + E // 8)) * images + lists
     assert sizes(H, I, T, T, 8, 9)[1] == 0 and sizes(H, I, T, T, 0, 0)[1] == 0
 
 

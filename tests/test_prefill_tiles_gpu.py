@@ -82,7 +82,7 @@ def test_experts_held_elsewhere(lib, cuda, H, I, counts, away):
                                              (256, 512, MANY, (50,)), (256, 256, MANY, range(51)), (512, 512, SHORT16, (8,)), (768, 768, SHORT8, (6, 8)), (256, 256, [49], (0,)),
                                              (256, 512, [1, 120], (1,))])
 def test_rounds_over_the_room_of_an_even_share(lib, cuda, H, I, counts, here):
-    """rows that crowd onto the experts held here: more than twice an even share, so that the tile images take several rounds"""
+    """rows that crowd onto the experts held here, more than twice an even share: the exact scratch for these few holds all their images"""
     run(H, I, 0, counts, tuple(e for e in range(len(counts)) if e not in here), len(tuple(here)))
 
 
