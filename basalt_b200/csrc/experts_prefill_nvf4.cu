@@ -773,7 +773,9 @@ static PrefillCarve prefill_carve(const bsx_expert_layout& L, int64_t n_tokens, 
 
 extern "C" size_t bsx_experts_prefill_packed_held_scratch_bytes(const bsx_expert_layout* L, int64_t n_tokens, int64_t cap_rows, int32_t n_expert, int32_t n_held) {
     if (!L || n_tokens < 0 || cap_rows < 0 || n_expert < 1 || n_held < 0 || n_held > n_expert || !bsx_expert_packed_bytes(L)) return 0;
-    return prefill_carve(*L, n_tokens, cap_rows, n_expert, n_held).bytes;
+    // A caller may size its scratch by its largest call, and the longest short one can need a little more than the next: its pass records.
+    return std::max(prefill_carve(*L, n_tokens, cap_rows, n_expert, n_held).bytes,
+                    prefill_carve(*L, n_tokens, std::min(cap_rows, short_rows(*L) * n_expert), n_expert, n_held).bytes);
 }
 
 // the most that any number of experts needs: of each route, for the largest number that takes it

@@ -300,8 +300,8 @@ BSX_API int32_t bsx_experts_prefill_packed(const bsx_expert_layout* layout, cons
                                            const void* x, int32_t x_kind, int64_t n_tokens, int32_t n_expert, void* scratch, float* dm,
                                            int32_t* status, void* stream);
 /* The same for a caller that says how many of the experts have a blob here (n_held non-zero entries of blob_table).  The scratch size is
- * exact for these numbers; with n_held = n_expert it is what bsx_experts_prefill_packed needs for n_expert experts
- * (bsx_experts_prefill_packed_scratch_bytes covers any number of them). */
+ * that of these numbers and covers every call of fewer rows or tokens; with n_held = n_expert it is what bsx_experts_prefill_packed needs
+ * for n_expert experts (bsx_experts_prefill_packed_scratch_bytes covers any number of them). */
 BSX_API size_t bsx_experts_prefill_packed_held_scratch_bytes(const bsx_expert_layout* layout, int64_t n_tokens, int64_t cap_rows, int32_t n_expert,
                                                              int32_t n_held);
 BSX_API int32_t bsx_experts_prefill_packed_held(const bsx_expert_layout* layout, const unsigned long long* blob_table, const int32_t* off,

@@ -60,3 +60,16 @@ def test_rows_an_expert_up_to_which_a_call_is_short(lib, I, most):
         tiles = rows // 128 + E
         want = size(rows, rows, min(tiles, rows // 65 + 1), rows // 8 + tiles) if short else size(rows, rows, tiles, 0)
         assert sizes(H, I, rows, rows, E, E)[1] == want, (per, want)
+
+
+def test_scratch_of_the_largest_call_covers_the_smaller(lib):
+    """around the numbers of rows where the route changes, at each of which the buffers differ"""
+    rng = random.Random(3)
+    for _ in range(150):
+        H, I, E, k = 256 * rng.randint(1, 28), 256 * rng.choice([1, 1, 2, 3, 9]), rng.choice([1, 3, 8, 64, 257, 513, 1025]), rng.randint(1, 10)
+        held = rng.choice([E, max(1, E // 8)])
+        last = (0, 0)
+        for T in sorted({max(1, r * E // k + d) for r in (1, 4, 28, 29, 30, 37, 38, 39, 48, 49, 60) for d in (-1, 0, 1)}):
+            now = sizes(H, I, T, T * k, E, held)
+            assert now[0] >= last[0] and now[1] >= last[1], (H, I, E, k, held, T)
+            last = now
